@@ -72,6 +72,7 @@ extern "C" int32_t b200nn_matmul(b200nn_ctx *ctx, const b200nn_tensor *a, const 
         w.K = (int)K;
         w.N = (int)N;
         w.w_kn = b->buf; // shared, not copied; no fp16 copy: the FMA kernels run
+        w.volatile_w = true;
         Epilogue e;
         e.out = y->data();
         e.ldo = (int)N;

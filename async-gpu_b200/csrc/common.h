@@ -212,7 +212,10 @@ int int4_weight_ln_fold(b200nn_ctx *ctx, const Int4Weight &w, const float *g_dev
 struct F32Weight {
     int K = 0, N = 0;
     bool exact = false;
+    int ldw = 0;             // floats between rows of w_kn (0: N); uploaded weights have rows that start on 16 bytes
+    bool volatile_w = false; // w_kn is a tensor that work before this may write: not read ahead of that
     std::shared_ptr<DevBuf> w_kn, bias, w_nk_h;
+    int ld() const { return ldw ? ldw : N; }
 };
 // weight given as [out,in] (Linear layout) or [in,out] (checkpoint layout)
 int f32_weight_upload(b200nn_ctx *ctx, const float *w, bool is_out_in, const float *bias, size_t K, size_t N,
@@ -303,16 +306,28 @@ struct Epilogue {
     int kv_at = 0, kv_w = 0, kv_heads = 0, kv_cap = 0;
 };
 
+// A LayerNorm that a GEMV of few rows applies to its f32 input rows itself (g null: none); rows of at most
+// NORM_IN_MAX values.
+struct NormIn {
+    const float *g = nullptr, *b = nullptr;
+    float eps = 0.0f;
+};
+static constexpr int NORM_IN_MAX = 2048;
+static constexpr int F32_GEMV_ROWS = 4; // rows that the f32 GEMV serves
+
 // ---------------------------------------------------------------------------------------------
 // kernel launchers (each in its own translation unit)
 // ---------------------------------------------------------------------------------------------
 // x: [M,K] f32 or fp16 (x_half).  Dispatches GEMV / tensor-core GEMM / generic kernel.
-int launch_int4_linear(b200nn_ctx *ctx, const Int4Weight &w, const void *x, bool x_half, int M, const Epilogue &epi);
-int launch_int4_gemv(b200nn_ctx *ctx, const Int4Weight &w, const void *x, bool x_half, int M, const Epilogue &epi);
+int launch_int4_linear(b200nn_ctx *ctx, const Int4Weight &w, const void *x, bool x_half, int M, const Epilogue &epi, const NormIn &ln = NormIn());
+int launch_int4_gemv(b200nn_ctx *ctx, const Int4Weight &w, const void *x, bool x_half, int M, const Epilogue &epi, const NormIn &ln = NormIn());
+bool int4_linear_takes_norm(const Int4Weight &w, int M);
 int launch_int4_naive(b200nn_ctx *ctx, const Int4Weight &w, const void *x, bool x_half, int M, const Epilogue &epi);
 bool int4_gemm_tc_supported(const Int4Weight &w, int M);
 int launch_int4_gemm_tc(b200nn_ctx *ctx, const Int4Weight &w, const __half *x, int M, const Epilogue &epi);
-int launch_f32_linear(b200nn_ctx *ctx, const F32Weight &w, const void *x, bool x_half, int M, const Epilogue &epi);
+int launch_f32_linear(b200nn_ctx *ctx, const F32Weight &w, const void *x, bool x_half, int M, const Epilogue &epi, const NormIn &ln = NormIn());
+bool f32_linear_takes_norm(const F32Weight &w, int M);
+bool f32_gemv_fits(const F32Weight &w); // the GEMV's shared memory holds this K
 bool f16_gemm_tc_supported(const b200nn_ctx *ctx, const F32Weight &w, int M);
 int launch_f16_gemm_tc(b200nn_ctx *ctx, const F32Weight &w, const __half *x, int M, const Epilogue &epi);
 // x: bf16 [M, ldx] (ldx >= the activation columns the weight reads, a multiple of 8)

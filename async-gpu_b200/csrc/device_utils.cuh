@@ -54,7 +54,7 @@ __device__ __forceinline__ void epi_store(const Epilogue &e, int m, int n, float
     if (e.no_store) return;
     if (e.mode == EPI_RESID) {
         size_t i = (size_t)m * e.ldo + n;
-        e.resid[i] += v;
+        e.resid[i] = __ldcg(e.resid + i) + v; // not from L1: see load_fresh
         return;
     }
     if (e.mode == EPI_QKV && n >= e.d_model) {
@@ -364,9 +364,96 @@ template <>
 __device__ __forceinline__ float load_as_float<__half>(const __half *p, size_t i) { return __half2float(p[i]); }
 template <>
 __device__ __forceinline__ float load_as_float<__nv_bfloat16>(const __nv_bfloat16 *p, size_t i) { return __bfloat162float(p[i]); }
+// A value that the kernel before wrote, read after pdl_wait: from L2.  The block may have been resident while that
+// kernel ran on the same SM, so a line that came into L1 since this kernel's start (or through the read-only
+// path, which a plain load from a const __restrict__ pointer takes) can be older than the wait: the second of four f32 rows
+// got its MLP from the residual stream without the attention's sum.
+__device__ __forceinline__ float load_fresh(const float *p, size_t i) { return __ldcg(p + i); }
+__device__ __forceinline__ float load_fresh(const __half *p, size_t i) {
+    return __half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short *>(p) + i)));
+}
 __device__ __forceinline__ void store_from_float(float *p, float v) { *p = v; }
 __device__ __forceinline__ void store_from_float(__half *p, float v) { *p = __float2half_rn(v); }
 __device__ __forceinline__ void store_from_float(__nv_bfloat16 *p, float v) { *p = __float2bfloat16_rn(v); }
+
+// The two halves of a cluster-wide barrier, and a store into the same shared variable of another block of the cluster.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void st_cluster(float *p, int rank, float v) {
+    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.f32 [a], %2;\n\t}" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(p)),
+                 "r"(rank), "f"(v)
+                 : "memory");
+}
+
+// LayerNorm of up to MT f32 rows x [m_valid][K] (K <= NORM_IN_MAX) by one block: the values of columns k0 .. k0+cols go
+// to xs [MT][ld] (zero past them and past m_valid).  Mean, then the mean square about it, as layernorm_kernel has it.
+// Contains the wait on the previous kernel, after the loads of scale and shift.  red: THREADS / 32 * MT floats; the
+// caller synchronises before it reads xs or reuses red.
+template <int MT, int THREADS>
+__device__ __forceinline__ void norm_rows_to_smem(const NormIn &ln, const float *__restrict__ x, int m_valid, int K, int k0, int cols,
+                                                  int ld, float *xs, float *red) {
+    constexpr int VPT = NORM_IN_MAX / THREADS, WARPS = THREADS / 32;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float g[VPT], b[VPT], v[MT][VPT], s[MT];
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+        const int k = tid + i * THREADS;
+        const bool mine = k >= k0 && k < k0 + cols;
+        g[i] = mine ? __ldg(ln.g + k) : 0.0f;
+        b[i] = mine ? __ldg(ln.b + k) : 0.0f;
+    }
+    pdl_wait();
+    auto sums = [&]() { // s[m] over the block, divided by K
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+            s[m] = warp_sum(s[m]);
+            if (lane == 0) red[warp * MT + m] = s[m];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+            float t = 0.0f;
+#pragma unroll
+            for (int wi = 0; wi < WARPS; ++wi) t += red[wi * MT + m];
+            s[m] = t / (float)K;
+        }
+        __syncthreads();
+    };
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+        s[m] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) {
+            const int k = tid + i * THREADS;
+            v[m][i] = m < m_valid && k < K ? load_fresh(x, (size_t)m * K + k) : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) s[m] += v[m][i];
+    }
+    sums();
+    float mean[MT];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+        mean[m] = s[m];
+        s[m] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) {
+            const float t = tid + i * THREADS < K ? v[m][i] - mean[m] : 0.0f;
+            s[m] += t * t;
+        }
+    }
+    sums();
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+        const float inv_std = rsqrtf(s[m] + ln.eps);
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) {
+            const int kk = tid + i * THREADS - k0;
+            if (kk >= 0 && kk < ld) xs[m * ld + kk] = m < m_valid && kk < cols ? (v[m][i] - mean[m]) * inv_std * g[i] + b[i] : 0.0f;
+        }
+    }
+}
 
 __device__ __forceinline__ float sigmoid_f(float v) { return 1.0f / (1.0f + expf(-v)); }
 

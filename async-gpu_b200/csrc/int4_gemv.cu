@@ -1,26 +1,22 @@
 // Group-wise int4 weight-only Linear on CUDA cores.
 //
 //   int4_gemv_kernel   few input rows (decode of one or two sequences): HBM-bound streaming of the
-//                      tiled nibbles with 128-bit coalesced loads (two K blocks per thread in
+//                      tiled nibbles with 128-bit coalesced loads (three K blocks per thread in
 //                      flight, the first ones issued before the wait on the preceding kernel:
 //                      weights do not depend on it), in-register dequantisation, f32 accumulation.
-//                      K is split four ways inside a block and up to eight ways across the blocks of
-//                      a thread-block cluster; the cluster's partial sums are reduced through
-//                      distributed shared memory by the cluster's first block (fixed order, no
-//                      global scratch, no atomics), which then runs the fused bias / activation /
-//                      residual / KV-cache epilogue.
+//                      K is split inside a block and up to eight ways across the blocks of
+//                      a thread-block cluster; the blocks store their partial sums into the
+//                      shared memory of the cluster's first block, which adds them (fixed order, no
+//                      global scratch, no atomics) and runs the fused bias / activation /
+//                      residual / KV-cache epilogue.  A LayerNorm of the input rows can ride along.
 //   int4_naive_kernel  any K%8==0 and any group size, reference layout, one thread per output as
 //                      crates/kernel/gpu-kernel-compute/src/compute_gemm.rs:2849-2910 does.
 //
 // Both compute y[m,n] = sum_k x[m,k] * (nibble(k,n)-8) * scale[k/group,n] (+ bias[n]).
-#include <cooperative_groups.h>
-
 #include "device_utils.cuh"
 
-namespace cg = cooperative_groups;
-
-static constexpr int GEMV_THREADS = 512; // 128 weight rows x 4 K slices
-static constexpr int GEMV_SLICES = 4;
+static constexpr int GEMV_THREADS = 512;
+static constexpr int GEMV_AHEAD = 3;     // K blocks of a thread in flight
 
 template <int MT>
 __device__ __forceinline__ void gemv_block_fma(const uint4 &wa, const uint4 &wb, float s, const float *xb, int len,
@@ -51,88 +47,92 @@ __device__ __forceinline__ void gemv_block_fma(const uint4 &wa, const uint4 &wb,
     for (int m = 0; m < MT; ++m) acc[m] = fmaf(s, part[m], acc[m]);
 }
 
-// grid (n_tiles, splits), cluster (1, splits, 1): the blocks of a cluster share one 128-row tile.
-template <int MT, typename XT>
-__global__ void __launch_bounds__(GEMV_THREADS)
+// grid (weight rows / RW, splits), cluster (1, splits, 1): the blocks of a cluster share RW rows of the weight.  A thread
+// has one row and every SLICES-th K block of its block's range.  RW 128: four slices.  RW 32: sixteen, for weights of
+// few rows, so that a thread has two or three K blocks, all of them requested before the wait, and most weights need no
+// second block per tile.
+template <int MT, int RW, typename XT>
+__global__ void __launch_bounds__(GEMV_THREADS, 2)
 int4_gemv_kernel(const uint4 *__restrict__ tiles, const __half *__restrict__ scales, const XT *__restrict__ x,
                  int m_valid, int m0, int K, int N, int k_blocks, int n_pad, int group, int kb_per_split,
-                 Epilogue epi) {
+                 NormIn ln, Epilogue epi) {
+    constexpr int SLICES = GEMV_THREADS / RW;
     extern __shared__ float smem_f[];
-    cg::cluster_group cluster = cg::this_cluster();
-    const int nt = blockIdx.x, split = blockIdx.y, splits = gridDim.y;
-    const int tid = threadIdx.x, r = tid & 127, slice = tid >> 7;
+    const int split = blockIdx.y, splits = gridDim.y;
+    const int tid = threadIdx.x, r = tid % RW, slice = tid / RW;
+    const int n = blockIdx.x * RW + r, tile_row = n & 127;
     const int kb0 = split * kb_per_split;
     const int kb1 = min(kb0 + kb_per_split, k_blocks);
     const int len = kb_per_split * 64;
-    const int n = nt * TILE_N + r;
-    float *xs = smem_f;                       // [MT][len] activations of this block's K range
-    float *red = smem_f + MT * len;           // [GEMV_SLICES][MT][128] slice sums
-    float *part = red + GEMV_SLICES * MT * 128; // [MT][128] this block's partial tile (read by the cluster)
+    float *xs = smem_f;                        // [MT][len] activations of this block's K range
+    float *red = smem_f + MT * len;            // [SLICES][MT][RW] slice sums
+    float *part = red + SLICES * MT * RW;      // [splits][MT][RW] partial tiles, in the cluster's first block
     pdl_trigger();
+    if (splits > 1) cluster_arrive(); // waited for before the first store into another block
 
-    // weights and scales of the first two K blocks of this thread: issued before the wait on the
+    // weights and scales of this thread's first K blocks: issued before the wait on the
     // previous kernel (they are constants), so that their DRAM latency overlaps its tail
-    const uint4 *tile0 = tiles + (size_t)nt * k_blocks * (TILE_BYTES / 16);
-    auto load_block = [&](int kb, uint4 &a, uint4 &b, float &s) {
+    const uint4 *tile0 = tiles + (size_t)(n >> 7) * k_blocks * (TILE_BYTES / 16) + tile_row;
+    uint4 wa[GEMV_AHEAD], wb[GEMV_AHEAD];
+    float sc[GEMV_AHEAD];
+    auto load_block = [&](int i, int kb) {
+        if (kb >= kb1) return;
         const uint4 *tp = tile0 + (size_t)kb * (TILE_BYTES / 16);
-        a = __ldg(tp + r);
-        b = __ldg(tp + 128 + r);
-        s = __half2float(scales[(size_t)((kb * 64) / group) * n_pad + n]);
+        wa[i] = __ldg(tp);
+        wb[i] = __ldg(tp + 128);
+        sc[i] = __half2float(scales[(size_t)((kb * 64) / group) * n_pad + n]);
     };
-    int kb = kb0 + slice;
-    uint4 a0 = make_uint4(0, 0, 0, 0), b0 = a0, a1 = a0, b1 = a0;
-    float s0 = 0.0f, s1 = 0.0f;
-    bool v0 = kb < kb1, v1 = kb + GEMV_SLICES < kb1;
-    if (v0) load_block(kb, a0, b0, s0);
-    if (v1) load_block(kb + GEMV_SLICES, a1, b1, s1);
+#pragma unroll
+    for (int i = 0; i < GEMV_AHEAD; ++i) load_block(i, kb0 + slice + i * SLICES);
 
-    pdl_wait();
-    for (int i = tid; i < MT * len; i += GEMV_THREADS) {
-        const int m = i / len, kk = i - m * len;
-        const int k = kb0 * 64 + kk;
-        xs[i] = (m < m_valid && k < kb1 * 64) ? load_as_float<XT>(x, (size_t)m * K + k) : 0.0f;
+    if constexpr (sizeof(XT) == 4) {
+        if (ln.g) norm_rows_to_smem<MT, GEMV_THREADS>(ln, x, m_valid, K, kb0 * 64, (kb1 - kb0) * 64, len, xs, red);
+    }
+    if (sizeof(XT) != 4 || !ln.g) {
+        pdl_wait();
+        for (int i = tid; i < MT * len; i += GEMV_THREADS) {
+            const int m = i / len, kk = i - m * len;
+            const int k = kb0 * 64 + kk;
+            xs[i] = (m < m_valid && k < kb1 * 64) ? load_fresh(x, (size_t)m * K + k) : 0.0f;
+        }
     }
     __syncthreads();
 
     float acc[MT];
 #pragma unroll
     for (int m = 0; m < MT; ++m) acc[m] = 0.0f;
-    while (v0) {
-        const uint4 ca = a0, cb = b0;
-        const float cs = s0;
-        const int ckb = kb;
-        a0 = a1; b0 = b1; s0 = s1; v0 = v1;
-        kb += GEMV_SLICES;
-        v1 = kb + GEMV_SLICES < kb1;
-        if (v1) load_block(kb + GEMV_SLICES, a1, b1, s1); // stays two K blocks ahead
-        gemv_block_fma<MT>(ca, cb, cs, xs + (ckb - kb0) * 64, len, acc);
+    for (int kb = kb0 + slice; kb < kb1; kb += GEMV_AHEAD * SLICES) {
+#pragma unroll
+        for (int i = 0; i < GEMV_AHEAD; ++i) {
+            const int k = kb + i * SLICES;
+            if (k < kb1) gemv_block_fma<MT>(wa[i], wb[i], sc[i], xs + (k - kb0) * 64, len, acc);
+            load_block(i, k + GEMV_AHEAD * SLICES);
+        }
     }
 
 #pragma unroll
-    for (int m = 0; m < MT; ++m) red[(slice * MT + m) * 128 + r] = acc[m];
+    for (int m = 0; m < MT; ++m) red[(slice * MT + m) * RW + r] = acc[m];
     __syncthreads();
-    if (slice == 0) {
+    float t = 0.0f; // thread m * RW + r: feature r of row m (MT * RW <= GEMV_THREADS)
+    const int m = slice;
+    if (m < MT)
 #pragma unroll
-        for (int m = 0; m < MT; ++m) {
-            float t = 0.0f;
-#pragma unroll
-            for (int sl = 0; sl < GEMV_SLICES; ++sl) t += red[(sl * MT + m) * 128 + r];
-            part[m * 128 + r] = t;
-        }
-    }
-    cluster.sync(); // every block's partial tile is in its shared memory
-    if (cluster.block_rank() == 0 && slice == 0) { // warps 0..3: 32 consecutive features each
-#pragma unroll
-        for (int m = 0; m < MT; ++m) {
-            if (m >= m_valid) break;
-            float t = 0.0f;
+        for (int sl = 0; sl < SLICES; ++sl) t += red[(sl * MT + m) * RW + r];
+    if (splits > 1) {
+        cluster_wait();
+        if (m < MT) st_cluster(&part[(split * MT + m) * RW + r], 0, t);
+        cluster_arrive();
+        cluster_wait(); // every block's partial tile is in the first block
+        if (split != 0) return;
+        t = 0.0f;
+        if (m < MT)
             for (int sp = 0; sp < splits; ++sp) // fixed order: the result does not depend on timing
-                t += cluster.map_shared_rank(part, sp)[m * 128 + r];
-            if (n < N) epi_apply(epi, m0 + m, n, t);
-            if (epi.amax_val) epi_argmax1(epi, m0 + m, n, t + (epi.bias && n < N ? epi.bias[n] : 0.0f), n < N);
-        }
+                t += part[(sp * MT + m) * RW + r];
     }
-    cluster.sync(); // no block leaves while its shared memory may still be read
+    if (m < min(MT, m_valid)) { // RW / 32 warps per row: 32 consecutive features each
+        if (n < N) epi_apply(epi, m0 + m, n, t);
+        if (epi.amax_val) epi_argmax1(epi, m0 + m, n, t + (epi.bias && n < N ? epi.bias[n] : 0.0f), n < N);
+    }
 }
 
 template <typename XT>
@@ -174,76 +174,93 @@ int launch_int4_naive(b200nn_ctx *ctx, const Int4Weight &w, const void *x, bool 
     return B200NN_OK;
 }
 
-template <int MT, typename XT>
-static int gemv_chunk(b200nn_ctx *ctx, const Int4Weight &w, const XT *x, int m_valid, int m0, const Epilogue &epi) {
-    // K split across a cluster of up to eight blocks so that about one block per SM is resident
-    int splits = (ctx->sm_count + w.n_tiles - 1) / w.n_tiles;
+template <int MT, int RW, typename XT>
+static int gemv_launch(b200nn_ctx *ctx, const Int4Weight &w, const XT *x, int m_valid, int m0, const NormIn &ln, const Epilogue &epi) {
+    constexpr int SLICES = GEMV_THREADS / RW;
+    constexpr size_t SMEM_MAX = 216 * 1024;
+    // K split across a cluster of up to eight blocks so that about one block per SM is resident; the sixteen slices of
+    // a narrow block have a K block each at least
+    const int tiles = (w.N + RW - 1) / RW;
+    int splits = RW == 32 ? ctx->sm_count / tiles : (ctx->sm_count + tiles - 1) / tiles;
     splits = std::max(1, std::min(splits, 8));
-    splits = std::min(splits, std::max(1, w.k_blocks / GEMV_SLICES));
+    splits = std::min(splits, std::max(1, w.k_blocks / SLICES));
     const int per = (w.k_blocks + splits - 1) / splits;
     splits = (w.k_blocks + per - 1) / per;
-    const size_t smem = ((size_t)MT * per * 64 + (size_t)(GEMV_SLICES + 1) * MT * 128) * sizeof(float);
-    auto kern = int4_gemv_kernel<MT, XT>;
+    const size_t smem = ((size_t)MT * per * 64 + (size_t)(SLICES + splits) * MT * RW) * sizeof(float);
+    auto kern = int4_gemv_kernel<MT, RW, XT>;
     static bool attr_done[16] = {}; // function attributes are per device
     if (!attr_done[ctx->device & 15]) {
-        CK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        CK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
         prefer_max_smem(kern);
         attr_done[ctx->device & 15] = true;
     }
-    if (smem > 200 * 1024) return set_error(ctx, B200NN_ERR_UNSUPPORTED, "int4 GEMV: K too large for one cluster");
+    if (smem > SMEM_MAX) return set_error(ctx, B200NN_ERR_UNSUPPORTED, "int4 GEMV: K too large for one cluster");
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(w.n_tiles, splits);
+    cfg.gridDim = dim3(tiles, splits);
     cfg.blockDim = dim3(GEMV_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1;
-    attr[0].val.clusterDim.y = splits;
-    attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = ctx->pdl ? 2 : 1;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1;
+    attr[1].val.clusterDim.y = splits;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = ctx->pdl ? attr : attr + 1;
+    cfg.numAttrs = (ctx->pdl ? 1 : 0) + (splits > 1 ? 1 : 0);
     CK(ctx, cudaLaunchKernelEx(&cfg, kern, (const uint4 *)w.tiled->p, (const __half *)w.scales_h->p, x, m_valid, m0, w.K,
-                               w.N, w.k_blocks, w.n_pad, w.group, per, epi));
+                               w.N, w.k_blocks, w.n_pad, w.group, per, ln, epi));
     CK_LAUNCH(ctx, "int4_gemv_kernel");
     return B200NN_OK;
 }
+template <int MT, typename XT>
+static int gemv_chunk(b200nn_ctx *ctx, const Int4Weight &w, const XT *x, int m_valid, int m0, const NormIn &ln, const Epilogue &epi) {
+    // 32 rows a block while the blocks stay under two per SM and the activations of a block's K range small (an output
+    // matrix has its blocks in 128 rows: ten blocks per SM would each pay for the start)
+    const int tiles = (w.N + 31) / 32, splits = std::max(1, std::min(8, ctx->sm_count / tiles)), per = (w.k_blocks + splits - 1) / splits;
+    if (tiles <= 2 * ctx->sm_count && (size_t)MT * per * 64 * sizeof(float) <= 96 * 1024) return gemv_launch<MT, 32, XT>(ctx, w, x, m_valid, m0, ln, epi);
+    return gemv_launch<MT, 128, XT>(ctx, w, x, m_valid, m0, ln, epi);
+}
 
 template <typename XT>
-static int gemv_all(b200nn_ctx *ctx, const Int4Weight &w, const XT *x, int M, const Epilogue &epi) {
+static int gemv_all(b200nn_ctx *ctx, const Int4Weight &w, const XT *x, int M, const NormIn &ln, const Epilogue &epi) {
     int m0 = 0;
     while (m0 < M) {
         int left = M - m0;
         const XT *xp = x + (size_t)m0 * w.K;
         if (left >= 4) {
-            TRY((gemv_chunk<4, XT>(ctx, w, xp, 4, m0, epi)));
+            TRY((gemv_chunk<4, XT>(ctx, w, xp, 4, m0, ln, epi)));
             m0 += 4;
         } else if (left >= 2) {
-            TRY((gemv_chunk<2, XT>(ctx, w, xp, 2, m0, epi)));
+            TRY((gemv_chunk<2, XT>(ctx, w, xp, 2, m0, ln, epi)));
             m0 += 2;
         } else {
-            TRY((gemv_chunk<1, XT>(ctx, w, xp, 1, m0, epi)));
+            TRY((gemv_chunk<1, XT>(ctx, w, xp, 1, m0, ln, epi)));
             m0 += 1;
         }
     }
     return B200NN_OK;
 }
 
-int launch_int4_gemv(b200nn_ctx *ctx, const Int4Weight &w, const void *x, bool x_half, int M, const Epilogue &epi) {
+bool int4_linear_takes_norm(const Int4Weight &w, int M) { return w.fast && M >= 1 && M <= 4 && w.K <= NORM_IN_MAX; }
+
+int launch_int4_gemv(b200nn_ctx *ctx, const Int4Weight &w, const void *x, bool x_half, int M, const Epilogue &epi, const NormIn &ln) {
     if (M <= 0) return B200NN_OK;
+    if (ln.g && (x_half || !int4_linear_takes_norm(w, M)))
+        return set_error(ctx, B200NN_ERR_UNSUPPORTED, "int4 Linear: only the GEMV of few rows takes a LayerNorm with its input");
     if (epi.ln_stats || epi.mode == EPI_RESID_LN) { // folded LayerNorms exist in the tensor-core GEMM's epilogue only
         if (!(w.fast && M > ctx->gemv_max_rows && x_half && int4_gemm_tc_supported(w, M)) || int4_via_f16_supported(ctx, w, M))
             return set_error(ctx, B200NN_ERR_UNSUPPORTED, "folded LayerNorm: this Linear does not run on the tensor-core GEMM");
         return launch_int4_gemm_tc(ctx, w, (const __half *)x, M, epi);
     }
     if (!w.fast) return launch_int4_naive(ctx, w, x, x_half, M, epi);
-    return x_half ? gemv_all<__half>(ctx, w, (const __half *)x, M, epi) : gemv_all<float>(ctx, w, (const float *)x, M, epi);
+    return x_half ? gemv_all<__half>(ctx, w, (const __half *)x, M, ln, epi) : gemv_all<float>(ctx, w, (const float *)x, M, ln, epi);
 }
 
-int launch_int4_linear(b200nn_ctx *ctx, const Int4Weight &w, const void *x, bool x_half, int M, const Epilogue &epi) {
+int launch_int4_linear(b200nn_ctx *ctx, const Int4Weight &w, const void *x, bool x_half, int M, const Epilogue &epi, const NormIn &ln) {
     if (M <= 0) return B200NN_OK;
+    if (ln.g) return launch_int4_gemv(ctx, w, x, x_half, M, epi, ln);
     if (epi.ln_stats || epi.mode == EPI_RESID_LN) { // folded LayerNorms exist in the tensor-core GEMM's epilogue only
         if (!(w.fast && M > ctx->gemv_max_rows && x_half && int4_gemm_tc_supported(w, M)) || int4_via_f16_supported(ctx, w, M))
             return set_error(ctx, B200NN_ERR_UNSUPPORTED, "folded LayerNorm: this Linear does not run on the tensor-core GEMM");

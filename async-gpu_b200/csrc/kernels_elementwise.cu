@@ -37,8 +37,8 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const float *__restrict_
         int j = tid + i * 256;
         float t = 0.0f;
         if (j < d) {
-            t = xr[j];
-            if (rr) t += rr[j];
+            t = load_fresh(xr, j);
+            if (rr) t += load_fresh(rr, j);
             if (sum_out) sum_out[(size_t)row * d + j] = t;
         }
         v[i] = t;

@@ -1,81 +1,136 @@
 // f32 Linear (y = x * W + b with W stored [K,N]) on CUDA cores with the shared fused epilogue.
 // Replaces the reference's matmul dispatch + bias_add pair (ops/gemm.rs:20-299, reshape.rs:112-156)
 // for the f32 model family.  Two kernels:
-//   f32_gemv_kernel  M <= 4 rows: one thread per output column, weights read once, coalesced
-//                    along N, K split across blocks with the deterministic last-block reduction.
+//   f32_gemv_kernel  M <= 4 rows: weights read once, 32 columns per block, K split over the block's warps
+//                    and the blocks of a cluster (fixed order of sums).
 //   f32_gemm_kernel  64x64x16 shared-memory tiles, 4x4 outputs per thread, any M.
+#include <algorithm>
+
 #include "device_utils.cuh"
 
-template <int MT, typename XT>
-__global__ void __launch_bounds__(256)
-f32_gemv_kernel(const float *__restrict__ w, const XT *__restrict__ x, int m_valid, int m0, int K, int N,
-                int k_per_split, Epilogue epi, float *__restrict__ scratch, unsigned *__restrict__ counters) {
-    extern __shared__ float xs[]; // [MT][k_per_split]
-    __shared__ int is_last;
-    const int n = blockIdx.x * 256 + threadIdx.x;
+static constexpr int FGEMV_THREADS = 256;
+static constexpr int FGEMV_COLS = 32;          // columns per block: one 128-byte line of every weight row
+static constexpr int FGEMV_AHEAD = 12;         // weight loads a thread has in flight
+static constexpr size_t FGEMV_XS = 160 * 1024; // bytes of activations a block holds at most
+
+bool f32_gemv_fits(const F32Weight &w) { return (size_t)F32_GEMV_ROWS * w.K * sizeof(float) <= 8 * FGEMV_XS; }
+
+// grid (column tiles, splits), cluster (1, splits, 1).  A decode step of one sequence is bound by the weights'
+// bytes and by the hand-over from kernel to kernel, so: the block's tile is narrow and its K range short enough that
+// most of its weights are requested before the wait on the previous kernel (they are constants), 16 bytes per
+// lane (VEC 4: eight lanes per row, 32 K slices in a block; VEC 1, rows that do not start on 16 bytes: eight slices).
+// The partial sums of a cluster are stored into its first block's shared memory, one barrier, no scratch in memory.
+// With `ln.g` the activations are the LayerNorm of the f32 rows x: every block takes the statistics of the whole
+// row itself, which saves a kernel between two Linears (norm_rows_to_smem).
+// GPT-2 Small, one sequence, 64 tokens after a prompt of 64: 52.5 ms with 4-byte loads, four in flight, plain launches and
+// a reduction through memory, 24.7 ms with this.
+template <int MT, int VEC, typename XT>
+__global__ void __launch_bounds__(FGEMV_THREADS)
+f32_gemv_kernel(const float *__restrict__ w, int ldw, const XT *__restrict__ x, int m_valid, int m0, int K, int N, int k_per_split,
+                NormIn ln, Epilogue epi) {
+    constexpr int LANES = FGEMV_COLS / VEC;             // lanes across a row of the tile
+    constexpr int SLICES = FGEMV_THREADS / LANES, WARPS = FGEMV_THREADS / 32;
+    extern __shared__ float smem_f[];
     const int split = blockIdx.y, splits = gridDim.y;
-    const int k0 = split * k_per_split, k1 = min(k0 + k_per_split, K);
-    for (int i = threadIdx.x; i < MT * k_per_split; i += 256) {
-        int m = i / k_per_split, kk = i - m * k_per_split;
-        xs[i] = (m < m_valid && k0 + kk < k1) ? load_as_float<XT>(x, (size_t)m * K + k0 + kk) : 0.0f;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int slice = tid / LANES, c = (tid % LANES) * VEC, n_base = blockIdx.x * FGEMV_COLS;
+    const int k0 = split * k_per_split, rows = min(k_per_split, K - k0);
+    float *xs = smem_f;                                 // [MT][k_per_split] activations of this block's K range
+    float *red = xs + MT * k_per_split;                 // [WARPS][MT][32]
+    float *part = red + WARPS * MT * FGEMV_COLS;        // [splits][MT][32] in the cluster's first block
+    pdl_trigger();
+    if (splits > 1) cluster_arrive(); // waited for before the first store into another block
+
+    const float *wp = w + (size_t)(k0 + slice) * ldw + n_base + c;
+    const bool n_ok = n_base + c < (VEC == 4 ? ldw : N);
+    float buf[FGEMV_AHEAD][VEC];
+    auto load = [&](float (&v)[VEC], int r) { // row `slice + r` of the range
+        if (!n_ok || slice + r >= rows) return;
+        if constexpr (VEC == 4) {
+            const float4 t = __ldg(reinterpret_cast<const float4 *>(wp + (size_t)r * ldw));
+            v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+        } else {
+            v[0] = __ldg(wp + (size_t)r * ldw);
+        }
+    };
+#pragma unroll
+    for (int j = 0; j < FGEMV_AHEAD; ++j) {
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) buf[j][i] = 0.0f;
+        load(buf[j], j * SLICES);
+    }
+    if constexpr (sizeof(XT) == 4) {
+        if (ln.g) norm_rows_to_smem<MT, FGEMV_THREADS>(ln, x, m_valid, K, k0, rows, k_per_split, xs, red);
+    }
+    if (sizeof(XT) != 4 || !ln.g) {
+        pdl_wait();
+        for (int i = tid; i < MT * k_per_split; i += FGEMV_THREADS) {
+            const int m = i / k_per_split, kk = i - m * k_per_split;
+            xs[i] = (m < m_valid && kk < rows) ? load_fresh(x, (size_t)m * K + k0 + kk) : 0.0f;
+        }
     }
     __syncthreads();
-    float acc[MT];
+
+    float acc[MT][VEC];
 #pragma unroll
-    for (int m = 0; m < MT; ++m) acc[m] = 0.0f;
-    if (n < N) {
-        const float *wp = w + (size_t)k0 * N + n;
-        int k = 0, len = k1 - k0;
-        for (; k + 4 <= len; k += 4) {
-            float w0 = wp[(size_t)k * N], w1 = wp[(size_t)(k + 1) * N], w2 = wp[(size_t)(k + 2) * N],
-                  w3 = wp[(size_t)(k + 3) * N];
+    for (int m = 0; m < MT; ++m)
 #pragma unroll
-            for (int m = 0; m < MT; ++m) {
-                const float *xm = xs + m * k_per_split + k;
-                acc[m] = fmaf(xm[0], w0, acc[m]);
-                acc[m] = fmaf(xm[1], w1, acc[m]);
-                acc[m] = fmaf(xm[2], w2, acc[m]);
-                acc[m] = fmaf(xm[3], w3, acc[m]);
+        for (int i = 0; i < VEC; ++i) acc[m][i] = 0.0f;
+    for (int r0 = 0; r0 < rows; r0 += FGEMV_AHEAD * SLICES) {
+#pragma unroll
+        for (int j = 0; j < FGEMV_AHEAD; ++j) {
+            const int r = r0 + j * SLICES;
+            if (slice + r < rows) {
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    const float xv = xs[m * k_per_split + slice + r];
+#pragma unroll
+                    for (int i = 0; i < VEC; ++i) acc[m][i] = fmaf(xv, buf[j][i], acc[m][i]);
+                }
             }
-        }
-        for (; k < len; ++k) {
-            float w0 = wp[(size_t)k * N];
-#pragma unroll
-            for (int m = 0; m < MT; ++m) acc[m] = fmaf(xs[m * k_per_split + k], w0, acc[m]);
+            load(buf[j], r + FGEMV_AHEAD * SLICES);
         }
     }
-    if (splits == 1) {
-        if (n < N)
+    // the four K slices of a warp by shuffles, the warps through shared memory, the blocks of the cluster in its first
+    if constexpr (VEC == 4) {
 #pragma unroll
-            for (int m = 0; m < MT; ++m)
-                if (m < m_valid) epi_apply(epi, m0 + m, n, acc[m]);
-        return;
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) {
+                acc[m][i] += __shfl_xor_sync(0xffffffffu, acc[m][i], 8);
+                acc[m][i] += __shfl_xor_sync(0xffffffffu, acc[m][i], 16);
+            }
     }
-    if (n < N)
+    if (lane < LANES)
 #pragma unroll
-        for (int m = 0; m < MT; ++m) scratch[((size_t)split * MT + m) * N + n] = acc[m];
-    __threadfence();
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) red[(warp * MT + m) * FGEMV_COLS + c + i] = acc[m][i];
     __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned prev = atomicAdd(&counters[blockIdx.x], 1u);
-        is_last = (prev == (unsigned)(splits - 1));
-        if (is_last) counters[blockIdx.x] = 0u;
+    float t = 0.0f;
+    if (warp < MT)
+#pragma unroll
+        for (int s = 0; s < WARPS; ++s) t += red[(s * MT + warp) * FGEMV_COLS + lane];
+    if (splits > 1) {
+        cluster_wait();
+        if (warp < MT) st_cluster(&part[(split * MT + warp) * FGEMV_COLS + lane], 0, t);
+        cluster_arrive();
+        cluster_wait(); // every block's sums are in the first block
+        if (split != 0) return;
+        t = 0.0f;
+        if (warp < MT)
+            for (int sp = 0; sp < splits; ++sp) t += part[(sp * MT + warp) * FGEMV_COLS + lane];
     }
-    __syncthreads();
-    if (!is_last || n >= N) return;
-    __threadfence();
-#pragma unroll
-    for (int m = 0; m < MT; ++m) {
-        if (m >= m_valid) break;
-        float t = 0.0f;
-        for (int sp = 0; sp < splits; ++sp) t += __ldcg(&scratch[((size_t)sp * MT + m) * N + n]);
-        epi_apply(epi, m0 + m, n, t);
+    if (warp < min(MT, m_valid)) { // one warp per row: 32 consecutive features
+        const int n = n_base + lane;
+        if (n < N) epi_apply(epi, m0 + warp, n, t);
+        if (epi.amax_val) epi_argmax1(epi, m0 + warp, n, t + (epi.bias && n < N ? epi.bias[n] : 0.0f), n < N);
     }
 }
 
 template <typename XT>
 __global__ void __launch_bounds__(256)
-f32_gemm_kernel(const float *__restrict__ w, const XT *__restrict__ x, int M, int K, int N, Epilogue epi) {
+f32_gemm_kernel(const float *__restrict__ w, int ldw, const XT *__restrict__ x, int M, int K, int N, Epilogue epi) {
     __shared__ float xs[16][64 + 1]; // [k][m]
     __shared__ float ws[16][64];     // [k][n]
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
@@ -94,7 +149,7 @@ f32_gemm_kernel(const float *__restrict__ w, const XT *__restrict__ x, int M, in
         for (int i = threadIdx.x; i < 16 * 64; i += 256) {
             int kk = i >> 6, nn = i & 63;
             int k = k0 + kk, n = n_base + nn;
-            ws[kk][nn] = (k < K && n < N) ? w[(size_t)k * N + n] : 0.0f;
+            ws[kk][nn] = (k < K && n < N) ? w[(size_t)k * ldw + n] : 0.0f;
         }
         __syncthreads();
 #pragma unroll
@@ -123,45 +178,77 @@ f32_gemm_kernel(const float *__restrict__ w, const XT *__restrict__ x, int M, in
     }
 }
 
-template <int MT, typename XT>
-static int f32_gemv_chunk(b200nn_ctx *ctx, const F32Weight &w, const XT *x, int m_valid, int m0, const Epilogue &epi) {
-    int col_blocks = (w.N + 255) / 256;
-    int target = 2 * ctx->sm_count;
-    int splits = (target + col_blocks - 1) / col_blocks;
-    int per = (w.K + splits - 1) / splits;
-    if (per < 64) per = 64;
-    if (per > 2048) per = 2048;
-    per = (per + 3) & ~3;
+template <int MT, int VEC, typename XT>
+static int f32_gemv_launch(b200nn_ctx *ctx, const F32Weight &w, const XT *x, int m_valid, int m0, const NormIn &ln, const Epilogue &epi) {
+    // K split over a cluster until there is about a block per SM (GPT-2 Small, 64 tokens after a prompt of 64: 24.7 ms; two
+    // blocks per SM 27.0, three 27.6), none of under 64 rows unless the activations need it
+    const int tiles = (w.N + FGEMV_COLS - 1) / FGEMV_COLS;
+    int splits = std::min(8, std::max(1, ctx->sm_count / tiles));
+    splits = std::min(splits, std::max(1, w.K / 64));
+    splits = std::max(splits, (int)(((size_t)MT * w.K * sizeof(float) + FGEMV_XS - 1) / FGEMV_XS));
+    const int per = (w.K + splits - 1) / splits;
     splits = (w.K + per - 1) / per;
-    if (splits > 1) TRY(ensure_scratch(ctx, (size_t)splits * MT * w.N * 4, (size_t)col_blocks));
-    dim3 grid(col_blocks, splits);
-    PREFER_SMEM_ONCE((f32_gemv_kernel<MT, XT>));
-    f32_gemv_kernel<MT, XT><<<grid, 256, (size_t)MT * per * 4, ctx->stream>>>(
-        (const float *)w.w_kn->p, x, m_valid, m0, w.K, w.N, per, epi, ctx->scratch, ctx->counters);
+    auto kern = f32_gemv_kernel<MT, VEC, XT>;
+    const size_t smem = ((size_t)MT * per + (size_t)(FGEMV_THREADS / 32 + splits) * MT * FGEMV_COLS) * sizeof(float);
+    static bool attr_done[16] = {}; // function attributes are per device
+    if (!attr_done[ctx->device & 15]) {
+        CK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        prefer_max_smem(kern);
+        attr_done[ctx->device & 15] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(tiles, splits);
+    cfg.blockDim = dim3(FGEMV_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = splits;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = ctx->pdl && !w.volatile_w ? 2 : 1;
+    CK(ctx, cudaLaunchKernelEx(&cfg, kern, (const float *)w.w_kn->p, w.ld(), x, m_valid, m0, w.K, w.N, per, ln, epi));
     CK_LAUNCH(ctx, "f32_gemv_kernel");
     return B200NN_OK;
 }
+template <int MT, typename XT>
+static int f32_gemv_chunk(b200nn_ctx *ctx, const F32Weight &w, const XT *x, int m_valid, int m0, const NormIn &ln, const Epilogue &epi) {
+    // rows of the weight that all start on 16 bytes: vector loads
+    if (w.ld() % 4 == 0 && !((uintptr_t)w.w_kn->p & 15)) return f32_gemv_launch<MT, 4, XT>(ctx, w, x, m_valid, m0, ln, epi);
+    return f32_gemv_launch<MT, 1, XT>(ctx, w, x, m_valid, m0, ln, epi);
+}
 
 template <typename XT>
-static int f32_linear_t(b200nn_ctx *ctx, const F32Weight &w, const XT *x, int M, const Epilogue &epi) {
-    if (M <= 4) {
-        if (M == 4) return f32_gemv_chunk<4, XT>(ctx, w, x, 4, 0, epi);
+static int f32_linear_t(b200nn_ctx *ctx, const F32Weight &w, const XT *x, int M, const NormIn &ln, const Epilogue &epi) {
+    // a K range that a cluster's shared memory does not hold goes to the tiled kernel
+    if (M <= F32_GEMV_ROWS && f32_gemv_fits(w)) {
+        if (M == 4) return f32_gemv_chunk<4, XT>(ctx, w, x, 4, 0, ln, epi);
         if (M >= 2) {
-            TRY((f32_gemv_chunk<2, XT>(ctx, w, x, 2, 0, epi)));
-            if (M == 3) return f32_gemv_chunk<1, XT>(ctx, w, x + (size_t)2 * w.K, 1, 2, epi);
+            TRY((f32_gemv_chunk<2, XT>(ctx, w, x, 2, 0, ln, epi)));
+            if (M == 3) return f32_gemv_chunk<1, XT>(ctx, w, x + (size_t)2 * w.K, 1, 2, ln, epi);
             return B200NN_OK;
         }
-        return f32_gemv_chunk<1, XT>(ctx, w, x, 1, 0, epi);
+        return f32_gemv_chunk<1, XT>(ctx, w, x, 1, 0, ln, epi);
     }
     dim3 grid((w.N + 63) / 64, (M + 63) / 64);
     PREFER_SMEM_ONCE(f32_gemm_kernel<XT>);
-    f32_gemm_kernel<XT><<<grid, 256, 0, ctx->stream>>>((const float *)w.w_kn->p, x, M, w.K, w.N, epi);
+    f32_gemm_kernel<XT><<<grid, 256, 0, ctx->stream>>>((const float *)w.w_kn->p, w.ld(), x, M, w.K, w.N, epi);
     CK_LAUNCH(ctx, "f32_gemm_kernel");
     return B200NN_OK;
 }
 
-int launch_f32_linear(b200nn_ctx *ctx, const F32Weight &w, const void *x, bool x_half, int M, const Epilogue &epi) {
+bool f32_linear_takes_norm(const F32Weight &w, int M) { return M >= 1 && M <= F32_GEMV_ROWS && w.K <= NORM_IN_MAX; }
+
+int launch_f32_linear(b200nn_ctx *ctx, const F32Weight &w, const void *x, bool x_half, int M, const Epilogue &epi, const NormIn &ln) {
     if (M <= 0) return B200NN_OK;
+    if (ln.g) {
+        if (x_half || !f32_linear_takes_norm(w, M))
+            return set_error(ctx, B200NN_ERR_UNSUPPORTED, "f32 Linear: only the GEMV of few rows takes a LayerNorm with its input");
+        return f32_linear_t<float>(ctx, w, (const float *)x, M, ln, epi);
+    }
     if (f16_gemm_tc_supported(ctx, w, M) && !((uintptr_t)x & 15)) {
         // more than four rows: fp16 operands on the tensor cores.  f32 activations are converted once
         // into a buffer the context keeps (grown outside stream capture only).
@@ -175,6 +262,6 @@ int launch_f32_linear(b200nn_ctx *ctx, const F32Weight &w, const void *x, bool x
         TRY(launch_f32_to_half(ctx, (const float *)x, (__half *)ctx->xh->p, (size_t)M * w.K));
         return launch_f16_gemm_tc(ctx, w, (const __half *)ctx->xh->p, M, epi);
     }
-    return x_half ? f32_linear_t<__half>(ctx, w, (const __half *)x, M, epi)
-                  : f32_linear_t<float>(ctx, w, (const float *)x, M, epi);
+    return x_half ? f32_linear_t<__half>(ctx, w, (const __half *)x, M, ln, epi)
+                  : f32_linear_t<float>(ctx, w, (const float *)x, M, ln, epi);
 }

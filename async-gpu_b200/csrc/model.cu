@@ -6,14 +6,18 @@
 
 #include "model.h"
 
-int linear_forward(b200nn_ctx *ctx, const LinearAny &l, const void *x, bool x_half, int M, Epilogue epi, int ldx) {
+int linear_forward(b200nn_ctx *ctx, const LinearAny &l, const void *x, bool x_half, int M, Epilogue epi, int ldx, const NormIn &ln) {
     if (l.b16) {
         if (!x_half) return set_error(ctx, B200NN_ERR_UNSUPPORTED, "a bfloat16 Linear takes bfloat16 activations");
         return launch_b16_linear(ctx, l.b, static_cast<const __nv_bfloat16 *>(x), ldx ? ldx : l.b.K, M, epi);
     }
     if (!epi.ln_stats) epi.bias = l.bias(); // a folded LayerNorm brings its own combined bias
-    if (l.int4) return launch_int4_linear(ctx, l.q, x, x_half, M, epi);
-    return launch_f32_linear(ctx, l.f, x, x_half, M, epi);
+    if (l.int4) return launch_int4_linear(ctx, l.q, x, x_half, M, epi, ln);
+    return launch_f32_linear(ctx, l.f, x, x_half, M, epi, ln);
+}
+bool linear_takes_norm(const LinearAny &l, int M) {
+    if (l.b16) return false;
+    return l.int4 ? int4_linear_takes_norm(l.q, M) : f32_linear_takes_norm(l.f, M);
 }
 
 static int upload_vec(b200nn_ctx *ctx, const float *h, size_t n, std::shared_ptr<DevBuf> *out) {
@@ -234,8 +238,11 @@ static void fold_producer(const Workspace &ws, int slot, const std::shared_ptr<D
     e->stats_nt = ws.ln_nt;
 }
 
+// With f32 activations (few rows) the GEMV behind a LayerNorm applies it: one kernel less in a step's chain.
+static bool norm_rides(const LinearAny &l, bool act_half, int rows) { return !act_half && linear_takes_norm(l, rows); }
+
 int BlockLaunch::ln1() const {
-    if (fold) return B200NN_OK;
+    if (fold || norm_rides(m->blocks[l].qkv, act_half, B * S)) return B200NN_OK;
     const BlockW &b = m->blocks[l];
     return launch_layernorm(m->ctx, (const float *)ws.x->p, nullptr, nullptr, (const float *)b.ln1_g->p, (const float *)b.ln1_b->p,
                             m->cfg.layer_norm_epsilon, B * S, m->cfg.n_embd, ws.ln->p, act_half);
@@ -256,7 +263,11 @@ int BlockLaunch::qkv() const {
     e.pos_ptr = pos_ptr;
     e.pos_off = pos_off;
     if (fold) fold_consumer(m, ws, 2 * l, m->blocks[l].qkv_gsum, m->blocks[l].qkv_bc, &e);
-    return linear_forward(m->ctx, m->blocks[l].qkv, ws.ln->p, act_half, B * S, e);
+    const BlockW &b = m->blocks[l];
+    if (norm_rides(b.qkv, act_half, B * S))
+        return linear_forward(m->ctx, b.qkv, ws.x->p, false, B * S, e, 0,
+                              NormIn{(const float *)b.ln1_g->p, (const float *)b.ln1_b->p, m->cfg.layer_norm_epsilon});
+    return linear_forward(m->ctx, b.qkv, ws.ln->p, act_half, B * S, e);
 }
 int BlockLaunch::attention() const {
     const int d = m->cfg.n_embd, H = m->cfg.n_head;
@@ -275,7 +286,7 @@ int BlockLaunch::proj() const {
     return linear_forward(m->ctx, m->blocks[l].proj, ws.att->p, act_half, B * S, r);
 }
 int BlockLaunch::ln2() const {
-    if (fold) return B200NN_OK;
+    if (fold || norm_rides(m->blocks[l].fc, act_half, B * S)) return B200NN_OK;
     const BlockW &b = m->blocks[l];
     return launch_layernorm(m->ctx, (const float *)ws.x->p, nullptr, nullptr, (const float *)b.ln2_g->p, (const float *)b.ln2_b->p,
                             m->cfg.layer_norm_epsilon, B * S, m->cfg.n_embd, ws.ln->p, act_half);
@@ -288,7 +299,11 @@ int BlockLaunch::fc() const {
     f.ldo = 4 * m->cfg.n_embd;
     f.out_half = act_half;
     if (fold) fold_consumer(m, ws, 2 * l + 1, m->blocks[l].fc_gsum, m->blocks[l].fc_bc, &f);
-    return linear_forward(m->ctx, m->blocks[l].fc, ws.ln->p, act_half, B * S, f);
+    const BlockW &b = m->blocks[l];
+    if (norm_rides(b.fc, act_half, B * S))
+        return linear_forward(m->ctx, b.fc, ws.x->p, false, B * S, f, 0,
+                              NormIn{(const float *)b.ln2_g->p, (const float *)b.ln2_b->p, m->cfg.layer_norm_epsilon});
+    return linear_forward(m->ctx, b.fc, ws.ln->p, act_half, B * S, f);
 }
 int BlockLaunch::fcproj() const {
     Epilogue r;
@@ -355,10 +370,10 @@ int run_head(b200nn_gpt2 *m, Workspace &ws, const float *x, int rows, bool act_h
 }
 
 // Which LM-head launches take the greedy pick in their epilogue: the tensor-core GEMMs and the two
-// GEMV kernels of an int4 head in the tiled layout, and the fp16 tensor-core GEMM of an f32 head.
+// GEMV kernels of an int4 head in the tiled layout, and the GEMV and the fp16 tensor-core GEMM of an f32 head.
 static bool head_fuses_pick(const b200nn_gpt2 *m, int rows, bool head_half) {
     if (m->lm_head.int4) return m->lm_head.q.fast && rows < 2048;
-    return head_half && f16_gemm_tc_supported(m->ctx, m->lm_head.f, rows);
+    return (rows <= F32_GEMV_ROWS && f32_gemv_fits(m->lm_head.f)) || (head_half && f16_gemm_tc_supported(m->ctx, m->lm_head.f, rows));
 }
 
 int run_head_pick(b200nn_gpt2 *m, Workspace &ws, const float *x, int rows, bool act_half, bool keep_last, bool tokens_only,

@@ -21,7 +21,8 @@ struct LinearAny {
 };
 // x_half: the activations are 16-bit (fp16, or bfloat16 for a bfloat16 weight), K elements per row unless
 // ldx says otherwise (bfloat16 only).
-int linear_forward(b200nn_ctx *ctx, const LinearAny &l, const void *x, bool x_half, int M, Epilogue epi, int ldx = 0);
+int linear_forward(b200nn_ctx *ctx, const LinearAny &l, const void *x, bool x_half, int M, Epilogue epi, int ldx = 0, const NormIn &ln = NormIn());
+bool linear_takes_norm(const LinearAny &l, int M); // the Linear can apply the LayerNorm of its f32 input rows itself
 
 struct b200nn_linear {
     b200nn_ctx *ctx;

@@ -320,14 +320,16 @@ int f32_weight_upload(b200nn_ctx *ctx, const float *wsrc, bool is_out_in, const 
     w->exact = exact;
     w->K = (int)K;
     w->N = (int)N;
-    if (is_out_in) { // [N,K] -> [K,N]
-        std::vector<float> t(K * N);
+    const size_t ld = (N + 3) & ~(size_t)3; // rows start on 16 bytes
+    w->ldw = (int)ld;
+    if (is_out_in || ld != N) { // [N,K] -> [K,ld], or wider rows
+        std::vector<float> t(K * ld, 0.0f);
         float *tp = t.data();
         parallel_for(N, [=](size_t n0, size_t n1) {
             for (size_t n = n0; n < n1; ++n)
-                for (size_t k = 0; k < K; ++k) tp[k * N + n] = wsrc[n * K + k];
+                for (size_t k = 0; k < K; ++k) tp[k * ld + n] = is_out_in ? wsrc[n * K + k] : wsrc[k * N + n];
         });
-        TRY(upload(ctx, t.data(), K * N * sizeof(float), &w->w_kn));
+        TRY(upload(ctx, t.data(), K * ld * sizeof(float), &w->w_kn));
     } else {
         TRY(upload(ctx, wsrc, K * N * sizeof(float), &w->w_kn));
     }
