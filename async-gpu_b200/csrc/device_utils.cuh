@@ -35,6 +35,10 @@ __device__ __forceinline__ float apply_act(float v, int act) {
     }
 }
 
+__device__ __forceinline__ float4 f4_add(float4 a, float4 b) {
+    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<const uint32_t *>(&h);
@@ -81,60 +85,119 @@ __device__ __forceinline__ void epi_store(const Epilogue &e, int m, int n, float
         static_cast<float *>(e.out)[i] = v;
 }
 
-// Four consecutive columns n..n+3 (n % 4 == 0) of row m in one go: 16-byte (f32) or 8-byte (fp16)
-// stores when the destination allows it, element-wise otherwise.  pos_ptr must already be folded
-// into e.pos_off by the caller (it is not dereferenced here for the vector path).
-template <bool B16 = false>
-__device__ __forceinline__ void epi_store4(const Epilogue &e, int m, int n, float4 v, int N) {
+// U token rows' finished values at once, the activation chosen once for all of them.
+template <int ACT, int U>
+__device__ __forceinline__ void act_rows(float4 (&v)[U]) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        v[u].x = apply_act(v[u].x, ACT); v[u].y = apply_act(v[u].y, ACT);
+        v[u].z = apply_act(v[u].z, ACT); v[u].w = apply_act(v[u].w, ACT);
+    }
+}
+template <int U>
+__device__ __forceinline__ void act_rows(float4 (&v)[U], int act) {
+    switch (act) {
+        case B200NN_ACT_GELU_TANH: return act_rows<B200NN_ACT_GELU_TANH>(v);
+        case B200NN_ACT_GELU_SIGMOID: return act_rows<B200NN_ACT_GELU_SIGMOID>(v);
+        case B200NN_ACT_RELU: return act_rows<B200NN_ACT_RELU>(v);
+        case B200NN_ACT_SILU: return act_rows<B200NN_ACT_SILU>(v);
+        case B200NN_ACT_SIGMOID: return act_rows<B200NN_ACT_SIGMOID>(v);
+        default: return;
+    }
+}
+
+// Four consecutive columns n..n+3 (n % 4 == 0) of the token rows m0, m0 + step, ... (cnt <= U of them; values past cnt are
+// not looked at): 16-byte (f32) or 8-byte (fp16) stores when the destination allows it, element-wise otherwise.  pos_ptr
+// must already be folded into e.pos_off by the caller (it is not dereferenced here for the vector path).
+// What to do with a value is decided once for the U rows, and their chains (activation, position, rotation) run under each
+// other (the hybrid decoder's prompts of 64 x 1024 and 32 steps: 50.2 -> 49.1 ms with four rows).
+template <int U, bool B16 = false>
+__device__ __forceinline__ void epi_store4_rows(const Epilogue &e, int m0, int step, int cnt, int n, float4 (&v)[U], int N) {
     if (e.no_store) return;
     if (B16 && e.mode == EPI_GLU) { // N and ldo are multiples of 4
         if (n >= N) return;
-        const size_t i = (size_t)m * e.ldo + (n >> 1);
-        *reinterpret_cast<uint32_t *>(static_cast<__nv_bfloat16 *>(e.out) + i) =
-            pack_bf16x2(apply_act(v.x, e.act) * v.z, apply_act(v.y, e.act) * v.w);
+        float4 g[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) g[u] = make_float4(v[u].x, v[u].y, 0.0f, 0.0f);
+        act_rows<U>(g, e.act);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (u < cnt)
+                *reinterpret_cast<uint32_t *>(static_cast<__nv_bfloat16 *>(e.out) + (size_t)(m0 + u * step) * e.ldo + (n >> 1)) =
+                    pack_bf16x2(g[u].x * v[u].z, g[u].y * v[u].w);
         return;
     }
     if (B16 && e.mode == EPI_ROPE) {
         if (n >= N) return;
         const int p = (n % e.rope_head - e.rope_at) >> 1;
         if (p >= 0 && p < e.rope_pairs) {
-            const float2 *t = e.rope_tab + (size_t)row_pos(e.rows, m) * e.rope_pairs + p;
-            const float2 c0 = t[0];
-            const float2 c1 = p + 1 < e.rope_pairs ? t[1] : make_float2(1.0f, 0.0f);
-            v = make_float4(v.x * c0.x - v.y * c0.y, v.y * c0.x + v.x * c0.y, v.z * c1.x - v.w * c1.y, v.w * c1.x + v.z * c1.y);
+            float2 c0[U], c1[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const float2 *t = e.rope_tab + (size_t)row_pos(e.rows, m0 + (u < cnt ? u : 0) * step) * e.rope_pairs + p;
+                c0[u] = t[0];
+                c1[u] = p + 1 < e.rope_pairs ? t[1] : make_float2(1.0f, 0.0f);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                v[u] = make_float4(v[u].x * c0[u].x - v[u].y * c0[u].y, v[u].y * c0[u].x + v[u].x * c0[u].y,
+                                   v[u].z * c1[u].x - v[u].w * c1[u].y, v[u].w * c1[u].x + v[u].z * c1[u].y);
         }
     }
     if (B16 && e.tail_out && n >= e.tail_at) {
-        const float f[4] = {v.x, v.y, v.z, v.w};
-        const size_t i = (size_t)m * e.tail_ld + (n - e.tail_at);
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (n + j < N) {
-                if (e.tail_type == OUT_BF16) static_cast<__nv_bfloat16 *>(e.tail_out)[i + j] = __float2bfloat16_rn(f[j]);
-                else static_cast<float *>(e.tail_out)[i + j] = f[j];
-            }
+        for (int u = 0; u < U; ++u) {
+            if (u >= cnt) break;
+            const float f[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+            const size_t i = (size_t)(m0 + u * step) * e.tail_ld + (n - e.tail_at);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (n + j < N) {
+                    if (e.tail_type == OUT_BF16) static_cast<__nv_bfloat16 *>(e.tail_out)[i + j] = __float2bfloat16_rn(f[j]);
+                    else static_cast<float *>(e.tail_out)[i + j] = f[j];
+                }
+        }
         return;
     }
     if (B16 && e.kv_cache && n >= e.kv_at) { // kv_w is a multiple of 16
         if (n >= N) return;
         const int c = n - e.kv_at, head = c / e.kv_w;
-        const size_t row = ((size_t)row_slot(e.rows, m) * e.kv_heads + head) * e.kv_cap + row_pos(e.rows, m);
-        *reinterpret_cast<uint2 *>(e.kv_cache + row * e.kv_w + (c - head * e.kv_w)) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+        int pos[U], slot[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int m = m0 + (u < cnt ? u : 0) * step;
+            pos[u] = row_pos(e.rows, m);
+            slot[u] = row_slot(e.rows, m);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (u < cnt) {
+                const size_t row = ((size_t)slot[u] * e.kv_heads + head) * e.kv_cap + pos[u];
+                *reinterpret_cast<uint2 *>(e.kv_cache + row * e.kv_w + (c - head * e.kv_w)) =
+                    make_uint2(pack_bf16x2(v[u].x, v[u].y), pack_bf16x2(v[u].z, v[u].w));
+            }
         return;
     }
     const bool vec = (n + 3 < N) && ((e.ldo & 3) == 0) && (e.pos_ptr == nullptr);
     if (!vec) {
-        if (n < N) epi_store<B16>(e, m, n, v.x);
-        if (n + 1 < N) epi_store<B16>(e, m, n + 1, v.y);
-        if (n + 2 < N) epi_store<B16>(e, m, n + 2, v.z);
-        if (n + 3 < N) epi_store<B16>(e, m, n + 3, v.w);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (u >= cnt) break;
+            if (n < N) epi_store<B16>(e, m0 + u * step, n, v[u].x);
+            if (n + 1 < N) epi_store<B16>(e, m0 + u * step, n + 1, v[u].y);
+            if (n + 2 < N) epi_store<B16>(e, m0 + u * step, n + 2, v[u].z);
+            if (n + 3 < N) epi_store<B16>(e, m0 + u * step, n + 3, v[u].w);
+        }
         return;
     }
     if (e.mode == EPI_RESID) {
-        float4 *p = reinterpret_cast<float4 *>(e.resid + (size_t)m * e.ldo + n);
-        float4 r = *p;
-        r.x += v.x; r.y += v.y; r.z += v.z; r.w += v.w;
-        *p = r;
+        float4 r[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (u < cnt) r[u] = __ldcg(reinterpret_cast<const float4 *>(e.resid + (size_t)(m0 + u * step) * e.ldo + n));
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (u < cnt) *reinterpret_cast<float4 *>(e.resid + (size_t)(m0 + u * step) * e.ldo + n) = f4_add(r[u], v[u]);
         return;
     }
     if (e.mode == EPI_QKV && n >= e.d_model) {
@@ -144,29 +207,35 @@ __device__ __forceinline__ void epi_store4(const Epilogue &e, int m, int n, floa
             c -= e.d_model;
             cache = e.vc;
         }
-        const int head = c >> 6, el = c & 63;
-        const int b = m / e.rows_per_seq, s = m - b * e.rows_per_seq;
-        const int pos = e.pos_off + s;
-        if (pos < e.cap) {
-            __half2 lo = __floats2half2_rn(v.x, v.y), hi = __floats2half2_rn(v.z, v.w);
-            uint2 u = make_uint2(*reinterpret_cast<uint32_t *>(&lo), *reinterpret_cast<uint32_t *>(&hi));
-            *reinterpret_cast<uint2 *>(cache + (((size_t)b * e.n_head + head) * e.cap + pos) * 64 + el) = u;
+        cache += (size_t)(c >> 6) * e.cap * 64 + (c & 63);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int m = m0 + u * step, b = e.rows_per_seq == 1 ? m : m / e.rows_per_seq, pos = e.pos_off + m - b * e.rows_per_seq;
+            if (u < cnt && pos < e.cap)
+                *reinterpret_cast<uint2 *>(cache + ((size_t)b * e.n_head * e.cap + pos) * 64) =
+                    make_uint2(pack_f16x2(v[u].x, v[u].y), pack_f16x2(v[u].z, v[u].w));
         }
         return;
     }
-    v.x = apply_act(v.x, e.act); v.y = apply_act(v.y, e.act);
-    v.z = apply_act(v.z, e.act); v.w = apply_act(v.w, e.act);
+    act_rows<U>(v, e.act);
     if (B16 && e.row_scale) {
-        const float rs = e.row_scale[(size_t)m * e.rs_ld + n / e.rs_cols];
-        v.x *= rs; v.y *= rs; v.z *= rs; v.w *= rs;
+        float rs[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) rs[u] = e.row_scale[(size_t)(m0 + (u < cnt ? u : 0) * step) * e.rs_ld + n / e.rs_cols];
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = make_float4(v[u].x * rs[u], v[u].y * rs[u], v[u].z * rs[u], v[u].w * rs[u]);
     }
-    const size_t i = (size_t)m * e.ldo + n;
-    if (e.out_half) {
-        const uint2 u = B16 && e.out_half == OUT_BF16 ? make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w))
-                                                      : make_uint2(pack_f16x2(v.x, v.y), pack_f16x2(v.z, v.w));
-        *reinterpret_cast<uint2 *>(static_cast<__half *>(e.out) + i) = u;
-    } else {
-        *reinterpret_cast<float4 *>(static_cast<float *>(e.out) + i) = v;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        if (u >= cnt) break;
+        const size_t i = (size_t)(m0 + u * step) * e.ldo + n;
+        if (e.out_half) {
+            *reinterpret_cast<uint2 *>(static_cast<__half *>(e.out) + i) =
+                B16 && e.out_half == OUT_BF16 ? make_uint2(pack_bf16x2(v[u].x, v[u].y), pack_bf16x2(v[u].z, v[u].w))
+                                              : make_uint2(pack_f16x2(v[u].x, v[u].y), pack_f16x2(v[u].z, v[u].w));
+        } else {
+            *reinterpret_cast<float4 *>(static_cast<float *>(e.out) + i) = v[u];
+        }
     }
 }
 
@@ -248,10 +317,6 @@ __device__ __forceinline__ void epi_resid_red4(const Epilogue &e, int m, int n, 
     }
 }
 
-__device__ __forceinline__ float4 f4_add(float4 a, float4 b) {
-    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
-}
-
 // ---- LayerNorm folded into the neighbouring GEMMs (see Epilogue) ---------------------------------
 // A row's (mean, 1/sqrt(var + eps)) from the partial sums its producer left, added in tile order.
 __device__ __forceinline__ float2 epi_row_mean_rstd(const Epilogue &e, int m) {
@@ -314,16 +379,30 @@ __device__ __forceinline__ void epi_resid_ln4(const Epilogue &e, int m, int n, f
     if ((threadIdx.x & 31) == 0)
         *reinterpret_cast<float2 *>(e.stats_out + ((size_t)m * e.stats_nt + (n >> 7)) * 2) = make_float2(s1, s2);
 }
+// cnt <= U finished rows (m0, m0 + step, ...) of a 128-feature tile leave the GEMM (warp-collective): v = the complete sums,
+// bias not yet added.
+template <int U, bool B16 = false>
+__device__ __forceinline__ void epi_emit4_rows(const Epilogue &e2, const Epilogue &epi, int m0, int step, int cnt, int n, float4 (&v)[U],
+                                               float4 b4, int N) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = f4_add(v[u], b4);
+    if (epi.amax_val)
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (u < cnt) epi_argmax4(epi, m0 + u * step, n, v[u], N);
+    epi_store4_rows<U, B16>(e2, m0, step, cnt, n, v, N);
+}
 // One finished row of a 128-feature tile leaves the GEMM (warp-collective as above): acc = the complete
 // sums of products, f4 = epi_fold4, mr = the row's (mean, rstd) when ln_stats is set, r = epi_resid_old4.
 __device__ __forceinline__ void epi_emit4(const Epilogue &e2, const Epilogue &epi, int m, int n, float4 acc, float4 f4,
                                           float4 b4, float2 mr, float4 r, int N) {
-    const float4 v = epi_finish4(epi, acc, f4, b4, mr);
+    float4 v[1] = {epi_finish4(epi, acc, f4, b4, mr)};
     if (epi.mode == EPI_RESID_LN) {
-        epi_resid_ln4(epi, m, n, v, r, f4, N);
+        epi_resid_ln4(epi, m, n, v[0], r, f4, N);
     } else {
-        epi_store4(e2, m, n, v, N);
-        if (epi.amax_val) epi_argmax4(epi, m, n, v, N);
+        epi_store4_rows<1>(e2, m, 1, 1, n, v, N);
+        v[0] = epi_finish4(epi, acc, f4, b4, mr);
+        if (epi.amax_val) epi_argmax4(epi, m, n, v[0], N);
     }
 }
 
@@ -368,9 +447,17 @@ __device__ __forceinline__ float load_as_float<__nv_bfloat16>(const __nv_bfloat1
 // kernel ran on the same SM, so a line that came into L1 since this kernel's start (or through the read-only
 // path, which a plain load from a const __restrict__ pointer takes) can be older than the wait: the second of four f32 rows
 // got its MLP from the residual stream without the attention's sum.
-__device__ __forceinline__ float load_fresh(const float *p, size_t i) { return __ldcg(p + i); }
+// (volatile: it stays behind the wait, and in the order of the source, so values that should be in flight together are
+// loaded before the first of them is used)
+__device__ __forceinline__ float load_fresh(const float *p, size_t i) {
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p + i));
+    return v;
+}
 __device__ __forceinline__ float load_fresh(const __half *p, size_t i) {
-    return __half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short *>(p) + i)));
+    unsigned short v;
+    asm volatile("ld.global.cg.u16 %0, [%1];" : "=h"(v) : "l"(p + i));
+    return __half2float(__ushort_as_half(v));
 }
 __device__ __forceinline__ void store_from_float(float *p, float v) { *p = v; }
 __device__ __forceinline__ void store_from_float(__half *p, float v) { *p = __float2half_rn(v); }
@@ -453,6 +540,23 @@ __device__ __forceinline__ void norm_rows_to_smem(const NormIn &ln, const float 
             if (kk >= 0 && kk < ld) xs[m * ld + kk] = m < m_valid && kk < cols ? (v[m][i] - mean[m]) * inv_std * g[i] + b[i] : 0.0f;
         }
     }
+}
+
+// Columns k0 .. k0+cols of up to MT rows x [m_valid][K] as f32 in xs [MT][ld], zero past them and past m_valid.
+template <int MT, int THREADS, typename XT>
+__device__ __forceinline__ void rows_to_smem(const XT *__restrict__ x, int m_valid, int K, int k0, int cols, int ld, float *xs) {
+    constexpr int U = 4; // loads of a thread in flight
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+        for (int base = threadIdx.x; base < ld; base += U * THREADS) {
+            float v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                v[u] = m < m_valid && base + u * THREADS < cols ? load_fresh(x, (size_t)m * K + k0 + base + u * THREADS) : 0.0f;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (base + u * THREADS < ld) xs[m * ld + base + u * THREADS] = v[u];
+        }
 }
 
 __device__ __forceinline__ float sigmoid_f(float v) { return 1.0f / (1.0f + expf(-v)); }

@@ -225,10 +225,13 @@ f16_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             const float4 *stage4 = reinterpret_cast<const float4 *>(stage);
             const int rows = min(MB, M - mt * MB);
             if (splits == 1) {
-                for (int c = w8; c < rows; c += NW) {
-                    const float4 v = f4_add(stage4[c * 32 + lane], b4);
-                    epi_store4<B16>(e2, mt * MB + c, n4, v, n_lim);
-                    if (epi.amax_val) epi_argmax4(epi, mt * MB + c, n4, v, n_lim);
+                constexpr int U = MB / NW < 4 ? MB / NW : 4; // token rows a warp finishes at a time
+                for (int c = w8; c < rows; c += U * NW) {
+                    float4 v[U];
+                    const int cnt = min(U, (rows - c + NW - 1) / NW);
+#pragma unroll
+                    for (int u = 0; u < U; ++u) v[u] = stage4[(c + (u < cnt ? u : 0) * NW) * 32 + lane];
+                    epi_emit4_rows<U, B16>(e2, epi, mt * MB + c, NW, cnt, n4, v, b4, n_lim);
                 }
             } else if (epi.mode == EPI_RESID) {
                 // every split adds its partial tile into the f32 residual stream with vector
@@ -252,12 +255,20 @@ f16_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             const int w8 = warp - 2;
             const float4 *stage4 = reinterpret_cast<const float4 *>(gen_base);
             const int rows = min(MB, M - mt * MB);
-            for (int c = split + splits * w8; c < rows; c += splits * NW) {
-                float4 sum = b4;
-                for (int sp = 0; sp < splits; ++sp)
-                    sum = f4_add(sum, cluster.map_shared_rank(stage4, sp)[c * 32 + lane]);
-                epi_store4<B16>(e2, mt * MB + c, n4, sum, n_lim);
-                if (epi.amax_val) epi_argmax4(epi, mt * MB + c, n4, sum, n_lim);
+            constexpr int U = MB / (2 * NW) < 1 ? 1 : MB / (2 * NW) < 4 ? MB / (2 * NW) : 4; // two splits at least share the rows
+            const int step = splits * NW;
+            for (int c = split + splits * w8; c < rows; c += U * step) {
+                float4 v[U];
+                const int cnt = min(U, (rows - c + step - 1) / step);
+#pragma unroll
+                for (int u = 0; u < U; ++u) v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+                for (int sp = 0; sp < splits; ++sp) {
+                    const float4 *p = cluster.map_shared_rank(stage4, sp);
+#pragma unroll
+                    for (int u = 0; u < U; ++u) v[u] = f4_add(v[u], p[(c + (u < cnt ? u : 0) * step) * 32 + lane]);
+                }
+                epi_emit4_rows<U, B16>(e2, epi, mt * MB + c, step, cnt, n4, v, b4, n_lim);
             }
         }
         cluster.sync(); // no block leaves while its shared memory may still be read
@@ -454,10 +465,13 @@ f16_gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const 
                     for (int c = w8; c < lim; c += NW)
                         epi_resid_red4(epi, mt * MB + c0 + c, n4, f4_add(stage4[c * 32 + lane], b4), n_lim);
                 } else {
-                    for (int c = w8; c < lim; c += NW) {
-                        const float4 v = f4_add(stage4[c * 32 + lane], b4);
-                        epi_store4<B16>(e2, mt * MB + c0 + c, n4, v, n_lim);
-                        if (epi.amax_val) epi_argmax4(epi, mt * MB + c0 + c, n4, v, n_lim);
+                    constexpr int U = CH / NW < 4 ? CH / NW : 4; // token rows a warp finishes at a time
+                    for (int c = w8; c < lim; c += U * NW) {
+                        float4 v[U];
+                        const int cnt = min(U, (lim - c + NW - 1) / NW);
+#pragma unroll
+                        for (int u = 0; u < U; ++u) v[u] = stage4[(c + (u < cnt ? u : 0) * NW) * 32 + lane];
+                        epi_emit4_rows<U, B16>(e2, epi, mt * MB + c0 + c, NW, cnt, n4, v, b4, n_lim);
                     }
                 }
                 bar_sync_epi<EPI>(); // the stage is free for the next pass

@@ -50,6 +50,59 @@ struct Smem {
     uint32_t acc_full, tmem_slot, sc;
 };
 
+// The epilogues of a decode step have kernels of their own.  A block runs its epilogue once, so what it costs is mostly the
+// fetching of its instructions and the chain of one row's decisions: with all modes in one kernel a token row took 900
+// cycles.  The plain ones want rows that leave as 16- or 8-byte pieces (N and ldo multiples of 4).
+enum EpiKind {
+    EK_ANY,   // every mode and shape
+    EK_STORE, // y = sums + bias, f32 or fp16
+    EK_GELU,  // the same through tanh-GELU
+    EK_QKV,   // fp16 q and cache rows
+    EK_RESID, // splits added into the residual stream
+    EK_ROWS   // y = sums + bias in f32, rows of any length, greedy pick or not: the output matrix
+};
+int epi_kind(const Epilogue &e, int N, int splits) {
+    const bool plain = !e.ln_stats && !e.row_scale && !e.tail_out && !e.kv_cache;
+    if (!plain) return EK_ANY;
+    if (e.mode == EPI_RESID) return splits > 1 ? EK_RESID : EK_ANY;
+    if (e.mode == EPI_STORE && splits == 1 && e.act == B200NN_ACT_NONE && e.out_half == OUT_F32 && (e.amax_val || ((N | e.ldo) & 3))) return EK_ROWS;
+    if (e.no_store || e.amax_val || ((N | e.ldo) & 3) || splits > 8) return EK_ANY;
+    if (e.mode == EPI_QKV) return e.out_half == OUT_F16 && e.act == B200NN_ACT_NONE && e.d_model % 64 == 0 ? EK_QKV : EK_ANY;
+    if (e.mode != EPI_STORE || e.out_half == OUT_BF16) return EK_ANY;
+    return e.act == B200NN_ACT_NONE ? EK_STORE : e.act == B200NN_ACT_GELU_TANH ? EK_GELU : EK_ANY;
+}
+// The finished sums of token rows m0, m0 + step, ... (cnt <= U), features n .. n+3 of each, for EK_STORE, EK_GELU and EK_QKV.
+template <int EK, int U>
+__device__ __forceinline__ void plain_rows(const Epilogue &e, int pos_off, int m0, int step, int cnt, int n, float4 (&v)[U], float4 b4, int N) {
+    if (n >= N) return;
+    if constexpr (EK == EK_QKV) {
+        const int part = n / e.d_model, c = n - part * e.d_model;
+        __half *cache = (part == 1 ? e.kc : e.vc) + (size_t)(c >> 6) * e.cap * 64 + (c & 63);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int m = m0 + u * step, b = e.rows_per_seq == 1 ? m : m / e.rows_per_seq, pos = pos_off + m - b * e.rows_per_seq;
+            if (u >= cnt || (part && pos >= e.cap)) continue;
+            __half *dst = part ? cache + ((size_t)b * e.n_head * e.cap + pos) * 64 : static_cast<__half *>(e.out) + (size_t)m * e.ldo + n;
+            *reinterpret_cast<uint2 *>(dst) = make_uint2(pack_f16x2(v[u].x + b4.x, v[u].y + b4.y), pack_f16x2(v[u].z + b4.z, v[u].w + b4.w));
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            v[u] = f4_add(v[u], b4);
+            if constexpr (EK == EK_GELU) v[u] = make_float4(gelu_tanh_f(v[u].x), gelu_tanh_f(v[u].y), gelu_tanh_f(v[u].z), gelu_tanh_f(v[u].w));
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (u >= cnt) continue;
+            const size_t i = (size_t)(m0 + u * step) * e.ldo + n;
+            if (e.out_half)
+                *reinterpret_cast<uint2 *>(static_cast<__half *>(e.out) + i) = make_uint2(pack_f16x2(v[u].x, v[u].y), pack_f16x2(v[u].z, v[u].w));
+            else
+                *reinterpret_cast<float4 *>(static_cast<float *>(e.out) + i) = v[u];
+        }
+    }
+}
+
 template <int NTHREADS>
 __device__ __forceinline__ void bar_sync_dequant() {
     asm volatile("bar.sync 1, %0;" ::"n"(NTHREADS) : "memory");
@@ -57,7 +110,8 @@ __device__ __forceinline__ void bar_sync_dequant() {
 
 // MB: token-tile width; NS: operand stages (activation tiles in shared memory, dequantised weight
 // tiles in TMEM); NP: packed-weight stages; NG: dequant groups; TC: TMEM columns to allocate.
-template <int MB, int NS, int NP, int NG, int TC>
+// EK: what becomes of the sums (EpiKind).
+template <int MB, int NS, int NP, int NG, int TC, int EK>
 __global__ void __launch_bounds__(96 + 128 * NG, NG == 2 ? 2 : 1)
 int4_gemm_tc_kernel(const uint8_t *__restrict__ tiles, const __half *__restrict__ scales,
                     const __grid_constant__ CUtensorMap tmap_x, int M, int N, int k_blocks, int n_pad, int group,
@@ -223,26 +277,22 @@ int4_gemm_tc_kernel(const uint8_t *__restrict__ tiles, const __half *__restrict_
             const __half2 s2 = __half2half2(sc_s[(((kb0 + i) * TILE_K) / group - g0) * TILE_N + row]);
             __syncwarp();
             if (dw_lane0) tc::mbar_arrive(S.p_empty + 8 * sp); // this warp has its packed words in registers
+            // the whole row is worked out before the stage is waited for: the arithmetic runs under the MMAs that still read it
+            uint32_t o[32];
+            const uint32_t ww[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                __half2 q[4];
+                unpack8_int4(ww[j], q);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    __half2 r = __hmul2(q[e], s2); // (k, k+1) -> low, high half of one 32-bit column
+                    o[4 * j + e] = *reinterpret_cast<uint32_t *>(&r);
+                }
+            }
             if (i >= NS && !tc::mbar_wait(S.ax_empty + 8 * sa, pha ^ 1, &abort_flag, dev_err, ERR_A_EMPTY)) break;
             tc::tc_fence_after_sync();
-            const uint32_t a_addr = tmem_a + ((uint32_t)(quad * 32) << 16) + sa * A_COLS;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint4 w = h ? w1 : w0;
-                const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-                uint32_t o[16];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    __half2 q[4];
-                    unpack8_int4(ww[j], q);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        __half2 r = __hmul2(q[e], s2); // (k, k+1) -> low, high half of one 32-bit column
-                        o[4 * j + e] = *reinterpret_cast<uint32_t *>(&r);
-                    }
-                }
-                tc::tmem_st_x16(a_addr + 16 * h, o);
-            }
+            tc::tmem_st_x32(tmem_a + ((uint32_t)(quad * 32) << 16) + sa * A_COLS, o);
             tc::tmem_st_wait();
             tc::tc_fence_before_sync();
             __syncwarp();
@@ -252,10 +302,10 @@ int4_gemm_tc_kernel(const uint8_t *__restrict__ tiles, const __half *__restrict_
         pdl_wait(); // the epilogue touches buffers the previous kernel may still be using
         // bias and the device-side position are fetched now, under the wait for the last MMAs
         b4 = epi_bias4(epi, n4, N);
-        g4 = epi_fold4(epi, n4, N);
+        if constexpr (EK == EK_ANY) g4 = epi_fold4(epi, n4, N);
         // folded LayerNorm: one thread per token row adds up the row's partial sums (the barrier below publishes them)
-        if (epi.ln_stats && t < MB && mt * MB + t < M) rowstat[t] = epi_row_mean_rstd(epi, mt * MB + t);
-        if (epi.mode == EPI_QKV && epi.pos_ptr) e2.pos_off = epi.pos_off + *epi.pos_ptr;
+        if (EK == EK_ANY && epi.ln_stats && t < MB && mt * MB + t < M) rowstat[t] = epi_row_mean_rstd(epi, mt * MB + t);
+        if ((EK == EK_ANY || EK == EK_QKV) && epi.mode == EPI_QKV && epi.pos_ptr) e2.pos_off = epi.pos_off + *epi.pos_ptr;
         bar_sync_dequant<DQ>();
         if (!abort_flag) tc::mbar_wait(S.acc_full, 0, &abort_flag, dev_err, ERR_ACC);
         bar_sync_dequant<DQ>();
@@ -287,6 +337,36 @@ int4_gemm_tc_kernel(const uint8_t *__restrict__ tiles, const __half *__restrict_
             const int tile_lin = mt * gridDim.x + nt;
             const float4 *stage4 = reinterpret_cast<const float4 *>(stage);
             const int rows = min(MB, M - mt * MB);
+            constexpr int U = MB >= 128 ? 4 : 2; // token rows a warp finishes at a time
+            if constexpr (EK == EK_ROWS) { // lane l stores features l, l + 32, ...: whole lines also where rows start anywhere
+                float bs[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int n = nt * TILE_N + 32 * j + lane;
+                    bs[j] = epi.bias && n < N ? epi.bias[n] : 0.0f;
+                }
+                for (int c = w8; c < rows; c += NW) {
+                    if (epi.amax_val) epi_argmax4(epi, mt * MB + c, n4, f4_add(stage4[c * 32 + lane], b4), N);
+                    if (epi.no_store) continue;
+                    float *dst = static_cast<float *>(epi.out) + (size_t)(mt * MB + c) * epi.ldo + nt * TILE_N + lane;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (nt * TILE_N + 32 * j + lane < N) dst[32 * j] = stage[c * TILE_N + 32 * j + lane] + bs[j];
+                }
+            } else if constexpr (EK == EK_STORE || EK == EK_GELU || EK == EK_QKV) {
+                if (splits == 1)
+                    for (int c = w8; c < rows; c += U * NW) {
+                        float4 v[U];
+                        const int cnt = min(U, (rows - c + NW - 1) / NW);
+#pragma unroll
+                        for (int u = 0; u < U; ++u) v[u] = stage4[(c + (u < cnt ? u : 0) * NW) * 32 + lane];
+                        plain_rows<EK, U>(epi, e2.pos_off, mt * MB + c, NW, cnt, n4, v, b4, N);
+                    }
+            } else if constexpr (EK == EK_RESID) {
+                const float4 add0 = (split == 0) ? b4 : make_float4(0.f, 0.f, 0.f, 0.f); // the bias goes in with split 0
+                for (int c = w8; c < rows; c += NW)
+                    epi_resid_red4(epi, mt * MB + c, n4, f4_add(stage4[c * 32 + lane], add0), N);
+            } else
             if (splits == 1) {
                 for (int c = w8; c < rows; c += NW)
                     epi_emit4(e2, epi, mt * MB + c, n4, stage4[c * 32 + lane], g4, b4, ROWSTAT(c),
@@ -341,7 +421,7 @@ int4_gemm_tc_kernel(const uint8_t *__restrict__ tiles, const __half *__restrict_
     // ---- split K inside a cluster: block `split` finishes the token rows c = split, split+splits, ...
     //      of the tile, adding the partial rows of all blocks in split order (deterministic).  Both
     //      cluster barriers are reached by every thread on every path, aborted or not. ----
-    if (cluster_mode) {
+    if (EK != EK_RESID && EK != EK_ROWS && cluster_mode) {
         cg::cluster_group cluster = cg::this_cluster();
         cluster.sync(); // every block of the cluster has staged its partial tile
         if (warp >= 3 && !abort_flag) {
@@ -349,6 +429,23 @@ int4_gemm_tc_kernel(const uint8_t *__restrict__ tiles, const __half *__restrict_
             const int w8 = warp - 3;
             const float4 *stage4 = reinterpret_cast<const float4 *>(gen_base);
             const int rows = min(MB, M - mt * MB);
+            constexpr int U = MB >= 128 ? 2 : 1;
+            const int step = splits * NW;
+            if constexpr (EK == EK_STORE || EK == EK_GELU || EK == EK_QKV) {
+                for (int c = split + splits * w8; c < rows; c += U * step) {
+                    float4 v[U];
+                    const int cnt = min(U, (rows - c + step - 1) / step);
+#pragma unroll
+                    for (int u = 0; u < U; ++u) v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+                    for (int sp = 0; sp < splits; ++sp) {
+                        const float4 *p = cluster.map_shared_rank(stage4, sp);
+#pragma unroll
+                        for (int u = 0; u < U; ++u) v[u] = f4_add(v[u], p[(c + (u < cnt ? u : 0) * step) * 32 + lane]);
+                    }
+                    plain_rows<EK, U>(epi, e2.pos_off, mt * MB + c, step, cnt, n4, v, b4, N);
+                }
+            } else
             for (int c = split + splits * w8; c < rows; c += splits * NW) {
                 const float4 r_old = epi_resid_old4(epi, mt * MB + c, n4, N); // in flight under the partial rows' reads
                 float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -379,6 +476,11 @@ constexpr int kMaxScaleGroups = 64; // group scales of one block's K range held 
 
 template <int MB, int NS, int NP, int NG, int TC>
 int launch_cfg(b200nn_ctx *ctx, const Int4Weight &w, const __half *x, int M, const Epilogue &epi) {
+    using Kernel = decltype(&int4_gemm_tc_kernel<MB, NS, NP, NG, TC, EK_ANY>);
+    static const Kernel kernels[] = {
+        int4_gemm_tc_kernel<MB, NS, NP, NG, TC, EK_ANY>,   int4_gemm_tc_kernel<MB, NS, NP, NG, TC, EK_STORE>,
+        int4_gemm_tc_kernel<MB, NS, NP, NG, TC, EK_GELU>,  int4_gemm_tc_kernel<MB, NS, NP, NG, TC, EK_QKV>,
+        int4_gemm_tc_kernel<MB, NS, NP, NG, TC, EK_RESID>, int4_gemm_tc_kernel<MB, NS, NP, NG, TC, EK_ROWS>};
     constexpr size_t ring = (size_t)NS * MB * 128 + (size_t)NP * TILE_BYTES;
     static_assert(ring >= (size_t)MB * TILE_N * sizeof(float), "epilogue stage must fit in the operand rings");
     // barriers behind the rings: NP*16 + NS*24 + 16 bytes, then 16-byte alignment of the scale buffer
@@ -387,10 +489,11 @@ int launch_cfg(b200nn_ctx *ctx, const Int4Weight &w, const __half *x, int M, con
     constexpr size_t smem_max = 1024 + ring + bar_bytes + (size_t)kMaxScaleGroups * TILE_N * sizeof(__half);
     static_assert(smem_max <= 227 * 1024, "shared memory budget exceeded");
     static bool attr_done[16] = {};
-    auto kern = int4_gemm_tc_kernel<MB, NS, NP, NG, TC>;
     if (!attr_done[ctx->device & 15]) {
-        CK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
-        prefer_max_smem(kern);
+        for (Kernel k : kernels) {
+            CK(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
+            prefer_max_smem(k);
+        }
         attr_done[ctx->device & 15] = true;
     }
     // activations as a 2-D tensor [M rows, K cols] fp16, box [MB x 64] with 128-byte swizzle
@@ -459,6 +562,7 @@ int launch_cfg(b200nn_ctx *ctx, const Int4Weight &w, const __half *x, int M, con
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
+    const Kernel kern = kernels[epi_kind(epi, w.N, splits)];
     CK(ctx, cudaLaunchKernelEx(&cfg, kern, (const uint8_t *)w.tiled->p, (const __half *)w.scales_h->p, tmap, M, w.N,
                                w.k_blocks, w.n_pad, w.group, per, cluster_mode, epi, ctx->scratch, ctx->counters,
                                ctx->dev_err, ctx->trace));

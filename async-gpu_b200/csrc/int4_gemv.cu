@@ -90,11 +90,7 @@ int4_gemv_kernel(const uint4 *__restrict__ tiles, const __half *__restrict__ sca
     }
     if (sizeof(XT) != 4 || !ln.g) {
         pdl_wait();
-        for (int i = tid; i < MT * len; i += GEMV_THREADS) {
-            const int m = i / len, kk = i - m * len;
-            const int k = kb0 * 64 + kk;
-            xs[i] = (m < m_valid && k < kb1 * 64) ? load_fresh(x, (size_t)m * K + k) : 0.0f;
-        }
+        rows_to_smem<MT, GEMV_THREADS>(x, m_valid, K, kb0 * 64, (kb1 - kb0) * 64, len, xs);
     }
     __syncthreads();
 

@@ -33,17 +33,17 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const float *__restrict_
     float v[VPT];
     float s = 0.0f;
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-        int j = tid + i * 256;
-        float t = 0.0f;
-        if (j < d) {
-            t = load_fresh(xr, j);
-            if (rr) t += load_fresh(rr, j);
-            if (sum_out) sum_out[(size_t)row * d + j] = t;
-        }
-        v[i] = t;
-        s += t;
-    }
+    for (int i = 0; i < VPT; ++i) v[i] = tid + i * 256 < d ? load_fresh(xr, tid + i * 256) : 0.0f; // all in flight at once
+    if (rr)
+#pragma unroll
+        for (int i = 0; i < VPT; ++i)
+            if (tid + i * 256 < d) v[i] += load_fresh(rr, tid + i * 256);
+    if (sum_out)
+#pragma unroll
+        for (int i = 0; i < VPT; ++i)
+            if (tid + i * 256 < d) sum_out[(size_t)row * d + tid + i * 256] = v[i];
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) s += v[i];
     float mean = block_sum(s, red) / (float)d;
     float q = 0.0f;
 #pragma unroll

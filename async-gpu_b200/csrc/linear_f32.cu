@@ -64,10 +64,7 @@ f32_gemv_kernel(const float *__restrict__ w, int ldw, const XT *__restrict__ x, 
     }
     if (sizeof(XT) != 4 || !ln.g) {
         pdl_wait();
-        for (int i = tid; i < MT * k_per_split; i += FGEMV_THREADS) {
-            const int m = i / k_per_split, kk = i - m * k_per_split;
-            xs[i] = (m < m_valid && kk < rows) ? load_fresh(x, (size_t)m * K + k0 + kk) : 0.0f;
-        }
+        rows_to_smem<MT, FGEMV_THREADS>(x, m_valid, K, k0, rows, k_per_split, xs);
     }
     __syncthreads();
 
