@@ -1,23 +1,26 @@
 // Causal prefill attention on the tensor cores (tcgen05, accumulators in tensor memory), pipelined.
 //
-// One block per (128-query tile, head, sequence), six warps with fixed roles:
+// One block per (128-query tile, head, sequence), ten warps with fixed roles:
 //   warp 0      copies: the Q tile once, then the K and V tiles of every 128-key step through tensor maps
 //               (cp.async.bulk.tensor, 128-byte swizzle, zero fill past the last cached row) into two-stage
 //               rings; no hand-written shared-memory stores anywhere
 //   warp 1      MMA issue: S_j = Q K_j^T into one of two score buffers in TMEM, then O_j = P_j V_j with
 //               P read from tensor memory (A operand) and V straight from its row-major tile (B operand
 //               MN-major: no transposition)
-//   warps 2..5  softmax: thread r owns query row r (= TMEM lane r).  Pass 1 takes the row maximum of S_j;
-//               then the previous step's O_{j-1} is fetched from TMEM and folded into the running output
-//               (64 f32 per thread, rescaled by that step's correction); pass 2 writes
-//               p = exp2(s*scale - max) back over S_j as packed fp16.
+//   warps 2..9  softmax: two threads per query row (= TMEM lane r), in two warps of the same lane quarter; each takes half of
+//               the keys of a step and half of the 64 output columns.  Pass 1 takes the maximum of the half row, the two
+//               threads exchange theirs through shared memory; then the previous step's O_{j-1} is fetched
+//               from TMEM and folded into the running output (32 f32 per thread, rescaled by that step's
+//               correction); pass 2 writes p = exp2(s*scale - max) back over S_j as packed fp16.
 // Per step the tensor pipe therefore works on S_{j+1} and O_{j-1} while the softmax warps are busy
-// with step j; two blocks per SM cover what is left of each other's gaps.
+// with step j; two blocks per SM cover what is left of each other's gaps.  What bounds it is the softmax's chain of
+// TMEM round trips, exponentials and hand-overs (the exponentials alone take a third of the time): hence sixteen
+// softmax warps per SM (8 prompts of 1024, 12 heads: 42.5 us with one thread per row, 38.9 with two).
 //
-// TMEM (256 columns per block): score buffer b at columns 128 b .. 128 b + 127.  P_j (64 columns of fp16
-// pairs) overwrites columns 0..63 of its own buffer as pass 2 goes along (the 16 P columns written at
-// score column c0 cover score columns c0/2 .. c0/2+15, all loaded by then; a thread only touches its
-// own lane); O_j lands in columns 64..127 of the same buffer, free once pass 2 is over.
+// TMEM (256 columns per block): score buffer b at columns 128 b .. 128 b + 127.  P_j (fp16 pairs) goes over columns 0..31
+// (keys 0..63) and 96..127 (keys 64..127) of its own buffer: each thread writes only over scores that it has
+// loaded itself, the second half of the keys from the last column down.  O_j lands in columns 32..95 of the
+// same buffer, free once pass 2 is over.
 //
 // Replaces flash_attention_v2 / flash_attn_v3.cu of the reference (compute_transformer.rs:597-816,
 // cuda/flash_attn_v3.cu:29-283) for the model path, where q and the output are fp16.
@@ -38,7 +41,7 @@ constexpr int TM_COLS = 256;                // two score buffers
 constexpr int KV_STAGES = 2;
 constexpr int TILE = 16384;                 // 128 rows x 64 fp16
 constexpr int SMEM_BYTES = (1 + 2 * KV_STAGES) * TILE + 1024; // Q, K ring, V ring + alignment slack
-constexpr int NTHREADS = 192;
+constexpr int NTHREADS = 320, SOFTMAX = 256;
 
 __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
     __half2 h = __floats2half2_rn(a, b);
@@ -59,6 +62,7 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     __shared__ __align__(8) Bars bars;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
+    __shared__ float pair_x[2][2][128]; // what the two threads of a row tell each other: [step parity][half][row]
 
     // the query tiles with the most key tiles are scheduled first (blocks start in index order)
     const int qt = gridDim.z - 1 - blockIdx.z, h = blockIdx.y, b = blockIdx.x;
@@ -78,9 +82,9 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         }
         for (int i = 0; i < 2; ++i) {
             tc::mbar_init(bar(bars.s_full[i]), 1);
-            tc::mbar_init(bar(bars.p_full[i]), 128); // every softmax thread
+            tc::mbar_init(bar(bars.p_full[i]), SOFTMAX); // every softmax thread
             tc::mbar_init(bar(bars.o_full[i]), 1);
-            tc::mbar_init(bar(bars.s_free[i]), 128);
+            tc::mbar_init(bar(bars.s_free[i]), SOFTMAX);
         }
         tc::fence_mbar_init();
     }
@@ -151,7 +155,7 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                     const uint32_t buf = tmem_base + bp * 128;
 #pragma unroll
                     for (int k = 0; k < 8; ++k) // 16 keys per MMA: 8 TMEM columns of P, 2048 bytes of V
-                        tc::umma_f16_ts(buf + 64, buf + 8 * k, dv + (uint64_t)(k * (2048 >> 4)), idesc_o, k != 0);
+                        tc::umma_f16_ts(buf + 32, buf + (k < 4 ? 8 * k : 64 + 8 * k), dv + (uint64_t)(k * (2048 >> 4)), idesc_o, k != 0);
                     tc::umma_commit(bar(bars.o_full[bp]));
                     tc::umma_commit(bar(bars.v_empty[st]));
                 }
@@ -159,86 +163,101 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             }
         }
     } else {
-        // ---- softmax and the running output: thread = query row = TMEM lane ----
-        const int quad = warp & 3, row = quad * 32 + (tid & 31);
+        // ---- softmax and the running output: two threads per query row (= TMEM lane) ----
+        const int quad = warp & 3, row = quad * 32 + (tid & 31), half = (warp - 2) >> 2;
         const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
         const int s_row = qt * 128 + row;
         const bool row_valid = s_row < S;
         const int a_pos = past + s_row; // absolute position of this thread's query
-        float m = NEG_BIG, l = 0.0f, corr_prev = 1.0f, acc[64];
+        float m = NEG_BIG, l = 0.0f, corr_prev = 1.0f;
+        float2 acc[16]; // output columns 32 half .. + 31
 #pragma unroll
-        for (int e = 0; e < 64; ++e) acc[e] = 0.0f;
+        for (int e = 0; e < 16; ++e) acc[e] = make_float2(0.0f, 0.0f);
         bool ok = true;
+        // the value of the row's other thread (the two warps of a quarter meet at a barrier of their own)
+        auto exchange = [&](float x, int parity) {
+            pair_x[parity][half][row] = x;
+            asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory");
+            return pair_x[parity][half ^ 1][row];
+        };
         // acc = acc * c + O_tile of score buffer bp (one TMEM round trip)
         auto fold_output = [&](int bp, float c) {
-            uint32_t v[64];
-            tc::tmem_ld_x64(lane_base + bp * 128 + 64, v);
+            uint32_t v[32];
+            tc::tmem_ld_x32(lane_base + bp * 128 + 32 + 32 * half, v);
+            const float2 c2 = make_float2(c, c);
 #pragma unroll
-            for (int e = 0; e < 64; ++e) acc[e] = fmaf(acc[e], c, __uint_as_float(v[e]));
+            for (int e = 0; e < 16; ++e)
+                acc[e] = __ffma2_rn(acc[e], c2, make_float2(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1])));
         };
         for (int j = 0; j < n_tiles; ++j) {
-            const int bf = j & 1, j0 = j * 128;
-            const uint32_t sbuf = lane_base + bf * 128;
-            ok = tc::mbar_wait(bar(bars.s_full[bf]), (j >> 1) & 1, &abort_flag, dev_err, ERR_ATT_S);
-            if (!ok) break;
-            tc::tc_fence_after_sync();
-            // columns of this tile the row may attend to: keys j0 .. min(a_pos, kv_end-1); only the tile on
+            const int bf = j & 1, j0 = j * 128 + 64 * half;
+            const uint32_t sbuf = lane_base + bf * 128 + 64 * half;
+            // A warp whose wait gives up skips the step's work but still meets its partner at every exchange.
+            if (ok) ok = tc::mbar_wait(bar(bars.s_full[bf]), (j >> 1) & 1, &abort_flag, dev_err, ERR_ATT_S);
+            if (ok) tc::tc_fence_after_sync();
+            // columns of this half the row may attend to: keys j0 .. min(a_pos, kv_end-1); only the tile on
             // the diagonal (and rows past the sequence) need the mask, the others take the short loops
             int nvalid = row_valid ? min(a_pos, kv_end - 1) - j0 + 1 : 0;
-            nvalid = max(0, min(nvalid, 128));
-            const bool full = __all_sync(0xffffffffu, nvalid == 128);
+            nvalid = max(0, min(nvalid, 64));
+            const bool full = __all_sync(0xffffffffu, nvalid == 64);
             float mx[4] = {NEG_BIG, NEG_BIG, NEG_BIG, NEG_BIG}; // four independent chains
+            if (ok)
 #pragma unroll 1
-            for (int hf = 0; hf < 2; ++hf) { // pass 1: row maximum, 64 scores per round trip
-                uint32_t v[64];
-                tc::tmem_ld_x64(sbuf + 64 * hf, v);
-                if (full) {
+                for (int hf = 0; hf < 2; ++hf) { // pass 1: maximum of the half row, 32 scores per round trip
+                    uint32_t v[32];
+                    tc::tmem_ld_x32(sbuf + 32 * hf, v);
+                    if (full) {
 #pragma unroll
-                    for (int e = 0; e < 64; e += 8) {
-                        mx[0] = tc::fmax3(mx[0], __uint_as_float(v[e]), __uint_as_float(v[e + 1]));
-                        mx[1] = tc::fmax3(mx[1], __uint_as_float(v[e + 2]), __uint_as_float(v[e + 3]));
-                        mx[2] = tc::fmax3(mx[2], __uint_as_float(v[e + 4]), __uint_as_float(v[e + 5]));
-                        mx[3] = tc::fmax3(mx[3], __uint_as_float(v[e + 6]), __uint_as_float(v[e + 7]));
+                        for (int e = 0; e < 32; e += 8) {
+                            mx[0] = tc::fmax3(mx[0], __uint_as_float(v[e]), __uint_as_float(v[e + 1]));
+                            mx[1] = tc::fmax3(mx[1], __uint_as_float(v[e + 2]), __uint_as_float(v[e + 3]));
+                            mx[2] = tc::fmax3(mx[2], __uint_as_float(v[e + 4]), __uint_as_float(v[e + 5]));
+                            mx[3] = tc::fmax3(mx[3], __uint_as_float(v[e + 6]), __uint_as_float(v[e + 7]));
+                        }
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 32; ++e)
+                            if (32 * hf + e < nvalid) mx[e & 3] = fmaxf(mx[e & 3], __uint_as_float(v[e]));
                     }
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 64; ++e)
-                        if (64 * hf + e < nvalid) mx[e & 3] = fmaxf(mx[e & 3], __uint_as_float(v[e]));
                 }
-            }
             const float mloc = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-            const float m_new = fmaxf(m, mloc * SCALE_LOG2E);
+            const float m_new = fmaxf(m, fmaxf(mloc, exchange(mloc, j & 1)) * SCALE_LOG2E);
             const float corr = tc::ex2_approx(m - m_new);
-            if (j >= 1) { // the previous step's P V has had pass 1 to finish
+            if (j >= 1 && ok) { // the previous step's P V has had pass 1 to finish
                 ok = tc::mbar_wait(bar(bars.o_full[bf ^ 1]), ((j - 1) >> 1) & 1, &abort_flag, dev_err, ERR_ATT_O);
-                if (!ok) break;
-                tc::tc_fence_after_sync();
-                fold_output(bf ^ 1, corr_prev);
-                tc::tc_fence_before_sync();
-                tc::mbar_arrive(bar(bars.s_free[bf ^ 1])); // that buffer may take S_{j+1}
-            }
-            float ls[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 1
-            for (int hf = 0; hf < 2; ++hf) { // pass 2: p = 2^(s*scale - max) as fp16 pairs over the scores
-                uint32_t v[64], o[32];
-                tc::tmem_ld_x64(sbuf + 64 * hf, v);
-#pragma unroll
-                for (int e = 0; e < 64; e += 2) {
-                    float p0 = tc::ex2_approx(fmaf(__uint_as_float(v[e]), SCALE_LOG2E, -m_new));
-                    float p1 = tc::ex2_approx(fmaf(__uint_as_float(v[e + 1]), SCALE_LOG2E, -m_new));
-                    if (!full) {
-                        if (64 * hf + e >= nvalid) p0 = 0.0f;
-                        if (64 * hf + e + 1 >= nvalid) p1 = 0.0f;
-                    }
-                    ls[(e >> 1) & 3] += p0 + p1;
-                    o[e >> 1] = pack_half2(p0, p1);
+                if (ok) {
+                    tc::tc_fence_after_sync();
+                    fold_output(bf ^ 1, corr_prev);
+                    tc::tc_fence_before_sync();
+                    tc::mbar_arrive(bar(bars.s_free[bf ^ 1])); // that buffer may take S_{j+1}
                 }
-                tc::tmem_st_x32(sbuf + 32 * hf, o);
             }
-            tc::tmem_st_wait();
-            tc::tc_fence_before_sync();
-            tc::mbar_arrive(bar(bars.p_full[bf]));
-            l = l * corr + ((ls[0] + ls[1]) + (ls[2] + ls[3]));
+            if (ok) {
+                float2 ls[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+                const float2 sc2 = make_float2(SCALE_LOG2E, SCALE_LOG2E), nm2 = make_float2(-m_new, -m_new);
+#pragma unroll 1
+                for (int i = 0; i < 2; ++i) { // pass 2: p = 2^(s*scale - max) as fp16 pairs over the scores
+                    const int hf = half ? 1 - i : i; // the second half from its last column down
+                    uint32_t v[32], o[16];
+                    tc::tmem_ld_x32(sbuf + 32 * hf, v);
+#pragma unroll
+                    for (int e = 0; e < 32; e += 2) {
+                        const float2 x = __ffma2_rn(make_float2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), sc2, nm2);
+                        float2 p = make_float2(tc::ex2_approx(x.x), tc::ex2_approx(x.y));
+                        if (!full) {
+                            if (32 * hf + e >= nvalid) p.x = 0.0f;
+                            if (32 * hf + e + 1 >= nvalid) p.y = 0.0f;
+                        }
+                        ls[(e >> 1) & 1] = __fadd2_rn(ls[(e >> 1) & 1], p);
+                        o[e >> 1] = pack_half2(p.x, p.y);
+                    }
+                    tc::tmem_st_x16(sbuf + (half ? 32 : 0) + 16 * hf, o);
+                }
+                tc::tmem_st_wait();
+                tc::tc_fence_before_sync();
+                tc::mbar_arrive(bar(bars.p_full[bf]));
+                l = l * corr + ((ls[0].x + ls[0].y) + (ls[1].x + ls[1].y));
+            }
             m = m_new;
             corr_prev = corr;
         }
@@ -250,16 +269,17 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                 fold_output(bl, corr_prev);
             }
         }
+        l += exchange(l, n_tiles & 1);
         if (ok && row_valid) {
             const float inv = 1.0f / l;
-            uint4 *dst = reinterpret_cast<uint4 *>(out + ((size_t)b * S + s_row) * ldo + h * 64);
+            uint4 *dst = reinterpret_cast<uint4 *>(out + ((size_t)b * S + s_row) * ldo + h * 64 + 32 * half);
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
+            for (int c = 0; c < 4; ++c) {
                 uint4 v;
-                v.x = pack_half2(acc[8 * c + 0] * inv, acc[8 * c + 1] * inv);
-                v.y = pack_half2(acc[8 * c + 2] * inv, acc[8 * c + 3] * inv);
-                v.z = pack_half2(acc[8 * c + 4] * inv, acc[8 * c + 5] * inv);
-                v.w = pack_half2(acc[8 * c + 6] * inv, acc[8 * c + 7] * inv);
+                v.x = pack_half2(acc[4 * c + 0].x * inv, acc[4 * c + 0].y * inv);
+                v.y = pack_half2(acc[4 * c + 1].x * inv, acc[4 * c + 1].y * inv);
+                v.z = pack_half2(acc[4 * c + 2].x * inv, acc[4 * c + 2].y * inv);
+                v.w = pack_half2(acc[4 * c + 3].x * inv, acc[4 * c + 3].y * inv);
                 dst[c] = v;
             }
         }
