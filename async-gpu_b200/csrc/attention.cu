@@ -75,7 +75,7 @@ decode_attn_kernel(const QT *__restrict__ q, int ldq, const __half *__restrict__
         if (bytes > 0) tc::bulk_prefetch_l2((tid ? vp : kp) + (size_t)p0 * 8, (uint32_t)bytes);
     }
     pdl_wait();
-    int ctx = (pos_ptr ? *pos_ptr : 0) + pos_off + 1;
+    int ctx = (pos_ptr ? load_fresh_int(pos_ptr) : 0) + pos_off + 1;
     if (ctx > cap) ctx = cap;
     range(ctx, p0, p1);
 
@@ -305,7 +305,7 @@ decode_attn_stream_kernel(const QT *__restrict__ q, int ldq, const __half *__res
         }
     }
     pdl_wait();
-    int ctx = (pos_ptr ? *pos_ptr : 0) + pos_off + 1;
+    int ctx = (pos_ptr ? load_fresh_int(pos_ptr) : 0) + pos_off + 1;
     if (ctx > cap) ctx = cap;
     const int nch = (ctx + ROWS - 1) / ROWS;
     const uint32_t ring = ((tc::smem_u32(smem_raw) + 127u) & ~127u) + warp * NST * STAGE_BYTES;

@@ -47,7 +47,13 @@ __device__ __forceinline__ uint32_t pack_f16x2(float a, float b) {
     const __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<const uint32_t *>(&h);
 }
-__device__ __forceinline__ int row_pos(const RowMap &r, int m) { return r.pos[(size_t)m * r.pos_stride]; }
+// A number that the kernels before this one write (positions, picked tokens), from L2: see load_fresh.
+__device__ __forceinline__ int load_fresh_int(const void *p) {
+    int v;
+    asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ int row_pos(const RowMap &r, int m) { return load_fresh_int(r.pos + (size_t)m * r.pos_stride); }
 __device__ __forceinline__ int row_slot(const RowMap &r, int m) { return r.slot ? r.slot[m] : m; }
 
 // Consumes one finished output value v (bias already added) for row m (token), column n (feature).
@@ -70,7 +76,7 @@ __device__ __forceinline__ void epi_store(const Epilogue &e, int m, int n, float
         }
         int head = c >> 6, el = c & 63;
         int b = m / e.rows_per_seq, s = m - b * e.rows_per_seq;
-        int pos = (e.pos_ptr ? *e.pos_ptr : 0) + e.pos_off + s;
+        int pos = (e.pos_ptr ? load_fresh_int(e.pos_ptr) : 0) + e.pos_off + s;
         if (pos < e.cap) cache[(((size_t)b * e.n_head + head) * e.cap + pos) * 64 + el] = __float2half_rn(v);
         return;
     }

@@ -197,7 +197,7 @@ f16_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         pdl_wait(); // the epilogue touches buffers the previous kernel may still be using
         // bias and the device-side position are fetched under the wait for the accumulator
         b4 = epi_bias4(epi, n4, n_lim);
-        if (epi.mode == EPI_QKV && epi.pos_ptr) e2.pos_off = epi.pos_off + *epi.pos_ptr;
+        if (epi.mode == EPI_QKV && epi.pos_ptr) e2.pos_off = epi.pos_off + load_fresh_int(epi.pos_ptr);
         // (the vote keeps the warp converged for the warp-collective wait)
         if (!__any_sync(0xffffffffu, abort_flag != 0)) tc::mbar_wait(acc_full, 0, &abort_flag, dev_err, ERR_ACC);
         bar_sync_epi<EPI>();
@@ -430,7 +430,7 @@ f16_gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const 
         const float4 *stage4 = reinterpret_cast<const float4 *>(stage);
         Epilogue e2 = epi;
         pdl_wait(); // the epilogue writes buffers the previous kernel may still be using
-        if (epi.mode == EPI_QKV && epi.pos_ptr) e2.pos_off = epi.pos_off + *epi.pos_ptr;
+        if (epi.mode == EPI_QKV && epi.pos_ptr) e2.pos_off = epi.pos_off + load_fresh_int(epi.pos_ptr);
         e2.pos_ptr = nullptr;
         int j = 0;
         for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++j) {

@@ -305,7 +305,7 @@ int4_gemm_tc_kernel(const uint8_t *__restrict__ tiles, const __half *__restrict_
         if constexpr (EK == EK_ANY) g4 = epi_fold4(epi, n4, N);
         // folded LayerNorm: one thread per token row adds up the row's partial sums (the barrier below publishes them)
         if (EK == EK_ANY && epi.ln_stats && t < MB && mt * MB + t < M) rowstat[t] = epi_row_mean_rstd(epi, mt * MB + t);
-        if ((EK == EK_ANY || EK == EK_QKV) && epi.mode == EPI_QKV && epi.pos_ptr) e2.pos_off = epi.pos_off + *epi.pos_ptr;
+        if ((EK == EK_ANY || EK == EK_QKV) && epi.mode == EPI_QKV && epi.pos_ptr) e2.pos_off = epi.pos_off + load_fresh_int(epi.pos_ptr);
         bar_sync_dequant<DQ>();
         if (!abort_flag) tc::mbar_wait(S.acc_full, 0, &abort_flag, dev_err, ERR_ACC);
         bar_sync_dequant<DQ>();

@@ -186,9 +186,9 @@ __global__ void embedding_kernel(const uint32_t *__restrict__ ids, const float *
     int r = blockIdx.x;
     pdl_trigger();
     pdl_wait();
-    uint32_t tok = ids[r];
+    uint32_t tok = (uint32_t)load_fresh_int(ids + r);
     if (tok >= (uint32_t)vocab) tok = vocab - 1; // ids are validated on the host; never read out of range
-    int pos = (pos_ptr ? *pos_ptr : 0) + pos_off + r % rows_per_seq;
+    int pos = (pos_ptr ? load_fresh_int(pos_ptr) : 0) + pos_off + r % rows_per_seq;
     if (pos >= n_positions) pos = n_positions - 1;
     const float *a = wte + (size_t)tok * d, *b = wpe + (size_t)pos * d;
     for (int j = threadIdx.x; j < d; j += blockDim.x) out[(size_t)r * d + j] = a[j] + b[j];
@@ -215,9 +215,9 @@ __global__ void __launch_bounds__(256) embedding_ln_kernel(const uint32_t *__res
     const int r = blockIdx.x;
     pdl_trigger();
     pdl_wait();
-    uint32_t tok = ids[r];
+    uint32_t tok = (uint32_t)load_fresh_int(ids + r);
     if (tok >= (uint32_t)vocab) tok = vocab - 1;
-    int pos = *pos_ptr;
+    int pos = load_fresh_int(pos_ptr);
     if (pos >= n_positions) pos = n_positions - 1;
     const float *a = wte + (size_t)tok * d, *b = wpe + (size_t)pos * d;
     float s1 = 0.0f, s2 = 0.0f;
@@ -513,13 +513,13 @@ __global__ void record_tokens_kernel(const uint32_t *__restrict__ tok, int rows,
                                      int hist_cap, int *step_ptr, int *pos_ptr) {
     pdl_trigger();
     pdl_wait();
-    int step = *step_ptr;
+    const int step = load_fresh_int(step_ptr);
     for (int r = threadIdx.x; r < rows; r += blockDim.x)
-        if (step < hist_cap) history[(size_t)r * hist_cap + step] = tok[r];
+        if (step < hist_cap) history[(size_t)r * hist_cap + step] = (uint32_t)load_fresh_int(tok + r);
     __syncthreads();
     if (threadIdx.x == 0) {
         *step_ptr = step + 1;
-        if (pos_ptr) *pos_ptr += 1;
+        if (pos_ptr) *pos_ptr = load_fresh_int(pos_ptr) + 1;
     }
 }
 int launch_record_tokens(b200nn_ctx *ctx, const uint32_t *tok, int rows, uint32_t *history, int hist_cap,

@@ -1,0 +1,104 @@
+"""Edges of the kernels that serve few rows: the f32 and int4 GEMVs (column and row tiles, K slices, splits over a
+cluster, a LayerNorm taken along), the split-context decode attention (stages, splits, clusters) and the int4 GEMM's
+epilogues.  Each is compared with float64 of the same operands; sums of n f32 terms may differ from it by
+n * 2^-24 of the terms' magnitudes at most, and the bounds below are a fraction of that for the longest sum.
+"""
+import numpy as np
+import pytest
+
+import b200nn
+import np_ref
+from b200nn import Gpt2Config, GpuTensor, Int4Linear, Linear, TransformerBlock, ops, synth
+from oracle import oracle
+from test_gpu_block import _slices
+
+pytestmark = pytest.mark.gpu
+
+
+def _close(got, ref, mag):
+    """f32 sums in another order: within 2e-6 of the sum of the terms' magnitudes."""
+    assert np.isfinite(got).all()
+    assert (np.abs(got - ref) <= 2e-6 * mag + 1e-30).all(), np.max(np.abs(got - ref) / mag)
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4])
+@pytest.mark.parametrize("k,n", [(1, 1), (63, 33), (64, 32), (65, 31), (768, 2304), (3072, 770), (20000, 40), (100, 50257)])
+def test_f32_linear_few_rows(reg, m, k, n):
+    rng = np.random.default_rng(k * 7 + n + m)
+    w, b, x = (rng.standard_normal(s).astype(np.float32) for s in ((n, k), (n,), (m, k)))
+    ref, mag = x.astype(np.float64) @ w.T + b, np.abs(x).astype(np.float64) @ np.abs(w).T + np.abs(b)
+    _close(Linear(w, b, k, n, reg).forward(GpuTensor.from_host(x, (m, k), reg)).to_host(), ref, mag)
+    # a matrix product takes the weight as it is: rows that need not start on 16 bytes
+    got = ops.matmul(GpuTensor.from_host(x, (m, k), reg), GpuTensor.from_host(np.ascontiguousarray(w.T), (k, n), reg), reg).to_host()
+    _close(got, ref - b, mag)
+
+
+def _int4(rng, k, n, group):
+    q = rng.integers(-8, 8, (k, n))
+    s = (rng.random(((k + group - 1) // group, n)) * 0.015 + 0.005).astype(np.float16).astype(np.float32)
+    packed = ((q + 8).reshape(k // 8, 8, n).astype(np.uint64) << (4 * np.arange(8, dtype=np.uint64)).reshape(1, 8, 1)).sum(1).astype(np.uint32)
+    return q * np.repeat(s.astype(np.float64), group, 0)[:k], packed, s
+
+
+@pytest.mark.parametrize("m", [1, 2])
+# one block of K, ragged rows, K split over a cluster, the last weight of 32-row blocks and the first of 128-row ones
+@pytest.mark.parametrize("k,n,group", [(64, 1, 64), (128, 33, 128), (1600, 1600, 128), (6400, 130, 128), (3072, 768, 64),
+                                       (1088, 9472, 64), (128, 9473, 128), (64, 50257, 64)])
+def test_int4_linear_one_and_two_rows(reg, m, k, n, group):
+    rng = np.random.default_rng(k + n + m)
+    w, packed, s = _int4(rng, k, n, group)
+    x, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal(n).astype(np.float32)
+    got = Int4Linear(packed, s, b, k, n, group, reg).forward(GpuTensor.from_host(x, (m, k), reg)).to_host()
+    _close(got, x.astype(np.float64) @ w + b, np.abs(x).astype(np.float64) @ np.abs(w) + np.abs(b))
+
+
+@pytest.mark.parametrize("m", [3, 32, 33, 65, 130, 300])
+@pytest.mark.parametrize("k,n", [(128, 128), (192, 132), (1600, 257), (64, 19000)])
+def test_int4_linear_epilogues(reg, m, k, n):
+    """Rows that leave in 16-byte pieces and rows that start anywhere, with and without splits; fp16 operands, so the reference
+    multiplies the rounded ones."""
+    rng = np.random.default_rng(m * 31 + n)
+    w, packed, s = _int4(rng, k, n, 64)
+    x, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal(n).astype(np.float32)
+    got = Int4Linear(packed, s, b, k, n, 64, reg).forward(GpuTensor.from_host(x, (m, k), reg)).to_host()
+    xh, wh = x.astype(np.float16).astype(np.float64), w.astype(np.float16).astype(np.float64)
+    _close(got, xh @ wh + b, np.abs(xh) @ np.abs(wh) + np.abs(b))
+
+
+def test_rows_after_rows(reg):
+    """Blocks of one to four f32 rows one after another: every kernel is resident before its input is written, so an old line
+    of the residual stream or of the buffers that the calls share would show."""
+    d = 192
+    cfg = Gpt2Config(n_layer=1, n_embd=d, n_head=d // 64, vocab_size=64, n_positions=64)
+    w = synth.gpt2_weights(cfg, base_seed=5, std=0.06, random_ln=True)
+    blk, om = TransformerBlock(*_slices(w), cfg, reg), oracle.Model(cfg.as_dict(), w)
+    for turn, n in enumerate((1, 2, 3, 4, 4, 3, 4, 1, 4)):
+        x = np.random.default_rng(turn).standard_normal((20, d)).astype(np.float32)
+        ref = om.block_forward(0, x, flags=oracle.KV_FP16)[0]
+        past = 20 - n
+        _, k0, v0 = blk.forward_cached(GpuTensor.from_host(x[:past], (past, d), reg), None, None, 0)
+        got = blk.forward_cached(GpuTensor.from_host(x[past:], (n, d), reg), k0, v0, past)[0].to_host()
+        for i in range(n):
+            assert np_ref.rel_rms(got[i], ref[past + i]) < 1e-3, (turn, n, i)
+
+
+# one row, a stage's edge, a split's edge, the most splits, and the pairs around which the split count changes
+@pytest.mark.parametrize("batch,heads,ctx,cap", [(1, 1, 1, 1), (1, 1, 64, 64), (1, 2, 65, 65), (1, 1, 129, 300), (1, 3, 1024, 1024),
+                                                 (1, 1, 5000, 5000), (37, 3, 513, 520), (37, 12, 200, 256), (37, 13, 77, 128), (74, 12, 130, 130),
+                                                 (75, 12, 131, 131)])
+def test_decode_attention_splits(reg, batch, heads, ctx, cap):
+    import torch
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(ctx * 100 + batch)
+    q = torch.randn(batch, heads * 64, generator=g, device="cuda").half()
+    k, v = (torch.randn(batch, heads, cap, 64, generator=g, device="cuda").half() for _ in range(2))
+    k[:, :, ctx:], v[:, :, ctx:] = float("nan"), float("nan")  # rows past the context are not looked at
+    out = torch.zeros_like(q)
+    torch.cuda.synchronize()
+    ops.decode_attention_f16(q.data_ptr(), k.data_ptr(), v.data_ptr(), batch, heads, cap, ctx, out.data_ptr(), reg)
+    reg.synchronize()
+    s = torch.einsum("bhd,bhnd->bhn", q.double().reshape(batch, heads, 64), k[:, :, :ctx].double()) / 8
+    ref = torch.einsum("bhn,bhnd->bhd", torch.softmax(s, -1), v[:, :, :ctx].double()).reshape(batch, heads * 64)
+    # the result is rounded to fp16: 2^-11 of a value, and f32 sums below that
+    assert ((out.double() - ref).abs() <= 2.0 ** -10 * ref.abs() + 2e-5).all()
