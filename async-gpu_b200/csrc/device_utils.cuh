@@ -245,6 +245,79 @@ __device__ __forceinline__ void epi_store4_rows(const Epilogue &e, int m0, int s
     }
 }
 
+// ---- plain epilogues --------------------------------------------------------------------------------
+// The epilogues that most tensor-core GEMMs of a pass have, each in a kernel of its own.  A block runs its epilogue once, so
+// what it costs is mostly the fetching of its instructions and the chain of one row's decisions: with all modes in
+// one kernel a token row took 900 cycles.  They want rows that leave as 16- or 8-byte pieces (N and ldo multiples of 4).
+enum EpiKind {
+    EK_ANY,   // every mode and shape
+    EK_STORE, // y = sums + bias
+    EK_GELU,  // the same through tanh-GELU (f32 or fp16)
+    EK_QKV,   // fp16 q and cache rows
+    EK_RESID, // splits added into the residual stream
+    EK_ROWS,  // y = sums + bias in f32, rows of any length, greedy pick or not: the output matrix (int4 GEMM)
+    EK_GLU    // act(gate) * up in bfloat16 (bfloat16 GEMM)
+};
+inline int epi_kind(const Epilogue &e, int N, int splits, bool b16) {
+    if (e.ln_stats || e.row_scale || e.tail_out || e.kv_cache) return EK_ANY;
+    if (e.mode == EPI_RESID) return splits > 1 ? EK_RESID : EK_ANY;
+    if (!b16 && e.mode == EPI_STORE && splits == 1 && e.act == B200NN_ACT_NONE && e.out_half == OUT_F32 && (e.amax_val || ((N | e.ldo) & 3)))
+        return EK_ROWS;
+    if (e.no_store || e.amax_val || ((N | e.ldo) & 3) || splits > 8) return EK_ANY;
+    if (b16 && e.mode == EPI_GLU) return e.act == B200NN_ACT_SILU || e.act == B200NN_ACT_GELU_TANH ? EK_GLU : EK_ANY;
+    if (!b16 && e.mode == EPI_QKV) return e.out_half == OUT_F16 && e.act == B200NN_ACT_NONE && e.d_model % 64 == 0 ? EK_QKV : EK_ANY;
+    if (e.mode != EPI_STORE || (!b16 && e.out_half == OUT_BF16)) return EK_ANY;
+    return e.act == B200NN_ACT_NONE ? EK_STORE : !b16 && e.act == B200NN_ACT_GELU_TANH ? EK_GELU : EK_ANY;
+}
+// The finished sums of token rows m0, m0 + step, ... (cnt <= U), features n .. n+3 of each, for EK_STORE, EK_GELU, EK_QKV
+// and EK_GLU.
+template <int EK, int U, bool B16 = false>
+__device__ __forceinline__ void plain_rows(const Epilogue &e, int pos_off, int m0, int step, int cnt, int n, float4 (&v)[U], float4 b4, int N) {
+    if (n >= N) return;
+    if constexpr (EK == EK_QKV) {
+        const int part = n / e.d_model, c = n - part * e.d_model;
+        __half *cache = (part == 1 ? e.kc : e.vc) + (size_t)(c >> 6) * e.cap * 64 + (c & 63);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int m = m0 + u * step, b = e.rows_per_seq == 1 ? m : m / e.rows_per_seq, pos = pos_off + m - b * e.rows_per_seq;
+            if (u >= cnt || (part && pos >= e.cap)) continue;
+            __half *dst = part ? cache + ((size_t)b * e.n_head * e.cap + pos) * 64 : static_cast<__half *>(e.out) + (size_t)m * e.ldo + n;
+            *reinterpret_cast<uint2 *>(dst) = make_uint2(pack_f16x2(v[u].x + b4.x, v[u].y + b4.y), pack_f16x2(v[u].z + b4.z, v[u].w + b4.w));
+        }
+    } else if constexpr (EK == EK_GLU) {
+        float4 g[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            v[u] = f4_add(v[u], b4);
+            g[u] = make_float4(v[u].x, v[u].y, 0.0f, 0.0f);
+        }
+        if (e.act == B200NN_ACT_SILU) act_rows<B200NN_ACT_SILU>(g);
+        else act_rows<B200NN_ACT_GELU_TANH>(g);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (u < cnt)
+                *reinterpret_cast<uint32_t *>(static_cast<__nv_bfloat16 *>(e.out) + (size_t)(m0 + u * step) * e.ldo + (n >> 1)) =
+                    pack_bf16x2(g[u].x * v[u].z, g[u].y * v[u].w);
+    } else {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            v[u] = f4_add(v[u], b4);
+            if constexpr (EK == EK_GELU) v[u] = make_float4(gelu_tanh_f(v[u].x), gelu_tanh_f(v[u].y), gelu_tanh_f(v[u].z), gelu_tanh_f(v[u].w));
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (u >= cnt) continue;
+            const size_t i = (size_t)(m0 + u * step) * e.ldo + n;
+            if (e.out_half)
+                *reinterpret_cast<uint2 *>(static_cast<__half *>(e.out) + i) =
+                    B16 && e.out_half == OUT_BF16 ? make_uint2(pack_bf16x2(v[u].x, v[u].y), pack_bf16x2(v[u].z, v[u].w))
+                                                  : make_uint2(pack_f16x2(v[u].x, v[u].y), pack_f16x2(v[u].z, v[u].w));
+            else
+                *reinterpret_cast<float4 *>(static_cast<float *>(e.out) + i) = v[u];
+        }
+    }
+}
+
 // ---- greedy pick fused into the epilogue ---------------------------------------------------------
 // The better of two (value, index) candidates: larger value; on equal values the lower index, or the
 // higher with keep_last (Rust's max_by, gpt2.rs:991-997).  NaN never wins, as in argmax_kernel.

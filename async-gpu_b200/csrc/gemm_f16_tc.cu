@@ -71,8 +71,8 @@ __device__ __forceinline__ void bar_sync_epi() {
 
 // MB: token-tile width (the MMA's N); NS: operand stages; NE: epilogue groups of four warps;
 // TW: fp16 terms of the weight (1: hi, 2: hi + lo; tmap_w2 is read only with TW = 2);
-// B16: both operands bfloat16, with those Linears' epilogues and block-diagonal form.
-template <int MB, int NS, int NE, int TW, bool B16>
+// B16: both operands bfloat16, with those Linears' epilogues and block-diagonal form; EK: what becomes of the sums (EpiKind).
+template <int MB, int NS, int NE, int TW, bool B16, int EK>
 __global__ void __launch_bounds__(64 + 128 * NE, 1)
 f16_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_w2,
                    const __grid_constant__ CUtensorMap tmap_x, int M, int N, int k_blocks, int kb_per_split,
@@ -197,7 +197,7 @@ f16_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         pdl_wait(); // the epilogue touches buffers the previous kernel may still be using
         // bias and the device-side position are fetched under the wait for the accumulator
         b4 = epi_bias4(epi, n4, n_lim);
-        if (epi.mode == EPI_QKV && epi.pos_ptr) e2.pos_off = epi.pos_off + load_fresh_int(epi.pos_ptr);
+        if ((EK == EK_ANY || EK == EK_QKV) && epi.mode == EPI_QKV && epi.pos_ptr) e2.pos_off = epi.pos_off + load_fresh_int(epi.pos_ptr);
         // (the vote keeps the warp converged for the warp-collective wait)
         if (!__any_sync(0xffffffffu, abort_flag != 0)) tc::mbar_wait(acc_full, 0, &abort_flag, dev_err, ERR_ACC);
         bar_sync_epi<EPI>();
@@ -224,16 +224,17 @@ f16_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             constexpr int NW = 4 * NE;
             const float4 *stage4 = reinterpret_cast<const float4 *>(stage);
             const int rows = min(MB, M - mt * MB);
-            if (splits == 1) {
+            if (EK != EK_RESID && splits == 1) {
                 constexpr int U = MB / NW < 4 ? MB / NW : 4; // token rows a warp finishes at a time
                 for (int c = w8; c < rows; c += U * NW) {
                     float4 v[U];
                     const int cnt = min(U, (rows - c + NW - 1) / NW);
 #pragma unroll
                     for (int u = 0; u < U; ++u) v[u] = stage4[(c + (u < cnt ? u : 0) * NW) * 32 + lane];
-                    epi_emit4_rows<U, B16>(e2, epi, mt * MB + c, NW, cnt, n4, v, b4, n_lim);
+                    if constexpr (EK == EK_ANY) epi_emit4_rows<U, B16>(e2, epi, mt * MB + c, NW, cnt, n4, v, b4, n_lim);
+                    else if constexpr (EK != EK_RESID) plain_rows<EK, U, B16>(epi, e2.pos_off, mt * MB + c, NW, cnt, n4, v, b4, n_lim);
                 }
-            } else if (epi.mode == EPI_RESID) {
+            } else if (EK == EK_RESID || (EK == EK_ANY && epi.mode == EPI_RESID)) {
                 // every split adds its partial tile into the f32 residual stream with vector
                 // reductions at L2; the bias goes in with split 0.  The order of the additions is not
                 // fixed, so the last bits of the sum can differ between runs.
@@ -247,7 +248,7 @@ f16_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     // ---- split K inside a cluster: block `split` finishes token rows split, split+splits, ... of the
     //      tile, adding the partial rows of all blocks in split order.  Both cluster barriers are
     //      reached by every thread on every path, aborted or not. ----
-    if (cluster_mode) {
+    if (EK != EK_RESID && cluster_mode) {
         cg::cluster_group cluster = cg::this_cluster();
         cluster.sync(); // every block of the cluster has staged its partial tile
         if (warp >= 2 && !abort_flag) {
@@ -268,7 +269,8 @@ f16_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
 #pragma unroll
                     for (int u = 0; u < U; ++u) v[u] = f4_add(v[u], p[(c + (u < cnt ? u : 0) * step) * 32 + lane]);
                 }
-                epi_emit4_rows<U, B16>(e2, epi, mt * MB + c, step, cnt, n4, v, b4, n_lim);
+                if constexpr (EK == EK_ANY) epi_emit4_rows<U, B16>(e2, epi, mt * MB + c, step, cnt, n4, v, b4, n_lim);
+                else plain_rows<EK, U, B16>(epi, e2.pos_off, mt * MB + c, step, cnt, n4, v, b4, n_lim);
             }
         }
         cluster.sync(); // no block leaves while its shared memory may still be read
@@ -307,7 +309,7 @@ __device__ __forceinline__ bool bar_or_epi(bool pred) {
 //   full[s] / empty[s]      operand stage s loaded / its MMAs retired (as above);
 //   acc_full[b] / acc_empty[b]  accumulator b complete (tcgen05.commit) / read out (one arrival per
 //                               epilogue warp).
-template <int MB, int NS, int NE, int TW, bool B16>
+template <int MB, int NS, int NE, int TW, bool B16, int EK>
 __global__ void __launch_bounds__(64 + 128 * NE, 1)
 f16_gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_w2,
                               const __grid_constant__ CUtensorMap tmap_x, int M, int N, int k_blocks, int n_tiles,
@@ -430,7 +432,7 @@ f16_gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const 
         const float4 *stage4 = reinterpret_cast<const float4 *>(stage);
         Epilogue e2 = epi;
         pdl_wait(); // the epilogue writes buffers the previous kernel may still be using
-        if (epi.mode == EPI_QKV && epi.pos_ptr) e2.pos_off = epi.pos_off + load_fresh_int(epi.pos_ptr);
+        if ((EK == EK_ANY || EK == EK_QKV) && epi.mode == EPI_QKV && epi.pos_ptr) e2.pos_off = epi.pos_off + load_fresh_int(epi.pos_ptr);
         e2.pos_ptr = nullptr;
         int j = 0;
         for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++j) {
@@ -459,7 +461,7 @@ f16_gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const 
                 }
                 bar_sync_epi<EPI>();
                 const int lim = min(CH, rows - c0);
-                if (epi.mode == EPI_RESID) {
+                if (EK == EK_RESID || (EK == EK_ANY && epi.mode == EPI_RESID)) {
                     // this block is the only one that adds to these elements: a reduction at L2 does
                     // the read-modify-write there, with no load for the warp to wait on
                     for (int c = w8; c < lim; c += NW)
@@ -471,7 +473,8 @@ f16_gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tmap_w, const 
                         const int cnt = min(U, (lim - c + NW - 1) / NW);
 #pragma unroll
                         for (int u = 0; u < U; ++u) v[u] = stage4[(c + (u < cnt ? u : 0) * NW) * 32 + lane];
-                        epi_emit4_rows<U, B16>(e2, epi, mt * MB + c0 + c, NW, cnt, n4, v, b4, n_lim);
+                        if constexpr (EK == EK_ANY) epi_emit4_rows<U, B16>(e2, epi, mt * MB + c0 + c, NW, cnt, n4, v, b4, n_lim);
+                        else if constexpr (EK != EK_RESID) plain_rows<EK, U, B16>(epi, e2.pos_off, mt * MB + c0 + c, NW, cnt, n4, v, b4, n_lim);
                     }
                 }
                 bar_sync_epi<EPI>(); // the stage is free for the next pass
@@ -529,11 +532,21 @@ int launch_cfg(b200nn_ctx *ctx, const WOperand &w, const __half *x, int M, const
     constexpr size_t smem = 1024 + ring + 256;
     static_assert(16 * NS + 16 <= 256, "barrier area too small");
     static_assert(smem <= 227 * 1024, "shared memory budget exceeded");
+    // by EpiKind; the kinds that this element type does not have are never asked for
+    using Kernel = decltype(&f16_gemm_tc_kernel<MB, NS, NE, TW, B16, EK_ANY>);
+    static const Kernel kernels[] = {f16_gemm_tc_kernel<MB, NS, NE, TW, B16, EK_ANY>,
+                                     f16_gemm_tc_kernel<MB, NS, NE, TW, B16, EK_STORE>,
+                                     f16_gemm_tc_kernel<MB, NS, NE, TW, B16, B16 ? EK_ANY : EK_GELU>,
+                                     f16_gemm_tc_kernel<MB, NS, NE, TW, B16, B16 ? EK_ANY : EK_QKV>,
+                                     f16_gemm_tc_kernel<MB, NS, NE, TW, B16, EK_RESID>,
+                                     f16_gemm_tc_kernel<MB, NS, NE, TW, B16, EK_ANY>,
+                                     f16_gemm_tc_kernel<MB, NS, NE, TW, B16, B16 ? EK_GLU : EK_ANY>};
     static bool attr_done[16] = {};
-    auto kern = f16_gemm_tc_kernel<MB, NS, NE, TW, B16>;
     if (!attr_done[ctx->device & 15]) {
-        CK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        prefer_max_smem(kern);
+        for (Kernel k : kernels) {
+            CK(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            prefer_max_smem(k);
+        }
         attr_done[ctx->device & 15] = true;
     }
     CUtensorMap tmap_w, tmap_w2, tmap_x;
@@ -580,6 +593,7 @@ int launch_cfg(b200nn_ctx *ctx, const WOperand &w, const __half *x, int M, const
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
+    const Kernel kern = kernels[w.form.group_stride ? EK_ANY : epi_kind(epi, w.N, splits, B16)]; // (block-diagonal Linears have limits of their own)
     CK(ctx, cudaLaunchKernelEx(&cfg, kern, tmap_w, tmap_w2, tmap_x, M, w.N, k_blocks, per, cluster_mode, w.form, epi, ctx->dev_err));
     CK_LAUNCH(ctx, "f16_gemm_tc_kernel");
     return B200NN_OK;
@@ -592,11 +606,21 @@ int launch_persistent(b200nn_ctx *ctx, const WOperand &w, const __half *x, int M
     constexpr size_t smem = 1024 + (size_t)NS * (TW * W_BYTES + MB * BK * 2) + 64 * 128 * 4 + 256;
     static_assert(16 * NS + 48 <= 256, "barrier area too small");
     static_assert(smem <= 227 * 1024, "shared memory budget exceeded");
+    // by EpiKind; the kinds that this element type does not have are never asked for
+    using Kernel = decltype(&f16_gemm_tc_persistent_kernel<MB, NS, NE, TW, B16, EK_ANY>);
+    static const Kernel kernels[] = {f16_gemm_tc_persistent_kernel<MB, NS, NE, TW, B16, EK_ANY>,
+                                     f16_gemm_tc_persistent_kernel<MB, NS, NE, TW, B16, EK_STORE>,
+                                     f16_gemm_tc_persistent_kernel<MB, NS, NE, TW, B16, B16 ? EK_ANY : EK_GELU>,
+                                     f16_gemm_tc_persistent_kernel<MB, NS, NE, TW, B16, B16 ? EK_ANY : EK_QKV>,
+                                     f16_gemm_tc_persistent_kernel<MB, NS, NE, TW, B16, EK_RESID>,
+                                     f16_gemm_tc_persistent_kernel<MB, NS, NE, TW, B16, EK_ANY>,
+                                     f16_gemm_tc_persistent_kernel<MB, NS, NE, TW, B16, B16 ? EK_GLU : EK_ANY>};
     static bool attr_done[16] = {};
-    auto kern = f16_gemm_tc_persistent_kernel<MB, NS, NE, TW, B16>;
     if (!attr_done[ctx->device & 15]) {
-        CK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        prefer_max_smem(kern);
+        for (Kernel k : kernels) {
+            CK(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            prefer_max_smem(k);
+        }
         attr_done[ctx->device & 15] = true;
     }
     CUtensorMap tmap_w, tmap_w2, tmap_x;
@@ -616,6 +640,8 @@ int launch_persistent(b200nn_ctx *ctx, const WOperand &w, const __half *x, int M
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = (ctx->pdl && w.constant) ? 1 : 0;
+    // (the residual epilogue adds at L2 here as split sums do)
+    const Kernel kern = kernels[w.form.group_stride ? EK_ANY : epi.mode == EPI_RESID ? EK_RESID : epi_kind(epi, w.N, 1, B16)];
     CK(ctx, cudaLaunchKernelEx(&cfg, kern, tmap_w, tmap_w2, tmap_x, M, w.N, k_blocks, n_tiles, total, w.form, epi, ctx->dev_err));
     CK_LAUNCH(ctx, "f16_gemm_tc_persistent_kernel");
     return B200NN_OK;

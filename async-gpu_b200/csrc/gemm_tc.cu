@@ -50,59 +50,6 @@ struct Smem {
     uint32_t acc_full, tmem_slot, sc;
 };
 
-// The epilogues of a decode step have kernels of their own.  A block runs its epilogue once, so what it costs is mostly the
-// fetching of its instructions and the chain of one row's decisions: with all modes in one kernel a token row took 900
-// cycles.  The plain ones want rows that leave as 16- or 8-byte pieces (N and ldo multiples of 4).
-enum EpiKind {
-    EK_ANY,   // every mode and shape
-    EK_STORE, // y = sums + bias, f32 or fp16
-    EK_GELU,  // the same through tanh-GELU
-    EK_QKV,   // fp16 q and cache rows
-    EK_RESID, // splits added into the residual stream
-    EK_ROWS   // y = sums + bias in f32, rows of any length, greedy pick or not: the output matrix
-};
-int epi_kind(const Epilogue &e, int N, int splits) {
-    const bool plain = !e.ln_stats && !e.row_scale && !e.tail_out && !e.kv_cache;
-    if (!plain) return EK_ANY;
-    if (e.mode == EPI_RESID) return splits > 1 ? EK_RESID : EK_ANY;
-    if (e.mode == EPI_STORE && splits == 1 && e.act == B200NN_ACT_NONE && e.out_half == OUT_F32 && (e.amax_val || ((N | e.ldo) & 3))) return EK_ROWS;
-    if (e.no_store || e.amax_val || ((N | e.ldo) & 3) || splits > 8) return EK_ANY;
-    if (e.mode == EPI_QKV) return e.out_half == OUT_F16 && e.act == B200NN_ACT_NONE && e.d_model % 64 == 0 ? EK_QKV : EK_ANY;
-    if (e.mode != EPI_STORE || e.out_half == OUT_BF16) return EK_ANY;
-    return e.act == B200NN_ACT_NONE ? EK_STORE : e.act == B200NN_ACT_GELU_TANH ? EK_GELU : EK_ANY;
-}
-// The finished sums of token rows m0, m0 + step, ... (cnt <= U), features n .. n+3 of each, for EK_STORE, EK_GELU and EK_QKV.
-template <int EK, int U>
-__device__ __forceinline__ void plain_rows(const Epilogue &e, int pos_off, int m0, int step, int cnt, int n, float4 (&v)[U], float4 b4, int N) {
-    if (n >= N) return;
-    if constexpr (EK == EK_QKV) {
-        const int part = n / e.d_model, c = n - part * e.d_model;
-        __half *cache = (part == 1 ? e.kc : e.vc) + (size_t)(c >> 6) * e.cap * 64 + (c & 63);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int m = m0 + u * step, b = e.rows_per_seq == 1 ? m : m / e.rows_per_seq, pos = pos_off + m - b * e.rows_per_seq;
-            if (u >= cnt || (part && pos >= e.cap)) continue;
-            __half *dst = part ? cache + ((size_t)b * e.n_head * e.cap + pos) * 64 : static_cast<__half *>(e.out) + (size_t)m * e.ldo + n;
-            *reinterpret_cast<uint2 *>(dst) = make_uint2(pack_f16x2(v[u].x + b4.x, v[u].y + b4.y), pack_f16x2(v[u].z + b4.z, v[u].w + b4.w));
-        }
-    } else {
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            v[u] = f4_add(v[u], b4);
-            if constexpr (EK == EK_GELU) v[u] = make_float4(gelu_tanh_f(v[u].x), gelu_tanh_f(v[u].y), gelu_tanh_f(v[u].z), gelu_tanh_f(v[u].w));
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (u >= cnt) continue;
-            const size_t i = (size_t)(m0 + u * step) * e.ldo + n;
-            if (e.out_half)
-                *reinterpret_cast<uint2 *>(static_cast<__half *>(e.out) + i) = make_uint2(pack_f16x2(v[u].x, v[u].y), pack_f16x2(v[u].z, v[u].w));
-            else
-                *reinterpret_cast<float4 *>(static_cast<float *>(e.out) + i) = v[u];
-        }
-    }
-}
-
 template <int NTHREADS>
 __device__ __forceinline__ void bar_sync_dequant() {
     asm volatile("bar.sync 1, %0;" ::"n"(NTHREADS) : "memory");
@@ -562,7 +509,7 @@ int launch_cfg(b200nn_ctx *ctx, const Int4Weight &w, const __half *x, int M, con
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    const Kernel kern = kernels[epi_kind(epi, w.N, splits)];
+    const Kernel kern = kernels[epi_kind(epi, w.N, splits, false)];
     CK(ctx, cudaLaunchKernelEx(&cfg, kern, (const uint8_t *)w.tiled->p, (const __half *)w.scales_h->p, tmap, M, w.N,
                                w.k_blocks, w.n_pad, w.group, per, cluster_mode, epi, ctx->scratch, ctx->counters,
                                ctx->dev_err, ctx->trace));
@@ -588,7 +535,10 @@ int launch_int4_gemm_tc(b200nn_ctx *ctx, const Int4Weight &w, const __half *x, i
     while (mb < M && mb < cap) mb <<= 1;
     switch (mb) { //            MB  NS  NP NG  TMEM columns
         case 32: return launch_cfg<32, 7, 16, 2, 256>(ctx, w, x, M, epi);
-        case 64: return launch_cfg<64, 6, 12, 4, 256>(ctx, w, x, M, epi);
+        case 64:
+            // more tiles than SMs (an output matrix): two smaller blocks per SM, so that one's epilogue runs under the other's loop
+            if (w.n_tiles > ctx->sm_count) return launch_cfg<64, 4, 8, 2, 256>(ctx, w, x, M, epi);
+            return launch_cfg<64, 6, 12, 4, 256>(ctx, w, x, M, epi);
         case 128: return launch_cfg<128, 4, 12, 4, 256>(ctx, w, x, M, epi); // 8 stages measured no faster
         default: return launch_cfg<256, 4, 8, 4, 512>(ctx, w, x, M, epi);
     }
