@@ -476,7 +476,9 @@ __global__ void __launch_bounds__(256) argmax_entries_kernel(const float *__rest
     const int *ri = idx + (size_t)blockIdx.x * n_entries;
     float best = -INFINITY;
     int bi = keep_last ? -1 : 0x7fffffff;
-    for (int j = threadIdx.x; j < n_entries; j += blockDim.x) amax_merge(best, bi, rv[j], ri[j], keep_last);
+    // (a row has entries for whole 128-feature tiles; those past the vocabulary may not have been written)
+    const int used = min(n_entries, (vocab + 31) / 32);
+    for (int j = threadIdx.x; j < used; j += blockDim.x) amax_merge(best, bi, rv[j], ri[j], keep_last);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, best, o);

@@ -8,7 +8,7 @@ import pytest
 
 import b200nn
 import np_ref
-from b200nn import Gpt2Config, GpuTensor, Int4Linear, Linear, TransformerBlock, ops, synth
+from b200nn import Gpt2Config, Gpt2Model, GpuTensor, Int4Gpt2Model, Int4Linear, Linear, TransformerBlock, ops, synth
 from oracle import oracle
 from test_gpu_block import _slices
 
@@ -80,6 +80,26 @@ def test_rows_after_rows(reg):
         got = blk.forward_cached(GpuTensor.from_host(x[past:], (n, d), reg), k0, v0, past)[0].to_host()
         for i in range(n):
             assert np_ref.rel_rms(got[i], ref[past + i]) < 1e-3, (turn, n, i)
+
+
+@pytest.mark.parametrize("int4", [False, True])
+def test_greedy_pick_of_a_vocabulary_between_tiles(reg, int4):
+    """The pick of one row reads the entries of whole 32-feature groups only: a model of 256 tokens with large logits has left
+    its entries in the buffers that a model of 130 then uses."""
+    for vocab, scale in ((256, 50.0), (130, 1.0), (256, 50.0), (97, 1.0)):
+        cfg = Gpt2Config(n_layer=1, n_embd=64, n_head=1, vocab_size=vocab, n_positions=16)
+        w = synth.gpt2_weights(cfg, base_seed=vocab, std=0.02)
+        w["wte"] = w["wte"] * scale
+        m = Int4Gpt2Model(w, cfg, reg, flags=b200nn.QUANT_LM_HEAD, group_size=64) if int4 else Gpt2Model.from_weights(w, cfg, reg)
+        prompt = np.array([1, 2, 3], dtype=np.uint32)
+        got = m.generate(prompt, 6, flags=0)
+        reg.set_tuning("fused_argmax", 0)
+        try:
+            ref = m.generate(prompt, 6, flags=0)
+        finally:
+            reg.set_tuning("fused_argmax", 1)
+        assert np.array_equal(got, ref) and got.max() < vocab
+        del m
 
 
 # one row, a stage's edge, a split's edge, the most splits, and the pairs around which the split count changes
