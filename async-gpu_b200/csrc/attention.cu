@@ -46,8 +46,7 @@ constexpr int SMEM_BYTES = NST * STAGE_U4 * 16;
 
 template <typename QT, typename OT>
 __global__ void __launch_bounds__(split_attn::THREADS, split_attn::BLOCKS_PER_SM)
-decode_attn_kernel(const QT *__restrict__ q, int ldq, const __half *__restrict__ kc, const __half *__restrict__ vc,
-                   int H, int cap, const int *__restrict__ pos_ptr, int pos_off, OT *__restrict__ out, int ldo, int pf_bytes) {
+decode_attn_kernel(Fresh<QT> q, int ldq, Fresh<__half> kc, Fresh<__half> vc, int H, int cap, Fresh<int> pos_ptr, int pos_off, OT *__restrict__ out, int ldo, int pf_bytes) {
     using namespace split_attn;
     extern __shared__ __align__(16) uint8_t smem_raw[];
     uint4 *ring = reinterpret_cast<uint4 *>(smem_raw);
@@ -58,8 +57,8 @@ decode_attn_kernel(const QT *__restrict__ q, int ldq, const __half *__restrict__
     pdl_trigger();
     if (n_splits > 1) cluster_arrive(); // waited for before the first store into another block
     const size_t base = ((size_t)b * H + h) * cap;
-    const uint4 *kp = reinterpret_cast<const uint4 *>(kc + base * 64);
-    const uint4 *vp = reinterpret_cast<const uint4 *>(vc + base * 64);
+    const uint4 *kp = reinterpret_cast<const uint4 *>(kc.p + base * 64);
+    const uint4 *vp = reinterpret_cast<const uint4 *>(vc.p + base * 64);
     auto range = [&](int ctx, int &p0, int &p1) {
         const int chunk = (((ctx + n_splits - 1) / n_splits) + 15) & ~15;
         p0 = split * chunk;
@@ -69,13 +68,13 @@ decode_attn_kernel(const QT *__restrict__ q, int ldq, const __half *__restrict__
     // Rows of earlier steps are asked into L2 while the projection before this kernel runs (a hint only: the position read
     // here may be a step behind).
     if (tid < 2 && pf_bytes > 0) {
-        const int old_rows = (pos_ptr ? *reinterpret_cast<const volatile int *>(pos_ptr) : 0) + pos_off;
+        const int old_rows = (pos_ptr ? pos_ptr[0] : 0) + pos_off;
         range(min(max(old_rows, 0), cap), p0, p1);
         const int bytes = min((p1 - p0) * 128, pf_bytes & ~127);
         if (bytes > 0) tc::bulk_prefetch_l2((tid ? vp : kp) + (size_t)p0 * 8, (uint32_t)bytes);
     }
     pdl_wait();
-    int ctx = (pos_ptr ? load_fresh_int(pos_ptr) : 0) + pos_off + 1;
+    int ctx = (pos_ptr ? pos_ptr[0] : 0) + pos_off + 1;
     if (ctx > cap) ctx = cap;
     range(ctx, p0, p1);
 
@@ -99,7 +98,7 @@ decode_attn_kernel(const QT *__restrict__ q, int ldq, const __half *__restrict__
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const size_t qi = (size_t)b * ldq + h * 64 + c * 8 + 2 * i;
-        qf2[i] = make_float2(load_fresh(q, qi) * ATT_SCALE_LOG2E, load_fresh(q, qi + 1) * ATT_SCALE_LOG2E);
+        qf2[i] = make_float2(q[qi] * ATT_SCALE_LOG2E, q[qi + 1] * ATT_SCALE_LOG2E);
         acc2[i] = make_float2(0.0f, 0.0f);
     }
     float m = NEG_BIG, l = 0.0f;
@@ -271,8 +270,7 @@ constexpr int REC_FLOATS = 80; // half-item record: [0] max, [1] sum, [8..71] ou
 
 template <typename QT, typename OT, int WARPS, int ROWS>
 __global__ void __launch_bounds__(WARPS * 32, 1)
-decode_attn_stream_kernel(const QT *__restrict__ q, int ldq, const __half *__restrict__ kc,
-                          const __half *__restrict__ vc, int H, int cap, const int *__restrict__ pos_ptr, int pos_off,
+decode_attn_stream_kernel(Fresh<QT> q, int ldq, Fresh<__half> kc, Fresh<__half> vc, int H, int cap, Fresh<int> pos_ptr, int pos_off,
                           OT *__restrict__ out, int ldo, int n_items, int pf_items, int split_items,
                           unsigned *__restrict__ work, float *__restrict__ scratch, unsigned *__restrict__ counters, uint32_t *__restrict__ dev_err) {
     using namespace stream_attn;
@@ -294,18 +292,18 @@ decode_attn_stream_kernel(const QT *__restrict__ q, int ldq, const __half *__res
     // be brought into L2 while that projection is still running.  The position read here may be one
     // step behind (the kernel that advances it may not have finished); fewer rows are harmless.
     if (lane == 0 && pf_items > 0) {
-        int old_rows = (pos_ptr ? *reinterpret_cast<const volatile int *>(pos_ptr) : 0) + pos_off;
+        int old_rows = (pos_ptr ? pos_ptr[0] : 0) + pos_off;
         old_rows = min(max(old_rows, 0), cap);
         if (old_rows > 0) {
             const int n_w = gridDim.x * WARPS;
             for (int it = blockIdx.x * WARPS + warp; it < pf_items; it += n_w) {
-                tc::bulk_prefetch_l2(kc + (size_t)it * cap * 64, (uint32_t)old_rows * 128u);
-                tc::bulk_prefetch_l2(vc + (size_t)it * cap * 64, (uint32_t)old_rows * 128u);
+                tc::bulk_prefetch_l2(kc.p + (size_t)it * cap * 64, (uint32_t)old_rows * 128u);
+                tc::bulk_prefetch_l2(vc.p + (size_t)it * cap * 64, (uint32_t)old_rows * 128u);
             }
         }
     }
     pdl_wait();
-    int ctx = (pos_ptr ? load_fresh_int(pos_ptr) : 0) + pos_off + 1;
+    int ctx = (pos_ptr ? pos_ptr[0] : 0) + pos_off + 1;
     if (ctx > cap) ctx = cap;
     const int nch = (ctx + ROWS - 1) / ROWS;
     const uint32_t ring = ((tc::smem_u32(smem_raw) + 127u) & ~127u) + warp * NST * STAGE_BYTES;
@@ -362,11 +360,11 @@ decode_attn_stream_kernel(const QT *__restrict__ q, int ldq, const __half *__res
                 const uint32_t bar = tc::smem_u32(&full_bar[warp][s]), dst = ring + s * STAGE_BYTES;
                 const size_t off = ((size_t)p_item * cap + (size_t)p_ch * ROWS) * 64;
                 tc::mbar_expect_tx(bar, rows * 256 + (first ? 64 * (uint32_t)sizeof(QT) : 0u));
-                tc::tma_load_1d(dst, kc + off, rows * 128, bar);
-                tc::tma_load_1d(dst + ROWS * 128, vc + off, rows * 128, bar);
+                tc::tma_load_1d(dst, kc.p + off, rows * 128, bar);
+                tc::tma_load_1d(dst + ROWS * 128, vc.p + off, rows * 128, bar);
                 if (first) {
                     const int pb = p_item / H, ph = p_item - pb * H;
-                    tc::tma_load_1d(dst + 2 * ROWS * 128, q + (size_t)pb * ldq + ph * 64, 64 * (uint32_t)sizeof(QT), bar);
+                    tc::tma_load_1d(dst + 2 * ROWS * 128, q.p + (size_t)pb * ldq + ph * 64, 64 * (uint32_t)sizeof(QT), bar);
                 }
                 meta[warp][s] = make_int2(p_item, p_ch | (first ? 0x100 : 0) | (last ? 0x200 : 0) | (p_part << 10));
             }

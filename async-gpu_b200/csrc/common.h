@@ -129,6 +129,7 @@ inline void prefer_max_smem(Kernel kern) {
 // Launch with programmatic dependent launch allowed: the kernel may start while its predecessor
 // on the stream is still running and must execute pdl_wait() (griddepcontrol.wait) before it reads
 // or writes anything the predecessor touches.  Only kernels that do so are launched this way.
+// Its blocks may be resident while those kernels run, so it takes what they write as Fresh<T> (device_utils.cuh).
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(b200nn_ctx *ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
                               Args &&...args) {
@@ -142,6 +143,17 @@ inline cudaError_t launch_pdl(b200nn_ctx *ctx, void (*kern)(KArgs...), dim3 grid
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = ctx->pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+// Launch behind the end of everything before it, for kernels that read what earlier kernels wrote through L1 (several
+// threads share the lines, or one walks along them).
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_ordered(b200nn_ctx *ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 

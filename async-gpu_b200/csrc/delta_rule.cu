@@ -32,7 +32,7 @@ __device__ __forceinline__ float decay_f(float a_exp, float a, float dt_bias) { 
 // step size.
 template <int RPW, bool CH, typename T>
 __global__ void __launch_bounds__(256, RPW <= 16 ? 2 : 1)
-delta_step_kernel(DeltaDims d, const float *__restrict__ proj, int ldp, const float *__restrict__ ext, DeltaWeights w, float *__restrict__ conv_state,
+delta_step_kernel(DeltaDims d, Fresh<float> proj, int ldp, Fresh<float> ext, DeltaWeights w, float *__restrict__ conv_state,
                   float *__restrict__ state, RowMap rows, T *__restrict__ out) {
     // q [dim_p], k [dim_p], v, gate, o [vdim_p], reduction [8][2][128], scalars [8], CH: decays [dim_p]
     extern __shared__ __align__(16) float sh[];
@@ -49,13 +49,13 @@ delta_step_kernel(DeltaDims d, const float *__restrict__ proj, int ldp, const fl
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
             const int i = warp + 8 * r;
-            st[r] = col && i < d.dim_p && pos > 0 ? *reinterpret_cast<const float4 *>(S + (size_t)i * d.vdim_p + c0 + lane * 4)
+            st[r] = col && i < d.dim_p && pos > 0 ? load_fresh4(S + (size_t)i * d.vdim_p + c0 + lane * 4)
                                                   : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     };
     load_chunk(0);
 
-    const float *p = proj + (size_t)row * ldp;
+    const Fresh<float> p = proj + (size_t)row * ldp;
     const int group = d.heads / d.kv_heads, kh = h / group;
     const int cw = d.conv_w(), here = pos % d.taps;
     float *cring = conv_state + (size_t)slot * d.taps * cw;
@@ -65,13 +65,13 @@ delta_step_kernel(DeltaDims d, const float *__restrict__ proj, int ldp, const fl
     };
     auto request = [&](int ch) {
         Taps t;
-        t.x[0] = *reinterpret_cast<const float4 *>(p + ch);
+        t.x[0] = p.four(ch);
         t.w[0] = __ldg(reinterpret_cast<const float4 *>(w.conv + (size_t)(d.taps - 1) * cw + ch));
 #pragma unroll
         for (int i = 1; i < 4; ++i) {
             const bool use = i < d.taps && pos >= i;
             const int at = use ? (here - i < 0 ? here - i + d.taps : here - i) : here, tap = use ? d.taps - 1 - i : d.taps - 1;
-            const float4 y = *reinterpret_cast<const float4 *>(cring + (size_t)at * cw + ch);
+            const float4 y = load_fresh4(cring + (size_t)at * cw + ch);
             t.x[i] = use ? y : make_float4(0.f, 0.f, 0.f, 0.f);
             t.w[i] = __ldg(reinterpret_cast<const float4 *>(w.conv + (size_t)tap * cw + ch));
         }
@@ -85,7 +85,7 @@ delta_step_kernel(DeltaDims d, const float *__restrict__ proj, int ldp, const fl
             a.z = fmaf(t.x[i].z, t.w[i].z, a.z); a.w = fmaf(t.x[i].w, t.w[i].w, a.w);
         }
         for (int i = 4; i < d.taps && pos >= i; ++i) {
-            const float4 y = *reinterpret_cast<const float4 *>(cring + (size_t)(here - i < 0 ? here - i + d.taps : here - i) * cw + ch);
+            const float4 y = load_fresh4(cring + (size_t)(here - i < 0 ? here - i + d.taps : here - i) * cw + ch);
             const float4 wt = __ldg(reinterpret_cast<const float4 *>(w.conv + (size_t)(d.taps - 1 - i) * cw + ch));
             a.x = fmaf(y.x, wt.x, a.x); a.y = fmaf(y.y, wt.y, a.y); a.z = fmaf(y.z, wt.z, a.z); a.w = fmaf(y.w, wt.w, a.w);
         }
@@ -105,8 +105,8 @@ delta_step_kernel(DeltaDims d, const float *__restrict__ proj, int ldp, const fl
         if (lane == 0) sc[2 + warp] = 1.0f / sqrtf(s + 1e-6f); // unit norms (the value's is not used)
     } else if (warp == 3) {
         for (int j = lane * 4; j < d.vdim_p; j += 128) { // the last columns may be padding: no norm weight there
-            const float *gate = CH ? ext + (size_t)row * 2 * d.ext() + d.ext() : p + d.g_at();
-            const float4 gg = *reinterpret_cast<const float4 *>(gate + h * d.vdim_p + j);
+            const Fresh<float> gate = CH ? ext + ((size_t)row * 2 * d.ext() + d.ext()) : p + d.g_at();
+            const float4 gg = gate.four(h * d.vdim_p + j);
             const float e[4] = {gg.x, gg.y, gg.z, gg.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i) sgn[j + i] = j + i < d.vdim ? w.norm[j + i] * (CH ? sigmoid_f(e[i]) : silu_f(e[i])) : 0.0f;
@@ -181,7 +181,7 @@ delta_step_kernel(DeltaDims d, const float *__restrict__ proj, int ldp, const fl
 // then per query/key head k . q; rows DeltaDims::conv_ld() apart.
 //
 // A warp takes four rows of one unit: a query/key head (both of its vectors) or a value head.  The eight warps of a
-// block take neighbouring rows, which share their convolution inputs in L1.
+// block take neighbouring rows, which share their convolution inputs in L1 (hence an ordered launch).
 // NCH: 128-channel chunks of a query/key head.
 constexpr int CONV_ROWS = 4;
 template <int NCH, bool CH>
@@ -189,7 +189,6 @@ __global__ void __launch_bounds__(256)
 delta_conv_kernel(DeltaDims d, const float *__restrict__ proj, int ldp, const float *__restrict__ ext, DeltaWeights w, const float *__restrict__ conv_state, RowMap rows,
                   SeqMap sm, const int *__restrict__ row_seq, int n_rows, float *__restrict__ conv) {
     pdl_trigger();
-    pdl_wait();
     const int r_first = (blockIdx.y * 8 + (threadIdx.x >> 5)) * CONV_ROWS, u = blockIdx.x, lane = threadIdx.x & 31;
     const int cw = d.conv_w(), ld = d.conv_ld();
     int pos[CONV_ROWS], back[CONV_ROWS]; // position; rows of the same sequence before it in the pass
@@ -328,7 +327,6 @@ delta_scan_kernel(DeltaDims d, const float *__restrict__ proj, int ldp, const fl
     const int cg = blockIdx.x, h = blockIdx.y, sidx = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int part = lane & 7, cl = (warp * 4 + (lane >> 3)) * NC, col = cg * CB + cl; // NC columns from col on
     for (int i = tid; i < (int)(2 * sizeof(Stage) / 4); i += 128) reinterpret_cast<float *>(smem_raw)[i] = 0.0f; // entries past dim stay zero
-    pdl_wait();
     const int n = sm.n[sidx], past = sm.past[sidx], slot = sm.slot[sidx], row0 = sm.row0[sidx];
     const int group = d.heads / d.kv_heads, kh = h / group, cw = d.conv_w(), ldc = d.conv_ld();
     float *S = state + ((size_t)slot * d.heads + h) * d.dim_p * d.vdim_p + col;
@@ -489,31 +487,34 @@ delta_scan_kernel(DeltaDims d, const float *__restrict__ proj, int ldp, const fl
 // One warp per (row, head).
 template <bool CH, typename T>
 __global__ void __launch_bounds__(256)
-delta_out_kernel(DeltaDims d, const float *__restrict__ gates, int ldg, const float *__restrict__ norm, const float *__restrict__ heads_out,
+delta_out_kernel(DeltaDims d, Fresh<float> gates, int ldg, const float *__restrict__ norm, Fresh<float> heads_out,
                  int n_rows, T *__restrict__ out) {
     pdl_trigger();
     pdl_wait();
     const int unit = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (unit >= n_rows * d.heads) return;
     const int row = unit / d.heads, h = unit - row * d.heads;
-    const float *o = heads_out + (size_t)unit * d.vdim_p, *g = gates + (size_t)row * ldg + h * d.vdim_p;
+    const Fresh<float> o = heads_out + (size_t)unit * d.vdim_p, g = gates + ((size_t)row * ldg + h * d.vdim_p);
     auto act = [](float z) { return CH ? sigmoid_f(z) : silu_f(z); };
     float4 v[2]; // the first 256 columns stay in registers
     float s = 0.0f;
 #pragma unroll
     for (int c = 0; c < 2; ++c) { // columns past vdim hold zeros
         const int j = lane * 4 + 128 * c;
-        v[c] = j < d.vdim_p ? __ldcs(reinterpret_cast<const float4 *>(o + j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[c] = j < d.vdim_p ? o.four(j) : make_float4(0.f, 0.f, 0.f, 0.f);
         s += (v[c].x * v[c].x + v[c].y * v[c].y) + (v[c].z * v[c].z + v[c].w * v[c].w);
     }
-    for (int j = 256 + lane; j < d.vdim_p; j += 32) s = fmaf(o[j], o[j], s);
+    for (int j = 256 + lane; j < d.vdim_p; j += 32) {
+        const float t = o[j];
+        s = fmaf(t, t, s);
+    }
     const float rn = 1.0f / sqrtf(warp_sum(s) / (float)d.vdim + d.eps);
     T *y = out + (size_t)unit * d.vdim_p;
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         const int j = lane * 4 + 128 * c;
         if (j >= d.vdim_p) continue;
-        const float4 gg = __ldcs(reinterpret_cast<const float4 *>(g + j));
+        const float4 gg = g.four(j);
         const float e[4] = {v[c].x * act(gg.x), v[c].y * act(gg.y), v[c].z * act(gg.z), v[c].w * act(gg.w)};
 #pragma unroll
         for (int i = 0; i < 4; ++i) store_from_float(y + j + i, j + i < d.vdim ? e[i] * rn * norm[j + i] : 0.0f);
@@ -547,9 +548,9 @@ int prompt_launch(b200nn_ctx *ctx, const DeltaDims &d, bool b16, const float *pr
     PREFER_SMEM_ONCE((delta_conv_kernel<1, CH>));
     PREFER_SMEM_ONCE((delta_conv_kernel<2, CH>));
     if (d.dim_p <= 128)
-        launch_pdl(ctx, delta_conv_kernel<1, CH>, cgrid, dim3(256), 0, d, proj, ldp, ext, w, conv_state, rows, sm, row_seq, n_rows, conv);
+        launch_ordered(ctx, delta_conv_kernel<1, CH>, cgrid, dim3(256), 0, d, proj, ldp, ext, w, conv_state, rows, sm, row_seq, n_rows, conv);
     else
-        launch_pdl(ctx, delta_conv_kernel<2, CH>, cgrid, dim3(256), 0, d, proj, ldp, ext, w, conv_state, rows, sm, row_seq, n_rows, conv);
+        launch_ordered(ctx, delta_conv_kernel<2, CH>, cgrid, dim3(256), 0, d, proj, ldp, ext, w, conv_state, rows, sm, row_seq, n_rows, conv);
     CK_LAUNCH(ctx, "delta_conv_kernel");
     // columns per lane: two when that leaves every SM a dozen warps, else one (more parallel, more instructions)
     const long long columns = (long long)d.vdim_p * d.heads * sm.n_seq;
@@ -565,8 +566,8 @@ int prompt_launch(b200nn_ctx *ctx, const DeltaDims &d, bool b16, const float *pr
             prefer_max_smem(delta_scan_kernel<M, C, CH>);                                                                     \
             done[ctx->device & 15] = true;                                                                                    \
         }                                                                                                                     \
-        CK(ctx, launch_pdl(ctx, delta_scan_kernel<M, C, CH>, dim3((d.vdim_p + 16 * C - 1) / (16 * C), d.heads, sm.n_seq),     \
-                           dim3(128), smem, d, proj, ldp, conv, conv_state, state, sm, heads_out));                           \
+        CK(ctx, launch_ordered(ctx, delta_scan_kernel<M, C, CH>, dim3((d.vdim_p + 16 * C - 1) / (16 * C), d.heads, sm.n_seq), \
+                               dim3(128), smem, d, proj, ldp, conv, conv_state, state, sm, heads_out));                           \
     } while (0)
 #define DSCAN_C(M)                                                                                                            \
     do {                                                                                                                      \

@@ -47,12 +47,44 @@ __device__ __forceinline__ uint32_t pack_f16x2(float a, float b) {
     const __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<const uint32_t *>(&h);
 }
-// A number that the kernels before this one write (positions, picked tokens), from L2: see load_fresh.
+// A value that an earlier kernel of the chain wrote, read after pdl_wait: from L2.  The block may have been resident while
+// that kernel ran on the same SM, so a line that came into L1 since this kernel's start (or through the read-only
+// path, which a plain load from a const __restrict__ pointer takes) can be older than the wait: the second of four f32 rows
+// got its MLP from the residual stream without the attention's sum.
+// (volatile: it stays behind the wait, and in the order of the source, so values that should be in flight together are
+// loaded before the first of them is used)
 __device__ __forceinline__ int load_fresh_int(const void *p) {
     int v;
     asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
+__device__ __forceinline__ float load_fresh(const float *p, size_t i) {
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p + i));
+    return v;
+}
+__device__ __forceinline__ float load_fresh(const __half *p, size_t i) {
+    unsigned short v;
+    asm volatile("ld.global.cg.u16 %0, [%1];" : "=h"(v) : "l"(p + i));
+    return __half2float(__ushort_as_half(v));
+}
+__device__ __forceinline__ uint32_t load_fresh(const uint32_t *p, size_t i) { return (uint32_t)load_fresh_int(p + i); }
+__device__ __forceinline__ int load_fresh(const int *p, size_t i) { return load_fresh_int(p + i); }
+__device__ __forceinline__ float2 load_fresh(const float2 *p, size_t i) { return __ldcg(p + i); }
+__device__ __forceinline__ float4 load_fresh(const float4 *p, size_t i) { return __ldcg(p + i); }
+__device__ __forceinline__ uint4 load_fresh(const uint4 *p, size_t i) { return __ldcg(p + i); }
+__device__ __forceinline__ float4 load_fresh4(const float *p) { return __ldcg(reinterpret_cast<const float4 *>(p)); }
+// The parameter through which a kernel launched with launch_pdl takes an array that earlier kernels of the chain write:
+// it has no plain reads.  (p is for copies that go past L1 anyway: cp.async.cg, bulk copies.)
+template <typename T>
+struct Fresh {
+    const T *p;
+    __host__ __device__ Fresh(const T *q) : p(q) {}
+    __device__ __forceinline__ explicit operator bool() const { return p != nullptr; }
+    __device__ __forceinline__ Fresh operator+(size_t n) const { return Fresh(p + n); }
+    __device__ __forceinline__ auto operator[](size_t i) const { return load_fresh(p, i); }
+    __device__ __forceinline__ float4 four(size_t i) const { return load_fresh4(p + i); } // floats i .. i+3, i a multiple of 4
+};
 __device__ __forceinline__ int row_pos(const RowMap &r, int m) { return load_fresh_int(r.pos + (size_t)m * r.pos_stride); }
 __device__ __forceinline__ int row_slot(const RowMap &r, int m) { return r.slot ? r.slot[m] : m; }
 
@@ -64,7 +96,7 @@ __device__ __forceinline__ void epi_store(const Epilogue &e, int m, int n, float
     if (e.no_store) return;
     if (e.mode == EPI_RESID) {
         size_t i = (size_t)m * e.ldo + n;
-        e.resid[i] = __ldcg(e.resid + i) + v; // not from L1: see load_fresh
+        e.resid[i] = load_fresh(e.resid, i) + v;
         return;
     }
     if (e.mode == EPI_QKV && n >= e.d_model) {
@@ -81,7 +113,7 @@ __device__ __forceinline__ void epi_store(const Epilogue &e, int m, int n, float
         return;
     }
     v = apply_act(v, e.act);
-    if (B16 && e.row_scale) v *= e.row_scale[(size_t)m * e.rs_ld + n / e.rs_cols];
+    if (B16 && e.row_scale) v *= load_fresh(e.row_scale, (size_t)m * e.rs_ld + n / e.rs_cols);
     size_t i = (size_t)m * e.ldo + n;
     if (B16 && e.out_half == OUT_BF16)
         static_cast<__nv_bfloat16 *>(e.out)[i] = __float2bfloat16_rn(v);
@@ -200,7 +232,7 @@ __device__ __forceinline__ void epi_store4_rows(const Epilogue &e, int m0, int s
         float4 r[U];
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            if (u < cnt) r[u] = __ldcg(reinterpret_cast<const float4 *>(e.resid + (size_t)(m0 + u * step) * e.ldo + n));
+            if (u < cnt) r[u] = load_fresh4(e.resid + (size_t)(m0 + u * step) * e.ldo + n);
 #pragma unroll
         for (int u = 0; u < U; ++u)
             if (u < cnt) *reinterpret_cast<float4 *>(e.resid + (size_t)(m0 + u * step) * e.ldo + n) = f4_add(r[u], v[u]);
@@ -227,7 +259,7 @@ __device__ __forceinline__ void epi_store4_rows(const Epilogue &e, int m0, int s
     if (B16 && e.row_scale) {
         float rs[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) rs[u] = e.row_scale[(size_t)(m0 + (u < cnt ? u : 0) * step) * e.rs_ld + n / e.rs_cols];
+        for (int u = 0; u < U; ++u) rs[u] = load_fresh(e.row_scale, (size_t)(m0 + (u < cnt ? u : 0) * step) * e.rs_ld + n / e.rs_cols);
 #pragma unroll
         for (int u = 0; u < U; ++u) v[u] = make_float4(v[u].x * rs[u], v[u].y * rs[u], v[u].z * rs[u], v[u].w * rs[u]);
     }
@@ -434,7 +466,7 @@ __device__ __forceinline__ float4 epi_fold4(const Epilogue &e, int n, int N) {
 // The residual values a producer row will be added to (fetched early, under the reduction of the sums).
 __device__ __forceinline__ float4 epi_resid_old4(const Epilogue &e, int m, int n, int N) {
     if (e.mode != EPI_RESID_LN || n >= N) return make_float4(0.f, 0.f, 0.f, 0.f);
-    return *reinterpret_cast<const float4 *>(e.resid + (size_t)m * e.ldo + n);
+    return load_fresh4(e.resid + (size_t)m * e.ldo + n);
 }
 // Residual epilogue that also prepares the next LayerNorm.  Warp-collective: the 32 lanes are converged on
 // one token row m, lane l holding features n..n+3 (n = 128 * tile + 4 l); v = the finished values (bias
@@ -522,22 +554,6 @@ template <>
 __device__ __forceinline__ float load_as_float<__half>(const __half *p, size_t i) { return __half2float(p[i]); }
 template <>
 __device__ __forceinline__ float load_as_float<__nv_bfloat16>(const __nv_bfloat16 *p, size_t i) { return __bfloat162float(p[i]); }
-// A value that the kernel before wrote, read after pdl_wait: from L2.  The block may have been resident while that
-// kernel ran on the same SM, so a line that came into L1 since this kernel's start (or through the read-only
-// path, which a plain load from a const __restrict__ pointer takes) can be older than the wait: the second of four f32 rows
-// got its MLP from the residual stream without the attention's sum.
-// (volatile: it stays behind the wait, and in the order of the source, so values that should be in flight together are
-// loaded before the first of them is used)
-__device__ __forceinline__ float load_fresh(const float *p, size_t i) {
-    float v;
-    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p + i));
-    return v;
-}
-__device__ __forceinline__ float load_fresh(const __half *p, size_t i) {
-    unsigned short v;
-    asm volatile("ld.global.cg.u16 %0, [%1];" : "=h"(v) : "l"(p + i));
-    return __half2float(__ushort_as_half(v));
-}
 __device__ __forceinline__ void store_from_float(float *p, float v) { *p = v; }
 __device__ __forceinline__ void store_from_float(__half *p, float v) { *p = __float2half_rn(v); }
 __device__ __forceinline__ void store_from_float(__nv_bfloat16 *p, float v) { *p = __float2bfloat16_rn(v); }
@@ -557,7 +573,7 @@ __device__ __forceinline__ void st_cluster(float *p, int rank, float v) {
 // Contains the wait on the previous kernel, after the loads of scale and shift.  red: THREADS / 32 * MT floats; the
 // caller synchronises before it reads xs or reuses red.
 template <int MT, int THREADS>
-__device__ __forceinline__ void norm_rows_to_smem(const NormIn &ln, const float *__restrict__ x, int m_valid, int K, int k0, int cols,
+__device__ __forceinline__ void norm_rows_to_smem(const NormIn &ln, Fresh<float> x, int m_valid, int K, int k0, int cols,
                                                   int ld, float *xs, float *red) {
     constexpr int VPT = NORM_IN_MAX / THREADS, WARPS = THREADS / 32;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -592,7 +608,7 @@ __device__ __forceinline__ void norm_rows_to_smem(const NormIn &ln, const float 
 #pragma unroll
         for (int i = 0; i < VPT; ++i) {
             const int k = tid + i * THREADS;
-            v[m][i] = m < m_valid && k < K ? load_fresh(x, (size_t)m * K + k) : 0.0f;
+            v[m][i] = m < m_valid && k < K ? x[(size_t)m * K + k] : 0.0f;
         }
 #pragma unroll
         for (int i = 0; i < VPT; ++i) s[m] += v[m][i];
@@ -623,7 +639,7 @@ __device__ __forceinline__ void norm_rows_to_smem(const NormIn &ln, const float 
 
 // Columns k0 .. k0+cols of up to MT rows x [m_valid][K] as f32 in xs [MT][ld], zero past them and past m_valid.
 template <int MT, int THREADS, typename XT>
-__device__ __forceinline__ void rows_to_smem(const XT *__restrict__ x, int m_valid, int K, int k0, int cols, int ld, float *xs) {
+__device__ __forceinline__ void rows_to_smem(Fresh<XT> x, int m_valid, int K, int k0, int cols, int ld, float *xs) {
     constexpr int U = 4; // loads of a thread in flight
 #pragma unroll
     for (int m = 0; m < MT; ++m)
@@ -631,7 +647,7 @@ __device__ __forceinline__ void rows_to_smem(const XT *__restrict__ x, int m_val
             float v[U];
 #pragma unroll
             for (int u = 0; u < U; ++u)
-                v[u] = m < m_valid && base + u * THREADS < cols ? load_fresh(x, (size_t)m * K + k0 + base + u * THREADS) : 0.0f;
+                v[u] = m < m_valid && base + u * THREADS < cols ? x[(size_t)m * K + k0 + base + u * THREADS] : 0.0f;
 #pragma unroll
             for (int u = 0; u < U; ++u)
                 if (base + u * THREADS < ld) xs[m * ld + base + u * THREADS] = v[u];

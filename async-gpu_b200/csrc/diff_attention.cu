@@ -15,7 +15,6 @@ diff_simple_kernel(DiffDims d, const T *__restrict__ q, int ldq, const T *__rest
                    T *__restrict__ out) {
     extern __shared__ float sh[]; // query [2 dim_p], weights [2][128], reduction [16]
     pdl_trigger();
-    pdl_wait();
     const int h = blockIdx.x, row = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kw = d.kv_w();
     float *sq = sh, *sp = sq + 2 * d.dim_p, *red = sp + 256;
@@ -93,7 +92,7 @@ diff_simple_kernel(DiffDims d, const T *__restrict__ q, int ldq, const T *__rest
     }
 }
 
-__global__ void __launch_bounds__(256) kv_store_f32_kernel(const float *__restrict__ proj, int ldp, int at, int kv_heads, int kv_w, int cap, RowMap rows,
+__global__ void __launch_bounds__(256) kv_store_f32_kernel(Fresh<float> proj, int ldp, int at, int kv_heads, int kv_w, int cap, RowMap rows,
                                                            float *__restrict__ cache) {
     pdl_trigger();
     pdl_wait();
@@ -132,11 +131,11 @@ int launch_diff_attention(b200nn_ctx *ctx, const DiffDims &d, bool b16, const vo
     const size_t smem = (2 * d.dim_p + 256 + 16) * sizeof(float);
     if (b16) {
         PREFER_SMEM_ONCE(diff_simple_kernel<__nv_bfloat16>);
-        launch_pdl(ctx, diff_simple_kernel<__nv_bfloat16>, grid, dim3(128), smem, d, (const __nv_bfloat16 *)q, ldq, (const __nv_bfloat16 *)cache, cap, rows,
+        launch_ordered(ctx, diff_simple_kernel<__nv_bfloat16>, grid, dim3(128), smem, d, (const __nv_bfloat16 *)q, ldq, (const __nv_bfloat16 *)cache, cap, rows,
                    gate, gate_ld, (__nv_bfloat16 *)out);
     } else {
         PREFER_SMEM_ONCE(diff_simple_kernel<float>);
-        launch_pdl(ctx, diff_simple_kernel<float>, grid, dim3(128), smem, d, (const float *)q, ldq, (const float *)cache, cap, rows, gate, gate_ld,
+        launch_ordered(ctx, diff_simple_kernel<float>, grid, dim3(128), smem, d, (const float *)q, ldq, (const float *)cache, cap, rows, gate, gate_ld,
                    (float *)out);
     }
     CK_LAUNCH(ctx, "diff_simple_kernel");

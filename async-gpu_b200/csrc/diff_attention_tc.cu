@@ -50,7 +50,7 @@ __device__ __forceinline__ float rcp_approx(float x) {
 template <int KB, int VB, int VS, bool CAP>
 __global__ void __launch_bounds__(NTHREADS, 1)
 diff_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_c, DiffDims d, int cap_rows, SeqMap sm,
-                       const float *__restrict__ gate, int gate_ld, __nv_bfloat16 *__restrict__ out, uint32_t *__restrict__ dev_err) {
+                       Fresh<float> gate, int gate_ld, __nv_bfloat16 *__restrict__ out, uint32_t *__restrict__ dev_err) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) Bars bars;
     __shared__ float row_sum[128]; // of map 1

@@ -181,7 +181,7 @@ diff_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_c, const DiffDecode
                 const int box = i / (N * 8), c = (i >> 3) % N, ch = i & 7, col = box * 64 + ch * 8, map = c / NH, hh = c % NH;
                 uint4 v = make_uint4(0, 0, 0, 0);
                 if (hh < nh && col >= map * d.dim_p && col < (map + 1) * d.dim_p)
-                    v = *reinterpret_cast<const uint4 *>(a.q + (size_t)row * a.ldq + (size_t)(h0 + hh) * 2 * d.dim_p + col);
+                    v = load_fresh(reinterpret_cast<const uint4 *>(a.q + (size_t)row * a.ldq + (size_t)(h0 + hh) * 2 * d.dim_p + col), 0);
                 *reinterpret_cast<uint4 *>(gen_base + (sQ - base) + box * QBOX + c * 128 + ((ch ^ (c & 7)) << 4)) = v;
             }
             tc::fence_proxy_async_smem();
@@ -304,7 +304,7 @@ diff_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_c, const DiffDecode
 
 // Adds up the splits of one (head, row), then the two maps, norm and gate.
 __global__ void __launch_bounds__(128)
-diff_merge_kernel(DiffDims d, const float *__restrict__ part_o, const float *__restrict__ part_ml, int splits, const float *__restrict__ gate, int gate_ld,
+diff_merge_kernel(DiffDims d, Fresh<float> part_o, Fresh<float> part_ml, int splits, Fresh<float> gate, int gate_ld,
                   __nv_bfloat16 *__restrict__ out) {
     __shared__ float red[4];
     pdl_trigger();
@@ -313,7 +313,7 @@ diff_merge_kernel(DiffDims d, const float *__restrict__ part_o, const float *__r
     const size_t unit = ((size_t)row * d.heads + h) * 2, stride = (size_t)gridDim.y * d.heads * 2;
     float m[2] = {NEG_BIG, NEG_BIG}, total[2] = {0.0f, 0.0f};
     for (int s = 0; s < splits; ++s) {
-        const float4 ml = __ldcg(reinterpret_cast<const float4 *>(part_ml + (s * stride + unit) * 2)); // (max, sum) of both maps
+        const float4 ml = part_ml.four((s * stride + unit) * 2); // (max, sum) of both maps
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
             const float mm = x ? ml.z : ml.x, ll = x ? ml.w : ml.y, mn = fmaxf(m[x], mm);
@@ -324,14 +324,14 @@ diff_merge_kernel(DiffDims d, const float *__restrict__ part_o, const float *__r
     const float inv[2] = {1.0f / total[0], -d.lambda / total[1]};
     float acc[4] = {0.f, 0.f, 0.f, 0.f}, ss = 0.0f; // vdim_p <= 512
     for (int s = 0; s < splits; ++s) {
-        const float4 ml = __ldcg(reinterpret_cast<const float4 *>(part_ml + (s * stride + unit) * 2));
+        const float4 ml = part_ml.four((s * stride + unit) * 2);
         if (ml.y == 0.0f) continue; // a split without keys left nothing
         const float f0 = tc::ex2_approx(ml.x - m[0]) * inv[0], f1 = tc::ex2_approx(ml.z - m[1]) * inv[1];
-        const float *o = part_o + (s * stride + unit) * d.vdim_p;
+        const Fresh<float> o = part_o + (s * stride + unit) * d.vdim_p;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             const int e = tid + 128 * c;
-            if (e < d.vdim_p) acc[c] += f0 * __ldcg(o + e) + f1 * __ldcg(o + d.vdim_p + e);
+            if (e < d.vdim_p) acc[c] += f0 * o[e] + f1 * o[d.vdim_p + e];
         }
     }
 #pragma unroll

@@ -53,7 +53,7 @@ __device__ __forceinline__ void gemv_block_fma(const uint4 &wa, const uint4 &wb,
 // second block per tile.
 template <int MT, int RW, typename XT>
 __global__ void __launch_bounds__(GEMV_THREADS, 2)
-int4_gemv_kernel(const uint4 *__restrict__ tiles, const __half *__restrict__ scales, const XT *__restrict__ x,
+int4_gemv_kernel(const uint4 *__restrict__ tiles, const __half *__restrict__ scales, Fresh<XT> x,
                  int m_valid, int m0, int K, int N, int k_blocks, int n_pad, int group, int kb_per_split,
                  NormIn ln, Epilogue epi) {
     constexpr int SLICES = GEMV_THREADS / RW;

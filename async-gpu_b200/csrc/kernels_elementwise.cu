@@ -11,7 +11,7 @@
 // (ops/norm.rs:248-400 `layer_norm_residual_dual`).
 // ---------------------------------------------------------------------------------------------
 template <int VPT, typename TOut>
-__global__ void __launch_bounds__(256) layernorm_kernel(const float *__restrict__ x, const float *__restrict__ res_in,
+__global__ void __launch_bounds__(256) layernorm_kernel(Fresh<float> x, Fresh<float> res_in,
                                                         float *__restrict__ sum_out, const float *__restrict__ gamma,
                                                         const float *__restrict__ beta, float eps, int d,
                                                         TOut *__restrict__ out) {
@@ -28,16 +28,15 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const float *__restrict_
         bt[i] = (j < d) ? beta[j] : 0.0f;
     }
     pdl_wait();
-    const float *xr = x + (size_t)row * d;
-    const float *rr = res_in ? res_in + (size_t)row * d : nullptr;
+    const Fresh<float> xr = x + (size_t)row * d, rr = res_in ? res_in + (size_t)row * d : res_in;
     float v[VPT];
     float s = 0.0f;
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) v[i] = tid + i * 256 < d ? load_fresh(xr, tid + i * 256) : 0.0f; // all in flight at once
-    if (rr)
+    for (int i = 0; i < VPT; ++i) v[i] = tid + i * 256 < d ? xr[tid + i * 256] : 0.0f; // all in flight at once
+    if (rr) // (asked of rr: with res_in the compiler makes a second copy of what follows, 2.4 -> 2.9 us in a decode step)
 #pragma unroll
         for (int i = 0; i < VPT; ++i)
-            if (tid + i * 256 < d) v[i] += load_fresh(rr, tid + i * 256);
+            if (tid + i * 256 < d) v[i] += rr[tid + i * 256];
     if (sum_out)
 #pragma unroll
         for (int i = 0; i < VPT; ++i)
@@ -72,7 +71,7 @@ __global__ void __launch_bounds__(256) layernorm_kernel(const float *__restrict_
 // shuffles, nothing waits on a block barrier, and scale / shift come from shared memory; 16-byte loads and
 // 8-byte (fp16) or 16-byte (f32) stores, all coalesced.  d a multiple of 4, at most 128 * NV.
 template <int NV, typename TOut>
-__global__ void __launch_bounds__(256) layernorm_rows_kernel(const float *__restrict__ x, const float *__restrict__ gamma,
+__global__ void __launch_bounds__(256) layernorm_rows_kernel(Fresh<float> x, const float *__restrict__ gamma,
                                                              const float *__restrict__ beta, float eps, int rows, int d,
                                                              TOut *__restrict__ out) {
     extern __shared__ float4 gb[]; // [d/4] scale, then [d/4] shift
@@ -86,13 +85,13 @@ __global__ void __launch_bounds__(256) layernorm_rows_kernel(const float *__rest
     pdl_wait();
     const float inv_d = 1.0f / (float)d;
     for (int row = blockIdx.x * 8 + warp; row < rows; row += gridDim.x * 8) {
-        const float4 *xr = reinterpret_cast<const float4 *>(x + (size_t)row * d);
+        const Fresh<float> xr = x + (size_t)row * d;
         float4 v[NV];
         float s = 0.0f;
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int c = lane + 32 * i;
-            v[i] = c < d4 ? __ldcs(xr + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[i] = c < d4 ? xr.four(c * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
             s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
         }
         const float mean = warp_sum(s) * inv_d;
@@ -180,15 +179,15 @@ int launch_layernorm(b200nn_ctx *ctx, const float *x, const float *res_in, float
 // Embedding: out[r,:] = wte[ids[r],:] + wpe[pos(r),:], pos(r) = *pos_ptr + pos_off + r % rows_per_seq
 // (layers/embedding.rs:59-93 computes the offset form on the host; here it is one gather).
 // ---------------------------------------------------------------------------------------------
-__global__ void embedding_kernel(const uint32_t *__restrict__ ids, const float *__restrict__ wte,
-                                 const float *__restrict__ wpe, int d, int rows_per_seq, const int *pos_ptr,
+__global__ void embedding_kernel(Fresh<uint32_t> ids, const float *__restrict__ wte,
+                                 const float *__restrict__ wpe, int d, int rows_per_seq, Fresh<int> pos_ptr,
                                  int pos_off, int vocab, int n_positions, float *__restrict__ out) {
     int r = blockIdx.x;
     pdl_trigger();
     pdl_wait();
-    uint32_t tok = (uint32_t)load_fresh_int(ids + r);
+    uint32_t tok = ids[r];
     if (tok >= (uint32_t)vocab) tok = vocab - 1; // ids are validated on the host; never read out of range
-    int pos = (pos_ptr ? load_fresh_int(pos_ptr) : 0) + pos_off + r % rows_per_seq;
+    int pos = (pos_ptr ? pos_ptr[0] : 0) + pos_off + r % rows_per_seq;
     if (pos >= n_positions) pos = n_positions - 1;
     const float *a = wte + (size_t)tok * d, *b = wpe + (size_t)pos * d;
     for (int j = threadIdx.x; j < d; j += blockDim.x) out[(size_t)r * d + j] = a[j] + b[j];
@@ -206,8 +205,8 @@ int launch_embedding(b200nn_ctx *ctx, const uint32_t *ids, const float *wte, con
 
 // The decode-step embedding when the first LayerNorm is folded into the q/k/v GEMM (see Epilogue): one
 // row per block at position *pos_ptr.
-__global__ void __launch_bounds__(256) embedding_ln_kernel(const uint32_t *__restrict__ ids, const float *__restrict__ wte,
-                                                           const float *__restrict__ wpe, int d, const int *pos_ptr, int vocab,
+__global__ void __launch_bounds__(256) embedding_ln_kernel(Fresh<uint32_t> ids, const float *__restrict__ wte,
+                                                           const float *__restrict__ wpe, int d, Fresh<int> pos_ptr, int vocab,
                                                            int n_positions, float *__restrict__ out,
                                                            const float *__restrict__ g, __half *__restrict__ xg,
                                                            float *__restrict__ stats, int stats_nt) {
@@ -215,9 +214,9 @@ __global__ void __launch_bounds__(256) embedding_ln_kernel(const uint32_t *__res
     const int r = blockIdx.x;
     pdl_trigger();
     pdl_wait();
-    uint32_t tok = (uint32_t)load_fresh_int(ids + r);
+    uint32_t tok = ids[r];
     if (tok >= (uint32_t)vocab) tok = vocab - 1;
-    int pos = load_fresh_int(pos_ptr);
+    int pos = pos_ptr[0];
     if (pos >= n_positions) pos = n_positions - 1;
     const float *a = wte + (size_t)tok * d, *b = wpe + (size_t)pos * d;
     float s1 = 0.0f, s2 = 0.0f;
@@ -265,17 +264,17 @@ __global__ void add_kernel(float *__restrict__ a, const float *__restrict__ b, s
 // int4 Linears of GPT-2 Small's shapes with 8 rows 45 -> 34 us, with 64 rows 61 -> 51 us.
 // VEC: both buffers start on 16 bytes and n is a multiple of 4.
 template <bool VEC>
-__global__ void f32_to_half_kernel(const float *__restrict__ x, __half *__restrict__ y, size_t n) {
+__global__ void f32_to_half_kernel(Fresh<float> x, __half *__restrict__ y, size_t n) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, st = (size_t)gridDim.x * blockDim.x;
     pdl_trigger();
     pdl_wait();
     if constexpr (VEC) {
         for (; i < n / 4; i += st) {
-            const float4 v = __ldcg(reinterpret_cast<const float4 *>(x) + i);
+            const float4 v = x.four(i * 4);
             reinterpret_cast<uint2 *>(y)[i] = make_uint2(pack_f16x2(v.x, v.y), pack_f16x2(v.z, v.w));
         }
     } else {
-        for (; i < n; i += st) y[i] = __float2half_rn(load_fresh(x, i));
+        for (; i < n; i += st) y[i] = __float2half_rn(x[i]);
     }
 }
 __global__ void half_to_f32_kernel(const __half *__restrict__ x, float *__restrict__ y, size_t n) {
@@ -412,20 +411,26 @@ int launch_pack_kv(b200nn_ctx *ctx, const float *src, int H, int len, int cap, _
 // maximum (the CPU f64 reference, tests_inference.rs:4504-4515); keep_last=true keeps the last
 // (Rust max_by, models/gpt2.rs:991-997).
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) argmax_kernel(const float *__restrict__ logits, int vocab, int ld,
+__global__ void __launch_bounds__(1024) argmax_kernel(Fresh<float> logits, int vocab, int ld,
                                                       int keep_last, uint32_t *__restrict__ tok_out) {
     __shared__ float sv[32];
     __shared__ int si[32];
     pdl_trigger();
     pdl_wait();
-    const float *row = logits + (size_t)blockIdx.x * ld;
+    const Fresh<float> row = logits + (size_t)blockIdx.x * ld;
     float best = -INFINITY;
     int bi = keep_last ? -1 : 0x7fffffff;
-    for (int j = threadIdx.x; j < vocab; j += blockDim.x) {
-        float v = row[j];
-        if (v > best || (v == best && (keep_last ? j > bi : j < bi))) {
-            best = v;
-            bi = j;
+    for (int j0 = threadIdx.x; j0 < vocab; j0 += 4 * blockDim.x) {
+        float v[4]; // in flight together
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = j0 + u * blockDim.x < vocab ? row[j0 + u * blockDim.x] : -INFINITY;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int j = j0 + u * blockDim.x;
+            if (j < vocab && (v[u] > best || (v[u] == best && (keep_last ? j > bi : j < bi)))) {
+                best = v[u];
+                bi = j;
+            }
         }
     }
     auto better = [&](float v, int i, float bv, int bidx) {
@@ -465,15 +470,15 @@ int launch_argmax(b200nn_ctx *ctx, const float *logits, int rows, int vocab, int
 // Second stage of the greedy pick fused into the LM head's epilogue: the (value, index) entries of a
 // row, one per 32 features, reduced with the same tie rule as argmax_kernel (same token, bit for bit:
 // a maximum does not depend on the order it is taken in).
-__global__ void __launch_bounds__(256) argmax_entries_kernel(const float *__restrict__ val, const int *__restrict__ idx,
+__global__ void __launch_bounds__(256) argmax_entries_kernel(Fresh<float> val, Fresh<int> idx,
                                                             int n_entries, int vocab, int keep_last,
                                                             uint32_t *__restrict__ tok_out) {
     __shared__ float sv[8];
     __shared__ int si[8];
     pdl_trigger();
     pdl_wait();
-    const float *rv = val + (size_t)blockIdx.x * n_entries;
-    const int *ri = idx + (size_t)blockIdx.x * n_entries;
+    const Fresh<float> rv = val + (size_t)blockIdx.x * n_entries;
+    const Fresh<int> ri = idx + (size_t)blockIdx.x * n_entries;
     float best = -INFINITY;
     int bi = keep_last ? -1 : 0x7fffffff;
     // (a row has entries for whole 128-feature tiles; those past the vocabulary may not have been written)
@@ -511,13 +516,13 @@ int launch_argmax_entries(b200nn_ctx *ctx, const float *val, const int *idx, int
 
 // Appends this step's token of every sequence to the history and advances the step / position
 // counters that the next step's kernels read (single block, so the increment is ordered).
-__global__ void record_tokens_kernel(const uint32_t *__restrict__ tok, int rows, uint32_t *__restrict__ history,
+__global__ void record_tokens_kernel(Fresh<uint32_t> tok, int rows, uint32_t *__restrict__ history,
                                      int hist_cap, int *step_ptr, int *pos_ptr) {
     pdl_trigger();
     pdl_wait();
     const int step = load_fresh_int(step_ptr);
     for (int r = threadIdx.x; r < rows; r += blockDim.x)
-        if (step < hist_cap) history[(size_t)r * hist_cap + step] = (uint32_t)load_fresh_int(tok + r);
+        if (step < hist_cap) history[(size_t)r * hist_cap + step] = tok[r];
     __syncthreads();
     if (threadIdx.x == 0) {
         *step_ptr = step + 1;
@@ -582,7 +587,7 @@ int launch_tensor_transpose(b200nn_ctx *ctx, const float *in, float *out, const 
 // ---------------------------------------------------------------------------------------------
 // x / sqrt(mean(x^2) + eps) * w, one block per row; output rows ldo apart.
 template <int VPT, typename TOut>
-__global__ void __launch_bounds__(256) rmsnorm_kernel(const float *__restrict__ x, const float *__restrict__ w, float eps, int d, int ldo,
+__global__ void __launch_bounds__(256) rmsnorm_kernel(Fresh<float> x, const float *__restrict__ w, float eps, int d, int ldo,
                                                       TOut *__restrict__ out) {
     __shared__ float red[32];
     const int row = blockIdx.x, tid = threadIdx.x;
@@ -593,10 +598,9 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float *__restrict__ 
     pdl_wait();
     float v[VPT], s = 0.0f;
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-        v[i] = tid + i * 256 < d ? x[(size_t)row * d + tid + i * 256] : 0.0f;
-        s = fmaf(v[i], v[i], s);
-    }
+    for (int i = 0; i < VPT; ++i) v[i] = tid + i * 256 < d ? x[(size_t)row * d + tid + i * 256] : 0.0f; // all in flight at once
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) s = fmaf(v[i], v[i], s);
     const float r = 1.0f / sqrtf(block_sum(s, red) / (float)d + eps);
 #pragma unroll
     for (int i = 0; i < VPT; ++i)
@@ -605,19 +609,19 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const float *__restrict__ 
 
 // Many rows (prompt passes): one warp per row, the row in registers (NV float4 per lane); d a multiple of 4.
 template <int NV>
-__global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const float *__restrict__ x, const float *__restrict__ w, float eps, int rows,
+__global__ void __launch_bounds__(256) rmsnorm_rows_kernel(Fresh<float> x, const float *__restrict__ w, float eps, int rows,
                                                            int d, int ldo, __nv_bfloat16 *__restrict__ out) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d4 = d >> 2;
     pdl_trigger();
     pdl_wait();
     for (int row = blockIdx.x * 8 + warp; row < rows; row += gridDim.x * 8) {
-        const float4 *xr = reinterpret_cast<const float4 *>(x + (size_t)row * d);
+        const Fresh<float> xr = x + (size_t)row * d;
         float4 v[NV];
         float s = 0.0f;
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int c = lane + 32 * i;
-            v[i] = c < d4 ? __ldcs(xr + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[i] = c < d4 ? xr.four(c * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
             s += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
         }
         const float r = 1.0f / sqrtf(warp_sum(s) / (float)d + eps);
@@ -672,7 +676,7 @@ int launch_rmsnorm(b200nn_ctx *ctx, const float *x, const float *w, float eps, i
 }
 
 template <typename T>
-__global__ void embedding_rows_kernel(const uint32_t *__restrict__ ids, const T *__restrict__ table, int ldt, int d, int vocab,
+__global__ void embedding_rows_kernel(Fresh<uint32_t> ids, const T *__restrict__ table, int ldt, int d, int vocab,
                                       const T *__restrict__ pos_table, int max_pos, RowMap rows, float *__restrict__ out) {
     const int r = blockIdx.x;
     pdl_trigger();
@@ -697,7 +701,7 @@ int launch_embedding_rows(b200nn_ctx *ctx, const uint32_t *ids, const void *tabl
     return B200NN_OK;
 }
 
-__global__ void glu_kernel(const float4 *__restrict__ gu, size_t quads, int act, float2 *__restrict__ out) {
+__global__ void glu_kernel(Fresh<float4> gu, size_t quads, int act, float2 *__restrict__ out) {
     pdl_trigger();
     pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -714,10 +718,10 @@ int launch_glu(b200nn_ctx *ctx, const float *gu, int rows, int n2, int act, floa
     return B200NN_OK;
 }
 
-__global__ void gather_rows_kernel(const float *__restrict__ src, const int *__restrict__ idx, int d, float *__restrict__ dst) {
+__global__ void gather_rows_kernel(Fresh<float> src, const int *__restrict__ idx, int d, float *__restrict__ dst) {
     pdl_trigger();
     pdl_wait();
-    const float *s = src + (size_t)idx[blockIdx.x] * d;
+    const Fresh<float> s = src + (size_t)idx[blockIdx.x] * d;
     for (int j = threadIdx.x; j < d; j += blockDim.x) dst[(size_t)blockIdx.x * d + j] = s[j];
 }
 int launch_gather_rows(b200nn_ctx *ctx, const float *src, const int *idx, int n_rows, int d, float *dst) {
@@ -729,7 +733,7 @@ int launch_gather_rows(b200nn_ctx *ctx, const float *src, const int *idx, int n_
 }
 
 // One warp per output: the weight rows are contiguous along K.
-__global__ void __launch_bounds__(256) grouped_f32_kernel(const float *__restrict__ w, int groups, int Ng, int Kg, const float *__restrict__ x,
+__global__ void __launch_bounds__(256) grouped_f32_kernel(const float *__restrict__ w, int groups, int Ng, int Kg, Fresh<float> x,
                                                           int ldx, int x_stride, int M, Epilogue epi, int out_stride) {
     pdl_trigger();
     pdl_wait();
@@ -737,8 +741,10 @@ __global__ void __launch_bounds__(256) grouped_f32_kernel(const float *__restric
     const int lane = threadIdx.x & 31;
     if (unit >= (size_t)M * groups * Ng) return;
     const int gn = (int)(unit % ((size_t)groups * Ng)), m = (int)(unit / ((size_t)groups * Ng)), g = gn / Ng, n = gn - g * Ng;
-    const float *wr = w + (size_t)gn * Kg, *xr = x + (size_t)m * ldx + (size_t)g * x_stride;
+    const float *wr = w + (size_t)gn * Kg;
+    const Fresh<float> xr = x + ((size_t)m * ldx + (size_t)g * x_stride);
     float a = 0.0f;
+#pragma unroll 4
     for (int k = lane; k < Kg; k += 32) a = fmaf(wr[k], xr[k], a);
     a = warp_sum(a);
     if (lane == 0) epi_apply<true>(epi, m, g * out_stride + n, a);

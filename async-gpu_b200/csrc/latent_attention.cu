@@ -18,19 +18,23 @@ namespace {
 
 template <typename T>
 __global__ void __launch_bounds__(128)
-latent_prep_kernel(LatentDims d, const float *__restrict__ proj, int ldp, const float *__restrict__ q_norm,
+latent_prep_kernel(LatentDims d, Fresh<float> proj, int ldp, const float *__restrict__ q_norm,
                    const float *__restrict__ kv_norm, const float2 *__restrict__ rope, RowMap rows, T *__restrict__ cq,
                    T *__restrict__ cache, int ring, float *__restrict__ gate) {
     __shared__ float red[2];
     pdl_trigger();
     pdl_wait();
     const int r = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const float *p = proj + (size_t)r * ldp, *pc = p + d.q_rank, *pr = pc + d.rank, *pg = pr + d.rot;
+    const Fresh<float> p = proj + (size_t)r * ldp, pc = p + d.q_rank, pr = pc + d.rank, pg = pr + d.rot;
     if (warp < 2) { // one warp per norm
-        const float *src = warp ? pc : p;
+        const Fresh<float> src = warp ? pc : p;
         const int n = warp ? d.rank : d.q_rank;
         float s = 0.0f;
-        for (int j = lane; j < n; j += 32) s = fmaf(src[j], src[j], s);
+        #pragma unroll 4
+        for (int j = lane; j < n; j += 32) {
+            const float v = src[j];
+            s = fmaf(v, v, s);
+        }
         s = warp_sum(s);
         if (lane == 0) red[warp] = 1.0f / sqrtf(s / (float)n + d.eps);
     }
@@ -65,14 +69,14 @@ __global__ void rope_heads_kernel(float *__restrict__ q, int n_rows, int heads, 
         const int i = t % pairs, h = (t / pairs) % heads, r = t / (pairs * heads);
         float *x = q + ((size_t)r * heads + h) * head_w + at + 2 * i;
         const float2 cs = tab[(size_t)row_pos(rows, r) * pairs + i];
-        const float u = x[0], v = x[1];
+        const float u = load_fresh(x, 0), v = load_fresh(x, 1);
         x[0] = u * cs.x - v * cs.y;
         x[1] = v * cs.x + u * cs.y;
     }
 }
 
 // 16-byte pieces: rows are multiples of 32 bytes.
-__global__ void latent_gather_kernel(const uint4 *__restrict__ cache, int ring, int pieces, SeqMap sm, uint4 *__restrict__ lin) {
+__global__ void latent_gather_kernel(Fresh<uint4> cache, int ring, int pieces, SeqMap sm, uint4 *__restrict__ lin) {
     pdl_trigger();
     pdl_wait();
     const int s = blockIdx.y, klen = sm.klen[s];
@@ -90,7 +94,6 @@ latent_prefill_simple_kernel(LatentDims d, const T *__restrict__ q, const T *__r
                              const float *__restrict__ gate, T *__restrict__ out) {
     extern __shared__ float sh[]; // query [head_w], weights [128], red [8]
     pdl_trigger();
-    pdl_wait();
     const int h = blockIdx.x, s = blockIdx.z, i = blockIdx.y, tid = threadIdx.x;
     if (i >= sm.n[s]) return;
     const int hw = d.dim_p + d.rot_p, ld = d.rank_p + d.rot_p, kvw = d.heads * (d.dim_p + d.vdim_p);
@@ -152,7 +155,6 @@ latent_decode_simple_kernel(LatentDims d, const T *__restrict__ q, const T *__re
                             RowMap rows, T *__restrict__ out) {
     extern __shared__ float sh[]; // query [rank_p + rot_p], weights [128], red [8]
     pdl_trigger();
-    pdl_wait();
     const int h = blockIdx.x, row = blockIdx.y, tid = threadIdx.x;
     const int hw = d.dim_p + d.rot_p, ld = d.rank_p + d.rot_p;
     float *sq = sh, *sp = sh + ld, *red = sp + 128;
@@ -256,11 +258,11 @@ int launch_latent_prefill(b200nn_ctx *ctx, const LatentDims &d, bool b16, int n_
     const size_t smem = (d.head_w() + 136) * sizeof(float);
     if (b16) {
         PREFER_SMEM_ONCE(latent_prefill_simple_kernel<__nv_bfloat16>);
-        launch_pdl(ctx, latent_prefill_simple_kernel<__nv_bfloat16>, grid, dim3(128), smem, d, (const __nv_bfloat16 *)q,
+        launch_ordered(ctx, latent_prefill_simple_kernel<__nv_bfloat16>, grid, dim3(128), smem, d, (const __nv_bfloat16 *)q,
                    (const __nv_bfloat16 *)kvx, (const __nv_bfloat16 *)lin, sm, gate, (__nv_bfloat16 *)out);
     } else {
         PREFER_SMEM_ONCE(latent_prefill_simple_kernel<float>);
-        launch_pdl(ctx, latent_prefill_simple_kernel<float>, grid, dim3(128), smem, d, (const float *)q, (const float *)kvx,
+        launch_ordered(ctx, latent_prefill_simple_kernel<float>, grid, dim3(128), smem, d, (const float *)q, (const float *)kvx,
                    (const float *)lin, sm, gate, (float *)out);
     }
     CK_LAUNCH(ctx, "latent_prefill_simple_kernel");
@@ -282,11 +284,11 @@ int launch_latent_decode(b200nn_ctx *ctx, const LatentDims &d, bool b16, const v
     const size_t smem = (d.ld() + 136) * sizeof(float);
     if (b16) {
         PREFER_SMEM_ONCE(latent_decode_simple_kernel<__nv_bfloat16>);
-        launch_pdl(ctx, latent_decode_simple_kernel<__nv_bfloat16>, grid, dim3(128), smem, d, (const __nv_bfloat16 *)q,
+        launch_ordered(ctx, latent_decode_simple_kernel<__nv_bfloat16>, grid, dim3(128), smem, d, (const __nv_bfloat16 *)q,
                    (const __nv_bfloat16 *)qlat, (const __nv_bfloat16 *)cache, ring, rows, (__nv_bfloat16 *)out);
     } else {
         PREFER_SMEM_ONCE(latent_decode_simple_kernel<float>);
-        launch_pdl(ctx, latent_decode_simple_kernel<float>, grid, dim3(128), smem, d, (const float *)q, (const float *)qlat,
+        launch_ordered(ctx, latent_decode_simple_kernel<float>, grid, dim3(128), smem, d, (const float *)q, (const float *)qlat,
                    (const float *)cache, ring, rows, (float *)out);
     }
     CK_LAUNCH(ctx, "latent_decode_simple_kernel");

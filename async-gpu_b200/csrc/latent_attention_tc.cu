@@ -40,7 +40,7 @@ template <int VB>
 __global__ void __launch_bounds__(NTHREADS, 1)
 latent_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                          const __grid_constant__ CUtensorMap tm_r, const __grid_constant__ CUtensorMap tm_v, LatentDims d, SeqMap sm,
-                         float scale_log2e, const float *__restrict__ gate, __nv_bfloat16 *__restrict__ out, uint32_t *__restrict__ dev_err) {
+                         float scale_log2e, Fresh<float> gate, __nv_bfloat16 *__restrict__ out, uint32_t *__restrict__ dev_err) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) Bars bars;
     __shared__ uint32_t tmem_slot;

@@ -305,26 +305,26 @@ latent_decode_tc_kernel(const __grid_constant__ CUtensorMap tm_c, const __grid_c
 
 // Adds up the splits of one (head, row).
 __global__ void __launch_bounds__(128)
-latent_merge_kernel(const float *__restrict__ part_o, const float *__restrict__ part_ml, int splits, int heads, int rank_p,
+latent_merge_kernel(Fresh<float> part_o, Fresh<float2> part_ml, int splits, int heads, int rank_p,
                     __nv_bfloat16 *__restrict__ out) {
     pdl_trigger();
     pdl_wait();
     const size_t unit = (size_t)blockIdx.y * heads + blockIdx.x, stride = (size_t)gridDim.y * heads;
     float m = NEG_BIG;
-    for (int s = 0; s < splits; ++s) m = fmaxf(m, __ldcg(part_ml + (s * stride + unit) * 2));
+    for (int s = 0; s < splits; ++s) m = fmaxf(m, part_ml[s * stride + unit].x);
     float total = 0.0f;
     for (int s = 0; s < splits; ++s) {
-        const float2 ml = __ldcg(reinterpret_cast<const float2 *>(part_ml) + s * stride + unit);
+        const float2 ml = part_ml[s * stride + unit];
         total += ml.y * tc::ex2_approx(ml.x - m);
     }
     const float inv = 1.0f / total;
     for (int c = threadIdx.x * 4; c < rank_p; c += 512) {
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int s = 0; s < splits; ++s) {
-            const float2 ml = __ldcg(reinterpret_cast<const float2 *>(part_ml) + s * stride + unit);
+            const float2 ml = part_ml[s * stride + unit];
             if (ml.y == 0.0f) continue; // a split without keys left nothing
             const float f = tc::ex2_approx(ml.x - m) * inv;
-            const float4 o = __ldcg(reinterpret_cast<const float4 *>(part_o + (s * stride + unit) * rank_p + c));
+            const float4 o = part_o.four((s * stride + unit) * rank_p + c);
             acc.x = fmaf(f, o.x, acc.x); acc.y = fmaf(f, o.y, acc.y); acc.z = fmaf(f, o.z, acc.z); acc.w = fmaf(f, o.w, acc.w);
         }
         *reinterpret_cast<uint2 *>(out + unit * rank_p + c) = make_uint2(pack_bf16x2(acc.x, acc.y), pack_bf16x2(acc.z, acc.w));
@@ -429,7 +429,7 @@ int launch_latent_decode_tc(b200nn_ctx *ctx, const LatentDims &d, const __nv_bfl
     TRY(n == 16 ? launch_n<16>(ctx, a, tcm, tr, tql, tqr, n_rows, smem) : launch_n<32>(ctx, a, tcm, tr, tql, tqr, n_rows, smem));
     if (a.splits > 1) {
         PREFER_SMEM_ONCE(latent_merge_kernel);
-        CK(ctx, launch_pdl(ctx, latent_merge_kernel, dim3(d.heads, n_rows), dim3(128), 0, a.part_o, a.part_ml, a.splits, d.heads, d.rank_p, out));
+        CK(ctx, launch_pdl(ctx, latent_merge_kernel, dim3(d.heads, n_rows), dim3(128), 0, a.part_o, (const float2 *)a.part_ml, a.splits, d.heads, d.rank_p, out));
         CK_LAUNCH(ctx, "latent_merge_kernel");
     }
     return B200NN_OK;

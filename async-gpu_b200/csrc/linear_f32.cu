@@ -26,7 +26,7 @@ bool f32_gemv_fits(const F32Weight &w) { return (size_t)F32_GEMV_ROWS * w.K * si
 // a reduction through memory, 24.7 ms with this.
 template <int MT, int VEC, typename XT>
 __global__ void __launch_bounds__(FGEMV_THREADS)
-f32_gemv_kernel(const float *__restrict__ w, int ldw, const XT *__restrict__ x, int m_valid, int m0, int K, int N, int k_per_split,
+f32_gemv_kernel(const float *__restrict__ w, int ldw, Fresh<XT> x, int m_valid, int m0, int K, int N, int k_per_split,
                 NormIn ln, Epilogue epi) {
     constexpr int LANES = FGEMV_COLS / VEC;             // lanes across a row of the tile
     constexpr int SLICES = FGEMV_THREADS / LANES, WARPS = FGEMV_THREADS / 32;

@@ -28,7 +28,7 @@ __device__ __forceinline__ float gate_f(float v) { return __fdividef(1.0f, 1.0f 
 // chunk.  Under the state's loads the threads fetch q, k, v, the gates and their entry of the normaliser.
 template <int RPW, typename T>
 __global__ void __launch_bounds__(256, RPW <= 16 ? 2 : 1)
-mlstm_step_kernel(MlstmDims d, const float *__restrict__ proj, int ldp, MlstmWeights w, MlstmState state, RowMap rows, T *__restrict__ out) {
+mlstm_step_kernel(MlstmDims d, Fresh<float> proj, int ldp, MlstmWeights w, MlstmState state, RowMap rows, T *__restrict__ out) {
     extern __shared__ __align__(16) float sh[]; // q, k [dim_p], v, o [vdim_p], reduction [8][128], scalars [16]
     const int h = blockIdx.x, row = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     float *sq = sh, *sk = sq + d.dim_p, *sv = sk + d.dim_p, *so = sv + d.vdim_p, *red = so + d.vdim_p, *sc = red + 1024;
@@ -43,24 +43,24 @@ mlstm_step_kernel(MlstmDims d, const float *__restrict__ proj, int ldp, MlstmWei
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
             const int i = warp + 8 * r;
-            st[r] = col && i < d.dim_p && pos > 0 ? *reinterpret_cast<const float4 *>(S + (size_t)i * d.vdim_p + c0 + lane * 4)
+            st[r] = col && i < d.dim_p && pos > 0 ? load_fresh4(S + (size_t)i * d.vdim_p + c0 + lane * 4)
                                                   : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     };
     load_chunk(0);
-    const float *p = proj + (size_t)row * ldp;
+    const Fresh<float> p = proj + (size_t)row * ldp;
     float ni = 0.0f, qi = 0.0f, ki = 0.0f; // this thread's entry of the normaliser (dim <= 256)
     if (tid < d.dim_p) {
         qi = p[d.q_at() + h * d.dim_p + tid] / sqrtf((float)d.dim);
         ki = p[d.k_at() + h * d.dim_p + tid];
-        if (pos > 0) ni = state.normaliser[unit * d.dim_p + tid];
+        if (pos > 0) ni = load_fresh(state.normaliser, unit * d.dim_p + tid);
         sq[tid] = qi;
         sk[tid] = ki;
     }
     for (int j = tid; j < d.vdim_p; j += 256) sv[j] = p[d.v_at() + h * d.vdim_p + j];
     if (tid == 255) {
         const float i = soft_cap(p[d.i_at() + h] + w.i_bias[h], d.cap), f = log_sigmoid_f(soft_cap(p[d.f_at() + h] + w.f_bias[h], d.cap));
-        const float m0 = pos > 0 ? state.maximum[unit] : 0.0f, m = fmaxf(f + m0, i);
+        const float m0 = pos > 0 ? load_fresh(state.maximum, unit) : 0.0f, m = fmaxf(f + m0, i);
         state.maximum[unit] = m;
         sc[0] = expf(f + m0 - m);
         sc[1] = expf(i - m);
@@ -124,7 +124,7 @@ mlstm_step_kernel(MlstmDims d, const float *__restrict__ proj, int ldp, MlstmWei
 // tokens makes the segments' maps, the second starts from the maximum that enters its segment.  gates [row][head]: keep
 // e^(f + m - m'), write e^(i - m'), floor e^(-m'), and room for n . q.
 __global__ void __launch_bounds__(256)
-mlstm_gate_kernel(MlstmDims d, const float *__restrict__ proj, int ldp, MlstmWeights w, MlstmState state, SeqMap sm, float4 *__restrict__ gates) {
+mlstm_gate_kernel(MlstmDims d, Fresh<float> proj, int ldp, MlstmWeights w, MlstmState state, SeqMap sm, float4 *__restrict__ gates) {
     __shared__ float2 seg[8];
     const int h = blockIdx.x, sidx = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     pdl_trigger();
@@ -132,12 +132,13 @@ mlstm_gate_kernel(MlstmDims d, const float *__restrict__ proj, int ldp, MlstmWei
     pdl_wait();
     const int n = sm.n[sidx], row0 = sm.row0[sidx], per = (n + 255) / 256 * 32, t_beg = warp * per, t_end = min(n, t_beg + per);
     float *mp = state.maximum + (size_t)sm.slot[sidx] * d.heads + h;
-    float m = sm.past[sidx] > 0 ? *mp : 0.0f;
+    float m = sm.past[sidx] > 0 ? load_fresh(mp, 0) : 0.0f;
     float i = 0.0f, f = 0.0f, a, b;
     auto scan = [&](int t) { // the lane's gates and the map from the group's start through its token; past the end the map is the identity
-        const float *p = proj + (size_t)(row0 + min(t, n - 1)) * ldp;
-        i = soft_cap(p[d.i_at() + h] + ib, d.cap);
-        f = log_sigmoid_f(soft_cap(p[d.f_at() + h] + fb, d.cap));
+        const Fresh<float> p = proj + (size_t)(row0 + min(t, n - 1)) * ldp;
+        const float pi = p[d.i_at() + h], pf = p[d.f_at() + h];
+        i = soft_cap(pi + ib, d.cap);
+        f = log_sigmoid_f(soft_cap(pf + fb, d.cap));
         a = t < t_end ? f : 0.0f;
         b = t < t_end ? i : -INFINITY;
 #pragma unroll
@@ -195,7 +196,6 @@ mlstm_scan_kernel(MlstmDims d, const float *__restrict__ proj, int ldp, MlstmSta
     for (int i = tid; i < (int)(2 * sizeof(Stage) / 4); i += 128) reinterpret_cast<float *>(smem_raw)[i] = 0.0f; // entries past dim stay zero
     __syncthreads();
     if (norm && tid < 2 * TOK) stages[tid / TOK].v[tid % TOK][0] = 1.0f;
-    pdl_wait();
     const int n = sm.n[sidx], past = sm.past[sidx], slot = sm.slot[sidx], row0 = sm.row0[sidx];
     const size_t unit = (size_t)slot * d.heads + h;
     float *S = norm ? state.normaliser + unit * d.dim_p : state.memory + unit * d.dim_p * d.vdim_p;
@@ -327,14 +327,14 @@ mlstm_scan_kernel(MlstmDims d, const float *__restrict__ proj, int ldp, MlstmSta
 // One warp per (row, head).
 template <typename T>
 __global__ void __launch_bounds__(256)
-mlstm_out_kernel(MlstmDims d, const float *__restrict__ proj, int ldp, const float *__restrict__ norm, const float4 *__restrict__ gates,
-                 const float *__restrict__ heads_out, int n_rows, T *__restrict__ out) {
+mlstm_out_kernel(MlstmDims d, Fresh<float> proj, int ldp, const float *__restrict__ norm, Fresh<float4> gates,
+                 Fresh<float> heads_out, int n_rows, T *__restrict__ out) {
     pdl_trigger();
     pdl_wait();
     const int unit = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (unit >= n_rows * d.heads) return;
     const int row = unit / d.heads, h = unit - row * d.heads;
-    const float *o = heads_out + (size_t)unit * d.vdim_p, *g = proj + (size_t)row * ldp + d.g_at() + h * d.vdim_p;
+    const Fresh<float> o = heads_out + (size_t)unit * d.vdim_p, g = proj + ((size_t)row * ldp + d.g_at() + h * d.vdim_p);
     const float4 gt = gates[unit];
     const float inv = 1.0f / (fmaxf(fabsf(gt.w), gt.z) + 1e-6f);
     float4 v[2]; // the first 256 columns stay in registers
@@ -342,11 +342,14 @@ mlstm_out_kernel(MlstmDims d, const float *__restrict__ proj, int ldp, const flo
 #pragma unroll
     for (int c = 0; c < 2; ++c) { // columns past vdim hold zeros
         const int j = lane * 4 + 128 * c;
-        v[c] = j < d.vdim_p ? __ldcs(reinterpret_cast<const float4 *>(o + j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[c] = j < d.vdim_p ? o.four(j) : make_float4(0.f, 0.f, 0.f, 0.f);
         v[c].x *= inv; v[c].y *= inv; v[c].z *= inv; v[c].w *= inv;
         s += (v[c].x * v[c].x + v[c].y * v[c].y) + (v[c].z * v[c].z + v[c].w * v[c].w);
     }
-    for (int j = 256 + lane; j < d.vdim_p; j += 32) s = fmaf(o[j] * inv, o[j] * inv, s);
+    for (int j = 256 + lane; j < d.vdim_p; j += 32) {
+        const float t = o[j] * inv;
+        s = fmaf(t, t, s);
+    }
     const float rn = 1.0f / sqrtf(warp_sum(s) / (float)d.vdim + d.eps);
     const float *nw = norm + h * d.vdim_p; // zero past vdim
     T *y = out + (size_t)unit * d.vdim_p;
@@ -354,7 +357,7 @@ mlstm_out_kernel(MlstmDims d, const float *__restrict__ proj, int ldp, const flo
     for (int c = 0; c < 2; ++c) {
         const int j = lane * 4 + 128 * c;
         if (j >= d.vdim_p) continue;
-        const float4 gg = __ldcs(reinterpret_cast<const float4 *>(g + j)), ww = __ldg(reinterpret_cast<const float4 *>(nw + j));
+        const float4 gg = g.four(j), ww = __ldg(reinterpret_cast<const float4 *>(nw + j));
         store_from_float(y + j, v[c].x * rn * ww.x * gate_f(gg.x));
         store_from_float(y + j + 1, v[c].y * rn * ww.y * gate_f(gg.y));
         store_from_float(y + j + 2, v[c].z * rn * ww.z * gate_f(gg.z));
@@ -413,8 +416,8 @@ int launch_mlstm_prompt(b200nn_ctx *ctx, const MlstmDims &d, bool b16, const flo
             prefer_max_smem(mlstm_scan_kernel<M, C>);                                                                         \
             done[ctx->device & 15] = true;                                                                                    \
         }                                                                                                                     \
-        CK(ctx, launch_pdl(ctx, mlstm_scan_kernel<M, C>, dim3((d.vdim_p + 16 * C - 1) / (16 * C) + 1, d.heads, sm.n_seq),     \
-                           dim3(128), smem, d, proj, ldp, st, sm, (float4 *)gates, heads_out));                               \
+        CK(ctx, launch_ordered(ctx, mlstm_scan_kernel<M, C>, dim3((d.vdim_p + 16 * C - 1) / (16 * C) + 1, d.heads, sm.n_seq), \
+                               dim3(128), smem, d, proj, ldp, st, sm, (float4 *)gates, heads_out));                               \
     } while (0)
 #define MSCAN_C(M)                                                                                                            \
     do {                                                                                                                      \

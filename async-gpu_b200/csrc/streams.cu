@@ -18,6 +18,11 @@ __device__ __forceinline__ void load_cols(const float *p, float (&f)[V]) {
     *reinterpret_cast<typename Vec<V>::type *>(f) = *reinterpret_cast<const typename Vec<V>::type *>(p);
 }
 template <int V>
+__device__ __forceinline__ void load_cols(Fresh<float> p, float (&f)[V]) {
+    if constexpr (V == 4) *reinterpret_cast<float4 *>(f) = p.four(0);
+    else f[0] = p[0];
+}
+template <int V>
 __device__ __forceinline__ void store_cols(float *p, const float (&f)[V]) {
     *reinterpret_cast<typename Vec<V>::type *>(p) = *reinterpret_cast<const typename Vec<V>::type *>(f);
 }
@@ -25,7 +30,7 @@ __device__ __forceinline__ void store_cols(float *p, const float (&f)[V]) {
 // S: streams at most; V: columns per access; NV: accesses per thread; NT: threads
 template <int S, int V, int NV, int NT, typename T>
 __global__ void __launch_bounds__(NT)
-stream_step_kernel(int n, int d, float *__restrict__ xs, const float *__restrict__ x0, const float *__restrict__ y, StreamCoef prev, StreamCoef next,
+stream_step_kernel(int n, int d, float *xs, Fresh<float> x0, Fresh<float> y, StreamCoef prev, StreamCoef next,
                    const float *__restrict__ norm, float eps, int ldo, T *__restrict__ out, float *__restrict__ x_sum) {
     __shared__ float red[32];
     const int row = blockIdx.x, tid = threadIdx.x;
@@ -51,10 +56,10 @@ stream_step_kernel(int n, int d, float *__restrict__ xs, const float *__restrict
         float o[S][V];
         if (y) {
             float x[S][V], yy[V];
-            load_cols<V>(y + (size_t)row * d + c, yy);
+            load_cols<V>(y + ((size_t)row * d + c), yy);
 #pragma unroll
             for (int s = 0; s < S; ++s)
-                if (s < n) load_cols<V>(xr + (size_t)s * d + c, x[s]);
+                if (s < n) load_cols<V>(Fresh<float>(xr + (size_t)s * d + c), x[s]);
                 else
 #pragma unroll
                     for (int e = 0; e < V; ++e) x[s][e] = 0.0f;
@@ -69,7 +74,7 @@ stream_step_kernel(int n, int d, float *__restrict__ xs, const float *__restrict
                 }
         } else {
             float x[V];
-            load_cols<V>(x0 + (size_t)row * d + c, x);
+            load_cols<V>(x0 + ((size_t)row * d + c), x);
 #pragma unroll
             for (int t = 0; t < S; ++t)
 #pragma unroll

@@ -8,6 +8,8 @@ import pytest
 
 import b200nn
 import np_ref
+import test_gpu_vivezen as vivezen
+import test_gpu_zufilorn as zufilorn
 from b200nn import Gpt2Config, Gpt2Model, GpuTensor, Int4Gpt2Model, Int4Linear, Linear, TransformerBlock, ops, synth
 from oracle import oracle
 from test_gpu_block import _slices
@@ -80,6 +82,22 @@ def test_rows_after_rows(reg):
         got = blk.forward_cached(GpuTensor.from_host(x[past:], (n, d), reg), k0, v0, past)[0].to_host()
         for i in range(n):
             assert np_ref.rel_rms(got[i], ref[past + i]) < 1e-3, (turn, n, i)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("family", [vivezen, zufilorn])
+def test_rows_after_rows_of_hybrid_models(reg, family, dtype):
+    """The same of the hybrid decoders: steps of one to four requests' single tokens, with that family's tolerances."""
+    reqs = {k: family.tokens("small", 40 + k, k) for k in range(4)}
+    rb = b200nn.RequestBatch(family.model(reg, "small", dtype), 4, 64)
+    got = {k: list(rb.step([(k, t[:10 + k], range(10 + k))])) for k, t in reqs.items()}
+    for turn in range(24):
+        live = [(turn + j) % 4 for j in range((1, 2, 3, 4, 4, 3, 4, 1)[turn % 8])]
+        for k, row in zip(live, rb.step([(k, [reqs[k][len(got[k])]], [0]) for k in live])):
+            got[k].append(row)
+    for k, rows in got.items():
+        ref = family.reference("small", reqs[k][:len(rows)])
+        family.check(np.stack(rows), ref, family.TOL[dtype] if family is vivezen else dtype, f"request {k}")
 
 
 @pytest.mark.parametrize("int4", [False, True])
