@@ -339,7 +339,6 @@ bool int4_gemm_tc_supported(const Int4Weight &w, int M);
 int launch_int4_gemm_tc(b200nn_ctx *ctx, const Int4Weight &w, const __half *x, int M, const Epilogue &epi);
 int launch_f32_linear(b200nn_ctx *ctx, const F32Weight &w, const void *x, bool x_half, int M, const Epilogue &epi, const NormIn &ln = NormIn());
 bool f32_linear_takes_norm(const F32Weight &w, int M);
-bool f32_gemv_fits(const F32Weight &w); // the GEMV's shared memory holds this K
 bool f16_gemm_tc_supported(const b200nn_ctx *ctx, const F32Weight &w, int M);
 int launch_f16_gemm_tc(b200nn_ctx *ctx, const F32Weight &w, const __half *x, int M, const Epilogue &epi);
 // x: bf16 [M, ldx] (ldx >= the activation columns the weight reads, a multiple of 8)

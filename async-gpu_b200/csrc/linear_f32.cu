@@ -11,9 +11,7 @@
 static constexpr int FGEMV_THREADS = 256;
 static constexpr int FGEMV_COLS = 32;          // columns per block: one 128-byte line of every weight row
 static constexpr int FGEMV_AHEAD = 12;         // weight loads a thread has in flight
-static constexpr size_t FGEMV_XS = 160 * 1024; // bytes of activations a block holds at most
-
-bool f32_gemv_fits(const F32Weight &w) { return (size_t)F32_GEMV_ROWS * w.K * sizeof(float) <= 8 * FGEMV_XS; }
+static constexpr size_t FGEMV_XS = 160 * 1024; // bytes of activations a block holds at a time
 
 // grid (column tiles, splits), cluster (1, splits, 1).  A decode step of one sequence is bound by the weights'
 // bytes and by the hand-over from kernel to kernel, so: the block's tile is narrow and its K range short enough that
@@ -22,21 +20,23 @@ bool f32_gemv_fits(const F32Weight &w) { return (size_t)F32_GEMV_ROWS * w.K * si
 // The partial sums of a cluster are stored into its first block's shared memory, one barrier, no scratch in memory.
 // With `ln.g` the activations are the LayerNorm of the f32 rows x: every block takes the statistics of the whole
 // row itself, which saves a kernel between two Linears (norm_rows_to_smem).
+// PIECES: K ranges whose activations exceed x_rows rows (whole trips of the loop) are staged piece by piece.  One row,
+// 100000 x 64: 11 ms on the tiled kernel, which has one block per 64 columns, 28 us here.
 // GPT-2 Small, one sequence, 64 tokens after a prompt of 64: 52.5 ms with 4-byte loads, four in flight, plain launches and
 // a reduction through memory, 24.7 ms with this.
-template <int MT, int VEC, typename XT>
+template <int MT, int VEC, bool PIECES, typename XT>
 __global__ void __launch_bounds__(FGEMV_THREADS)
-f32_gemv_kernel(const float *__restrict__ w, int ldw, Fresh<XT> x, int m_valid, int m0, int K, int N, int k_per_split,
+f32_gemv_kernel(const float *__restrict__ w, int ldw, Fresh<XT> x, int m_valid, int m0, int K, int N, int k_per_split, int x_rows,
                 NormIn ln, Epilogue epi) {
     constexpr int LANES = FGEMV_COLS / VEC;             // lanes across a row of the tile
-    constexpr int SLICES = FGEMV_THREADS / LANES, WARPS = FGEMV_THREADS / 32;
+    constexpr int SLICES = FGEMV_THREADS / LANES, WARPS = FGEMV_THREADS / 32, TRIP = FGEMV_AHEAD * SLICES;
     extern __shared__ float smem_f[];
     const int split = blockIdx.y, splits = gridDim.y;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int slice = tid / LANES, c = (tid % LANES) * VEC, n_base = blockIdx.x * FGEMV_COLS;
     const int k0 = split * k_per_split, rows = min(k_per_split, K - k0);
-    float *xs = smem_f;                                 // [MT][k_per_split] activations of this block's K range
-    float *red = xs + MT * k_per_split;                 // [WARPS][MT][32]
+    float *xs = smem_f;                                 // [MT][x_rows] activations of this block's K range
+    float *red = xs + MT * x_rows;                      // [WARPS][MT][32]
     float *part = red + WARPS * MT * FGEMV_COLS;        // [splits][MT][32] in the cluster's first block
     pdl_trigger();
     if (splits > 1) cluster_arrive(); // waited for before the first store into another block
@@ -60,11 +60,11 @@ f32_gemv_kernel(const float *__restrict__ w, int ldw, Fresh<XT> x, int m_valid, 
         load(buf[j], j * SLICES);
     }
     if constexpr (sizeof(XT) == 4) {
-        if (ln.g) norm_rows_to_smem<MT, FGEMV_THREADS>(ln, x, m_valid, K, k0, rows, k_per_split, xs, red);
+        if (ln.g) norm_rows_to_smem<MT, FGEMV_THREADS>(ln, x, m_valid, K, k0, rows, x_rows, xs, red);
     }
     if (sizeof(XT) != 4 || !ln.g) {
         pdl_wait();
-        rows_to_smem<MT, FGEMV_THREADS>(x, m_valid, K, k0, rows, k_per_split, xs);
+        rows_to_smem<MT, FGEMV_THREADS>(x, m_valid, K, k0, PIECES ? min(rows, x_rows) : rows, x_rows, xs);
     }
     __syncthreads();
 
@@ -73,19 +73,26 @@ f32_gemv_kernel(const float *__restrict__ w, int ldw, Fresh<XT> x, int m_valid, 
     for (int m = 0; m < MT; ++m)
 #pragma unroll
         for (int i = 0; i < VEC; ++i) acc[m][i] = 0.0f;
-    for (int r0 = 0; r0 < rows; r0 += FGEMV_AHEAD * SLICES) {
+    int piece = 0; // first row of the range in xs
+    for (int r0 = 0; r0 < rows; r0 += TRIP) {
+        if (PIECES && r0 == piece + x_rows) {
+            piece = r0;
+            __syncthreads();
+            rows_to_smem<MT, FGEMV_THREADS>(x, m_valid, K, k0 + r0, min(rows - r0, x_rows), x_rows, xs);
+            __syncthreads();
+        }
 #pragma unroll
         for (int j = 0; j < FGEMV_AHEAD; ++j) {
             const int r = r0 + j * SLICES;
             if (slice + r < rows) {
 #pragma unroll
                 for (int m = 0; m < MT; ++m) {
-                    const float xv = xs[m * k_per_split + slice + r];
+                    const float xv = xs[m * x_rows + slice + r - piece];
 #pragma unroll
                     for (int i = 0; i < VEC; ++i) acc[m][i] = fmaf(xv, buf[j][i], acc[m][i]);
                 }
             }
-            load(buf[j], r + FGEMV_AHEAD * SLICES);
+            load(buf[j], r + TRIP);
         }
     }
     // the four K slices of a warp by shuffles, the warps through shared memory, the blocks of the cluster in its first
@@ -175,18 +182,12 @@ f32_gemm_kernel(const float *__restrict__ w, int ldw, const XT *__restrict__ x, 
     }
 }
 
-template <int MT, int VEC, typename XT>
-static int f32_gemv_launch(b200nn_ctx *ctx, const F32Weight &w, const XT *x, int m_valid, int m0, const NormIn &ln, const Epilogue &epi) {
-    // K split over a cluster until there is about a block per SM (GPT-2 Small, 64 tokens after a prompt of 64: 24.7 ms; two
-    // blocks per SM 27.0, three 27.6), none of under 64 rows unless the activations need it
+template <int MT, int VEC, bool PIECES, typename XT>
+static int f32_gemv_launch(b200nn_ctx *ctx, const F32Weight &w, const XT *x, int m_valid, int m0, int splits, int per, int x_rows, const NormIn &ln,
+                           const Epilogue &epi) {
     const int tiles = (w.N + FGEMV_COLS - 1) / FGEMV_COLS;
-    int splits = std::min(8, std::max(1, ctx->sm_count / tiles));
-    splits = std::min(splits, std::max(1, w.K / 64));
-    splits = std::max(splits, (int)(((size_t)MT * w.K * sizeof(float) + FGEMV_XS - 1) / FGEMV_XS));
-    const int per = (w.K + splits - 1) / splits;
-    splits = (w.K + per - 1) / per;
-    auto kern = f32_gemv_kernel<MT, VEC, XT>;
-    const size_t smem = ((size_t)MT * per + (size_t)(FGEMV_THREADS / 32 + splits) * MT * FGEMV_COLS) * sizeof(float);
+    auto kern = f32_gemv_kernel<MT, VEC, PIECES, XT>;
+    const size_t smem = ((size_t)MT * x_rows + (size_t)(FGEMV_THREADS / 32 + splits) * MT * FGEMV_COLS) * sizeof(float);
     static bool attr_done[16] = {}; // function attributes are per device
     if (!attr_done[ctx->device & 15]) {
         CK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -207,21 +208,33 @@ static int f32_gemv_launch(b200nn_ctx *ctx, const F32Weight &w, const XT *x, int
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = ctx->pdl && !w.volatile_w ? 2 : 1;
-    CK(ctx, cudaLaunchKernelEx(&cfg, kern, (const float *)w.w_kn->p, w.ld(), x, m_valid, m0, w.K, w.N, per, ln, epi));
+    CK(ctx, cudaLaunchKernelEx(&cfg, kern, (const float *)w.w_kn->p, w.ld(), x, m_valid, m0, w.K, w.N, per, x_rows, ln, epi));
     CK_LAUNCH(ctx, "f32_gemv_kernel");
     return B200NN_OK;
+}
+template <int MT, int VEC, typename XT>
+static int f32_gemv_plan(b200nn_ctx *ctx, const F32Weight &w, const XT *x, int m_valid, int m0, const NormIn &ln, const Epilogue &epi) {
+    // K split over a cluster until there is about a block per SM (GPT-2 Small, 64 tokens after a prompt of 64: 24.7 ms; two
+    // blocks per SM 27.0, three 27.6), none of under 64 rows; activations of a longer range are staged in whole trips
+    constexpr int TRIP = FGEMV_AHEAD * FGEMV_THREADS * VEC / FGEMV_COLS, X_ROWS = (int)(FGEMV_XS / (MT * sizeof(float))) / TRIP * TRIP;
+    const int tiles = (w.N + FGEMV_COLS - 1) / FGEMV_COLS;
+    int splits = std::min(8, std::max(1, ctx->sm_count / tiles));
+    splits = std::min(splits, std::max(1, w.K / 64));
+    const int per = (w.K + splits - 1) / splits;
+    splits = (w.K + per - 1) / per;
+    if (per <= X_ROWS) return f32_gemv_launch<MT, VEC, false, XT>(ctx, w, x, m_valid, m0, splits, per, per, ln, epi);
+    return f32_gemv_launch<MT, VEC, true, XT>(ctx, w, x, m_valid, m0, splits, per, X_ROWS, ln, epi);
 }
 template <int MT, typename XT>
 static int f32_gemv_chunk(b200nn_ctx *ctx, const F32Weight &w, const XT *x, int m_valid, int m0, const NormIn &ln, const Epilogue &epi) {
     // rows of the weight that all start on 16 bytes: vector loads
-    if (w.ld() % 4 == 0 && !((uintptr_t)w.w_kn->p & 15)) return f32_gemv_launch<MT, 4, XT>(ctx, w, x, m_valid, m0, ln, epi);
-    return f32_gemv_launch<MT, 1, XT>(ctx, w, x, m_valid, m0, ln, epi);
+    if (w.ld() % 4 == 0 && !((uintptr_t)w.w_kn->p & 15)) return f32_gemv_plan<MT, 4, XT>(ctx, w, x, m_valid, m0, ln, epi);
+    return f32_gemv_plan<MT, 1, XT>(ctx, w, x, m_valid, m0, ln, epi);
 }
 
 template <typename XT>
 static int f32_linear_t(b200nn_ctx *ctx, const F32Weight &w, const XT *x, int M, const NormIn &ln, const Epilogue &epi) {
-    // a K range that a cluster's shared memory does not hold goes to the tiled kernel
-    if (M <= F32_GEMV_ROWS && f32_gemv_fits(w)) {
+    if (M <= F32_GEMV_ROWS) {
         if (M == 4) return f32_gemv_chunk<4, XT>(ctx, w, x, 4, 0, ln, epi);
         if (M >= 2) {
             TRY((f32_gemv_chunk<2, XT>(ctx, w, x, 2, 0, ln, epi)));

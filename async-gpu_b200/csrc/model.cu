@@ -373,7 +373,7 @@ int run_head(b200nn_gpt2 *m, Workspace &ws, const float *x, int rows, bool act_h
 // GEMV kernels of an int4 head in the tiled layout, and the GEMV and the fp16 tensor-core GEMM of an f32 head.
 static bool head_fuses_pick(const b200nn_gpt2 *m, int rows, bool head_half) {
     if (m->lm_head.int4) return m->lm_head.q.fast && rows < 2048;
-    return (rows <= F32_GEMV_ROWS && f32_gemv_fits(m->lm_head.f)) || (head_half && f16_gemm_tc_supported(m->ctx, m->lm_head.f, rows));
+    return rows <= F32_GEMV_ROWS || (head_half && f16_gemm_tc_supported(m->ctx, m->lm_head.f, rows));
 }
 
 int run_head_pick(b200nn_gpt2 *m, Workspace &ws, const float *x, int rows, bool act_half, bool keep_last, bool tokens_only,

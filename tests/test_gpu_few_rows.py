@@ -3,6 +3,8 @@ cluster, a LayerNorm taken along), the split-context decode attention (stages, s
 epilogues.  Each is compared with float64 of the same operands; sums of n f32 terms may differ from it by
 n * 2^-24 of the terms' magnitudes at most, and the bounds below are a fraction of that for the longest sum.
 """
+import time
+
 import numpy as np
 import pytest
 
@@ -24,7 +26,8 @@ def _close(got, ref, mag):
 
 
 @pytest.mark.parametrize("m", [1, 2, 3, 4])
-@pytest.mark.parametrize("k,n", [(1, 1), (63, 33), (64, 32), (65, 31), (768, 2304), (3072, 770), (20000, 40), (100, 50257)])
+# the last two: activations staged in pieces, with and without a K split
+@pytest.mark.parametrize("k,n", [(1, 1), (63, 33), (64, 32), (65, 31), (768, 2304), (3072, 770), (20000, 40), (100, 50257), (100000, 64), (10500, 2401)])
 def test_f32_linear_few_rows(reg, m, k, n):
     rng = np.random.default_rng(k * 7 + n + m)
     w, b, x = (rng.standard_normal(s).astype(np.float32) for s in ((n, k), (n,), (m, k)))
@@ -33,6 +36,31 @@ def test_f32_linear_few_rows(reg, m, k, n):
     # a matrix product takes the weight as it is: rows that need not start on 16 bytes
     got = ops.matmul(GpuTensor.from_host(x, (m, k), reg), GpuTensor.from_host(np.ascontiguousarray(w.T), (k, n), reg), reg).to_host()
     _close(got, ref - b, mag)
+
+
+def _seconds(reg, f, n=20):
+    """A call's time, the best of five rounds."""
+    f()
+    best = []
+    for _ in range(5):
+        reg.synchronize()
+        t = time.perf_counter()
+        for _ in range(n):
+            f()
+        reg.synchronize()
+        best.append((time.perf_counter() - t) / n)
+    return min(best)
+
+
+def _linear_seconds(reg, k, n, m):
+    layer = Linear(np.ones((n, k), np.float32), None, k, n, reg)
+    x = GpuTensor.from_host(np.ones((m, k), np.float32), (m, k), reg)
+    return _seconds(reg, lambda: layer.forward(x))
+
+
+def test_f32_linear_of_very_long_rows_keeps_its_pace(reg):
+    """1.7 times the bytes; on the tiled kernel the longer one took 400 times as long."""
+    assert _linear_seconds(reg, 100000, 64, 1) < 6 * _linear_seconds(reg, 60000, 64, 1)
 
 
 def _int4(rng, k, n, group):
