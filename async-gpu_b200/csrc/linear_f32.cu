@@ -9,7 +9,6 @@
 #include "device_utils.cuh"
 
 static constexpr int FGEMV_THREADS = 256;
-static constexpr int FGEMV_COLS = 32;          // columns per block: one 128-byte line of every weight row
 static constexpr int FGEMV_AHEAD = 12;         // weight loads a thread has in flight
 static constexpr size_t FGEMV_XS = 160 * 1024; // bytes of activations a block holds at a time
 
@@ -22,22 +21,25 @@ static constexpr size_t FGEMV_XS = 160 * 1024; // bytes of activations a block h
 // row itself, which saves a kernel between two Linears (norm_rows_to_smem).
 // PIECES: K ranges whose activations exceed x_rows rows (whole trips of the loop) are staged piece by piece.  One row,
 // 100000 x 64: 11 ms on the tiled kernel, which has one block per 64 columns, 28 us here.
+// COLS: 32 columns, one 128-byte line of every weight row, or 128 for a weight that would have more than three blocks per
+// SM that way (an output matrix), each paying for its start and its activations (768 x 50257 with one / four rows: 65 / 147 us
+// in 32 columns, 44 / 65 in 128; 100 x 50257: 21 / 40 and 14 / 15).  Those are never split over a cluster and take no LayerNorm.
 // GPT-2 Small, one sequence, 64 tokens after a prompt of 64: 52.5 ms with 4-byte loads, four in flight, plain launches and
 // a reduction through memory, 24.7 ms with this.
-template <int MT, int VEC, bool PIECES, typename XT>
+template <int MT, int VEC, int COLS, bool PIECES, typename XT>
 __global__ void __launch_bounds__(FGEMV_THREADS)
 f32_gemv_kernel(const float *__restrict__ w, int ldw, Fresh<XT> x, int m_valid, int m0, int K, int N, int k_per_split, int x_rows,
                 NormIn ln, Epilogue epi) {
-    constexpr int LANES = FGEMV_COLS / VEC;             // lanes across a row of the tile
+    constexpr int LANES = COLS / VEC;                   // lanes across a row of the tile
     constexpr int SLICES = FGEMV_THREADS / LANES, WARPS = FGEMV_THREADS / 32, TRIP = FGEMV_AHEAD * SLICES;
     extern __shared__ float smem_f[];
     const int split = blockIdx.y, splits = gridDim.y;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int slice = tid / LANES, c = (tid % LANES) * VEC, n_base = blockIdx.x * FGEMV_COLS;
+    const int slice = tid / LANES, c = (tid % LANES) * VEC, n_base = blockIdx.x * COLS;
     const int k0 = split * k_per_split, rows = min(k_per_split, K - k0);
     float *xs = smem_f;                                 // [MT][x_rows] activations of this block's K range
-    float *red = xs + MT * x_rows;                      // [WARPS][MT][32]
-    float *part = red + WARPS * MT * FGEMV_COLS;        // [splits][MT][32] in the cluster's first block
+    float *red = xs + MT * x_rows;                      // [WARPS][MT][COLS]
+    float *part = red + WARPS * MT * COLS;              // [splits][MT][COLS] in the cluster's first block
     pdl_trigger();
     if (splits > 1) cluster_arrive(); // waited for before the first store into another block
 
@@ -59,10 +61,10 @@ f32_gemv_kernel(const float *__restrict__ w, int ldw, Fresh<XT> x, int m_valid, 
         for (int i = 0; i < VEC; ++i) buf[j][i] = 0.0f;
         load(buf[j], j * SLICES);
     }
-    if constexpr (sizeof(XT) == 4) {
+    if constexpr (sizeof(XT) == 4 && COLS == 32) {
         if (ln.g) norm_rows_to_smem<MT, FGEMV_THREADS>(ln, x, m_valid, K, k0, rows, x_rows, xs, red);
     }
-    if (sizeof(XT) != 4 || !ln.g) {
+    if (sizeof(XT) != 4 || COLS != 32 || !ln.g) {
         pdl_wait();
         rows_to_smem<MT, FGEMV_THREADS>(x, m_valid, K, k0, PIECES ? min(rows, x_rows) : rows, x_rows, xs);
     }
@@ -96,7 +98,7 @@ f32_gemv_kernel(const float *__restrict__ w, int ldw, Fresh<XT> x, int m_valid, 
         }
     }
     // the four K slices of a warp by shuffles, the warps through shared memory, the blocks of the cluster in its first
-    if constexpr (VEC == 4) {
+    if constexpr (LANES == 8) {
 #pragma unroll
         for (int m = 0; m < MT; ++m)
 #pragma unroll
@@ -109,21 +111,33 @@ f32_gemv_kernel(const float *__restrict__ w, int ldw, Fresh<XT> x, int m_valid, 
 #pragma unroll
         for (int m = 0; m < MT; ++m)
 #pragma unroll
-            for (int i = 0; i < VEC; ++i) red[(warp * MT + m) * FGEMV_COLS + c + i] = acc[m][i];
+            for (int i = 0; i < VEC; ++i) red[(warp * MT + m) * COLS + c + i] = acc[m][i];
     __syncthreads();
+    if constexpr (COLS > 32) {
+        for (int o = tid; o < MT * COLS; o += FGEMV_THREADS) { // a warp: 32 consecutive features of a row
+            const int m = o / COLS, n = n_base + o % COLS;
+            if (m >= m_valid) break;
+            float t = 0.0f;
+#pragma unroll
+            for (int s = 0; s < WARPS; ++s) t += red[s * MT * COLS + o];
+            if (n < N) epi_apply(epi, m0 + m, n, t);
+            if (epi.amax_val) epi_argmax1(epi, m0 + m, n, t + (epi.bias && n < N ? epi.bias[n] : 0.0f), n < N);
+        }
+        return;
+    }
     float t = 0.0f;
     if (warp < MT)
 #pragma unroll
-        for (int s = 0; s < WARPS; ++s) t += red[(s * MT + warp) * FGEMV_COLS + lane];
+        for (int s = 0; s < WARPS; ++s) t += red[(s * MT + warp) * COLS + lane];
     if (splits > 1) {
         cluster_wait();
-        if (warp < MT) st_cluster(&part[(split * MT + warp) * FGEMV_COLS + lane], 0, t);
+        if (warp < MT) st_cluster(&part[(split * MT + warp) * COLS + lane], 0, t);
         cluster_arrive();
         cluster_wait(); // every block's sums are in the first block
         if (split != 0) return;
         t = 0.0f;
         if (warp < MT)
-            for (int sp = 0; sp < splits; ++sp) t += part[(sp * MT + warp) * FGEMV_COLS + lane];
+            for (int sp = 0; sp < splits; ++sp) t += part[(sp * MT + warp) * COLS + lane];
     }
     if (warp < min(MT, m_valid)) { // one warp per row: 32 consecutive features
         const int n = n_base + lane;
@@ -182,12 +196,12 @@ f32_gemm_kernel(const float *__restrict__ w, int ldw, const XT *__restrict__ x, 
     }
 }
 
-template <int MT, int VEC, bool PIECES, typename XT>
+template <int MT, int VEC, int COLS, bool PIECES, typename XT>
 static int f32_gemv_launch(b200nn_ctx *ctx, const F32Weight &w, const XT *x, int m_valid, int m0, int splits, int per, int x_rows, const NormIn &ln,
                            const Epilogue &epi) {
-    const int tiles = (w.N + FGEMV_COLS - 1) / FGEMV_COLS;
-    auto kern = f32_gemv_kernel<MT, VEC, PIECES, XT>;
-    const size_t smem = ((size_t)MT * x_rows + (size_t)(FGEMV_THREADS / 32 + splits) * MT * FGEMV_COLS) * sizeof(float);
+    const int tiles = (w.N + COLS - 1) / COLS;
+    auto kern = f32_gemv_kernel<MT, VEC, COLS, PIECES, XT>;
+    const size_t smem = ((size_t)MT * x_rows + (size_t)(FGEMV_THREADS / 32 + splits) * MT * COLS) * sizeof(float);
     static bool attr_done[16] = {}; // function attributes are per device
     if (!attr_done[ctx->device & 15]) {
         CK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -212,24 +226,26 @@ static int f32_gemv_launch(b200nn_ctx *ctx, const F32Weight &w, const XT *x, int
     CK_LAUNCH(ctx, "f32_gemv_kernel");
     return B200NN_OK;
 }
-template <int MT, int VEC, typename XT>
+template <int MT, int VEC, int COLS, typename XT>
 static int f32_gemv_plan(b200nn_ctx *ctx, const F32Weight &w, const XT *x, int m_valid, int m0, const NormIn &ln, const Epilogue &epi) {
     // K split over a cluster until there is about a block per SM (GPT-2 Small, 64 tokens after a prompt of 64: 24.7 ms; two
     // blocks per SM 27.0, three 27.6), none of under 64 rows; activations of a longer range are staged in whole trips
-    constexpr int TRIP = FGEMV_AHEAD * FGEMV_THREADS * VEC / FGEMV_COLS, X_ROWS = (int)(FGEMV_XS / (MT * sizeof(float))) / TRIP * TRIP;
-    const int tiles = (w.N + FGEMV_COLS - 1) / FGEMV_COLS;
-    int splits = std::min(8, std::max(1, ctx->sm_count / tiles));
+    constexpr int TRIP = FGEMV_AHEAD * FGEMV_THREADS * VEC / COLS, X_ROWS = (int)(FGEMV_XS / (MT * sizeof(float))) / TRIP * TRIP;
+    const int tiles = (w.N + COLS - 1) / COLS;
+    int splits = COLS > 32 ? 1 : std::min(8, std::max(1, ctx->sm_count / tiles));
     splits = std::min(splits, std::max(1, w.K / 64));
     const int per = (w.K + splits - 1) / splits;
     splits = (w.K + per - 1) / per;
-    if (per <= X_ROWS) return f32_gemv_launch<MT, VEC, false, XT>(ctx, w, x, m_valid, m0, splits, per, per, ln, epi);
-    return f32_gemv_launch<MT, VEC, true, XT>(ctx, w, x, m_valid, m0, splits, per, X_ROWS, ln, epi);
+    if (per <= X_ROWS) return f32_gemv_launch<MT, VEC, COLS, false, XT>(ctx, w, x, m_valid, m0, splits, per, per, ln, epi);
+    return f32_gemv_launch<MT, VEC, COLS, true, XT>(ctx, w, x, m_valid, m0, splits, per, X_ROWS, ln, epi);
 }
 template <int MT, typename XT>
 static int f32_gemv_chunk(b200nn_ctx *ctx, const F32Weight &w, const XT *x, int m_valid, int m0, const NormIn &ln, const Epilogue &epi) {
     // rows of the weight that all start on 16 bytes: vector loads
-    if (w.ld() % 4 == 0 && !((uintptr_t)w.w_kn->p & 15)) return f32_gemv_plan<MT, 4, XT>(ctx, w, x, m_valid, m0, ln, epi);
-    return f32_gemv_plan<MT, 1, XT>(ctx, w, x, m_valid, m0, ln, epi);
+    if (w.ld() % 4 == 0 && !((uintptr_t)w.w_kn->p & 15))
+        return !ln.g && w.N > 3 * 32 * ctx->sm_count ? f32_gemv_plan<MT, 4, 128, XT>(ctx, w, x, m_valid, m0, ln, epi)
+                                                     : f32_gemv_plan<MT, 4, 32, XT>(ctx, w, x, m_valid, m0, ln, epi);
+    return f32_gemv_plan<MT, 1, 32, XT>(ctx, w, x, m_valid, m0, ln, epi);
 }
 
 template <typename XT>

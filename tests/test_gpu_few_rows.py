@@ -26,8 +26,10 @@ def _close(got, ref, mag):
 
 
 @pytest.mark.parametrize("m", [1, 2, 3, 4])
-# the last two: activations staged in pieces, with and without a K split
-@pytest.mark.parametrize("k,n", [(1, 1), (63, 33), (64, 32), (65, 31), (768, 2304), (3072, 770), (20000, 40), (100, 50257), (100000, 64), (10500, 2401)])
+# activations staged in pieces, with and without a K split; the last weight of 32-column tiles and the first of 128-column ones
+# (148 SMs)
+@pytest.mark.parametrize("k,n", [(1, 1), (63, 33), (64, 32), (65, 31), (768, 2304), (3072, 770), (20000, 40), (100, 50257), (100000, 64), (10500, 2401),
+                                 (97, 14208), (97, 14209), (1, 14336), (800, 14401)])
 def test_f32_linear_few_rows(reg, m, k, n):
     rng = np.random.default_rng(k * 7 + n + m)
     w, b, x = (rng.standard_normal(s).astype(np.float32) for s in ((n, k), (n,), (m, k)))
@@ -61,6 +63,24 @@ def _linear_seconds(reg, k, n, m):
 def test_f32_linear_of_very_long_rows_keeps_its_pace(reg):
     """1.7 times the bytes; on the tiled kernel the longer one took 400 times as long."""
     assert _linear_seconds(reg, 100000, 64, 1) < 6 * _linear_seconds(reg, 60000, 64, 1)
+
+
+def test_f32_linear_of_long_rows_and_many_columns(reg):
+    """Wide tiles whose activations are staged in pieces."""
+    import torch
+
+    k, n, m = 10300, 14212, 4
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    w, x = torch.randn(n, k, generator=g, device="cuda"), torch.randn(m, k, generator=g, device="cuda")
+    ref, mag = x.double() @ w.double().T, x.abs().double() @ w.abs().double().T
+    got = Linear(w.cpu().numpy(), None, k, n, reg).forward(GpuTensor.from_host(x.cpu().numpy(), (m, k), reg)).to_host()
+    _close(got, ref.cpu().numpy(), mag.cpu().numpy())
+
+
+def test_f32_output_matrix_of_four_rows_keeps_its_pace(reg):
+    """The weight's bytes bound it: four rows took 2.3 times as long as one while a block per SM was all their registers left."""
+    assert _linear_seconds(reg, 768, 50257, 4) < 1.9 * _linear_seconds(reg, 768, 50257, 1)
 
 
 def _int4(rng, k, n, group):
@@ -132,7 +152,7 @@ def test_rows_after_rows_of_hybrid_models(reg, family, dtype):
 def test_greedy_pick_of_a_vocabulary_between_tiles(reg, int4):
     """The pick of one row reads the entries of whole 32-feature groups only: a model of 256 tokens with large logits has left
     its entries in the buffers that a model of 130 then uses."""
-    for vocab, scale in ((256, 50.0), (130, 1.0), (256, 50.0), (97, 1.0)):
+    for vocab, scale in ((256, 50.0), (130, 1.0), (256, 50.0), (97, 1.0), (14300, 1.0)):
         cfg = Gpt2Config(n_layer=1, n_embd=64, n_head=1, vocab_size=vocab, n_positions=16)
         w = synth.gpt2_weights(cfg, base_seed=vocab, std=0.02)
         w["wte"] = w["wte"] * scale
