@@ -572,18 +572,31 @@ __device__ __forceinline__ void st_cluster(float *p, int rank, float v) {
 // to xs [MT][ld] (zero past them and past m_valid).  Mean, then the mean square about it, as layernorm_kernel has it.
 // Contains the wait on the previous kernel, after the loads of scale and shift.  red: THREADS / 32 * MT floats; the
 // caller synchronises before it reads xs or reuses red.
-template <int MT, int THREADS>
+// held: null, or [MT + 2][K] floats of shared memory in which the threads keep their values, scale and shift between the
+// sums, for kernels whose registers are full of weights (each thread reads back what it wrote itself).
+template <int MT, int THREADS, bool HELD = false>
 __device__ __forceinline__ void norm_rows_to_smem(const NormIn &ln, Fresh<float> x, int m_valid, int K, int k0, int cols,
-                                                  int ld, float *xs, float *red) {
+                                                  int ld, float *xs, float *red, float *held = nullptr) {
     constexpr int VPT = NORM_IN_MAX / THREADS, WARPS = THREADS / 32;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    float g[VPT], b[VPT], v[MT][VPT], s[MT];
+    float regs[HELD ? 1 : MT + 2][HELD ? 1 : VPT], s[MT];
+    auto put = [&](int row, int i, float v) {
+        if constexpr (HELD) {
+            if (tid + i * THREADS < K) held[row * K + tid + i * THREADS] = v;
+        } else {
+            regs[row][i] = v;
+        }
+    };
+    auto get = [&](int row, int i) { // 0 past K
+        if constexpr (HELD) return tid + i * THREADS < K ? held[row * K + tid + i * THREADS] : 0.0f;
+        else return regs[row][i];
+    };
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
         const int k = tid + i * THREADS;
         const bool mine = k >= k0 && k < k0 + cols;
-        g[i] = mine ? __ldg(ln.g + k) : 0.0f;
-        b[i] = mine ? __ldg(ln.b + k) : 0.0f;
+        put(MT, i, mine ? __ldg(ln.g + k) : 0.0f);
+        put(MT + 1, i, mine ? __ldg(ln.b + k) : 0.0f);
     }
     pdl_wait();
     auto sums = [&]() { // s[m] over the block, divided by K
@@ -605,13 +618,17 @@ __device__ __forceinline__ void norm_rows_to_smem(const NormIn &ln, Fresh<float>
 #pragma unroll
     for (int m = 0; m < MT; ++m) {
         s[m] = 0.0f;
+        float v[VPT];
 #pragma unroll
         for (int i = 0; i < VPT; ++i) {
             const int k = tid + i * THREADS;
-            v[m][i] = m < m_valid && k < K ? x[(size_t)m * K + k] : 0.0f;
+            v[i] = m < m_valid && k < K ? x[(size_t)m * K + k] : 0.0f;
         }
 #pragma unroll
-        for (int i = 0; i < VPT; ++i) s[m] += v[m][i];
+        for (int i = 0; i < VPT; ++i) {
+            put(m, i, v[i]);
+            s[m] += v[i];
+        }
     }
     sums();
     float mean[MT];
@@ -621,7 +638,7 @@ __device__ __forceinline__ void norm_rows_to_smem(const NormIn &ln, Fresh<float>
         s[m] = 0.0f;
 #pragma unroll
         for (int i = 0; i < VPT; ++i) {
-            const float t = tid + i * THREADS < K ? v[m][i] - mean[m] : 0.0f;
+            const float t = tid + i * THREADS < K ? get(m, i) - mean[m] : 0.0f;
             s[m] += t * t;
         }
     }
@@ -632,7 +649,7 @@ __device__ __forceinline__ void norm_rows_to_smem(const NormIn &ln, Fresh<float>
 #pragma unroll
         for (int i = 0; i < VPT; ++i) {
             const int kk = tid + i * THREADS - k0;
-            if (kk >= 0 && kk < ld) xs[m * ld + kk] = m < m_valid && kk < cols ? (v[m][i] - mean[m]) * inv_std * g[i] + b[i] : 0.0f;
+            if (kk >= 0 && kk < ld) xs[m * ld + kk] = m < m_valid && kk < cols ? (get(m, i) - mean[m]) * inv_std * get(MT, i) + get(MT + 1, i) : 0.0f;
         }
     }
 }

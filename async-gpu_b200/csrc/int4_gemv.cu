@@ -16,7 +16,10 @@
 #include "device_utils.cuh"
 
 static constexpr int GEMV_THREADS = 512;
-static constexpr int GEMV_AHEAD = 3;     // K blocks of a thread in flight
+// K blocks of a thread in flight: as many as the 64 registers of two blocks per SM hold beside the row sums and a LayerNorm's
+// values; three where the registers of a whole SM are there for one block.
+template <int MT, bool LN, int PER_SM>
+constexpr int gemv_ahead = MT == 1 || (MT == 2 && !LN) || PER_SM == 1 ? 3 : 2;
 
 template <int MT>
 __device__ __forceinline__ void gemv_block_fma(const uint4 &wa, const uint4 &wb, float s, const float *xb, int len,
@@ -50,13 +53,15 @@ __device__ __forceinline__ void gemv_block_fma(const uint4 &wa, const uint4 &wb,
 // grid (weight rows / RW, splits), cluster (1, splits, 1): the blocks of a cluster share RW rows of the weight.  A thread
 // has one row and every SLICES-th K block of its block's range.  RW 128: four slices.  RW 32: sixteen, for weights of
 // few rows, so that a thread has two or three K blocks, all of them requested before the wait, and most weights need no
-// second block per tile.
-template <int MT, int RW, typename XT>
-__global__ void __launch_bounds__(GEMV_THREADS, 2)
+// second block per tile.  LN: the rows' LayerNorm is taken here; one f32 row has one kernel for both and asks `ln.g`, two have
+// the values that the LayerNorm holds in shared memory and a kernel of their own for it (in registers they spilled: two
+// sequences of GPT-2 Small, 64 tokens after a prompt of 64: 23.6 -> 20.4 ms).
+template <int MT, int RW, bool LN, int PER_SM, typename XT>
+__global__ void __launch_bounds__(GEMV_THREADS, PER_SM)
 int4_gemv_kernel(const uint4 *__restrict__ tiles, const __half *__restrict__ scales, Fresh<XT> x,
                  int m_valid, int m0, int K, int N, int k_blocks, int n_pad, int group, int kb_per_split,
                  NormIn ln, Epilogue epi) {
-    constexpr int SLICES = GEMV_THREADS / RW;
+    constexpr int SLICES = GEMV_THREADS / RW, AHEAD = gemv_ahead<MT, LN, PER_SM>;
     extern __shared__ float smem_f[];
     const int split = blockIdx.y, splits = gridDim.y;
     const int tid = threadIdx.x, r = tid % RW, slice = tid / RW;
@@ -67,14 +72,15 @@ int4_gemv_kernel(const uint4 *__restrict__ tiles, const __half *__restrict__ sca
     float *xs = smem_f;                        // [MT][len] activations of this block's K range
     float *red = smem_f + MT * len;            // [SLICES][MT][RW] slice sums
     float *part = red + SLICES * MT * RW;      // [splits][MT][RW] partial tiles, in the cluster's first block
+    float *held = part + splits * MT * RW;     // two rows with a LayerNorm: [MT + 2][K]
     pdl_trigger();
     if (splits > 1) cluster_arrive(); // waited for before the first store into another block
 
     // weights and scales of this thread's first K blocks: issued before the wait on the
     // previous kernel (they are constants), so that their DRAM latency overlaps its tail
     const uint4 *tile0 = tiles + (size_t)(n >> 7) * k_blocks * (TILE_BYTES / 16) + tile_row;
-    uint4 wa[GEMV_AHEAD], wb[GEMV_AHEAD];
-    float sc[GEMV_AHEAD];
+    uint4 wa[AHEAD], wb[AHEAD];
+    float sc[AHEAD];
     auto load_block = [&](int i, int kb) {
         if (kb >= kb1) return;
         const uint4 *tp = tile0 + (size_t)kb * (TILE_BYTES / 16);
@@ -83,12 +89,12 @@ int4_gemv_kernel(const uint4 *__restrict__ tiles, const __half *__restrict__ sca
         sc[i] = __half2float(scales[(size_t)((kb * 64) / group) * n_pad + n]);
     };
 #pragma unroll
-    for (int i = 0; i < GEMV_AHEAD; ++i) load_block(i, kb0 + slice + i * SLICES);
+    for (int i = 0; i < AHEAD; ++i) load_block(i, kb0 + slice + i * SLICES);
 
-    if constexpr (sizeof(XT) == 4) {
-        if (ln.g) norm_rows_to_smem<MT, GEMV_THREADS>(ln, x, m_valid, K, kb0 * 64, (kb1 - kb0) * 64, len, xs, red);
+    if constexpr (LN) {
+        if (MT > 1 || ln.g) norm_rows_to_smem<MT, GEMV_THREADS, (MT > 1)>(ln, x, m_valid, K, kb0 * 64, (kb1 - kb0) * 64, len, xs, red, held);
     }
-    if (sizeof(XT) != 4 || !ln.g) {
+    if (!LN || (MT == 1 && !ln.g)) {
         pdl_wait();
         rows_to_smem<MT, GEMV_THREADS>(x, m_valid, K, kb0 * 64, (kb1 - kb0) * 64, len, xs);
     }
@@ -97,12 +103,12 @@ int4_gemv_kernel(const uint4 *__restrict__ tiles, const __half *__restrict__ sca
     float acc[MT];
 #pragma unroll
     for (int m = 0; m < MT; ++m) acc[m] = 0.0f;
-    for (int kb = kb0 + slice; kb < kb1; kb += GEMV_AHEAD * SLICES) {
+    for (int kb = kb0 + slice; kb < kb1; kb += AHEAD * SLICES) {
 #pragma unroll
-        for (int i = 0; i < GEMV_AHEAD; ++i) {
+        for (int i = 0; i < AHEAD; ++i) {
             const int k = kb + i * SLICES;
             if (k < kb1) gemv_block_fma<MT>(wa[i], wb[i], sc[i], xs + (k - kb0) * 64, len, acc);
-            load_block(i, k + GEMV_AHEAD * SLICES);
+            load_block(i, k + AHEAD * SLICES);
         }
     }
 
@@ -170,7 +176,7 @@ int launch_int4_naive(b200nn_ctx *ctx, const Int4Weight &w, const void *x, bool 
     return B200NN_OK;
 }
 
-template <int MT, int RW, typename XT>
+template <int MT, int RW, bool LN, int PER_SM, typename XT>
 static int gemv_launch(b200nn_ctx *ctx, const Int4Weight &w, const XT *x, int m_valid, int m0, const NormIn &ln, const Epilogue &epi) {
     constexpr int SLICES = GEMV_THREADS / RW;
     constexpr size_t SMEM_MAX = 216 * 1024;
@@ -182,8 +188,8 @@ static int gemv_launch(b200nn_ctx *ctx, const Int4Weight &w, const XT *x, int m_
     splits = std::min(splits, std::max(1, w.k_blocks / SLICES));
     const int per = (w.k_blocks + splits - 1) / splits;
     splits = (w.k_blocks + per - 1) / per;
-    const size_t smem = ((size_t)MT * per * 64 + (size_t)(SLICES + splits) * MT * RW) * sizeof(float);
-    auto kern = int4_gemv_kernel<MT, RW, XT>;
+    const size_t smem = ((size_t)MT * per * 64 + (size_t)(SLICES + splits) * MT * RW + (LN && MT > 1 ? (MT + 2) * w.K : 0)) * sizeof(float);
+    auto kern = int4_gemv_kernel<MT, RW, LN, PER_SM, XT>;
     static bool attr_done[16] = {}; // function attributes are per device
     if (!attr_done[ctx->device & 15]) {
         CK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
@@ -210,36 +216,45 @@ static int gemv_launch(b200nn_ctx *ctx, const Int4Weight &w, const XT *x, int m_
     CK_LAUNCH(ctx, "int4_gemv_kernel");
     return B200NN_OK;
 }
-template <int MT, typename XT>
+template <int MT, bool LN, typename XT>
 static int gemv_chunk(b200nn_ctx *ctx, const Int4Weight &w, const XT *x, int m_valid, int m0, const NormIn &ln, const Epilogue &epi) {
     // 32 rows a block while the blocks stay under two per SM and the activations of a block's K range small (an output
     // matrix has its blocks in 128 rows: ten blocks per SM would each pay for the start)
     const int tiles = (w.N + 31) / 32, splits = std::max(1, std::min(8, ctx->sm_count / tiles)), per = (w.k_blocks + splits - 1) / splits;
-    if (tiles <= 2 * ctx->sm_count && (size_t)MT * per * 64 * sizeof(float) <= 96 * 1024) return gemv_launch<MT, 32, XT>(ctx, w, x, m_valid, m0, ln, epi);
-    return gemv_launch<MT, 128, XT>(ctx, w, x, m_valid, m0, ln, epi);
+    const bool narrow = tiles <= 2 * ctx->sm_count && (size_t)MT * per * 64 * sizeof(float) <= 96 * 1024;
+    if constexpr (MT == 1 && sizeof(XT) == 4) {
+        return narrow ? gemv_launch<1, 32, true, 2, XT>(ctx, w, x, m_valid, m0, ln, epi) : gemv_launch<1, 128, true, 2, XT>(ctx, w, x, m_valid, m0, ln, epi);
+    } else if constexpr (LN) { // K is short, N a few times K
+        return gemv_launch<MT, 32, true, 2, XT>(ctx, w, x, m_valid, m0, ln, epi);
+    } else {
+        if constexpr (MT == 4) // a block per SM at most: its registers hold three K blocks (6400 x 1600, four rows: 13.3 -> 9.8 us)
+            if (narrow && tiles <= ctx->sm_count) return gemv_launch<4, 32, false, 1, XT>(ctx, w, x, m_valid, m0, ln, epi);
+        return narrow ? gemv_launch<MT, 32, false, 2, XT>(ctx, w, x, m_valid, m0, ln, epi) : gemv_launch<MT, 128, false, 2, XT>(ctx, w, x, m_valid, m0, ln, epi);
+    }
 }
 
-template <typename XT>
+template <bool LN, typename XT>
 static int gemv_all(b200nn_ctx *ctx, const Int4Weight &w, const XT *x, int M, const NormIn &ln, const Epilogue &epi) {
     int m0 = 0;
     while (m0 < M) {
         int left = M - m0;
         const XT *xp = x + (size_t)m0 * w.K;
         if (left >= 4) {
-            TRY((gemv_chunk<4, XT>(ctx, w, xp, 4, m0, ln, epi)));
+            TRY((gemv_chunk<4, false, XT>(ctx, w, xp, 4, m0, ln, epi)));
             m0 += 4;
         } else if (left >= 2) {
-            TRY((gemv_chunk<2, XT>(ctx, w, xp, 2, m0, ln, epi)));
+            TRY((gemv_chunk<2, LN, XT>(ctx, w, xp, 2, m0, ln, epi)));
             m0 += 2;
         } else {
-            TRY((gemv_chunk<1, XT>(ctx, w, xp, 1, m0, ln, epi)));
+            TRY((gemv_chunk<1, LN, XT>(ctx, w, xp, 1, m0, ln, epi)));
             m0 += 1;
         }
     }
     return B200NN_OK;
 }
 
-bool int4_linear_takes_norm(const Int4Weight &w, int M) { return w.fast && M >= 1 && M <= 4 && w.K <= NORM_IN_MAX; }
+// (four rows at a time and a LayerNorm do not fit the registers beside the weights in flight)
+bool int4_linear_takes_norm(const Int4Weight &w, int M) { return w.fast && M >= 1 && M <= 2 && w.K <= NORM_IN_MAX; }
 
 int launch_int4_gemv(b200nn_ctx *ctx, const Int4Weight &w, const void *x, bool x_half, int M, const Epilogue &epi, const NormIn &ln) {
     if (M <= 0) return B200NN_OK;
@@ -251,7 +266,8 @@ int launch_int4_gemv(b200nn_ctx *ctx, const Int4Weight &w, const void *x, bool x
         return launch_int4_gemm_tc(ctx, w, (const __half *)x, M, epi);
     }
     if (!w.fast) return launch_int4_naive(ctx, w, x, x_half, M, epi);
-    return x_half ? gemv_all<__half>(ctx, w, (const __half *)x, M, ln, epi) : gemv_all<float>(ctx, w, (const float *)x, M, ln, epi);
+    if (x_half) return gemv_all<false, __half>(ctx, w, (const __half *)x, M, ln, epi);
+    return ln.g ? gemv_all<true, float>(ctx, w, (const float *)x, M, ln, epi) : gemv_all<false, float>(ctx, w, (const float *)x, M, ln, epi);
 }
 
 int launch_int4_linear(b200nn_ctx *ctx, const Int4Weight &w, const void *x, bool x_half, int M, const Epilogue &epi, const NormIn &ln) {

@@ -12,9 +12,9 @@ import b200nn
 import np_ref
 import test_gpu_vivezen as vivezen
 import test_gpu_zufilorn as zufilorn
-from b200nn import Gpt2Config, Gpt2Model, GpuTensor, Int4Gpt2Model, Int4Linear, Linear, TransformerBlock, ops, synth
+from b200nn import Gpt2Config, Gpt2Model, GpuTensor, Int4Gpt2Model, Int4Linear, Int4TransformerBlock, Linear, TransformerBlock, ops, synth
 from oracle import oracle
-from test_gpu_block import _slices
+from test_gpu_block import _int4_oracle, _slices
 
 pytestmark = pytest.mark.gpu
 
@@ -90,15 +90,19 @@ def _int4(rng, k, n, group):
     return q * np.repeat(s.astype(np.float64), group, 0)[:k], packed, s
 
 
-@pytest.mark.parametrize("m", [1, 2])
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 7])
 # one block of K, ragged rows, K split over a cluster, the last weight of 32-row blocks and the first of 128-row ones
 @pytest.mark.parametrize("k,n,group", [(64, 1, 64), (128, 33, 128), (1600, 1600, 128), (6400, 130, 128), (3072, 768, 64),
                                        (1088, 9472, 64), (128, 9473, 128), (64, 50257, 64)])
-def test_int4_linear_one_and_two_rows(reg, m, k, n, group):
+def test_int4_linear_few_rows(reg, m, k, n, group):
     rng = np.random.default_rng(k + n + m)
     w, packed, s = _int4(rng, k, n, group)
     x, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal(n).astype(np.float32)
-    got = Int4Linear(packed, s, b, k, n, group, reg).forward(GpuTensor.from_host(x, (m, k), reg)).to_host()
+    reg.set_tuning("gemv_max_rows", 8)
+    try:
+        got = Int4Linear(packed, s, b, k, n, group, reg).forward(GpuTensor.from_host(x, (m, k), reg)).to_host()
+    finally:
+        reg.set_tuning("gemv_max_rows", -1)
     _close(got, x.astype(np.float64) @ w + b, np.abs(x).astype(np.float64) @ np.abs(w) + np.abs(b))
 
 
@@ -113,6 +117,25 @@ def test_int4_linear_epilogues(reg, m, k, n):
     got = Int4Linear(packed, s, b, k, n, 64, reg).forward(GpuTensor.from_host(x, (m, k), reg)).to_host()
     xh, wh = x.astype(np.float16).astype(np.float64), w.astype(np.float16).astype(np.float64)
     _close(got, xh @ wh + b, np.abs(xh) @ np.abs(wh) + np.abs(b))
+
+
+@pytest.mark.parametrize("d", [128, 768, 1600, 2048, 2112])
+@pytest.mark.parametrize("int4", [False, True])
+def test_block_with_a_layernorm_taken_along(reg, int4, d):
+    """One to four new rows on cached ones, the LayerNorms applied by the GEMV behind them up to 2048 columns (int4: one and two
+    rows), against float64."""
+    cfg = Gpt2Config(n_layer=1, n_embd=d, n_head=d // 64, vocab_size=64, n_positions=32)
+    w = synth.gpt2_weights(cfg, base_seed=d, std=1.5 / d ** 0.5, random_ln=True)
+    blk = Int4TransformerBlock(*_slices(w), cfg, reg, group_size=64) if int4 else TransformerBlock(*_slices(w), cfg, reg)
+    om = oracle.Model(cfg.as_dict(), _int4_oracle(w, cfg, 64) if int4 else w)
+    x = np.random.default_rng(d).standard_normal((12, d)).astype(np.float32)
+    ref = om.block_forward(0, x, flags=oracle.KV_FP16)[0]
+    for n in (1, 2) if int4 else (1, 2, 3, 4): # (more int4 rows go to the tensor cores)
+        past = 12 - n
+        _, k0, v0 = blk.forward_cached(GpuTensor.from_host(x[:past], (past, d), reg), None, None, 0)
+        got = blk.forward_cached(GpuTensor.from_host(x[past:], (n, d), reg), k0, v0, past)[0].to_host()
+        for i in range(n):
+            assert np_ref.rel_rms(got[i], ref[past + i]) < 1e-3, (n, i, np_ref.rel_rms(got[i], ref[past + i]))
 
 
 def test_rows_after_rows(reg):
