@@ -654,21 +654,24 @@ __device__ __forceinline__ void norm_rows_to_smem(const NormIn &ln, Fresh<float>
     }
 }
 
-// Columns k0 .. k0+cols of up to MT rows x [m_valid][K] as f32 in xs [MT][ld], zero past them and past m_valid.
+// Columns k0 .. k0+cols of up to MT rows x [m_valid][K] as f32 in xs [MT][ld], zero past them and past m_valid.  The rows
+// are requested together (one after the other, each waited out its own latency: four rows, int4 768 x 2304 4.0 -> 3.3 us, f32 3072 x 768 20.5 -> 18.3).
 template <int MT, int THREADS, typename XT>
 __device__ __forceinline__ void rows_to_smem(Fresh<XT> x, int m_valid, int K, int k0, int cols, int ld, float *xs) {
-    constexpr int U = 4; // loads of a thread in flight
+    constexpr int U = MT == 4 ? 2 : 4; // columns of a thread in flight, MT loads each
+    for (int base = threadIdx.x; base < ld; base += U * THREADS) {
+        float v[U][MT];
 #pragma unroll
-    for (int m = 0; m < MT; ++m)
-        for (int base = threadIdx.x; base < ld; base += U * THREADS) {
-            float v[U];
+        for (int u = 0; u < U; ++u)
 #pragma unroll
-            for (int u = 0; u < U; ++u)
-                v[u] = m < m_valid && base + u * THREADS < cols ? x[(size_t)m * K + k0 + base + u * THREADS] : 0.0f;
+            for (int m = 0; m < MT; ++m)
+                v[u][m] = m < m_valid && base + u * THREADS < cols ? x[(size_t)m * K + k0 + base + u * THREADS] : 0.0f;
 #pragma unroll
-            for (int u = 0; u < U; ++u)
-                if (base + u * THREADS < ld) xs[m * ld + base + u * THREADS] = v[u];
-        }
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int m = 0; m < MT; ++m)
+                if (base + u * THREADS < ld) xs[m * ld + base + u * THREADS] = v[u][m];
+    }
 }
 
 __device__ __forceinline__ float sigmoid_f(float v) { return 1.0f / (1.0f + expf(-v)); }
