@@ -37,20 +37,21 @@ __device__ __forceinline__ void half8_to_float(const uint4 &u, float (&f)[8]) {
 // triples are stored into the shared memory of the cluster's first block: one cluster barrier in the place of a record in
 // memory, a fence and a counter.  GPT-2 XL, one sequence: 6.7 -> 3.3 us a launch.
 namespace split_attn {
-constexpr int THREADS = 128, R = 4, NST = 2, MAX_SPLITS = 8;
-constexpr int BLOCKS_PER_SM = 6;                    // 32 KB of shared memory and at most 85 registers a thread
-constexpr int ROWS = 16 * R;                        // cached rows of a stage
-constexpr int STAGE_U4 = 2 * R * THREADS;           // 16-byte pieces
-constexpr int SMEM_BYTES = NST * STAGE_U4 * 16;
+constexpr int R = 4, NST = 2, MAX_SPLITS = 8;
+constexpr int BLOCKS_PER_SM = 6; // of four warps: 32 KB of shared memory and at most 85 registers a thread
 }  // namespace split_attn
 
-template <typename QT, typename OT>
-__global__ void __launch_bounds__(split_attn::THREADS, split_attn::BLOCKS_PER_SM)
-decode_attn_kernel(Fresh<QT> q, int ldq, Fresh<__half> kc, Fresh<__half> vc, int H, int cap, Fresh<int> pos_ptr, int pos_off, OT *__restrict__ out, int ldo, int pf_bytes) {
+// WARPS: see attn_warps
+template <typename QT, typename OT, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? split_attn::BLOCKS_PER_SM : 16 / WARPS)
+decode_attn_kernel(Fresh<QT> q, int ldq, Fresh<__half> kc, Fresh<__half> vc, int H, int cap, Fresh<int> pos_ptr, int pos_off,
+                   OT *__restrict__ out, int ldo, int pf_bytes) {
     using namespace split_attn;
+    constexpr int THREADS = WARPS * 32, STEP = WARPS * 4, ROWS = STEP * R; // cached rows of a step and of a stage
+    constexpr int STAGE_U4 = 2 * R * THREADS;                              // 16-byte pieces
     extern __shared__ __align__(16) uint8_t smem_raw[];
     uint4 *ring = reinterpret_cast<uint4 *>(smem_raw);
-    __shared__ float sm_m[4], sm_l[4], sm_acc[4][64];
+    __shared__ float sm_m[WARPS], sm_l[WARPS], sm_acc[WARPS][64];
     __shared__ float part_ml[MAX_SPLITS][2], part_o[MAX_SPLITS][64]; // in the cluster's first block
     const int h = blockIdx.x, b = blockIdx.y, split = blockIdx.z, n_splits = gridDim.z;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 3, c = lane & 7;
@@ -78,11 +79,11 @@ decode_attn_kernel(Fresh<QT> q, int ldq, Fresh<__half> kc, Fresh<__half> vc, int
     if (ctx > cap) ctx = cap;
     range(ctx, p0, p1);
 
-    auto request = [&](int stage, int jw) { // rows jw + g, + 16, ... of this thread
+    auto request = [&](int stage, int jw) { // rows jw + g, + STEP, ... of this thread
         uint4 *st = ring + stage * STAGE_U4 + tid;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const int j = jw + g + 16 * r;
+            const int j = jw + g + STEP * r;
             if (j < p1) {
                 cp_async16(st + 2 * r * THREADS, kp + (size_t)j * 8 + c);
                 cp_async16(st + (2 * r + 1) * THREADS, vp + (size_t)j * 8 + c);
@@ -112,7 +113,7 @@ decode_attn_kernel(Fresh<QT> q, int ldq, Fresh<__half> kc, Fresh<__half> vc, int
         float sc[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            valid[r] = jw + g + 16 * r < p1;
+            valid[r] = jw + g + STEP * r < p1;
             const uint4 kr = valid[r] ? st[2 * r * THREADS] : make_uint4(0, 0, 0, 0);
             const __half2 *kh = reinterpret_cast<const __half2 *>(&kr);
             float2 t2 = make_float2(0.0f, 0.0f);
@@ -169,9 +170,9 @@ decode_attn_kernel(Fresh<QT> q, int ldq, Fresh<__half> kc, Fresh<__half> vc, int
     float M = NEG_BIG, L = 0.0f, O = 0.0f;
     if (tid < 64) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) M = fmaxf(M, sm_m[i]);
+        for (int i = 0; i < WARPS; ++i) M = fmaxf(M, sm_m[i]);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < WARPS; ++i) {
             const float w = exp2f(sm_m[i] - M);
             L += sm_l[i] * w;
             O += sm_acc[i][tid] * w;
@@ -200,28 +201,38 @@ decode_attn_kernel(Fresh<QT> q, int ldq, Fresh<__half> kc, Fresh<__half> vc, int
     if (tid < 64) store_from_float(out + (size_t)b * ldo + h * 64 + tid, O / L);
 }
 
-// Splits of a pair's context: as many as keep all blocks resident at once (a second, partial wave runs at the latency of
-// its chain), none of under 64 rows, at most a cluster.
+// Splits of a pair's context: as many as the block slots of the GPU take at once (a second, partial wave runs at the
+// latency of its chain; clusters that do not pack into a GPC may still leave one), none of under 64 rows, at most a cluster.
 static int attn_splits(int blocks_per_sm, int sm_count, long long pairs, int max_ctx) {
     const long long room = (long long)blocks_per_sm * sm_count / pairs;
     return (int)std::max(1LL, std::min(std::min(room, (max_ctx + 63LL) / 64), (long long)split_attn::MAX_SPLITS));
 }
+// Warps of a block.  A cluster has at most eight blocks, whatever the context, and a warp's chain from one stage to the next
+// (scores, shuffles, maximum, exponentials) takes longer than its bytes: where that leaves an SM one or two blocks of long
+// ranges they get 16 or 8 warps, of at least two stages each (four / more warps, inputs beyond L2: one pair of 32768
+// positions 36 / 18 us, 12 pairs of 8192 15.4 / 9.3 and of 32768 45 / 22, 24 pairs of 8192 24 / 17; a ring of six stages
+// instead: 33, 14.3, 43 and 16).
+static int attn_warps(int sm_count, long long pairs, int n_splits, int max_ctx) {
+    const long long blocks = pairs * n_splits, rows = (max_ctx + n_splits - 1) / n_splits;
+    return blocks <= sm_count && rows >= 512 ? 16 : blocks <= 2LL * sm_count && rows >= 256 ? 8 : 4;
+}
 
-template <typename QT, typename OT>
-static cudaError_t launch_decode_attn(int device, cudaStream_t stream, bool pdl, const QT *q, int ldq, const __half *kc, const __half *vc,
+template <typename QT, typename OT, int WARPS>
+static cudaError_t launch_decode_attn_w(int device, cudaStream_t stream, bool pdl, const QT *q, int ldq, const __half *kc, const __half *vc,
                                       int B, int H, int cap, const int *pos_ptr, int pos_off, OT *out, int n_splits, size_t pf_total) {
-    auto kern = decode_attn_kernel<QT, OT>;
+    auto kern = decode_attn_kernel<QT, OT, WARPS>;
+    constexpr int SMEM_BYTES = split_attn::NST * 2 * split_attn::R * WARPS * 32 * 16;
     static bool attr_done[64] = {}; // function attributes are per device
     if (!attr_done[device & 63]) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, split_attn::SMEM_BYTES);
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
         if (e != cudaSuccess) return e;
         prefer_max_smem(kern);
         attr_done[device & 63] = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(H, B, n_splits);
-    cfg.blockDim = dim3(split_attn::THREADS);
-    cfg.dynamicSmemBytes = split_attn::SMEM_BYTES;
+    cfg.blockDim = dim3(WARPS * 32);
+    cfg.dynamicSmemBytes = SMEM_BYTES;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -235,6 +246,13 @@ static cudaError_t launch_decode_attn(int device, cudaStream_t stream, bool pdl,
     const size_t blocks = (size_t)H * B * n_splits;
     return cudaLaunchKernelEx(&cfg, kern, q, ldq, kc, vc, H, cap, pos_ptr, pos_off, out, H * 64,
                               (int)std::min<size_t>(pf_total / 2 / blocks, 1u << 20));
+}
+template <typename QT, typename OT>
+static cudaError_t launch_decode_attn(int device, int sm_count, cudaStream_t stream, bool pdl, const QT *q, int ldq, const __half *kc, const __half *vc,
+                                      int B, int H, int cap, const int *pos_ptr, int pos_off, OT *out, int n_splits, int max_ctx, size_t pf_total) {
+    const int warps = attn_warps(sm_count, (long long)B * H, n_splits, max_ctx);
+    auto launch = warps == 16 ? launch_decode_attn_w<QT, OT, 16> : warps == 8 ? launch_decode_attn_w<QT, OT, 8> : launch_decode_attn_w<QT, OT, 4>;
+    return launch(device, stream, pdl, q, ldq, kc, vc, B, H, cap, pos_ptr, pos_off, out, n_splits, pf_total);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -603,8 +621,8 @@ int launch_decode_attention(b200nn_ctx *ctx, const void *q, bool q_half, int ldq
     const int n_splits = attn_splits(ctx->attn_blocks_per_sm, ctx->sm_count, pairs, max_ctx_hint);
     const size_t pf = (size_t)ctx->kv_prefetch_mb << 20;
 #define DA(QT, OT)                                                                                                           \
-    CK(ctx, (launch_decode_attn<QT, OT>(ctx->device, ctx->stream, ctx->pdl, (const QT *)q, ldq, kc, vc, B, H, cap, pos_ptr, pos_off, \
-                                        (OT *)out, n_splits, pf)))
+    CK(ctx, (launch_decode_attn<QT, OT>(ctx->device, ctx->sm_count, ctx->stream, ctx->pdl, (const QT *)q, ldq, kc, vc, B, H, cap, pos_ptr, \
+                                        pos_off, (OT *)out, n_splits, max_ctx_hint, pf)))
     if (q_half && out_half) DA(__half, __half);
     else if (q_half) DA(__half, float);
     else if (out_half) DA(float, __half);
@@ -791,9 +809,9 @@ extern "C" int32_t b200nn_decode_attention_noalloc(int32_t device, void *stream,
     }
     if (rc == B200NN_OK) {
         const int n_splits = attn_splits(split_attn::BLOCKS_PER_SM, sms, pairs, ctx_len);
-        e = launch_decode_attn<float, float>(device, static_cast<cudaStream_t>(stream), false, q_dev, n_heads * 64,
+        e = launch_decode_attn<float, float>(device, sms, static_cast<cudaStream_t>(stream), false, q_dev, n_heads * 64,
                                              static_cast<const __half *>(k_cache_dev), static_cast<const __half *>(v_cache_dev), batch,
-                                             n_heads, capacity, nullptr, ctx_len - 1, out_dev, n_splits, 0);
+                                             n_heads, capacity, nullptr, ctx_len - 1, out_dev, n_splits, ctx_len, 0);
         if (e != cudaSuccess) rc = noalloc_fail(B200NN_ERR_CUDA, "kernel launch", e);
     }
     if (prev != device && prev >= 0) cudaSetDevice(prev);

@@ -194,7 +194,10 @@ def test_greedy_pick_of_a_vocabulary_between_tiles(reg, int4):
 # one row, a stage's edge, a split's edge, the most splits, and the pairs around which the split count changes
 @pytest.mark.parametrize("batch,heads,ctx,cap", [(1, 1, 1, 1), (1, 1, 64, 64), (1, 2, 65, 65), (1, 1, 129, 300), (1, 3, 1024, 1024),
                                                  (1, 1, 5000, 5000), (37, 3, 513, 520), (37, 12, 200, 256), (37, 13, 77, 128), (74, 12, 130, 130),
-                                                 (75, 12, 131, 131)])
+                                                 (75, 12, 131, 131),
+                                                 # blocks of 16 warps, of 8 (by rows, by blocks), and of 4 again
+                                                 (1, 1, 4089, 4100), (1, 1, 4088, 4088), (1, 2, 2041, 2041), (1, 2, 2040, 2050), (1, 18, 4100, 4100),
+                                                 (1, 19, 4100, 4101), (1, 37, 2049, 2049), (1, 38, 2049, 2049)])
 def test_decode_attention_splits(reg, batch, heads, ctx, cap):
     import torch
 
