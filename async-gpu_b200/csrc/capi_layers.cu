@@ -19,7 +19,7 @@ extern "C" int32_t b200nn_layer_norm(b200nn_ctx *ctx, const b200nn_tensor *x, co
     b200nn_tensor *y = nullptr;
     TRY(tensor_alloc(ctx, x->shape, false, &y));
     int rc = launch_layernorm(ctx, x->data(), nullptr, nullptr, gamma->data(), beta->data(), eps, (int)lead_rows(x),
-                              (int)d, y->data(), false);
+                              (int)d, y->data(), false, true);
     if (rc != B200NN_OK) { delete y; return rc; }
     *out = y;
     return B200NN_OK;
@@ -38,7 +38,7 @@ extern "C" int32_t b200nn_layer_norm_residual_dual(b200nn_ctx *ctx, const b200nn
     int rc = tensor_alloc(ctx, a->shape, false, &y);
     if (rc == B200NN_OK)
         rc = launch_layernorm(ctx, a->data(), b->data(), s->data(), gamma->data(), beta->data(), eps,
-                              (int)lead_rows(a), (int)d, y->data(), false);
+                              (int)lead_rows(a), (int)d, y->data(), false, true);
     if (rc != B200NN_OK) { delete s; delete y; return rc; }
     *sum_out = s;
     *norm_out = y;

@@ -11,6 +11,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "b200nn.h"
@@ -130,9 +131,10 @@ inline void prefer_max_smem(Kernel kern) {
 // on the stream is still running and must execute pdl_wait() (griddepcontrol.wait) before it reads
 // or writes anything the predecessor touches.  Only kernels that do so are launched this way.
 // Its blocks may be resident while those kernels run, so it takes what they write as Fresh<T> (device_utils.cuh).
+// early: whether it may (false: it starts behind the end of everything before it).
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(b200nn_ctx *ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                              Args &&...args) {
+inline cudaError_t launch_dependent(b200nn_ctx *ctx, bool early, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                    Args &&...args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -142,19 +144,18 @@ inline cudaError_t launch_pdl(b200nn_ctx *ctx, void (*kern)(KArgs...), dim3 grid
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = ctx->pdl ? 1 : 0;
+    cfg.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(b200nn_ctx *ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args &&...args) {
+    return launch_dependent(ctx, ctx->pdl != 0, kern, grid, block, smem, std::forward<Args>(args)...);
 }
 // Launch behind the end of everything before it, for kernels that read what earlier kernels wrote through L1 (several
 // threads share the lines, or one walks along them).
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_ordered(b200nn_ctx *ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args &&...args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = ctx->stream;
-    return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+    return launch_dependent(ctx, false, kern, grid, block, smem, std::forward<Args>(args)...);
 }
 
 #define TRY(expr)                       \
@@ -346,8 +347,9 @@ int launch_b16_linear(b200nn_ctx *ctx, const B16Weight &w, const __nv_bfloat16 *
 bool int4_via_f16_supported(const b200nn_ctx *ctx, const Int4Weight &w, int M);
 int launch_int4_via_f16(b200nn_ctx *ctx, const Int4Weight &w, const __half *x, int M, const Epilogue &epi);
 
+// params_written: gamma and beta are tensors that work before this may write (they are read ahead of the wait on it otherwise)
 int launch_layernorm(b200nn_ctx *ctx, const float *x, const float *res_in, float *sum_out, const float *gamma,
-                     const float *beta, float eps, int rows, int d, void *out, bool out_half);
+                     const float *beta, float eps, int rows, int d, void *out, bool out_half, bool params_written = false);
 // launch_embedding that also prepares the first LayerNorm for folding: xg = fp16(out * g) and each row's
 // (sum, sum of squares) in partial 0 of stats [n_rows][stats_nt][2] (the other partials zero).
 int launch_embedding_ln(b200nn_ctx *ctx, const uint32_t *ids, const float *wte, const float *wpe, int n_rows, int d,

@@ -126,31 +126,32 @@ __global__ void __launch_bounds__(256) layernorm_rows_kernel(Fresh<float> x, con
 }
 
 template <int NV>
-static void launch_layernorm_rows(b200nn_ctx *ctx, const float *x, const float *gamma, const float *beta, float eps, int rows,
+static void launch_layernorm_rows(b200nn_ctx *ctx, bool early, const float *x, const float *gamma, const float *beta, float eps, int rows,
                                   int d, void *out, bool out_half) {
     const int grid = std::min((rows + 7) / 8, 8 * ctx->sm_count);
     const size_t smem = (size_t)d * 2 * sizeof(float);
     PREFER_SMEM_ONCE((layernorm_rows_kernel<NV, __half>));
     PREFER_SMEM_ONCE((layernorm_rows_kernel<NV, float>));
     if (out_half)
-        launch_pdl(ctx, layernorm_rows_kernel<NV, __half>, dim3(grid), dim3(256), smem, x, gamma, beta, eps, rows, d, (__half *)out);
+        launch_dependent(ctx, early, layernorm_rows_kernel<NV, __half>, dim3(grid), dim3(256), smem, x, gamma, beta, eps, rows, d, (__half *)out);
     else
-        launch_pdl(ctx, layernorm_rows_kernel<NV, float>, dim3(grid), dim3(256), smem, x, gamma, beta, eps, rows, d, (float *)out);
+        launch_dependent(ctx, early, layernorm_rows_kernel<NV, float>, dim3(grid), dim3(256), smem, x, gamma, beta, eps, rows, d, (float *)out);
 }
 
 int launch_layernorm(b200nn_ctx *ctx, const float *x, const float *res_in, float *sum_out, const float *gamma,
-                     const float *beta, float eps, int rows, int d, void *out, bool out_half) {
+                     const float *beta, float eps, int rows, int d, void *out, bool out_half, bool params_written) {
     if (rows <= 0) return B200NN_OK;
+    const bool early = ctx->pdl && !params_written;
     if (d > 256 * 32) return set_error(ctx, B200NN_ERR_UNSUPPORTED, "layer_norm: d > 8192");
     // many rows without a residual (prefill passes): a warp per row
     if (rows >= ctx->ln_rows_min && !res_in && !sum_out && d % 4 == 0 && d <= 2048 && !((uintptr_t)x & 15) && !((uintptr_t)out & 15) &&
         !((uintptr_t)gamma & 15) && !((uintptr_t)beta & 15)) {
         const int nv = (d / 4 + 31) / 32;
-        if (nv <= 6) launch_layernorm_rows<6>(ctx, x, gamma, beta, eps, rows, d, out, out_half);
-        else if (nv <= 8) launch_layernorm_rows<8>(ctx, x, gamma, beta, eps, rows, d, out, out_half);
-        else if (nv <= 10) launch_layernorm_rows<10>(ctx, x, gamma, beta, eps, rows, d, out, out_half);
-        else if (nv <= 13) launch_layernorm_rows<13>(ctx, x, gamma, beta, eps, rows, d, out, out_half);
-        else launch_layernorm_rows<16>(ctx, x, gamma, beta, eps, rows, d, out, out_half);
+        if (nv <= 6) launch_layernorm_rows<6>(ctx, early, x, gamma, beta, eps, rows, d, out, out_half);
+        else if (nv <= 8) launch_layernorm_rows<8>(ctx, early, x, gamma, beta, eps, rows, d, out, out_half);
+        else if (nv <= 10) launch_layernorm_rows<10>(ctx, early, x, gamma, beta, eps, rows, d, out, out_half);
+        else if (nv <= 13) launch_layernorm_rows<13>(ctx, early, x, gamma, beta, eps, rows, d, out, out_half);
+        else launch_layernorm_rows<16>(ctx, early, x, gamma, beta, eps, rows, d, out, out_half);
         CK_LAUNCH(ctx, "layernorm_rows_kernel");
         return B200NN_OK;
     }
@@ -159,11 +160,11 @@ int launch_layernorm(b200nn_ctx *ctx, const float *x, const float *res_in, float
         PREFER_SMEM_ONCE((layernorm_kernel<V, __half>));                                                          \
         PREFER_SMEM_ONCE((layernorm_kernel<V, float>));                                                           \
         if (out_half)                                                                                             \
-            launch_pdl(ctx, layernorm_kernel<V, __half>, dim3(rows), dim3(256), 0, x, res_in, sum_out, gamma,    \
-                       beta, eps, d, (__half *)out);                                                             \
+            launch_dependent(ctx, early, layernorm_kernel<V, __half>, dim3(rows), dim3(256), 0, x, res_in, sum_out, gamma, \
+                             beta, eps, d, (__half *)out);                                                        \
         else                                                                                                      \
-            launch_pdl(ctx, layernorm_kernel<V, float>, dim3(rows), dim3(256), 0, x, res_in, sum_out, gamma,     \
-                       beta, eps, d, (float *)out);                                                              \
+            launch_dependent(ctx, early, layernorm_kernel<V, float>, dim3(rows), dim3(256), 0, x, res_in, sum_out, gamma, \
+                             beta, eps, d, (float *)out);                                                         \
     } while (0)
     int vpt = (d + 255) / 256;
     if (vpt <= 4) LN_LAUNCH(4);

@@ -155,6 +155,22 @@ def test_rows_after_rows(reg):
             assert np_ref.rel_rms(got[i], ref[past + i]) < 1e-3, (turn, n, i)
 
 
+def test_layer_norm_of_parameters_just_computed(reg):
+    """Scale and shift that the calls before it make: a LayerNorm that is given tensors must not read them ahead of its wait."""
+    k, d = 16384, 256
+    rng = np.random.default_rng(8)
+    w = GpuTensor.from_host(np.ones((k, d), np.float32), (k, d), reg)
+    x = rng.standard_normal((3, d)).astype(np.float32)
+    xd = GpuTensor.from_host(x, (3, d), reg)
+    plain = oracle.layer_norm(x, np.ones(d, np.float32), np.zeros(d, np.float32), 1e-5).reshape(3, d)
+    rows = [GpuTensor.from_host(np.full((1, k), v, np.float32), (1, k), reg) for v in (2.0 ** -10, 2.0 ** -12, 2.0 ** -14)]
+    for i in range(12):
+        gamma, beta = ops.matmul(rows[i % 3], w, reg), ops.matmul(rows[(i + 1) % 3], w, reg)
+        got = ops.layer_norm(xd, gamma, beta, 1e-5, reg).to_host()
+        g, b = (16.0, 4.0, 1.0)[i % 3], (16.0, 4.0, 1.0)[(i + 1) % 3]
+        assert np.abs(got - (plain * g + b)).max() < 1e-5 * 40, i
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("family", [vivezen, zufilorn])
 def test_rows_after_rows_of_hybrid_models(reg, family, dtype):
