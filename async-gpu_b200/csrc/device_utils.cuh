@@ -655,7 +655,8 @@ __device__ __forceinline__ void norm_rows_to_smem(const NormIn &ln, Fresh<float>
 }
 
 // Columns k0 .. k0+cols of up to MT rows x [m_valid][K] as f32 in xs [MT][ld], zero past them and past m_valid.  The rows
-// are requested together (one after the other, each waited out its own latency: four rows, int4 768 x 2304 4.0 -> 3.3 us, f32 3072 x 768 20.5 -> 18.3).
+// are requested together (one after the other, each waited out its own latency: four rows, int4 768 x 2304 4.0 -> 3.3 us,
+// f32 3072 x 768 20.5 -> 18.3).
 template <int MT, int THREADS, typename XT>
 __device__ __forceinline__ void rows_to_smem(Fresh<XT> x, int m_valid, int K, int k0, int cols, int ld, float *xs) {
     constexpr int U = MT == 4 ? 2 : 4; // columns of a thread in flight, MT loads each

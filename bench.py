@@ -793,6 +793,8 @@ def run_b200(args):
     roof["peak_source"] = peak_kind
     roof["launch_ms"] = fam[dominant] / max(1, fam_launches[dominant])
     roof["launches_per_step"] = fam_launches
+    # one or two sequences (f32: up to four): the blocks' LayerNorms run inside the Linears and count there
+    roof["block_layernorms_in_linear"] = batch <= (2 if family == "int4" else 4) and d <= 2048
     roof["step_family_ms"] = {k2: round(v, 4) for k2, v in fam.items()}
     roof["other"] = {k2: {"achieved": v["achieved"], "frac": v["achieved"] / v["peak"]} for k2, v in roofs.items()
                      if k2 != dominant}

@@ -110,10 +110,11 @@ B200NN_API int32_t b200nn_ctx_set_gemv_max_rows(b200nn_ctx *ctx, int32_t rows);
  * "attn_tc" (0 = run fp16 prefill attention on the CUDA cores instead of the tensor cores),
  * "attn_stream" (0 = never use the TMA-fed decode-attention kernel), "attn_stream_min10" (tenths of
  * a (sequence, head) pair per warp of its grid from which it is used; default 20), "attn_stream_wide_min10" (the same for
- * its 16-warp block shape; default 25, 0 = never), "kv_prefetch_mb" (KV-cache
- * megabytes that kernel asks into L2 before its dependency wait), "attn_split_items" (items it
- * hands out as two halves at the end of the grid; 0 = none), "attn_blocks_per_sm" (blocks per SM the
- * split-context decode attention splits the context of few pairs for; default 6: all blocks resident).
+ * its 16-warp block shape; default 25, 0 = never), "attn_split_items" (items it
+ * hands out as two halves at the end of the grid; 0 = none), "kv_prefetch_mb" (KV-cache megabytes that it and the
+ * split-context decode attention ask into L2 before their dependency wait), "attn_blocks_per_sm" (blocks per SM the
+ * split-context decode attention splits the context of few pairs for, into eight parts at most; default 6: the block slots
+ * of the GPU).
  * "f32_tc" selects how an f32 Linear (linear.rs:283-313) multiplies more than four rows: 2 (default;
  * negative restores it) fp16 activations times the weight held as fp16 hi + lo on the tensor cores,
  * f32 accumulation (the weight enters with about 22 bits, the activations with fp16's 11); 1 the
@@ -470,7 +471,9 @@ B200NN_API int32_t b200nn_session_tokens(b200nn_session *s, uint32_t *out, size_
 B200NN_API int32_t b200nn_session_logits(b200nn_session *s, float *out);
 /* Per-kernel-family device time of ONE decode step at the current position, measured with CUDA
  * events around each launch (Gpt2Model::forward_profiled, gpt2.rs:529-568).  times_ms has
- * B200NN_PROF_COUNT entries. */
+ * B200NN_PROF_COUNT entries.  Where a block's two LayerNorms ride along with the Linears behind them (models of up to
+ * 2048 columns with one or two sequences, f32 models up to four) their work counts as B200NN_PROF_LINEAR, here and in
+ * b200nn_session_time_family; B200NN_PROF_LAYERNORM is then the final norm alone. */
 enum {
     B200NN_PROF_EMBED = 0, B200NN_PROF_LAYERNORM, B200NN_PROF_LINEAR, B200NN_PROF_ATTENTION,
     B200NN_PROF_LM_HEAD, B200NN_PROF_ARGMAX, B200NN_PROF_RECURRENCE, B200NN_PROF_COUNT

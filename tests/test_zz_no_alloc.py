@@ -2,14 +2,13 @@
 
 Some hosts of this library may not let it allocate device memory: they have given away their whole
 memory budget up front, or they call from a place where cudaMalloc would stall the device.  For
-them `b200nn_decode_attention_noalloc` runs the split-context decode-attention kernel with its
-scratch in a fixed array inside the library image.  This test calls it through the C ABI on
-caller-owned buffers, twice in a row (the calls share the scratch, so the second call proves that
-nothing stale is left behind), and compares each result with the regular entry point
-(`b200nn_attention_kv`, one head at a time) and with the CPU oracle's f64 attention at the attention
-tests' tolerance of 1e-4.  That nothing is allocated is checked on the driver's own figure
-(free device bytes from cudaMemGetInfo, which a cudaMalloc inside the library would lower), after
-a first call has done the per-device set-up.
+them `b200nn_decode_attention_noalloc` runs the split-context decode-attention kernel, whose partial
+results stay in the shared memory of a cluster: nothing is left behind by a call, and calls on different
+streams share nothing.  The tests call it through the C ABI on caller-owned buffers and compare the
+results with the regular entry point (`b200nn_attention_kv`, one head at a time) and with the CPU
+oracle's f64 attention at the attention tests' tolerance of 1e-4.  That nothing is allocated is checked on
+the driver's own figure (free device bytes from cudaMemGetInfo, which a cudaMalloc inside the library
+would lower), after a first call has done the per-device set-up.
 
 The file sorts last on purpose: if it fails, `pytest -x` has already run every other test.
 """
@@ -55,7 +54,7 @@ def test_no_alloc_entry_matches_regular_entry_twice(reg, B, H, cap, ctx_lens):
     lib = b200nn.load_library()
     rng = np.random.default_rng(B * 100 + H)
     dev = torch.device("cuda", reg.device)
-    for call, ctx_len in enumerate(ctx_lens):  # two calls in a row on the same scratch, different shapes of work
+    for call, ctx_len in enumerate(ctx_lens):
         q = rng.standard_normal((B, H * 64)).astype(np.float32)
         k16 = rng.standard_normal((B, H, cap, 64)).astype(np.float16)
         v16 = rng.standard_normal((B, H, cap, 64)).astype(np.float16)
@@ -65,7 +64,7 @@ def test_no_alloc_entry_matches_regular_entry_twice(reg, B, H, cap, ctx_lens):
         v_d = torch.from_numpy(v16).to(dev)
         out_d = torch.full((B, H * 64), float("nan"), device=dev, dtype=torch.float32)
         args = (reg.device, None, q_d.data_ptr(), k_d.data_ptr(), v_d.data_ptr(), B, H, cap, ctx_len, out_d.data_ptr())
-        if call == 0:  # the first call on a device looks the scratch's address up (module load, symbol lookup)
+        if call == 0:  # the first call on a device sets the kernel up (module load, function attributes)
             assert lib.b200nn_decode_attention_noalloc(*args) == 0, lib.b200nn_noalloc_last_error()
         torch.cuda.synchronize()
         free_before = torch.cuda.mem_get_info(dev)[0]
@@ -82,9 +81,8 @@ def test_no_alloc_entry_matches_regular_entry_twice(reg, B, H, cap, ctx_lens):
 
 
 def test_no_alloc_entry_at_the_largest_accepted_size(reg):
-    """batch x heads = 4096, the most the fixed scratch takes: the split count is then limited by the
-    fixed record array (16384 / 4096 = 4 splits of a 300-row context), not by the kernel's own rule.
-    Checked against the oracle on a sample of sequences and for two calls in a row giving the same bits."""
+    """batch x heads = 4096: a block per pair, several waves of them, no splits.  Checked against the oracle on a
+    sample of sequences and for two calls in a row giving the same bits."""
     import torch
 
     lib = b200nn.load_library()
@@ -110,6 +108,57 @@ def test_no_alloc_entry_at_the_largest_accepted_size(reg):
     assert np.abs(outs[0][sample] - orc).max() < 1e-4
 
 
+@pytest.mark.parametrize("B,H,cap,ctx_len", [(1, 1, 4100, 4096), (1, 3, 9000, 8999), (2, 12, 2050, 2050), (3, 40, 700, 513), (1, 1, 600, 512)])
+def test_no_alloc_entry_of_few_pairs_and_long_contexts(reg, B, H, cap, ctx_len):
+    """Eight splits merged over a cluster, with blocks of 16, 8 and 4 warps."""
+    import torch
+
+    lib = b200nn.load_library()
+    rng = np.random.default_rng(ctx_len)
+    dev = torch.device("cuda", reg.device)
+    q = rng.standard_normal((B, H * 64)).astype(np.float32)
+    k16, v16 = (rng.standard_normal((B, H, cap, 64)).astype(np.float16) for _ in range(2))
+    k16[:, :, ctx_len:], v16[:, :, ctx_len:] = np.nan, np.nan  # not looked at
+    q_d, k_d, v_d = (torch.from_numpy(a).to(dev) for a in (q, k16, v16))
+    out_d = torch.full((B, H * 64), float("nan"), device=dev)
+    torch.cuda.synchronize()
+    assert lib.b200nn_decode_attention_noalloc(reg.device, None, q_d.data_ptr(), k_d.data_ptr(), v_d.data_ptr(), B, H, cap, ctx_len, out_d.data_ptr()) == 0
+    torch.cuda.synchronize()
+    assert np.abs(out_d.cpu().numpy() - _oracle_rows(q, k16, v16, ctx_len)).max() < 1e-4
+
+
+def test_no_alloc_calls_on_two_streams_do_not_meet(reg):
+    """Calls queued on two streams overlap on the GPU; each gives the bits it gives alone."""
+    import torch
+
+    lib = b200nn.load_library()
+    g = torch.Generator(device="cuda")
+    g.manual_seed(11)
+    H, cap = 2, 4096
+    q, k, v = [], [], []
+    for _ in range(2):
+        q.append(torch.randn(1, H * 64, generator=g, device="cuda"))
+        k.append(torch.randn(1, H, cap, 64, generator=g, device="cuda").half())
+        v.append(torch.randn(1, H, cap, 64, generator=g, device="cuda").half())
+
+    def call(i, stream, out):
+        assert lib.b200nn_decode_attention_noalloc(reg.device, stream, q[i].data_ptr(), k[i].data_ptr(), v[i].data_ptr(), 1, H, cap, cap - i, out.data_ptr()) == 0
+
+    alone = [torch.empty(1, H * 64, device="cuda") for _ in range(2)]
+    for i in range(2):
+        call(i, None, alone[i])
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    outs = [torch.zeros(20, H * 64, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    for turn in range(20):
+        for i in range(2):
+            call(i, streams[i].cuda_stream, outs[i][turn])
+    torch.cuda.synchronize()
+    for i in range(2):
+        assert torch.equal(outs[i], alone[i].expand(20, -1))
+
+
 def test_no_alloc_entry_rejects_oversized_and_bad_arguments(reg):
     import torch
 
@@ -117,7 +166,7 @@ def test_no_alloc_entry_rejects_oversized_and_bad_arguments(reg):
     dev = torch.device("cuda", reg.device)
     buf = torch.zeros(64, device=dev)
     p = buf.data_ptr()
-    # 4097 (sequence, head) pairs: beyond the fixed scratch
+    # 4097 (sequence, head) pairs: beyond the limit
     assert lib.b200nn_decode_attention_noalloc(reg.device, None, p, p, p, 4097, 1, 8, 4, p) == b200nn.ERR_SHAPE
     assert b"4096" in lib.b200nn_noalloc_last_error()
     assert lib.b200nn_decode_attention_noalloc(reg.device, None, p, p, p, 1, 1, 8, 9, p) == b200nn.ERR_SHAPE  # ctx > capacity
