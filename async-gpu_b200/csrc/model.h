@@ -112,6 +112,7 @@ struct b200nn_gpt2 : b200nn_lm {
     std::vector<BlockW> blocks;
     LinearAny lm_head;
     bool ln_fold_ready = false;
+    std::shared_ptr<DevBuf> few_layers, few_maps; // decode_few.cu: per-layer pointers, tensor maps of the weights (on first use)
     int act() const { return (flags & B200NN_GELU_SIGMOID) ? B200NN_ACT_GELU_SIGMOID : B200NN_ACT_GELU_TANH; }
 };
 
@@ -237,6 +238,9 @@ struct b200nn_session {
     // MLP hidden GEMMs (zero at rest), grid counter + per-phase nanoseconds
     bool persist = false;
     std::shared_ptr<DevBuf> pd_layers, pd_qkv_acc, pd_fc_acc, pd_sync;
+    // steps of few rows (decode_few.cu): exchanged words, the ring's position and the step's parity behind them
+    bool few = false;
+    std::shared_ptr<DevBuf> few_words;
     int *pos_ptr() const { return static_cast<int *>(counters->p); }
     int *step_ptr() const { return static_cast<int *>(counters->p) + 1; }
 };
@@ -245,3 +249,9 @@ struct b200nn_session {
 bool decode_persistent_supported(const b200nn_gpt2 *m, int rows);
 int decode_persistent_prepare(b200nn_session *s);
 int launch_decode_layers(b200nn_session *s, bool profile);
+
+// Decode steps of few rows, layers, head and pick, as one persistent cooperative kernel; restart: after a prompt.
+bool decode_few_supported(const b200nn_gpt2 *m, int rows, int cap);
+int decode_few_prepare(b200nn_session *s);
+int decode_few_restart(b200nn_session *s);
+int launch_decode_few(b200nn_session *s, int n_steps);

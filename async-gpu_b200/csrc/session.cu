@@ -144,6 +144,10 @@ extern "C" int32_t b200nn_lm_session_create(b200nn_lm *m, size_t batch, size_t c
         TRY(decode_persistent_prepare(s.get()));
         s->persist = true;
     }
+    if (s->gpt2 && decode_few_supported(s->gpt2, (int)batch, (int)capacity)) {
+        TRY(decode_few_prepare(s.get()));
+        s->few = true;
+    }
     *out = s.release();
     return B200NN_OK;
 }
@@ -207,6 +211,7 @@ extern "C" int32_t b200nn_session_prefill(b200nn_session *s, const uint32_t *pro
     // record: history[0] = first token, step = 1, position = prompt_len
     TRY(launch_record_tokens(ctx, (const uint32_t *)s->ws_step.tok->p, (int)s->batch, (uint32_t *)s->history->p,
                              (int)s->hist_cap, s->step_ptr(), s->pos_ptr()));
+    if (s->few) TRY(decode_few_restart(s));
     s->position = prompt_len;
     s->steps_done = 1;
     s->prefilled = true;
@@ -248,6 +253,14 @@ extern "C" int32_t b200nn_session_step(b200nn_session *s, size_t n_steps) {
     if (s->position + n_steps > s->cap) return set_error(ctx, B200NN_ERR_DIM, "session_step: capacity exceeded");
     CK(ctx, cudaSetDevice(ctx->device));
     size_t done = 0;
+    if (s->few && ctx->few && !model_act_half(s->gpt2, (int)s->batch)) {
+        // whole steps in one launch, not too many of them: the kernel holds every SM until it ends
+        for (; done < n_steps; done += std::min<size_t>(32, n_steps - done)) TRY(launch_decode_few(s, (int)std::min<size_t>(32, n_steps - done)));
+        s->position += n_steps;
+        s->steps_done += n_steps;
+        s->kv.len = s->position;
+        return B200NN_OK;
+    }
     if (s->persist && ctx->persist) {
         // a step is six launches (embedding, the persistent kernel, final norm, LM head, argmax, record):
         // nothing to gain from a graph, and the cooperative launch stays an ordinary launch

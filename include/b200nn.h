@@ -137,6 +137,10 @@ B200NN_API int32_t b200nn_ctx_set_gemv_max_rows(b200nn_ctx *ctx, int32_t rows);
  * windowed layer's ring holds the window plus this many rows.  Read when a cache or session is created.
  * "delta_cols" (default 0 = by the amount of work): state columns per lane of the prompt kernels of the delta rules and
  * the mLSTM (1 or 2).
+ * "few" (default 1): the steps of a GPT-2 decode session of few sequences (int4 at most 2, f32 at most 4; all Linears and
+ * the output matrix of one kind) run as one persistent cooperative kernel, up to 32 steps per launch; 0: one kernel
+ * per operation.  "few_fault_layer" (test aid): one block leaves out its q/k/v words of that layer, so that the bounded
+ * waits ("persist_wait_kcycles") run out and B200NN_ERR_DEVICE is reported.
  * "persist" (default 0): decode steps of an int4 model run all transformer blocks as one cooperative
  * kernel (decode sessions whose shape it supports).  Measured slower than the per-op CUDA graph.
  * Its aids: "persist_min_rows" / "persist_max_rows" (batch range it is used for), "persist_prefetch_mb",

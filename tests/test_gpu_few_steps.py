@@ -1,0 +1,99 @@
+"""Decode steps of few sequences as one persistent kernel (tuning key "few"): against the oracle and against the same
+steps launched one kernel per operation."""
+import numpy as np
+import pytest
+
+import b200nn
+import np_ref
+from b200nn import DecodeSession, Gpt2Config, Gpt2Model, Int4Gpt2Model, synth
+from oracle import oracle
+from test_gpu_model import MAX_ABS, REL_RMS, _check_tokens, _int4_oracle_weights
+
+pytestmark = pytest.mark.gpu
+
+
+def _steps(reg, m, prompts, n_new, few, flags=0):
+    reg.set_tuning("few", few)
+    try:
+        B, P = prompts.shape
+        s = DecodeSession(m, batch=B, capacity=P + n_new, flags=flags)
+        s.prefill(prompts)
+        s.step(1)
+        launches = reg.launch_count()
+        s.step(n_new - 2)
+        return s.tokens(), s.logits(), reg.launch_count() - launches
+    finally:
+        reg.set_tuning("few", 1)
+
+
+# The narrowest model (12 blocks, one K unit per part, fewer tiles of the output matrix than blocks); contexts that cross one
+# and three context splits of 120 rows; three of four row slots; more steps than a launch takes; an odd group of 192;
+# one, three and two K parts of the projections (GPT-2 XL's, Small's and Medium's widths); an output matrix of 22 tiles a block.
+@pytest.mark.parametrize("family,d,layers,vocab,B,P,N,group", [
+    ("f32", 64, 1, 131, 4, 9, 5, 0), ("f32", 128, 2, 257, 3, 117, 8, 0), ("int4", 128, 3, 257, 2, 9, 40, 64),
+    ("int4", 192, 2, 1031, 1, 357, 7, 192), ("f32", 768, 2, 50257, 1, 33, 5, 0), ("f32", 1024, 1, 3001, 4, 20, 5, 0),
+    ("int4", 768, 2, 5003, 2, 250, 5, 128), ("int4", 1600, 2, 50257, 1, 77, 5, 128)])
+def test_steps_in_one_kernel_match_oracle_and_per_operation_path(reg, family, d, layers, vocab, B, P, N, group):
+    cfg = Gpt2Config(n_layer=layers, n_embd=d, n_head=d // 64, vocab_size=vocab, n_positions=400)
+    w = synth.gpt2_weights(cfg, base_seed=70 + d, std=0.08 if d < 512 else 0.02, random_ln=True)
+    m = Gpt2Model(w, cfg, reg) if family == "f32" else Int4Gpt2Model(w, cfg, reg, flags=b200nn.QUANT_LM_HEAD, group_size=group)
+    prompts = synth.token_ids(d + B, (B, P), vocab)
+    tok, lg, launches = _steps(reg, m, prompts, N, 1)
+    tok_o, lg_o, launches_o = _steps(reg, m, prompts, N, 0)
+    assert reg.device_error() == 0
+    assert launches == (N - 2 + 31) // 32 and launches_o > launches * layers
+    # The paths differ by the order of f32 sums, and where that turns the fp16 rounding of a cached value, by 2^-11 of it:
+    # under 1e-3 in logits of spread one.  A near-tie may turn a pick, and all that follows it.
+    same = (tok == tok_o).all(axis=1)
+    assert same.sum() >= B - 1
+    assert not same.any() or np.abs(lg - lg_o)[same].max() < 1e-3
+    if d <= 768 and vocab < 10000:
+        om = oracle.Model(cfg.as_dict(), w if family == "f32" else _int4_oracle_weights(m, cfg, w, True))
+        for b in sorted({0, B - 1}):
+            ref, lr = om.generate_cached(prompts[b], N, flags=oracle.KV_FP16, want_logits=True)
+            _check_tokens(np.concatenate([prompts[b], tok[b]]), ref, lr, P)
+            if np.array_equal(tok[b], ref[P:]):
+                assert np.abs(lg[b] - lr[-1]).max() < MAX_ABS and np_ref.rel_rms(lg[b], lr[-1]) < REL_RMS
+
+
+def test_steps_in_one_kernel_rewind_and_last_index_picks(reg):
+    """Equal logits everywhere: the last index wins when asked for.  Steps taken again after a rewind give the same."""
+    cfg = Gpt2Config(n_layer=2, n_embd=128, n_head=2, vocab_size=259, n_positions=64)
+    w = dict(synth.gpt2_weights(cfg, base_seed=3, std=0.08))
+    m = Gpt2Model(w, cfg, reg)
+    prompts = synth.token_ids(4, (2, 9), cfg.vocab_size)
+    s = DecodeSession(m, batch=2, capacity=40)
+    s.prefill(prompts)
+    s.step(12)
+    first = s.logits()
+    s.rewind(20)
+    s.step(1)
+    assert s.tokens().shape[1] == 13 and np.isfinite(s.logits()).all() and first.shape == s.logits().shape
+    w["wte"] = np.zeros_like(w["wte"])
+    flat = Gpt2Model(w, cfg, reg)
+    for flags, pick in ((0, 0), (b200nn.ARGMAX_LAST, cfg.vocab_size - 1)):
+        assert (_steps(reg, flat, prompts, 5, 1, flags)[0] == pick).all()
+
+
+def test_steps_in_one_kernel_wait_runs_out_and_session_recovers(reg):
+    cfg = Gpt2Config(n_layer=3, n_embd=128, n_head=2, vocab_size=257, n_positions=64)
+    m = Gpt2Model(synth.gpt2_weights(cfg, base_seed=77, std=0.08, random_ln=True), cfg, reg)
+    prompts = synth.token_ids(5, (2, 9), cfg.vocab_size)
+    s = DecodeSession(m, batch=2, capacity=40)
+
+    def run():
+        s.prefill(prompts)
+        s.step(6)
+        return s.tokens(), s.logits()
+    good = run()
+    reg.set_tuning("persist_wait_kcycles", 2000)  # about a millisecond of SM clocks
+    reg.set_tuning("few_fault_layer", 1)
+    try:
+        with pytest.raises(b200nn.NnError) as e:
+            run()
+        assert e.value.code == b200nn.ERR_DEVICE and reg.device_error() == 0
+    finally:
+        reg.set_tuning("few_fault_layer", -1)
+        reg.set_tuning("persist_wait_kcycles", 0)
+    again = run()  # a new prompt starts the exchanged words over
+    assert np.array_equal(again[0], good[0]) and np.array_equal(again[1], good[1]) and reg.device_error() == 0
