@@ -71,6 +71,10 @@ extern "C" int32_t b200nn_int4_linear_forward_dev(b200nn_int4_linear *l, const f
     e.out = y_dev;
     e.ldo = l->l.N;
     const Int4Weight &w = l->l.q;
+    if (m <= 8 && int4_rows_supported(ctx, w, x_dev, (int)m)) { // takes the f32 rows as they are
+        e.bias = l->l.bias();
+        return launch_int4_rows(ctx, w, x_dev, (int)m, e);
+    }
     if (w.fast && (int)m > ctx->gemv_max_rows && int4_gemm_tc_supported(w, (int)m)) {
         // tensor-core path consumes fp16 activations
         size_t need = m * (size_t)w.K * sizeof(__half);

@@ -40,6 +40,7 @@ struct b200nn_ctx {
     int last_cuda = 0;
     int sm_count = 148;
     int gemv_max_rows = 2;       // rows at or below this take the CUDA-core GEMV
+    int int4_rows_max = 8;       // stand-alone int4 Linears of more f32 rows than that, and up to this, take the mma.sync kernel
     int ln_rows_min = 1024;      // LayerNorm of at least this many rows (no residual) takes the warp-per-row kernel
     int ln_fold = 0;             // 1: decode steps of int4 models fold each block LayerNorm into the GEMMs around it (measured slower than the LayerNorm kernels: the residual GEMMs then need complete sums, i.e. cluster splits)
     int fused_argmax = 1;        // greedy decode steps take the argmax in the LM head's epilogue (0: separate kernel)
@@ -337,6 +338,9 @@ static constexpr int F32_GEMV_ROWS = 4; // rows that the f32 GEMV serves
 int launch_int4_linear(b200nn_ctx *ctx, const Int4Weight &w, const void *x, bool x_half, int M, const Epilogue &epi, const NormIn &ln = NormIn());
 int launch_int4_gemv(b200nn_ctx *ctx, const Int4Weight &w, const void *x, bool x_half, int M, const Epilogue &epi, const NormIn &ln = NormIn());
 bool int4_linear_takes_norm(const Int4Weight &w, int M);
+// x: [M,K] f32, three to eight rows, bias, activation and f32 output of the epilogue
+bool int4_rows_supported(const b200nn_ctx *ctx, const Int4Weight &w, const float *x, int M);
+int launch_int4_rows(b200nn_ctx *ctx, const Int4Weight &w, const float *x, int M, const Epilogue &epi);
 int launch_int4_naive(b200nn_ctx *ctx, const Int4Weight &w, const void *x, bool x_half, int M, const Epilogue &epi);
 bool int4_gemm_tc_supported(const Int4Weight &w, int M);
 int launch_int4_gemm_tc(b200nn_ctx *ctx, const Int4Weight &w, const __half *x, int M, const Epilogue &epi);

@@ -137,6 +137,8 @@ B200NN_API int32_t b200nn_ctx_set_gemv_max_rows(b200nn_ctx *ctx, int32_t rows);
  * windowed layer's ring holds the window plus this many rows.  Read when a cache or session is created.
  * "delta_cols" (default 0 = by the amount of work): state columns per lane of the prompt kernels of the delta rules and
  * the mLSTM (1 or 2).
+ * "int4_rows_max" (default 8, at most that; negative restores it): a stand-alone int4 Linear of three f32 rows to this many runs as
+ * one mma.sync kernel (no conversion launch); 0: always the conversion and the tcgen05 GEMM.
  * "few" (default 1): the steps of a GPT-2 decode session of few sequences (int4 at most 2, f32 at most 4; all Linears and
  * the output matrix of one kind) run as one persistent cooperative kernel, up to 32 steps per launch; 0: one kernel
  * per operation.  "few_fault_layer" (test aid): one block leaves out its q/k/v words of that layer, so that the bounded
