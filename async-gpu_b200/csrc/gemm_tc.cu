@@ -59,7 +59,7 @@ __device__ __forceinline__ void bar_sync_dequant() {
 // tiles in TMEM); NP: packed-weight stages; NG: dequant groups; TC: TMEM columns to allocate.
 // EK: what becomes of the sums (EpiKind).
 template <int MB, int NS, int NP, int NG, int TC, int EK>
-__global__ void __launch_bounds__(96 + 128 * NG, NG == 2 ? 2 : 1)
+__global__ void __launch_bounds__(96 + 128 * NG, NG == 1 ? 4 : NG == 2 ? 2 : 1)
 int4_gemm_tc_kernel(const uint8_t *__restrict__ tiles, const __half *__restrict__ scales,
                     const __grid_constant__ CUtensorMap tmap_x, int M, int N, int k_blocks, int n_pad, int group,
                     int kb_per_split, int cluster_mode, Epilogue epi, float *__restrict__ scratch,
@@ -460,7 +460,7 @@ int launch_cfg(b200nn_ctx *ctx, const Int4Weight &w, const __half *x, int M, con
     constexpr size_t smem_fixed = 1024 + ring + bar_bytes;
     // Blocks an SM holds at once: two for the variants with two dequant groups (352 threads, built
     // for at most 93 registers) when their shared memory and TMEM columns fit twice, else one.
-    const int ctas_per_sm = (NG == 2 && smem_fixed + 8192 <= 113 * 1024 && 2 * TC <= 512) ? 2 : 1;
+    const int ctas_per_sm = NG == 1 ? 4 : (NG == 2 && smem_fixed + 8192 <= 113 * 1024 && 2 * TC <= 512) ? 2 : 1;
     // K split: fills the GPU when there are few (feature tile x token tile) pairs.  The count is
     // rounded down, because one block more than the SMs can hold costs a whole second wave.  The
     // residual epilogue reduces its splits with L2 vector adds, which is cheap, so it splits down to
@@ -534,7 +534,12 @@ int launch_int4_gemm_tc(b200nn_ctx *ctx, const Int4Weight &w, const __half *x, i
     int mb = 32;
     while (mb < M && mb < cap) mb <<= 1;
     switch (mb) { //            MB  NS  NP NG  TMEM columns
-        case 32: return launch_cfg<32, 7, 16, 2, 256>(ctx, w, x, M, epi);
+        case 32:
+            // more tiles than two blocks per SM hold (an output matrix): four blocks with a dequant group each leave no second
+            // wave (768 x 50257, 32 rows with their conversion 14.8 -> 11.4 us); from about 20 K blocks on the one group is what
+            // a block waits for (1600 x 50257: 20.9 and 21.7 us)
+            if (w.n_tiles > 2 * ctx->sm_count && w.k_blocks <= 16) return launch_cfg<32, 3, 8, 1, 128>(ctx, w, x, M, epi);
+            return launch_cfg<32, 7, 16, 2, 256>(ctx, w, x, M, epi);
         case 64:
             // more tiles than SMs (an output matrix): two smaller blocks per SM, so that one's epilogue runs under the other's loop
             if (w.n_tiles > ctx->sm_count) return launch_cfg<64, 4, 8, 2, 256>(ctx, w, x, M, epi);
