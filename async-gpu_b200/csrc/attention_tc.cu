@@ -1,26 +1,26 @@
 // Causal prefill attention on the tensor cores (tcgen05, accumulators in tensor memory), pipelined.
 //
-// One block per (128-query tile, head, sequence), ten warps with fixed roles:
-//   warp 0      copies: the Q tile once, then the K and V tiles of every 128-key step through tensor maps
+// Two persistent blocks per SM; each takes items (128-query tile, sequence, head) in turn, its copies and MMAs running on
+// into the next item while the last one's output leaves.  Two warpgroups with fixed roles:
+//   warp 0      copies: an item's Q tile, then the K and V tiles of its 128-key steps through tensor maps
 //               (cp.async.bulk.tensor, 128-byte swizzle, zero fill past the last cached row) into two-stage
 //               rings; no hand-written shared-memory stores anywhere
-//   warp 1      MMA issue: S_j = Q K_j^T into one of two score buffers in TMEM, then O_j = P_j V_j with
-//               P read from tensor memory (A operand) and V straight from its row-major tile (B operand
-//               MN-major: no transposition)
-//   warps 2..9  softmax: two threads per query row (= TMEM lane r), in two warps of the same lane quarter; each takes half of
-//               the keys of a step and half of the 64 output columns.  Pass 1 takes the maximum of the half row, the two
-//               threads exchange theirs through shared memory; then the previous step's O_{j-1} is fetched
-//               from TMEM and folded into the running output (32 f32 per thread, rescaled by that step's
-//               correction); pass 2 writes p = exp2(s*scale - max) back over S_j as packed fp16.
-// Per step the tensor pipe therefore works on S_{j+1} and O_{j-1} while the softmax warps are busy
-// with step j; two blocks per SM cover what is left of each other's gaps.  What bounds it is the softmax's chain of
-// TMEM round trips, exponentials and hand-overs (the exponentials alone take a third of the time): hence sixteen
-// softmax warps per SM (8 prompts of 1024, 12 heads: 42.5 us with one thread per row, 38.9 with two).
+//   warp 1      MMA issue: S_t = Q K_t^T as soon as the softmax threads have S_{t-1} in their registers, then
+//               O (+)= P_{t-1} V_{t-1} with P read from tensor memory (A operand) and V straight from its row-major tile
+//               (B operand MN-major: no transposition)
+//   warps 4..7  softmax: one thread per query row (= TMEM lane).  It takes the row's 128 scores once and keeps them in registers
+//               from the maximum to the exponentials; p = exp2(s*scale - max) goes to tensor memory as packed fp16 when
+//               the step before has finished with its own.  O stays in tensor memory over an item's steps and is
+//               rescaled where a maximum has moved.
+// A thread needs about 190 registers: the other warpgroup hands over its own (setmaxnreg: 40 + 208 of the 2 x 128 that the block
+// was launched with).  What bounds it is the exponentials (16 per cycle and SM: 1024 of the 1800 cycles of a 128 x 128
+// step) and the chain of a step that the other block's step has to cover: 125 cycles of TMEM loads, 250 of maxima, 1400 of
+// exponentials, 300 of hand-overs.  Against one block per item, two threads per row, scores read twice, O folded into
+// registers every step, 12 / 12 / 25 heads, us: 8 prompts of 1024 37.6 / 31.4 now, 32 of 512 49.7 / 37.6, 16 of 400 behind 100
+// 59.1 / 45.1.  A reference that moves only past 2^8 saves another microsecond, and loses the exactness of the
+// largest probabilities (error 2.51e-4 -> 2.55e-4): not taken.  A quarter of the exponentials as polynomials: no gain.
 //
-// TMEM (256 columns per block): score buffer b at columns 128 b .. 128 b + 127.  P_j (fp16 pairs) goes over columns 0..31
-// (keys 0..63) and 96..127 (keys 64..127) of its own buffer: each thread writes only over scores that it has
-// loaded itself, the second half of the keys from the last column down.  O_j lands in columns 32..95 of the
-// same buffer, free once pass 2 is over.
+// TMEM (256 columns per block): S at columns 0..127, P (fp16 pairs) at 128..191, O at 192..255.
 //
 // Replaces flash_attention_v2 / flash_attn_v3.cu of the reference (compute_transformer.rs:597-816,
 // cuda/flash_attn_v3.cu:29-283) for the model path, where q and the output are fp16.
@@ -29,6 +29,8 @@
 // roles leave their loops, nothing is stored, the TMEM columns are freed and the kernel returns.
 #include <cuda.h>
 
+#include <algorithm>
+
 #include "device_utils.cuh"
 #include "tc_ptx.cuh"
 
@@ -36,12 +38,12 @@ namespace {
 
 constexpr float SCALE_LOG2E = 0.125f * 1.4426950408889634f;
 constexpr float NEG_BIG = -1.0e30f;
-enum : uint32_t { ERR_ATT_Q = 0x41, ERR_ATT_K, ERR_ATT_V, ERR_ATT_S, ERR_ATT_P, ERR_ATT_O, ERR_ATT_FREE, ERR_ATT_KE, ERR_ATT_VE };
-constexpr int TM_COLS = 256;                // two score buffers
+enum : uint32_t { ERR_ATT_Q = 0x41, ERR_ATT_K, ERR_ATT_V, ERR_ATT_S, ERR_ATT_P, ERR_ATT_O, ERR_ATT_FREE, ERR_ATT_KE, ERR_ATT_VE, ERR_ATT_QE };
+constexpr int TM_COLS = 256, TM_P = 128, TM_O = 192;
 constexpr int KV_STAGES = 2;
 constexpr int TILE = 16384;                 // 128 rows x 64 fp16
-constexpr int SMEM_BYTES = (1 + 2 * KV_STAGES) * TILE + 1024; // Q, K ring, V ring + alignment slack
-constexpr int NTHREADS = 320, SOFTMAX = 256;
+constexpr int SMEM_BYTES = (2 + 2 * KV_STAGES) * TILE + 1024; // Q of two items, K ring, V ring + alignment slack
+constexpr int NTHREADS = 256, SOFTMAX = 128;
 
 __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
     __half2 h = __floats2half2_rn(a, b);
@@ -49,43 +51,56 @@ __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
 }
 
 struct Bars {
-    uint64_t q_full;
+    uint64_t q_full[2], q_empty[2];
     uint64_t k_full[KV_STAGES], k_empty[KV_STAGES], v_full[KV_STAGES], v_empty[KV_STAGES];
-    uint64_t s_full[2], p_full[2], o_full[2], s_free[2];
+    uint64_t s_full, s_free, p_full, o_full; // one phase per step
 };
 
 __global__ void __launch_bounds__(NTHREADS, 2)
 prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                       const __grid_constant__ CUtensorMap tm_v, int H, int cap, int S, int past, __half *__restrict__ out,
-                       int ldo, uint32_t *__restrict__ dev_err) {
+                       const __grid_constant__ CUtensorMap tm_v, int H, int pairs, int cap, int S, int past,
+                       __half *__restrict__ out, int ldo, uint32_t *__restrict__ dev_err) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) Bars bars;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
-    __shared__ float pair_x[2][2][128]; // what the two threads of a row tell each other: [step parity][half][row]
 
-    // the query tiles with the most key tiles are scheduled first (blocks start in index order)
-    const int qt = gridDim.z - 1 - blockIdx.z, h = blockIdx.y, b = blockIdx.x;
+    // Items are (query tile, sequence, head), those with the most key tiles first; a block's n-th is dealt out forwards and
+    // backwards in turn, so that blocks come out even.
+    const int q_tiles = (S + 127) / 128, n_items = q_tiles * pairs;
+    struct Item {
+        int qt, bh, kv_end, n_tiles;
+    };
+    auto item_at = [&](int n, Item &it) {
+        const int i = n * gridDim.x + ((n & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+        if (i >= n_items) return false;
+        it.qt = q_tiles - 1 - i / pairs;
+        it.bh = i % pairs;
+        it.kv_end = min(past + min(S, it.qt * 128 + 128), cap); // keys this tile's queries can see
+        it.n_tiles = (it.kv_end + 127) / 128;
+        return true;
+    };
     const int tid = threadIdx.x, warp = tid >> 5;
     const uint32_t base = (tc::smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t sQ = base, sK = base + TILE, sV = base + TILE * (1 + KV_STAGES);
+    const uint32_t sQ = base, sK = base + 2 * TILE, sV = base + TILE * (2 + KV_STAGES);
     auto bar = [&](const uint64_t &x) { return tc::smem_u32(&x); };
 
     if (tid == 0) {
         abort_flag = 0;
-        tc::mbar_init(bar(bars.q_full), 1);
+        for (int i = 0; i < 2; ++i) {
+            tc::mbar_init(bar(bars.q_full[i]), 1);
+            tc::mbar_init(bar(bars.q_empty[i]), 1);
+        }
         for (int i = 0; i < KV_STAGES; ++i) {
             tc::mbar_init(bar(bars.k_full[i]), 1);
             tc::mbar_init(bar(bars.k_empty[i]), 1);
             tc::mbar_init(bar(bars.v_full[i]), 1);
             tc::mbar_init(bar(bars.v_empty[i]), 1);
         }
-        for (int i = 0; i < 2; ++i) {
-            tc::mbar_init(bar(bars.s_full[i]), 1);
-            tc::mbar_init(bar(bars.p_full[i]), SOFTMAX); // every softmax thread
-            tc::mbar_init(bar(bars.o_full[i]), 1);
-            tc::mbar_init(bar(bars.s_free[i]), SOFTMAX);
-        }
+        tc::mbar_init(bar(bars.s_full), 1);
+        tc::mbar_init(bar(bars.s_free), SOFTMAX / 32); // every softmax warp
+        tc::mbar_init(bar(bars.p_full), SOFTMAX / 32);
+        tc::mbar_init(bar(bars.o_full), 1);
         tc::fence_mbar_init();
     }
     if (warp == 0) {
@@ -99,189 +114,211 @@ prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     tc::tc_fence_after_sync();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(&tmem_slot);
 
-    const int kv_end = min(past + min(S, qt * 128 + 128), cap); // keys this tile's queries can see
-    const int n_tiles = (kv_end + 127) / 128;
-    const int bh = b * H + h;
-
-    if (warp == 0) {
-        // ---- copies (one elected lane issues; the warp stays converged on the waits) ----
-        if (tc::elect_one()) {
-            tc::mbar_expect_tx(bar(bars.q_full), TILE);
-            tc::tma_load_2d(sQ, &tm_q, h * 64, b * S + qt * 128, bar(bars.q_full));
-        }
-        for (int j = 0; j < n_tiles; ++j) {
-            const int st = j % KV_STAGES, u = j / KV_STAGES;
-            if (j >= KV_STAGES && !tc::mbar_wait(bar(bars.k_empty[st]), (u - 1) & 1, &abort_flag, dev_err, ERR_ATT_KE)) break;
-            if (tc::elect_one()) {
-                tc::mbar_expect_tx(bar(bars.k_full[st]), TILE);
-                tc::tma_load_3d(sK + st * TILE, &tm_k, 0, j * 128, bh, bar(bars.k_full[st]));
-            }
-            if (j >= KV_STAGES && !tc::mbar_wait(bar(bars.v_empty[st]), (u - 1) & 1, &abort_flag, dev_err, ERR_ATT_VE)) break;
-            if (tc::elect_one()) {
-                tc::mbar_expect_tx(bar(bars.v_full[st]), TILE);
-                tc::tma_load_3d(sV + st * TILE, &tm_v, 0, j * 128, bh, bar(bars.v_full[st]));
-            }
-        }
-    } else if (warp == 1) {
-        // ---- MMA issue: S_j as early as its buffer and K tile allow, then O_{j-1} once P_{j-1} is written ----
-        constexpr uint32_t idesc_s = tc::umma_idesc_f16(128, 128);
-        constexpr uint32_t idesc_o = tc::umma_idesc_f16_bmn(128, 64);
-        const uint64_t dq = tc::umma_desc_sw128(sQ);
-        bool ok = tc::mbar_wait(bar(bars.q_full), 0, &abort_flag, dev_err, ERR_ATT_Q);
-        for (int j = 0; ok && j <= n_tiles; ++j) {
-            if (j < n_tiles) {
-                const int bf = j & 1, st = j % KV_STAGES, u = j / KV_STAGES;
-                if (j >= 2) ok = tc::mbar_wait(bar(bars.s_free[bf]), ((j >> 1) - 1) & 1, &abort_flag, dev_err, ERR_ATT_FREE);
-                if (ok) ok = tc::mbar_wait(bar(bars.k_full[st]), u & 1, &abort_flag, dev_err, ERR_ATT_K);
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        Item it;
+        int t = 0; // step over all items
+        if (warp == 0) {
+            // ---- copies (one elected lane issues; the warp stays converged on the waits) ----
+            bool ok = true;
+            for (int n = 0; ok && item_at(n, it); ++n) {
+                if (n >= 2) ok = tc::mbar_wait(bar(bars.q_empty[n & 1]), ((n >> 1) - 1) & 1, &abort_flag, dev_err, ERR_ATT_QE);
                 if (!ok) break;
-                tc::tc_fence_after_sync();
                 if (tc::elect_one()) {
-                    const uint64_t dk = tc::umma_desc_sw128(sK + st * TILE);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) tc::umma_f16_ss(tmem_base + bf * 128, dq + 2 * k, dk + 2 * k, idesc_s, k != 0);
-                    tc::umma_commit(bar(bars.s_full[bf]));
-                    tc::umma_commit(bar(bars.k_empty[st]));
+                    tc::mbar_expect_tx(bar(bars.q_full[n & 1]), TILE);
+                    tc::tma_load_2d(sQ + (n & 1) * TILE, &tm_q, it.bh % H * 64, it.bh / H * S + it.qt * 128, bar(bars.q_full[n & 1]));
                 }
-                __syncwarp();
+                for (int j = 0; j < it.n_tiles; ++j, ++t) {
+                    const int st = t % KV_STAGES, u = t / KV_STAGES;
+                    if (t >= KV_STAGES) ok = tc::mbar_wait(bar(bars.k_empty[st]), (u - 1) & 1, &abort_flag, dev_err, ERR_ATT_KE);
+                    if (!ok) break;
+                    if (tc::elect_one()) {
+                        tc::mbar_expect_tx(bar(bars.k_full[st]), TILE);
+                        tc::tma_load_3d(sK + st * TILE, &tm_k, 0, j * 128, it.bh, bar(bars.k_full[st]));
+                    }
+                    if (t >= KV_STAGES) ok = tc::mbar_wait(bar(bars.v_empty[st]), (u - 1) & 1, &abort_flag, dev_err, ERR_ATT_VE);
+                    if (!ok) break;
+                    if (tc::elect_one()) {
+                        tc::mbar_expect_tx(bar(bars.v_full[st]), TILE);
+                        tc::tma_load_3d(sV + st * TILE, &tm_v, 0, j * 128, it.bh, bar(bars.v_full[st]));
+                    }
+                }
             }
-            if (j >= 1) {
-                const int jp = j - 1, bp = jp & 1, st = jp % KV_STAGES, u = jp / KV_STAGES;
-                ok = tc::mbar_wait(bar(bars.p_full[bp]), (jp >> 1) & 1, &abort_flag, dev_err, ERR_ATT_P);
-                if (ok) ok = tc::mbar_wait(bar(bars.v_full[st]), u & 1, &abort_flag, dev_err, ERR_ATT_V);
-                if (!ok) break;
+        } else if (warp == 1) {
+            // ---- MMA issue: S_t once S_{t-1} has been read and K_t is there, O (+)= P_{t-1} V_{t-1} once P_{t-1} is written ----
+            constexpr uint32_t idesc_s = tc::umma_idesc_f16(128, 128);
+            constexpr uint32_t idesc_o = tc::umma_idesc_f16_bmn(128, 64);
+            auto output = [&](int tp, bool first) {
+                const int st = tp % KV_STAGES, u = tp / KV_STAGES;
+                if (!tc::mbar_wait(bar(bars.p_full), tp & 1, &abort_flag, dev_err, ERR_ATT_P) ||
+                    !tc::mbar_wait(bar(bars.v_full[st]), u & 1, &abort_flag, dev_err, ERR_ATT_V))
+                    return false;
                 tc::tc_fence_after_sync();
                 if (tc::elect_one()) {
                     const uint64_t dv = tc::umma_desc_sw128_mn64(sV + st * TILE);
-                    const uint32_t buf = tmem_base + bp * 128;
 #pragma unroll
                     for (int k = 0; k < 8; ++k) // 16 keys per MMA: 8 TMEM columns of P, 2048 bytes of V
-                        tc::umma_f16_ts(buf + 32, buf + (k < 4 ? 8 * k : 64 + 8 * k), dv + (uint64_t)(k * (2048 >> 4)), idesc_o, k != 0);
-                    tc::umma_commit(bar(bars.o_full[bp]));
+                        tc::umma_f16_ts(tmem_base + TM_O, tmem_base + TM_P + 8 * k, dv + (uint64_t)(k * (2048 >> 4)), idesc_o, !first || k != 0);
+                    tc::umma_commit(bar(bars.o_full));
                     tc::umma_commit(bar(bars.v_empty[st]));
                 }
                 __syncwarp();
+                return true;
+            };
+            bool ok = true, first = true; // whether step t - 1 is its item's first
+            for (int n = 0; ok && item_at(n, it); ++n) {
+                ok = tc::mbar_wait(bar(bars.q_full[n & 1]), (n >> 1) & 1, &abort_flag, dev_err, ERR_ATT_Q);
+                const uint64_t dq = tc::umma_desc_sw128(sQ + (n & 1) * TILE);
+                for (int j = 0; ok && j < it.n_tiles; ++j, ++t) {
+                    const int st = t % KV_STAGES, u = t / KV_STAGES;
+                    if (t >= 1) ok = tc::mbar_wait(bar(bars.s_free), (t - 1) & 1, &abort_flag, dev_err, ERR_ATT_FREE);
+                    if (ok) ok = tc::mbar_wait(bar(bars.k_full[st]), u & 1, &abort_flag, dev_err, ERR_ATT_K);
+                    if (!ok) break;
+                    tc::tc_fence_after_sync();
+                    if (tc::elect_one()) {
+                        const uint64_t dk = tc::umma_desc_sw128(sK + st * TILE);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) tc::umma_f16_ss(tmem_base, dq + 2 * k, dk + 2 * k, idesc_s, k != 0);
+                        tc::umma_commit(bar(bars.s_full));
+                        tc::umma_commit(bar(bars.k_empty[st]));
+                        if (j + 1 == it.n_tiles) tc::umma_commit(bar(bars.q_empty[n & 1]));
+                    }
+                    __syncwarp();
+                    if (t >= 1) ok = output(t - 1, first);
+                    first = j == 0;
+                }
             }
+            if (ok) output(t - 1, first);
         }
     } else {
-        // ---- softmax and the running output: two threads per query row (= TMEM lane) ----
-        const int quad = warp & 3, row = quad * 32 + (tid & 31), half = (warp - 2) >> 2;
+        // ---- softmax: one thread per query row (= TMEM lane) ----
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+        const int quad = warp & 3, row = quad * 32 + (tid & 31);
         const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
-        const int s_row = qt * 128 + row;
-        const bool row_valid = s_row < S;
-        const int a_pos = past + s_row; // absolute position of this thread's query
-        float m = NEG_BIG, l = 0.0f, corr_prev = 1.0f;
-        float2 acc[16]; // output columns 32 half .. + 31
+        float m = NEG_BIG;
+        float2 l2[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+        uint4 *dst = nullptr; // output row of the item before (null: none, or past the sequence)
+        // The finished O of an item leaves (its last MMA has completed).
+        auto finish = [&]() {
+            const float inv = 1.0f / ((l2[0].x + l2[0].y) + (l2[1].x + l2[1].y));
 #pragma unroll
-        for (int e = 0; e < 16; ++e) acc[e] = make_float2(0.0f, 0.0f);
+            for (int i = 0; i < 2; ++i) {
+                uint32_t o[32];
+                tc::tmem_ld_x32(lane_base + TM_O + 32 * i, o);
+                if (dst)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        uint32_t w[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            w[e] = pack_half2(__uint_as_float(o[8 * c + 2 * e]) * inv, __uint_as_float(o[8 * c + 2 * e + 1]) * inv);
+                        dst[4 * i + c] = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
+            }
+        };
+        Item it;
+        int t = 0;
         bool ok = true;
-        // the value of the row's other thread (the two warps of a quarter meet at a barrier of their own)
-        auto exchange = [&](float x, int parity) {
-            pair_x[parity][half][row] = x;
-            asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory");
-            return pair_x[parity][half ^ 1][row];
-        };
-        // acc = acc * c + O_tile of score buffer bp (one TMEM round trip)
-        auto fold_output = [&](int bp, float c) {
-            uint32_t v[32];
-            tc::tmem_ld_x32(lane_base + bp * 128 + 32 + 32 * half, v);
-            const float2 c2 = make_float2(c, c);
+        for (int n = 0; ok && item_at(n, it); ++n) {
+            // Rows past the sequence are worked out like the others (their queries are the next sequence's, or zeros) and not stored.
+            const int s_row = it.qt * 128 + row, a_pos = past + s_row; // absolute position of this thread's query
+            const int warp_row = it.qt * 128 + quad * 32, warp_first = past + warp_row; // last key that all rows of the warp see
+            const int warp_last = warp_row < S ? min(warp_first + 31, it.kv_end - 1) : -1; // last key that any of them sees
+            for (int j = 0; j < it.n_tiles; ++j, ++t) {
+                const int j0 = j * 128;
+                ok = tc::mbar_wait(bar(bars.s_full), t & 1, &abort_flag, dev_err, ERR_ATT_S);
+                if (!ok) break;
+                tc::tc_fence_after_sync();
+                uint32_t v[2][64];
+                tc::tmem_ld_x64(lane_base, v[0]);
+                tc::tmem_ld_x64(lane_base + 64, v[1]);
+                tc::tc_fence_before_sync();
+                __syncwarp();
+                if ((tid & 31) == 0) tc::mbar_arrive(bar(bars.s_free)); // S_{t+1} may take their place
+                // the row may attend to keys up to a_pos.  Only the tile on the diagonal needs the mask: masked scores lie so far below any other that their exponentials are zero.
+                float mx[4] = {NEG_BIG, NEG_BIG, NEG_BIG, NEG_BIG}; // four independent chains
+                auto maxima = [&](int c) {
 #pragma unroll
-            for (int e = 0; e < 16; ++e)
-                acc[e] = __ffma2_rn(acc[e], c2, make_float2(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1])));
-        };
-        for (int j = 0; j < n_tiles; ++j) {
-            const int bf = j & 1, j0 = j * 128 + 64 * half;
-            const uint32_t sbuf = lane_base + bf * 128 + 64 * half;
-            // A warp whose wait gives up skips the step's work but still meets its partner at every exchange.
-            if (ok) ok = tc::mbar_wait(bar(bars.s_full[bf]), (j >> 1) & 1, &abort_flag, dev_err, ERR_ATT_S);
-            if (ok) tc::tc_fence_after_sync();
-            // columns of this half the row may attend to: keys j0 .. min(a_pos, kv_end-1); only the tile on
-            // the diagonal (and rows past the sequence) need the mask, the others take the short loops
-            int nvalid = row_valid ? min(a_pos, kv_end - 1) - j0 + 1 : 0;
-            nvalid = max(0, min(nvalid, 64));
-            const bool full = __all_sync(0xffffffffu, nvalid == 64);
-            float mx[4] = {NEG_BIG, NEG_BIG, NEG_BIG, NEG_BIG}; // four independent chains
-            if (ok)
-#pragma unroll 1
-                for (int hf = 0; hf < 2; ++hf) { // pass 1: maximum of the half row, 32 scores per round trip
-                    uint32_t v[32];
-                    tc::tmem_ld_x32(sbuf + 32 * hf, v);
-                    if (full) {
+                    for (int e = 32 * c; e < 32 * c + 32; e += 8)
 #pragma unroll
-                        for (int e = 0; e < 32; e += 8) {
-                            mx[0] = tc::fmax3(mx[0], __uint_as_float(v[e]), __uint_as_float(v[e + 1]));
-                            mx[1] = tc::fmax3(mx[1], __uint_as_float(v[e + 2]), __uint_as_float(v[e + 3]));
-                            mx[2] = tc::fmax3(mx[2], __uint_as_float(v[e + 4]), __uint_as_float(v[e + 5]));
-                            mx[3] = tc::fmax3(mx[3], __uint_as_float(v[e + 6]), __uint_as_float(v[e + 7]));
-                        }
+                        for (int i = 0; i < 4; ++i)
+                            mx[i] = tc::fmax3(mx[i], __uint_as_float(v[e >> 6][(e & 63) + 2 * i]), __uint_as_float(v[e >> 6][(e & 63) + 2 * i + 1]));
+                };
+                if (j0 + 127 <= warp_first) { // (uniform)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) maxima(c);
+                } else {
+                    const int nvalid = a_pos - j0 + 1;
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        if (j0 + 32 * c > warp_last) break; // (uniform) nothing that a row of the warp sees
+                        if (j0 + 32 * c + 31 > warp_first)
+#pragma unroll
+                            for (int e = 0; e < 32; ++e)
+                                if (32 * c + e >= nvalid) v[c >> 1][(c & 1) * 32 + e] = __float_as_uint(NEG_BIG);
+                        maxima(c);
+                    }
+                }
+                const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * SCALE_LOG2E;
+                const float next = j == 0 ? top : fmaxf(m, top), corr = tc::ex2_approx(m - next);
+                const bool moved = __any_sync(0xffffffffu, next > m);
+                // p = 2^(s*scale - maximum), in the scores' registers; the MMAs of the step before run meanwhile
+                const float2 sc2 = make_float2(SCALE_LOG2E, SCALE_LOG2E), nm2 = make_float2(-next, -next);
+                float2 ls[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+                uint32_t o[4][16];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    if (j0 + 32 * c > warp_last) { // (uniform)
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) o[c][e] = 0u;
                     } else {
 #pragma unroll
-                        for (int e = 0; e < 32; ++e)
-                            if (32 * hf + e < nvalid) mx[e & 3] = fmaxf(mx[e & 3], __uint_as_float(v[e]));
-                    }
-                }
-            const float mloc = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-            const float m_new = fmaxf(m, fmaxf(mloc, exchange(mloc, j & 1)) * SCALE_LOG2E);
-            const float corr = tc::ex2_approx(m - m_new);
-            if (j >= 1 && ok) { // the previous step's P V has had pass 1 to finish
-                ok = tc::mbar_wait(bar(bars.o_full[bf ^ 1]), ((j - 1) >> 1) & 1, &abort_flag, dev_err, ERR_ATT_O);
-                if (ok) {
-                    tc::tc_fence_after_sync();
-                    fold_output(bf ^ 1, corr_prev);
-                    tc::tc_fence_before_sync();
-                    tc::mbar_arrive(bar(bars.s_free[bf ^ 1])); // that buffer may take S_{j+1}
-                }
-            }
-            if (ok) {
-                float2 ls[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
-                const float2 sc2 = make_float2(SCALE_LOG2E, SCALE_LOG2E), nm2 = make_float2(-m_new, -m_new);
-#pragma unroll 1
-                for (int i = 0; i < 2; ++i) { // pass 2: p = 2^(s*scale - max) as fp16 pairs over the scores
-                    const int hf = half ? 1 - i : i; // the second half from its last column down
-                    uint32_t v[32], o[16];
-                    tc::tmem_ld_x32(sbuf + 32 * hf, v);
-#pragma unroll
-                    for (int e = 0; e < 32; e += 2) {
-                        const float2 x = __ffma2_rn(make_float2(__uint_as_float(v[e]), __uint_as_float(v[e + 1])), sc2, nm2);
-                        float2 p = make_float2(tc::ex2_approx(x.x), tc::ex2_approx(x.y));
-                        if (!full) {
-                            if (32 * hf + e >= nvalid) p.x = 0.0f;
-                            if (32 * hf + e + 1 >= nvalid) p.y = 0.0f;
+                        for (int e = 0; e < 32; e += 2) {
+                            const float2 x = __ffma2_rn(make_float2(__uint_as_float(v[c >> 1][(c & 1) * 32 + e]), __uint_as_float(v[c >> 1][(c & 1) * 32 + e + 1])), sc2, nm2);
+                            const float2 p = make_float2(tc::ex2_approx(x.x), tc::ex2_approx(x.y));
+                            ls[(e >> 1) & 1] = __fadd2_rn(ls[(e >> 1) & 1], p);
+                            o[c][e >> 1] = pack_half2(p.x, p.y);
                         }
-                        ls[(e >> 1) & 1] = __fadd2_rn(ls[(e >> 1) & 1], p);
-                        o[e >> 1] = pack_half2(p.x, p.y);
                     }
-                    tc::tmem_st_x16(sbuf + (half ? 32 : 0) + 16 * hf, o);
                 }
+                if (t >= 1) { // P's place is free and O complete
+                    ok = tc::mbar_wait(bar(bars.o_full), (t - 1) & 1, &abort_flag, dev_err, ERR_ATT_O);
+                    if (!ok) break;
+                    tc::tc_fence_after_sync();
+                }
+                if (j == 0) {
+                    if (n) finish();
+                    dst = s_row < S ? reinterpret_cast<uint4 *>(out + ((size_t)(it.bh / H) * S + s_row) * ldo + it.bh % H * 64) : nullptr;
+                    l2[0] = ls[0];
+                    l2[1] = ls[1];
+                } else {
+                    if (moved) {
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            uint32_t w[32];
+                            tc::tmem_ld_x32(lane_base + TM_O + 32 * i, w);
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) w[e] = __float_as_uint(__uint_as_float(w[e]) * corr);
+                            tc::tmem_st_x32(lane_base + TM_O + 32 * i, w);
+                            l2[i] = make_float2(l2[i].x * corr, l2[i].y * corr);
+                        }
+                    }
+                    l2[0] = __fadd2_rn(l2[0], ls[0]);
+                    l2[1] = __fadd2_rn(l2[1], ls[1]);
+                }
+                m = next;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) tc::tmem_st_x16(lane_base + TM_P + 16 * c, o[c]);
                 tc::tmem_st_wait();
                 tc::tc_fence_before_sync();
-                tc::mbar_arrive(bar(bars.p_full[bf]));
-                l = l * corr + ((ls[0].x + ls[0].y) + (ls[1].x + ls[1].y));
-            }
-            m = m_new;
-            corr_prev = corr;
-        }
-        if (ok) {
-            const int bl = (n_tiles - 1) & 1;
-            ok = tc::mbar_wait(bar(bars.o_full[bl]), ((n_tiles - 1) >> 1) & 1, &abort_flag, dev_err, ERR_ATT_O);
-            if (ok) {
-                tc::tc_fence_after_sync();
-                fold_output(bl, corr_prev);
+                __syncwarp();
+                if ((tid & 31) == 0) tc::mbar_arrive(bar(bars.p_full));
             }
         }
-        l += exchange(l, n_tiles & 1);
-        if (ok && row_valid) {
-            const float inv = 1.0f / l;
-            uint4 *dst = reinterpret_cast<uint4 *>(out + ((size_t)b * S + s_row) * ldo + h * 64 + 32 * half);
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                uint4 v;
-                v.x = pack_half2(acc[4 * c + 0].x * inv, acc[4 * c + 0].y * inv);
-                v.y = pack_half2(acc[4 * c + 1].x * inv, acc[4 * c + 1].y * inv);
-                v.z = pack_half2(acc[4 * c + 2].x * inv, acc[4 * c + 2].y * inv);
-                v.w = pack_half2(acc[4 * c + 3].x * inv, acc[4 * c + 3].y * inv);
-                dst[c] = v;
-            }
+        if (ok) ok = tc::mbar_wait(bar(bars.o_full), (t - 1) & 1, &abort_flag, dev_err, ERR_ATT_O);
+        if (ok) { // (warp-uniform)
+            tc::tc_fence_after_sync();
+            finish();
         }
     }
 
@@ -335,9 +372,11 @@ int launch_prefill_attention_tc(b200nn_ctx *ctx, const __half *q, int ldq, const
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) return set_error(ctx, B200NN_ERR_CUDA, "cuTensorMapEncodeTiled (K/V) failed: " + std::to_string((int)r));
     }
-    if (B > 65535 || (S + 127) / 128 > 65535) return set_error(ctx, B200NN_ERR_SHAPE, "prefill attention: more than 65535 sequences or query tiles");
-    dim3 grid(B, H, (S + 127) / 128);
-    prefill_attn_tc_kernel<<<grid, NTHREADS, SMEM_BYTES, ctx->stream>>>(tq, tk, tv, H, cap, S, past, out, H * 64, ctx->dev_err);
+    const long long items = (long long)B * H * ((S + 127) / 128);
+    if (B > 65535 || (S + 127) / 128 > 65535 || items > 0x3fffffff)
+        return set_error(ctx, B200NN_ERR_SHAPE, "prefill attention: more than 65535 sequences or query tiles");
+    const int grid = (int)std::min<long long>(items, 2 * ctx->sm_count);
+    prefill_attn_tc_kernel<<<grid, NTHREADS, SMEM_BYTES, ctx->stream>>>(tq, tk, tv, H, B * H, cap, S, past, out, H * 64, ctx->dev_err);
     CK_LAUNCH(ctx, "prefill_attn_tc_kernel");
     return B200NN_OK;
 }
