@@ -15,8 +15,11 @@
 // reads the other rows and replaces its own, so heads that share a query/key head do not race.
 #include <algorithm>
 
+#include <cuda.h>
+
 #include "device_utils.cuh"
 #include "hybrid.h"
+#include "tc_ptx.cuh"
 
 namespace {
 
@@ -306,27 +309,47 @@ delta_conv_kernel(DeltaDims d, const float *__restrict__ proj, int ldp, const fl
     }
 }
 
-// Block = (16 NC state columns, head, sequence), four warps.  The eight lanes of a column group hold its dim entries
-// 4 l + 32 m .. + 3 of NC columns each (f32 pairs along dim).  Tokens come through shared memory TOK at a time, the next
-// TOK being copied under the current ones.  The state is held divided by the decay G accumulated since it was last
-// rescaled (S = G s), so that a token costs three multiply-adds per entry; it is rescaled when G falls below 2^-20.
-// With CH the decays differ along dim and are multiplied in directly (one multiply more per entry).
-// Per token: both products against the old state, one reduction over the eight lanes (transposing: 2 NC values in
-// log steps), the write.  Also leaves the convolution's last inputs in the cache (blocks of column group 0).
+enum : uint32_t { ERR_SCAN = 0x401 };
+constexpr int SCAN_TOKENS = 8, SCAN_THREADS = 8 * SCAN_TOKENS; // eight lanes make one of a stage's TOK / 2 x 2 cross products
 template <int DM, int NC, bool CH>
-__global__ void __launch_bounds__(128, DM > 4 ? 1 : 4)
-delta_scan_kernel(DeltaDims d, const float *__restrict__ proj, int ldp, const float *__restrict__ conv, float *__restrict__ conv_state,
-                  float *__restrict__ state, SeqMap sm, float *__restrict__ heads_out) {
-    constexpr int TOK = DM <= 4 ? 16 : 8, DP = DM * 32, CB = 16 * NC;
-    struct Stage {
-        float k[TOK][DP], q[TOK][DP], v[TOK][CB], s[TOK][4], g[CH ? TOK : 1][CH ? DP : 4]; // s: decay, step size, k . q; g: decays
-    };
-    extern __shared__ __align__(16) uint8_t smem_raw[];
-    Stage *stages = reinterpret_cast<Stage *>(smem_raw);
+struct alignas(128) ScanStage { // the parts that tensor copies fill start on 128 bytes
+    static constexpr int TOK = SCAN_TOKENS, DP = DM * 32;
+    float qk[TOK][2][DP], v[TOK][8 * NC], s[TOK][4], g[CH ? TOK : 1][CH ? DP : 4]; // s: decay, step size, k . q; g: decays
+    float cross[TOK / 2][2]; // k1 . k2 and k1 . q2 of each pair
+};
+
+// Block = (8 NC state columns, head, sequence), two warps.  The eight lanes of a column group hold its dim entries
+// 4 l + 32 m .. + 3 of NC columns each (f32 pairs along dim).  Tokens come through shared memory TOK at a time, the next
+// TOK being copied under the current ones, and are taken in pairs: all four products (k, q of both tokens) are taken on
+// the state before the pair,
+//     u1 = beta1 (v1 - g1 S^T k1),               o1 = g1 S^T q1 + (k1 . q1) u1,
+//     u2 = beta2 (v2 - g1 g2 S^T k2 - g2 (k1 . k2) u1),  o2 = g1 g2 S^T q2 + g2 (k1 . q2) u1 + (k2 . q2) u2,
+//     S <- g1 g2 S + g2 k1 u1^T + k2 u2^T,
+// one lane reduction for the eight values (transposing: each lane ends with one of them) and one chain for two tokens.
+// The state is held divided by the decay G accumulated since it was last rescaled (S = G s), so that a token costs three
+// multiply-adds per entry; a pair that brings G below 2^-20 applies its decays to the state instead.
+// With CH the decays differ along dim and are multiplied in directly (one multiply more per entry).
+// What bounds it: the packed multiply-adds read three different operand pairs and issue every 3 to 3.5 cycles (two when operands
+// repeat): 96 of them and 60 other instructions per warp and pair; and, per stage, 600 cycles of copies announced, cross
+// products and two barriers.  One token at a time, copies by cp.async, four warps a block: 16 sequences of 1024 tokens, 8 heads of
+// 128, 591 us, now 515; one of 512 133 / 100.  Tried: four lanes for two columns (half the reductions, half the warps: 506, and
+// 170 for one sequence), plain multiply-adds (576), a bulk copy per token and vector (920: one lane issues them), the
+// cross products with the pair (longer chains), pairs unrolled (spills).
+// Also leaves the convolution's last inputs in the cache (blocks of column group 0).
+template <int DM, int NC, bool CH>
+__global__ void __launch_bounds__(SCAN_THREADS, DM > 4 ? 4 : 8)
+delta_scan_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_g,
+                  DeltaDims d, const float *__restrict__ proj, int ldp, const float *__restrict__ conv, float *__restrict__ conv_state,
+                  float *__restrict__ state, SeqMap sm, float *__restrict__ heads_out, uint32_t *__restrict__ dev_err) {
+    constexpr int TOK = SCAN_TOKENS, T = SCAN_THREADS, DP = DM * 32, CB = T / 8 * NC;
+    using Stage = ScanStage<DM, NC, CH>;
+    extern __shared__ __align__(128) uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t full[2]; // a stage's copies have landed
+    __shared__ int abort_flag;
+    Stage *stages = reinterpret_cast<Stage *>(smem_raw + (-tc::smem_u32(smem_raw) & 127));
     pdl_trigger();
     const int cg = blockIdx.x, h = blockIdx.y, sidx = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int part = lane & 7, cl = (warp * 4 + (lane >> 3)) * NC, col = cg * CB + cl; // NC columns from col on
-    for (int i = tid; i < (int)(2 * sizeof(Stage) / 4); i += 128) reinterpret_cast<float *>(smem_raw)[i] = 0.0f; // entries past dim stay zero
+    const int part = lane & 7, cl = (tid >> 3) * NC, col = cg * CB + cl; // NC columns from col on
     const int n = sm.n[sidx], past = sm.past[sidx], slot = sm.slot[sidx], row0 = sm.row0[sidx];
     const int group = d.heads / d.kv_heads, kh = h / group, cw = d.conv_w(), ldc = d.conv_ld();
     float *S = state + ((size_t)slot * d.heads + h) * d.dim_p * d.vdim_p + col;
@@ -342,28 +365,30 @@ delta_scan_kernel(DeltaDims d, const float *__restrict__ proj, int ldp, const fl
                 s[c][2 * m + e / 2] = in ? f32x2(S[(size_t)i * d.vdim_p + c], S[(size_t)(i + 1) * d.vdim_p + c]) : 0ull;
             }
         }
-    auto copy = [&](int t0, Stage &st) {
-        const int nt = min(TOK, n - t0), dv = d.dim_p >> 2, cv = min(CB, d.vdim_p - cg * CB) >> 2;
-        const float *c = conv + (size_t)(row0 + t0) * ldc;
-        for (int i = tid; i < nt * dv; i += 128) {
-            const int t = i / dv, j = (i - t * dv) * 4;
-            cp_async16(&st.q[t][j], c + (size_t)t * ldc + d.q_at() + kh * d.dim_p + j);
-            cp_async16(&st.k[t][j], c + (size_t)t * ldc + d.k_at() + kh * d.dim_p + j);
-            if constexpr (CH) cp_async16(&st.g[t][j], c + (size_t)t * ldc + d.decay_at() + h * d.dim_p + j);
-        }
-        for (int i = tid; i < nt * cv; i += 128) {
-            const int t = i / cv, j = (i - t * cv) * 4;
-            cp_async16(&st.v[t][j], c + (size_t)t * ldc + d.v_at() + h * d.vdim_p + cg * CB + j);
-        }
-        for (int i = tid; i < nt * 3; i += 128) {
-            const int t = i / 3, j = i - t * 3;
-            if (CH && j == 0) continue;
-            cp_async4(&st.s[t][j], c + (size_t)t * ldc + (j == 0 ? d.decay_at() + h : j == 1 ? d.beta_at() + h : d.kq_at() + kh));
+    // the tokens' single values (the last warp): requested before a stage's work, put down after it
+    const int one = (T / 32 - 1) * 32, st_t = (tid - one) >> 2, st_j = tid & 3;
+    const bool fetches = tid >= one && st_j < 3 && !(CH && st_j == 0);
+    const float *single = conv + (size_t)row0 * ldc + (st_j == 0 ? d.decay_at() + h : st_j == 1 ? d.beta_at() + h : d.kq_at() + kh);
+    auto fetch = [&](int t0) { return fetches && t0 + st_t < n ? single[(size_t)(t0 + st_t) * ldc] : 0.0f; };
+    // A box of TOK rows of each part (entries past dim arrive as zeros; rows past the sequence's last are not used).
+    auto copy = [&](int t0, Stage &st, uint64_t *landed) {
+        if (tid == 0) {
+            const uint32_t bar = tc::smem_u32(landed);
+            tc::mbar_expect_tx(bar, TOK * (DP * (CH ? 3 : 2) + CB) * 4);
+            tc::tma_load_4d(tc::smem_u32(st.qk), &map_qk, 0, kh, 0, row0 + t0, bar);
+            tc::tma_load_4d(tc::smem_u32(st.v), &map_v, cg * CB, h, 0, row0 + t0, bar);
+            if constexpr (CH) tc::tma_load_4d(tc::smem_u32(st.g), &map_g, 0, h, 0, row0 + t0, bar);
         }
     };
+    if (tid == 0) {
+        abort_flag = 0;
+        for (int i = 0; i < 2; ++i) tc::mbar_init(tc::smem_u32(&full[i]), 1);
+        tc::fence_mbar_init();
+    }
     __syncthreads();
-    copy(0, stages[0]);
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    copy(0, stages[0], &full[0]);
+    if (tid >= one) stages[0].s[st_t][st_j] = fetch(0);
+    __syncthreads();
     float G = 1.0f;
     auto rescale = [&](float f) {
         const uint64_t f2 = f32x2(f, f);
@@ -372,88 +397,159 @@ delta_scan_kernel(DeltaDims d, const float *__restrict__ proj, int ldp, const fl
 #pragma unroll
             for (int m = 0; m < DM * 2; ++m) s[c][m] = mul2(f2, s[c][m]);
     };
+    // what a lane ends with: S^T k1, q1, k2 or q2, of column `mine`
+    const int type = part >> 1, mine = NC == 2 ? part & 1 : 0;
+    const bool writer = (type & 1) && (NC == 2 || !(part & 1)) && col + mine < d.vdim_p;
+    float *o = heads_out + ((size_t)(row0 + (type >> 1)) * d.heads + h) * d.vdim_p + col + mine;
+    const size_t o_step = (size_t)d.heads * d.vdim_p;
     for (int t0 = 0, b = 0; t0 < n; t0 += TOK, b ^= 1) {
-        if (t0 + TOK < n) copy(t0 + TOK, stages[b ^ 1]);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncthreads();
-        const Stage &st = stages[b];
+        if (t0 + TOK < n) copy(t0 + TOK, stages[b ^ 1], &full[b ^ 1]);
+        const float next = fetch(t0 + TOK);
+        Stage &st = stages[b];
         const int nt = min(TOK, n - t0);
-#pragma unroll 4
-        for (int t = 0; t < nt; ++t) {
-            const float4 sc = *reinterpret_cast<const float4 *>(st.s[t]);
-            if constexpr (CH) {
+        tc::mbar_wait(tc::smem_u32(&full[b]), t0 / (2 * TOK) & 1, &abort_flag, dev_err, ERR_SCAN);
+        if (nt & 1) { // the last token's partner: nothing read, nothing written
+            for (int j = tid; j < DP; j += T) {
+                st.qk[nt][0][j] = st.qk[nt][1][j] = 0.0f;
+                if constexpr (CH) st.g[nt][j] = 1.0f;
+            }
+            if (tid < CB) st.v[nt][tid] = 0.0f;
+            if (tid < 3) st.s[nt][tid] = tid == 0 ? 1.0f : 0.0f;
+            __syncthreads();
+        }
+        { // k1 . k2 (even groups) and k1 . q2 (odd ones) of pair `at`, k1 under the second token's decay
+            const int g = tid >> 3, at = g & ~1;
+            const float *y = st.qk[at + 1][~g & 1];
+            uint64_t a[2] = {};
 #pragma unroll
-                for (int m = 0; m < DM; ++m) {
-                    const ulonglong2 gg = *reinterpret_cast<const ulonglong2 *>(&st.g[t][32 * m + 4 * part]);
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        s[c][2 * m] = mul2(gg.x, s[c][2 * m]);
-                        s[c][2 * m + 1] = mul2(gg.y, s[c][2 * m + 1]);
-                    }
+            for (int m = 0; m < DM; ++m) {
+                ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(&st.qk[at][1][32 * m + 4 * part]);
+                const ulonglong2 z = *reinterpret_cast<const ulonglong2 *>(&y[32 * m + 4 * part]);
+                if constexpr (CH) {
+                    const ulonglong2 gg = *reinterpret_cast<const ulonglong2 *>(&st.g[at + 1][32 * m + 4 * part]);
+                    x.x = mul2(x.x, gg.x);
+                    x.y = mul2(x.y, gg.y);
                 }
-            } else {
-                G *= sc.x;
-                if (G < 9.5367431640625e-7f) { // the same in every thread of the block
+                a[0] = fma2(x.x, z.x, a[0]);
+                a[1] = fma2(x.y, z.y, a[1]);
+            }
+            const float2 a0 = f32x2_parts(a[0]), a1 = f32x2_parts(a[1]);
+            float dot = (a0.x + a0.y) + (a1.x + a1.y);
+#pragma unroll
+            for (int sh = 4; sh; sh >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, sh);
+            if (part == 0) st.cross[at >> 1][g & 1] = dot;
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int t = 0; t < nt; t += 2) {
+            const float4 sc1 = *reinterpret_cast<const float4 *>(st.s[t]), sc2 = *reinterpret_cast<const float4 *>(st.s[t + 1]);
+            const float2 cross = *reinterpret_cast<const float2 *>(st.cross[t >> 1]);
+            float e1 = 1.0f, e2 = 1.0f, g2 = 1.0f; // decays from the state as held to each token, from the first token to the second
+            bool fold = false;                     // the same in every thread of the block
+            if constexpr (!CH) {
+                g2 = sc2.x;
+                fold = G * sc1.x * g2 < 9.5367431640625e-7f;
+                if (fold) {
                     rescale(G);
                     G = 1.0f;
                 }
+                e1 = G * sc1.x;
+                e2 = e1 * g2;
             }
-            uint64_t k[DM * 2];
-            float r[2 * NC]; // s^T k of the NC columns, then s^T q
+            uint64_t k1[DM * 2], k2[DM * 2];
+            float r[4 * NC]; // s^T k1, s^T q1, s^T k2, s^T q2, each of the NC columns
             {
-                uint64_t ak[NC], aq[NC];
+                uint64_t acc[4 * NC];
 #pragma unroll
-                for (int c = 0; c < NC; ++c) ak[c] = aq[c] = 0ull;
+                for (int i = 0; i < 4 * NC; ++i) acc[i] = 0ull;
 #pragma unroll
                 for (int m = 0; m < DM; ++m) {
-                    const ulonglong2 kk = *reinterpret_cast<const ulonglong2 *>(&st.k[t][32 * m + 4 * part]);
-                    const ulonglong2 qq = *reinterpret_cast<const ulonglong2 *>(&st.q[t][32 * m + 4 * part]);
-                    k[2 * m] = kk.x;
-                    k[2 * m + 1] = kk.y;
+                    const int at = 32 * m + 4 * part;
+                    const ulonglong2 ka = *reinterpret_cast<const ulonglong2 *>(&st.qk[t][1][at]), qa = *reinterpret_cast<const ulonglong2 *>(&st.qk[t][0][at]);
+                    const ulonglong2 kb = *reinterpret_cast<const ulonglong2 *>(&st.qk[t + 1][1][at]), qb = *reinterpret_cast<const ulonglong2 *>(&st.qk[t + 1][0][at]);
+                    k1[2 * m] = ka.x;
+                    k1[2 * m + 1] = ka.y;
+                    k2[2 * m] = kb.x;
+                    k2[2 * m + 1] = kb.y;
+                    ulonglong2 ga, gb;
+                    if constexpr (CH) {
+                        ga = *reinterpret_cast<const ulonglong2 *>(&st.g[t][at]);
+                        gb = *reinterpret_cast<const ulonglong2 *>(&st.g[t + 1][at]);
+                        k1[2 * m] = mul2(gb.x, ka.x);
+                        k1[2 * m + 1] = mul2(gb.y, ka.y);
+                    }
 #pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        ak[c] = fma2(s[c][2 * m], kk.x, ak[c]);
-                        aq[c] = fma2(s[c][2 * m], qq.x, aq[c]);
-                        ak[c] = fma2(s[c][2 * m + 1], kk.y, ak[c]);
-                        aq[c] = fma2(s[c][2 * m + 1], qq.y, aq[c]);
+                    for (int e = 0; e < 2; ++e) { // the accumulators in turn: no sum waits for the one before
+                        const uint64_t kae = e ? ka.y : ka.x, qae = e ? qa.y : qa.x, kbe = e ? kb.y : kb.x, qbe = e ? qb.y : qb.x;
+#pragma unroll
+                        for (int c = 0; c < NC; ++c) {
+                            if constexpr (CH) s[c][2 * m + e] = mul2(e ? ga.y : ga.x, s[c][2 * m + e]);
+                            acc[c] = fma2(s[c][2 * m + e], kae, acc[c]);
+                            acc[NC + c] = fma2(s[c][2 * m + e], qae, acc[NC + c]);
+                        }
+#pragma unroll
+                        for (int c = 0; c < NC; ++c) {
+                            if constexpr (CH) s[c][2 * m + e] = mul2(e ? gb.y : gb.x, s[c][2 * m + e]);
+                            acc[2 * NC + c] = fma2(s[c][2 * m + e], kbe, acc[2 * NC + c]);
+                            acc[3 * NC + c] = fma2(s[c][2 * m + e], qbe, acc[3 * NC + c]);
+                        }
                     }
                 }
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    const float2 a = f32x2_parts(ak[c]), q = f32x2_parts(aq[c]);
-                    r[c] = a.x + a.y;
-                    r[NC + c] = q.x + q.y;
+                for (int i = 0; i < 4 * NC; ++i) {
+                    const float2 a = f32x2_parts(acc[i]);
+                    r[i] = a.x + a.y;
                 }
             }
-            // reduction over the eight lanes of the group: halve the values while there are several, then plain
-            int o = 4;
+            // reduction over the lanes of the group: halve the values while there are several, then plain
 #pragma unroll
-            for (int w = NC; w >= 1; w >>= 1, o >>= 1) {
-                const bool up = (lane & o) != 0;
+            for (int sh = 4, w = 2 * NC; sh; sh >>= 1, w >>= 1) {
+                const bool up = (lane & sh) != 0;
 #pragma unroll
                 for (int i = 0; i < w; ++i) {
                     const float send = up ? r[i] : r[i + w], keep = up ? r[i + w] : r[i];
-                    r[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                    r[i] = keep + __shfl_xor_sync(0xffffffffu, send, sh);
                 }
+                if (w == 0) r[0] += __shfl_xor_sync(0xffffffffu, r[0], sh);
             }
-            for (; o; o >>= 1) r[0] += __shfl_xor_sync(0xffffffffu, r[0], o);
-            // lanes with bit 4 clear now hold s^T k, the others s^T q, of column idx
-            const int idx = NC == 1 ? 0 : (lane >> 1) & 1;
-            const float mine = CH ? r[0] : G * r[0], other = __shfl_xor_sync(0xffffffffu, mine, 4);
-            const float u_own = sc.y * (st.v[t][cl + idx] - ((lane & 4) ? other : mine));
-            if ((lane & 4) && !(lane & 1) && (NC == 2 || !(lane & 2)) && col + idx < d.vdim_p)
-                heads_out[((size_t)(row0 + t0 + t) * d.heads + h) * d.vdim_p + col + idx] = fmaf(sc.z, u_own, mine);
-            const float us = CH ? u_own : __fdividef(u_own, G);
+            float u1[NC], u2[NC];
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
-                const float u = NC == 1 ? us : __shfl_sync(0xffffffffu, us, (lane & 24) | (c << 1));
-                const uint64_t u2 = f32x2(u, u);
+                const float a1 = __shfl_sync(0xffffffffu, r[0], (lane & 24) | c), a2 = __shfl_sync(0xffffffffu, r[0], (lane & 24) | 4 | c);
+                u1[c] = sc1.y * fmaf(-e1, a1, st.v[t][cl + c]);
+                u2[c] = sc2.y * fmaf(-g2 * cross.x, u1[c], fmaf(-e2, a2, st.v[t + 1][cl + c]));
+            }
+            {
+                const bool second = type & 2;
+                const float p1 = mine ? u1[NC - 1] : u1[0], p2 = mine ? u2[NC - 1] : u2[0];
+                const float out = second ? fmaf(sc2.z, p2, fmaf(g2 * cross.y, p1, e2 * r[0])) : fmaf(sc1.z, p1, e1 * r[0]);
+                if (writer && t + (type >> 1) < nt) *o = out;
+                o += 2 * o_step;
+            }
+            float f1 = 1.0f, f2 = 1.0f;
+            if constexpr (!CH) {
+                if (fold) {
+                    rescale(e2);
+                    f1 = g2;
+                } else {
+                    G = e2;
+                    f1 = __fdividef(1.0f, e1);
+                    f2 = __fdividef(1.0f, e2);
+                }
+            }
 #pragma unroll
-                for (int m = 0; m < DM * 2; ++m) s[c][m] = fma2(k[m], u2, s[c][m]);
+            for (int c = 0; c < NC; ++c) {
+                const uint64_t w1 = f32x2(f1 * u1[c], f1 * u1[c]), w2 = f32x2(f2 * u2[c], f2 * u2[c]);
+#pragma unroll
+                for (int m = 0; m < DM * 2; ++m) s[c][m] = fma2(k2[m], w2, fma2(k1[m], w1, s[c][m]));
             }
         }
+        if (tid >= one) stages[b ^ 1].s[st_t][st_j] = next;
         __syncthreads();
+        if (*(volatile int *)&abort_flag) { // a copy did not come: reported; leave once none is under way
+            for (int i = 0; i < 2; ++i) tc::mbar_try(tc::smem_u32(&full[i]), (t0 / TOK + 1 + i) / 2 & 1);
+            return;
+        }
     }
     if (!CH) rescale(G);
 #pragma unroll
@@ -475,11 +571,11 @@ delta_scan_kernel(DeltaDims d, const float *__restrict__ proj, int ldp, const fl
             const float *p = proj + (size_t)(row0 + t) * ldp;
             float *c = cring + (size_t)((past + t) % d.taps) * cw;
             if (h % group == 0)
-                for (int j = tid; j < d.dim_p; j += 128) {
+                for (int j = tid; j < d.dim_p; j += T) {
                     c[d.q_at() + kh * d.dim_p + j] = p[d.q_at() + kh * d.dim_p + j];
                     c[d.k_at() + kh * d.dim_p + j] = p[d.k_at() + kh * d.dim_p + j];
                 }
-            for (int j = tid; j < d.vdim_p; j += 128) c[d.v_at() + h * d.vdim_p + j] = p[d.v_at() + h * d.vdim_p + j];
+            for (int j = tid; j < d.vdim_p; j += T) c[d.v_at() + h * d.vdim_p + j] = p[d.v_at() + h * d.vdim_p + j];
         }
     }
 }
@@ -541,6 +637,19 @@ int step_launch(b200nn_ctx *ctx, const DeltaDims &d, const float *proj, int ldp,
     return B200NN_OK;
 }
 
+// [rows][parts][vectors][width] of f32 rows `ld` apart; a box holds SCAN_TOKENS rows of `box` entries of one vector of every part
+int map_rows(b200nn_ctx *ctx, CUtensorMap *map, const float *base, int width, int vectors, int parts, int rows, int ld, int box) {
+    if (!ctx->encode_tiled) return set_error(ctx, B200NN_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is unavailable");
+    auto encode = reinterpret_cast<decltype(&cuTensorMapEncodeTiled)>(ctx->encode_tiled);
+    const cuuint64_t dims[4] = {(cuuint64_t)width, (cuuint64_t)vectors, (cuuint64_t)parts, (cuuint64_t)rows};
+    const cuuint64_t strides[3] = {(cuuint64_t)width * 4, (cuuint64_t)width * vectors * 4, (cuuint64_t)ld * 4};
+    const cuuint32_t boxes[4] = {(cuuint32_t)box, 1, (cuuint32_t)parts, (cuuint32_t)SCAN_TOKENS}, steps[4] = {1, 1, 1, 1};
+    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(base), dims, strides, boxes, steps, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return set_error(ctx, B200NN_ERR_CUDA, "cuTensorMapEncodeTiled (delta rule) failed: " + std::to_string((int)r));
+    return B200NN_OK;
+}
+
 template <bool CH>
 int prompt_launch(b200nn_ctx *ctx, const DeltaDims &d, bool b16, const float *proj, int ldp, const float *ext, const DeltaWeights &w, float *conv_state,
                   float *state, const RowMap &rows, const SeqMap &sm, int n_rows, const int *row_seq, float *conv, float *heads_out, void *out) {
@@ -552,22 +661,29 @@ int prompt_launch(b200nn_ctx *ctx, const DeltaDims &d, bool b16, const float *pr
     else
         launch_ordered(ctx, delta_conv_kernel<2, CH>, cgrid, dim3(256), 0, d, proj, ldp, ext, w, conv_state, rows, sm, row_seq, n_rows, conv);
     CK_LAUNCH(ctx, "delta_conv_kernel");
-    // columns per lane: two when that leaves every SM a dozen warps, else one (more parallel, more instructions)
+    // columns per lane: one (shorter chains, more instructions) while that gives an SM no more than three blocks; 512 tokens,
+    // 8 heads of 128, one / two columns, us: 2 sequences 112 / 119, 4 149 / 126, 8 213 / 168, 16 404 / 267
     const long long columns = (long long)d.vdim_p * d.heads * sm.n_seq;
     const int dm = (d.dim_p + 31) / 32;
-    const int nc = dm > 4 ? 1 : ctx->delta_cols ? ctx->delta_cols : columns >= 4LL * 2 * 10 * ctx->sm_count ? 2 : 1;
+    const int nc = dm > 4 ? 1 : ctx->delta_cols ? ctx->delta_cols : columns > 8LL * 3 * ctx->sm_count ? 2 : 1;
+    CUtensorMap map_qk, map_v, map_g;
+    const int dp = dm <= 4 ? dm * 32 : dm <= 6 ? 192 : 256;
+    if (int e = map_rows(ctx, &map_qk, conv + d.q_at(), d.dim_p, d.kv_heads, 2, n_rows, d.conv_ld(), dp)) return e;
+    if (int e = map_rows(ctx, &map_v, conv + d.v_at(), d.vdim_p, d.heads, 1, n_rows, d.conv_ld(), nc == 1 ? 8 : 16)) return e;
+    map_g = map_v; // not read
+    if (CH)
+        if (int e = map_rows(ctx, &map_g, conv + d.decay_at(), d.dim_p, d.heads, 1, n_rows, d.conv_ld(), dp)) return e;
 #define DSCAN(M, C)                                                                                                           \
     do {                                                                                                                      \
-        constexpr int ch = M <= 4 ? 16 : 8;                                                                                   \
-        constexpr size_t smem = 2 * sizeof(float) * (ch * (2 * M * 32 + 16 * C + 4) + (CH ? ch * M * 32 : 4));                \
+        constexpr size_t smem = 2 * sizeof(ScanStage<M, C, CH>) + 128;                                                            \
         static bool done[16] = {};                                                                                            \
         if (!done[ctx->device & 15]) {                                                                                        \
             CK(ctx, cudaFuncSetAttribute(delta_scan_kernel<M, C, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
             prefer_max_smem(delta_scan_kernel<M, C, CH>);                                                                     \
             done[ctx->device & 15] = true;                                                                                    \
         }                                                                                                                     \
-        CK(ctx, launch_ordered(ctx, delta_scan_kernel<M, C, CH>, dim3((d.vdim_p + 16 * C - 1) / (16 * C), d.heads, sm.n_seq), \
-                               dim3(128), smem, d, proj, ldp, conv, conv_state, state, sm, heads_out));                           \
+        CK(ctx, launch_ordered(ctx, delta_scan_kernel<M, C, CH>, dim3((d.vdim_p + 8 * C - 1) / (8 * C), d.heads, sm.n_seq), \
+                               dim3(SCAN_THREADS), smem, map_qk, map_v, map_g, d, proj, ldp, conv, conv_state, state, sm, heads_out, ctx->dev_err));            \
     } while (0)
 #define DSCAN_C(M)                                                                                                            \
     do {                                                                                                                      \

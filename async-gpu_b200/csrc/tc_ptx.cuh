@@ -122,6 +122,13 @@ __device__ __forceinline__ void tma_load_3d(uint32_t smem_dst, const void *tmap,
                  "l"(tmap), "r"(bar), "r"(x), "r"(y), "r"(z)
                  : "memory");
 }
+// 4-D tiled copy through a tensor map (same alignment rule for x).
+__device__ __forceinline__ void tma_load_4d(uint32_t smem_dst, const void *tmap, int x, int y, int z, int w, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(
+                     smem_dst),
+                 "l"(tmap), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w)
+                 : "memory");
+}
 // Asks the memory system to bring [gsrc, gsrc+bytes) into L2 (16-byte aligned, size a multiple of
 // 16); nothing is written anywhere and nothing needs to be waited for.
 __device__ __forceinline__ void bulk_prefetch_l2(const void *gsrc, uint32_t bytes) {
