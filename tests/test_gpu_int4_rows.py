@@ -48,6 +48,18 @@ def test_int4_output_matrix_of_few_rows(reg, m, k, n):
     assert np.sqrt(((y - ref) ** 2).mean()) / np.sqrt((ref ** 2).mean()) < 5e-4
 
 
+# the same of a 64-row tile: its last row missing or all there, one K block, as many stages, sixteen
+@pytest.mark.parametrize("m,k,n", [(33, 64, 38001), (63, 128, 38001), (64, 1024, 38001), (64, 1088, 38001)])
+def test_int4_output_matrix_of_up_to_64_rows(reg, m, k, n):
+    packed, scales, x, _ = synth.int4_linear_case(m + k, m, k, n, 128)
+    layer = b200nn.Int4Linear(packed, scales, None, k, n, 128, reg)
+    y = layer.forward(GpuTensor.from_host(x, (m, k), reg)).to_host()
+    ref = oracle.int4_linear(x, packed, scales, None, m, n, k, 128)
+    # rows and scaled weights rounded to fp16: 2.8e-4 of a product on average each
+    assert np.sqrt(((y - ref) ** 2).mean()) / np.sqrt((ref ** 2).mean()) < 5e-4
+    assert reg.device_error() == 0
+
+
 def test_int4_linear_of_few_rows_at_any_address(reg):
     """Rows that start off 16 bytes take the way through the conversion kernel."""
     import torch
