@@ -46,7 +46,7 @@ struct b200nn_ctx {
     int fused_argmax = 1;        // greedy decode steps take the argmax in the LM head's epilogue (0: separate kernel)
     uint64_t launches = 0;       // kernels launched by this library
     uint32_t *dev_err = nullptr; // device error word (bounded waits report here)
-    uint32_t *host_err = nullptr; // pinned landing place of that word for stream_sync_check
+    uint32_t *host_err = nullptr; // pinned landing place of that word (and of a session's own) for stream_sync_check
     // split-K / split-KV scratch, grown on demand outside stream capture
     float *scratch = nullptr;
     size_t scratch_bytes = 0;
@@ -96,7 +96,8 @@ struct b200nn_ctx {
 int set_error(b200nn_ctx *ctx, int code, const std::string &msg);
 int set_cuda_error(b200nn_ctx *ctx, cudaError_t e, const char *what);
 int ensure_scratch(b200nn_ctx *ctx, size_t bytes, size_t counters);
-int stream_sync_check(b200nn_ctx *ctx); // stream synchronise + device error word -> B200NN_ERR_DEVICE
+// stream synchronise + device error word, and 1 in the session's own word if given -> B200NN_ERR_DEVICE
+int stream_sync_check(b200nn_ctx *ctx, const uint32_t *gave_up = nullptr);
 
 #define CK(ctx, call)                                                     \
     do {                                                                  \

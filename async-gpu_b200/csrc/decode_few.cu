@@ -29,8 +29,10 @@
 // 350 / 582 launched per operation, 186 / 239 / 309 here; GPT-2 Small int4 212 / 262, here 165 / 180; GPT-2 XL int4
 // 1235 / 1579, here 1000 / 1296.  More rows: the tensor-core GEMMs take over (their activations are fp16).
 //
-// Every wait is bounded: when one runs out the block records a code in the device error word, waits for nothing more and
-// leaves.
+// Every wait is bounded: when one runs out the block records a code in the device error word, marks the session's exchanged
+// words as broken (what was published and not taken back would pass for later values), waits for nothing more and leaves;
+// the mark ends the other blocks' waits too.  A launch that finds it reports E_BROKEN and touches nothing, until a prompt or a
+// rewind starts the words over.  Errors that other kernels of the context have left in its error word end nothing here.
 //
 // Replaces the per-operation launch structure of Gpt2Model::forward_cached / generate (crates/core/gpu-host/src/nn/
 // models/gpt2.rs:249-288, 712-783, 1284-1339) for decode steps of few rows.
@@ -50,7 +52,8 @@ constexpr int RING = 4;          // layers of exchange words
 constexpr int MAX_SPLITS = 4;    // context splits of a head (K splits of a projection: 3)
 constexpr int ATT_ROWS = 120;    // cached rows of a head that a block has in flight at a time
 constexpr uint32_t EMPTY = 0xffffffffu;
-enum : uint32_t { E_WAIT = 0x301, E_FULL, E_FREE };
+enum : uint32_t { E_WAIT = 0x301, E_FULL, E_FREE, E_BROKEN };
+constexpr uint32_t BROKEN = 1;   // of the session's state: a launch has given up (anything else: none has)
 enum { QKV = 0, OUT = 1, FC = 2, FP = 3, HEAD = 4, MATS = 5 };
 constexpr int UNIT_K[2] = {32, 64}; // inputs of a unit of K: f32, int4
 
@@ -80,7 +83,7 @@ struct Params {
     int keep_last;
     uint32_t *words;    // RING layers of slot_words each, then the picks of two steps
     int slot_words, o_att, o_lse, o_out, o_fc, o_fp; // words of a layer: q/k/v at 0
-    uint32_t *state;    // {ring position of the first layer, parity of the first step}
+    uint32_t *state;    // {ring position of the first layer, parity of the first step, BROKEN or not}
     uint32_t *dev_err;
     long long wait_cycles;
     int fault_layer;    // test hook: block 0 publishes no q/k/v word of that layer (-1: none)
@@ -92,18 +95,9 @@ struct Params {
 
 struct Waiter {
     volatile int *abort_flag;
-    uint32_t *dev_err;
+    uint32_t *dev_err, *broken;
     long long limit;
-    // Whether to stop waiting.  Called every few hundred looks.
-    __device__ __noinline__ bool give_up(long long &t0) const {
-        if (*abort_flag) return true;
-        const long long now = clock64();
-        if (!t0) t0 = now;
-        if (now - t0 <= limit && *reinterpret_cast<volatile uint32_t *>(dev_err) == 0u) return false;
-        *abort_flag = 1;
-        atomicCAS(dev_err, 0u, (uint32_t)E_WAIT);
-        return true;
-    }
+    __device__ bool give_up(long long &t0) const;
 };
 __device__ __forceinline__ uint4 look4(const uint32_t *p) {
     uint4 v;
@@ -121,6 +115,17 @@ __device__ __forceinline__ uint32_t look1(const uint32_t *p) {
     return v;
 }
 __device__ __forceinline__ void put(uint32_t *p, uint32_t v) { asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
+// Whether to stop waiting.  Called every few hundred looks.
+__device__ __noinline__ bool Waiter::give_up(long long &t0) const {
+    if (*abort_flag) return true;
+    const long long now = clock64();
+    if (!t0) t0 = now;
+    if (now - t0 <= limit && look1(broken) != BROKEN) return false;
+    *abort_flag = 1;
+    put(broken, BROKEN);
+    atomicCAS(dev_err, 0u, (uint32_t)E_WAIT);
+    return true;
+}
 __device__ __forceinline__ void publish(uint32_t *p, float f) {
     const uint32_t u = __float_as_uint(f);
     put(p, u == EMPTY ? 0x7fffffffu : u); // a NaN stays a NaN
@@ -208,7 +213,7 @@ __device__ __forceinline__ void stage4(uint8_t *xs, int ld, float *scale, int m,
 template <bool INT4, int MT>
 __global__ void __launch_bounds__(THREADS, 1) decode_few_kernel(const __grid_constant__ Params P) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    __shared__ int abort_flag, gone_s;
+    __shared__ int abort_flag, gone_s, ended_s, broken_s;
     __shared__ uint32_t tok_s[4];
     __shared__ int off_s[4][CT];    // word of the sum that this thread finishes in a phase (-1: none)
     __shared__ int bias_s[4][CT];   // its feature, if it adds the bias (-1: another part does)
@@ -238,6 +243,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_few_kernel(const __grid_con
     };
     if (tid == 0) {
         abort_flag = 0;
+        broken_s = look1(P.state + 2) == BROKEN;
 #pragma unroll 1
         for (int i = 0; i < P.slots; ++i) {
             tc::mbar_init(full + 8 * i, 1);
@@ -264,6 +270,10 @@ __global__ void __launch_bounds__(THREADS, 1) decode_few_kernel(const __grid_con
             bias_s[g][tid] = on && split == 0 ? n : -1;
         }
     __syncthreads();
+    if (broken_s) { // (by an earlier launch, or before this block had begun)
+        if (tid == 0) atomicCAS(P.dev_err, 0u, (uint32_t)E_BROKEN);
+        return;
+    }
 
     const int pos0 = P.counters[0], step0 = P.counters[1];
     if (warp == WARPS) {
@@ -324,7 +334,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_few_kernel(const __grid_con
         return;
     }
 
-    const Waiter wait{&abort_flag, P.dev_err, P.wait_cycles};
+    const Waiter wait{&abort_flag, P.dev_err, P.state + 2, P.wait_cycles};
     const uint32_t ring0 = P.state[0] % RING, par0 = P.state[1] & 1; // (EMPTY, the last of its kind, after a restart)
     uint32_t *picks = P.words + (size_t)RING * P.slot_words;
     const int gq = lane >> 2, tq = lane & 3;
@@ -861,12 +871,18 @@ __global__ void __launch_bounds__(THREADS, 1) decode_few_kernel(const __grid_con
             if (lane == 0) tok_s[warp] = bi < 0 || bi >= P.vocab ? 0u : (uint32_t)bi;
         }
         csync();
+        if (tid == 0) ended_s = abort_flag || (blk == 0 && step + 1 == P.n_steps && look1(P.state + 2) == BROKEN);
+        csync();
+        gone = ended_s != 0; // nothing of a step that was given up is stored
+        if (gone) break;
         // every block's candidates of this step are there, so those of the step before have been read; a layer's fence
         // comes before the next ones
         if (tid < 2 * MT) put(picks + (size_t)((par0 + step + 1) & 1) * nblk * MT * 2 + (size_t)blk * MT * 2 + tid, EMPTY);
         if (blk == 0 && tid < M && step0 + step < P.hist_cap) P.history[(size_t)tid * P.hist_cap + step0 + step] = tok_s[tid];
     }
-    if (blk == 0) { // every block has read these: it has published since
+    if (gone) {
+        if (tid == 0) put(P.state + 2, BROKEN); // (a copy that did not come ends a block too)
+    } else if (blk == 0) { // every block has read these: it has published since
         if (tid < M) P.tok[tid] = tok_s[tid];
         if (tid == 0) {
             P.counters[0] = pos0 + P.n_steps;
@@ -1007,7 +1023,8 @@ bool decode_few_supported(const b200nn_gpt2 *m, int rows, int cap) {
     return per_sm * ctx->sm_count >= p.grid;
 }
 
-// All words EMPTY (the ring's position and the parity too: any are as good): before the first step after a prompt.
+// All words EMPTY (the ring's position and the parity too: any are as good; not BROKEN): before the first step after a
+// prompt or a rewind.
 int decode_few_restart(b200nn_session *s) {
     CK(s->m->ctx, cudaMemsetAsync(s->few_words->p, 0xff, s->few_words->bytes, s->m->ctx->stream));
     return B200NN_OK;
@@ -1018,7 +1035,9 @@ int decode_few_prepare(b200nn_session *s) {
     b200nn_ctx *ctx = m->ctx;
     few::Plan p;
     if (!few::make_plan(m, (int)s->batch, (int)s->kv.cap, &p)) return set_error(ctx, B200NN_ERR_UNSUPPORTED, "decode_few: no plan");
-    TRY(dev_alloc(ctx, p.words * 4 + 8, &s->few_words));
+    TRY(dev_alloc(ctx, p.words * 4 + 16, &s->few_words));
+    s->few_broken = (const uint32_t *)s->few_words->p + p.words + 2;
+    TRY(decode_few_restart(s));
     if (m->few_maps) return B200NN_OK; // the chunks' shapes depend on the model alone
     const size_t L = m->cfg.n_layer;
     std::vector<few::LayerPtrs> h(L);

@@ -238,9 +238,10 @@ struct b200nn_session {
     // MLP hidden GEMMs (zero at rest), grid counter + per-phase nanoseconds
     bool persist = false;
     std::shared_ptr<DevBuf> pd_layers, pd_qkv_acc, pd_fc_acc, pd_sync;
-    // steps of few rows (decode_few.cu): exchanged words, the ring's position and the step's parity behind them
+    // steps of few rows (decode_few.cu): exchanged words, the ring's position, the step's parity and whether a launch gave up behind them
     bool few = false;
     std::shared_ptr<DevBuf> few_words;
+    const uint32_t *few_broken = nullptr; // 1: steps were given up, until a prompt or a rewind
     int *pos_ptr() const { return static_cast<int *>(counters->p); }
     int *step_ptr() const { return static_cast<int *>(counters->p) + 1; }
 };
@@ -250,7 +251,7 @@ bool decode_persistent_supported(const b200nn_gpt2 *m, int rows);
 int decode_persistent_prepare(b200nn_session *s);
 int launch_decode_layers(b200nn_session *s, bool profile);
 
-// Decode steps of few rows, layers, head and pick, as one persistent cooperative kernel; restart: after a prompt.
+// Decode steps of few rows, layers, head and pick, as one persistent cooperative kernel; restart: after a prompt or a rewind.
 bool decode_few_supported(const b200nn_gpt2 *m, int rows, int cap);
 int decode_few_prepare(b200nn_session *s);
 int decode_few_restart(b200nn_session *s);

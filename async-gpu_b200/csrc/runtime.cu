@@ -26,13 +26,16 @@ int set_cuda_error(b200nn_ctx *ctx, cudaError_t e, const char *what) {
 // Waits for the context's stream and brings the device error word back in the same step.  A kernel
 // whose bounded wait ran out leaves its output unwritten and a code in that word: the call that hands
 // results to the host then fails with B200NN_ERR_DEVICE instead of returning stale data.  The word is
-// cleared so that the context stays usable.
-int stream_sync_check(b200nn_ctx *ctx) {
-    if (!ctx->host_err) CK(ctx, cudaMallocHost((void **)&ctx->host_err, sizeof(uint32_t)));
-    *ctx->host_err = 0;
+// cleared so that the context stays usable.  gave_up: a word of the caller's that is 1 once its own work was given up; it
+// stays, so that another call that has reported and cleared the context's word does not hide it.
+int stream_sync_check(b200nn_ctx *ctx, const uint32_t *gave_up) {
+    if (!ctx->host_err) CK(ctx, cudaMallocHost((void **)&ctx->host_err, 2 * sizeof(uint32_t)));
+    ctx->host_err[0] = ctx->host_err[1] = 0;
+    if (gave_up) CK(ctx, cudaMemcpyAsync(ctx->host_err + 1, gave_up, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
     CK(ctx, cudaMemcpyAsync(ctx->host_err, ctx->dev_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
     CK(ctx, cudaStreamSynchronize(ctx->stream));
     const uint32_t w = *ctx->host_err;
+    if (!w && ctx->host_err[1] == 1) return set_error(ctx, B200NN_ERR_DEVICE, "steps of this session were given up; a prompt or a rewind starts it over");
     if (!w) return B200NN_OK;
     CK(ctx, cudaMemsetAsync(ctx->dev_err, 0, sizeof(uint32_t), ctx->stream));
     char msg[96];

@@ -314,6 +314,7 @@ extern "C" int32_t b200nn_session_rewind(b200nn_session *s, size_t position) {
     s->steps_done -= back;
     s->position = position;
     s->kv.len = position;
+    if (s->few) TRY(decode_few_restart(s));
     return set_counters(s, (int)position, (int)s->steps_done);
 }
 
@@ -327,7 +328,7 @@ extern "C" int32_t b200nn_session_tokens(b200nn_session *s, uint32_t *out, size_
     size_t n = std::min(s->steps_done, capacity_per_seq);
     CK(ctx, cudaMemcpy2DAsync(out, capacity_per_seq * 4, s->history->p, s->hist_cap * 4, n * 4, s->batch,
                               cudaMemcpyDeviceToHost, ctx->stream));
-    TRY(stream_sync_check(ctx));
+    TRY(stream_sync_check(ctx, s->few_broken));
     if (generated) *generated = n;
     return B200NN_OK;
 }
@@ -340,7 +341,7 @@ extern "C" int32_t b200nn_session_logits(b200nn_session *s, float *out) {
     CK(ctx, cudaSetDevice(ctx->device));
     CK(ctx, cudaMemcpyAsync(out, s->ws_step.logits->p, s->batch * (size_t)s->m->vocab() * 4,
                             cudaMemcpyDeviceToHost, ctx->stream));
-    return stream_sync_check(ctx);
+    return stream_sync_check(ctx, s->few_broken);
 }
 
 extern "C" int32_t b200nn_session_profile_step(b200nn_session *s, float *times_ms, uint64_t *linear_bytes) {

@@ -97,3 +97,43 @@ def test_steps_in_one_kernel_wait_runs_out_and_session_recovers(reg):
         reg.set_tuning("persist_wait_kcycles", 0)
     again = run()  # a new prompt starts the exchanged words over
     assert np.array_equal(again[0], good[0]) and np.array_equal(again[1], good[1]) and reg.device_error() == 0
+
+
+def test_steps_given_up_are_reported_until_the_session_starts_over(reg):
+    """Words that were published and not taken back must not pass for later values, whoever else has met the error."""
+    cfg = Gpt2Config(n_layer=3, n_embd=128, n_head=2, vocab_size=257, n_positions=64)
+    m = Gpt2Model(synth.gpt2_weights(cfg, base_seed=77, std=0.08, random_ln=True), cfg, reg)
+    prompts = synth.token_ids(5, (2, 9), cfg.vocab_size)
+    s, other = (DecodeSession(m, batch=2, capacity=40) for _ in range(2))
+
+    def read(x):
+        return x.tokens(), x.logits()
+
+    def given_up(x):
+        with pytest.raises(b200nn.NnError) as e:
+            x.tokens()
+        return e.value.code == b200nn.ERR_DEVICE
+
+    s.prefill(prompts)
+    s.step(6)
+    good = read(s)
+    other.prefill(prompts)
+    for layer in (0, 1, 2):
+        s.prefill(prompts)
+        reg.set_tuning("persist_wait_kcycles", 2000)  # about a millisecond of SM clocks
+        reg.set_tuning("few_fault_layer", layer)
+        try:
+            s.step(6)
+        finally:
+            reg.set_tuning("few_fault_layer", -1)
+            reg.set_tuning("persist_wait_kcycles", 0)
+        other.step(6)  # behind the error, which is not its own
+        assert given_up(other)  # the context's error word goes to whoever asks first
+        assert all(np.array_equal(a, b) for a, b in zip(read(other), good))
+        assert given_up(s) and given_up(s)  # kept although the context's word has been cleared
+        s.step(1)  # refused by the kernel
+        assert given_up(s)
+        s.rewind(9)
+        s.step(6)  # the prompt's pick is still in place: what was given up has stored nothing
+        assert all(np.array_equal(a, b) for a, b in zip(read(s), good)) and reg.device_error() == 0
+        other.prefill(prompts)
