@@ -389,7 +389,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_const
         tc::fence_mbar_init();
     }
     __syncthreads();
-    copy(0, stages[0], &full[0]);
+    if (n > 0) copy(0, stages[0], &full[0]); // (a sequence of no rows waits for nothing)
     if (tid >= one) stages[0].s[st_t][st_j] = fetch(0);
     __syncthreads();
     float G = 1.0f;

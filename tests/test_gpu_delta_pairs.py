@@ -65,3 +65,43 @@ def test_prompts_agree_with_single_tokens(reg, H, KH, dim, vdim, channel):
         assert torch.linalg.norm(a - b) <= 6e-5 * torch.linalg.norm(b) + 1e-30, f"state of {n}"
         assert torch.equal(states[0][0][slots[i]], states[1][0][slots[i]]), f"convolution inputs of {n}"
     assert reg.device_error() == 0
+
+
+@pytest.mark.parametrize("channel", [False, True])
+def test_sequences_of_no_rows_change_nothing(reg, channel):
+    """Entries of no rows first, last and between others, one of them behind the last row of the pass."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    H, KH, dim, vdim, taps = 3, 1, 64, 32, 4
+    lengths = [0, 5, 0, 0, 9, 0]
+    E, N = len(lengths), sum(lengths)
+    cw = 2 * KH * dim + H * vdim
+    pw = -(-(cw + H) // 16) * 16 if channel else -(-(cw + H * vdim + 2 * H) // 4) * 4
+    decays, ext = (H * dim if channel else H), H * max(dim, vdim)
+    proj, exts = torch.randn(N, pw, generator=g, device="cuda"), torch.randn(N, 2 * ext, generator=g, device="cuda")
+    conv, norm = torch.randn(taps, cw, generator=g, device="cuda"), torch.rand(vdim, generator=g, device="cuda") + 0.5
+    a_exp, dt = torch.ones(H, device="cuda"), torch.randn(decays, generator=g, device="cuda")
+    first = (torch.randn(E, taps, cw, generator=g, device="cuda"), torch.randn(E, H, dim, vdim, generator=g, device="cuda"))
+
+    def run(entries):
+        cs, st, out = first[0].clone(), first[1].clone(), torch.zeros(N, H, vdim, device="cuda")
+        scratch = torch.zeros(N * (cw + decays + H + KH + 4 + H * vdim), device="cuda")
+        ns = [lengths[i] for i in entries]
+        row0 = np.concatenate([[0], np.cumsum(ns)[:-1]])
+        meta = _ints(entries, row0, ns, [4] * len(ns), np.repeat(np.arange(len(ns)), ns))
+        pos, slot = _ints(np.concatenate([4 + np.arange(n) for n in ns])), _ints(np.repeat(entries, ns))
+        torch.cuda.synchronize()
+        shape, ptrs = (H, KH, dim, vdim, taps, 1e-5), tuple(t.data_ptr() for t in (conv, a_exp, dt, norm))
+        tail = (cs.data_ptr(), st.data_ptr(), pos.data_ptr(), slot.data_ptr(), N, out.data_ptr(), reg)
+        kw = dict(n_seq=len(ns), max_n=max(ns), seq_ptr=meta.data_ptr(), scratch_ptr=scratch.data_ptr(), flags=b200nn.LM_F32)
+        if channel:
+            ops.channel_delta_rule(shape, ptrs, proj.data_ptr(), exts.data_ptr(), *tail, **kw)
+        else:
+            ops.delta_rule(shape, ptrs, proj.data_ptr(), *tail, **kw)
+        reg.synchronize()
+        return out, cs, st
+    got, want = run(list(range(E))), run([1, 4])
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    for i in (0, 2, 3, 5):
+        assert torch.equal(got[1][i], first[0][i]) and torch.equal(got[2][i], first[1][i])
+    assert not torch.equal(got[2][1], first[1][1]) and reg.device_error() == 0
