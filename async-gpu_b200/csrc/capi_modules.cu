@@ -71,7 +71,10 @@ extern "C" int32_t b200nn_int4_linear_forward_dev(b200nn_int4_linear *l, const f
     e.out = y_dev;
     e.ldo = l->l.N;
     const Int4Weight &w = l->l.q;
-    if (m <= 8 && int4_rows_supported(ctx, w, x_dev, (int)m)) { // takes the f32 rows as they are
+    // One kernel takes the f32 rows as they are; results over the rows themselves have to go through the converted copy, which
+    // is complete before the first of them is stored.
+    const bool over = x_dev < y_dev + m * (size_t)w.N && y_dev < x_dev + m * (size_t)w.K;
+    if (m <= 8 && !over && int4_rows_supported(ctx, w, x_dev, (int)m)) {
         e.bias = l->l.bias();
         return launch_int4_rows(ctx, w, x_dev, (int)m, e);
     }

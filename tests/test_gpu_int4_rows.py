@@ -74,3 +74,27 @@ def test_int4_linear_of_few_rows_at_any_address(reg):
     layer.forward_dev(aligned.data_ptr(), 6, y[1].data_ptr())
     reg.synchronize()
     assert y[0].abs().max() > 0 and torch.linalg.norm(y[0] - y[1]) / torch.linalg.norm(y[1]) < 8e-4
+
+
+# the same buffer; results that begin in the rows' last values, and that end in their first
+@pytest.mark.parametrize("k,n,at", [(256, 256, 0), (256, 96, 5 * 256 - 4), (128, 320, 4 - 5 * 320)])
+def test_int4_linear_of_few_rows_over_its_own_rows(reg, k, n, at):
+    """Results may lie over the rows: they are converted before the first result is stored."""
+    import torch
+    m = 5
+    packed, scales, x, _ = synth.int4_linear_case(8, m, k, n, 128)
+    layer = b200nn.Int4Linear(packed, scales, None, k, n, 128, reg)
+    buf = torch.zeros(4 * m * 320, device="cuda")
+    start = 2 * m * 320
+    buf[start:start + m * k] = torch.from_numpy(x).cuda().reshape(-1)
+    torch.cuda.synchronize()
+    reg.set_tuning("int4_rows_max", 0)
+    try:
+        want = layer.forward(GpuTensor.from_host(x, (m, k), reg)).to_host()
+    finally:
+        reg.set_tuning("int4_rows_max", -1)
+    launches = reg.launch_count()
+    layer.forward_dev(buf.data_ptr() + 4 * start, m, buf.data_ptr() + 4 * (start + at))
+    reg.synchronize()
+    assert reg.launch_count() - launches == 2  # conversion, GEMM
+    assert np.array_equal(buf[start + at:start + at + m * n].cpu().numpy().reshape(m, n), want)
