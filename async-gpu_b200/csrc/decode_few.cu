@@ -842,7 +842,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_few_kernel(const __grid_con
             }
             if (lane < MT) {
                 publish(pick + (size_t)(blk * MT + lane) * 2, bv);
-                put(pick + (size_t)(blk * MT + lane) * 2 + 1, (uint32_t)(bi + 2)); // never EMPTY
+                put(pick + (size_t)(blk * MT + lane) * 2 + 1, (uint32_t)bi + 2u); // -1 .. 0x7fffffff: never EMPTY
             }
         }
         if (warp < M) { // a warp per row over all blocks' candidates
@@ -859,7 +859,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_few_kernel(const __grid_con
                     u = look2(p);
                     if ((++it & 255u) == 0 && wait.give_up(t0)) break;
                 }
-                amax_merge(bv, bi, __uint_as_float(u.x), (int)u.y - 2, P.keep_last);
+                amax_merge(bv, bi, __uint_as_float(u.x), (int)(u.y - 2u), P.keep_last);
             }
             __syncwarp();
 #pragma unroll
