@@ -10,8 +10,10 @@
 //     arithmetic makes) until the producer stores the value, and the consumer polls the value itself.  No counter, no
 //     fence and no barrier lies between a sum and the blocks that read it: one store and one load through L2.
 //   * Words are used again every RING layers.  Whoever publishes a word returns the one of the layer after next to all
-//     ones, when every block is known to have read it (every block owns a part of every q/k/v product, and nobody gets
-//     past a layer before all of those were published); one thread per block orders that by a fence per layer.
+//     ones.  What lies between the uses of a word (and between a cached row and the steps that read it) is ordered by one
+//     counter: in the middle of a layer one thread of every block fences and adds to it, and in the middle of the next one
+//     the same thread looks, while the block waits for words anyway, whether every block has, and fences.  That covers
+//     everything a block did up to the middle of the layer before last, both what it wrote and what it had read.
 //   * The residual rows live in the registers of every block (a thread holds four columns); every block adds the
 //     projections' words to its own copy and normalises it itself.
 //   * Weights never depend on activations: one warp streams the block's part of them through a ring of tensor copies, in
@@ -83,7 +85,8 @@ struct Params {
     int keep_last;
     uint32_t *words;    // RING layers of slot_words each, then the picks of two steps
     int slot_words, o_att, o_lse, o_out, o_fc, o_fp; // words of a layer: q/k/v at 0
-    uint32_t *state;    // {ring position of the first layer, parity of the first step, BROKEN or not}
+    uint32_t *state;    // {ring position of the first layer, parity of the first step, BROKEN or not, `fenced` at the start}
+    uint32_t *fenced;   // fences of all blocks in the middle of a layer, ever
     uint32_t *dev_err;
     long long wait_cycles;
     int fault_layer;    // test hook: block 0 publishes no q/k/v word of that layer (-1: none)
@@ -130,6 +133,7 @@ __device__ __forceinline__ void publish(uint32_t *p, float f) {
     const uint32_t u = __float_as_uint(f);
     put(p, u == EMPTY ? 0x7fffffffu : u); // a NaN stays a NaN
 }
+__device__ __forceinline__ void count(uint32_t *p) { asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory"); }
 __device__ __forceinline__ uint32_t most(uint4 v) { return max(max(v.x, v.y), max(v.z, v.w)); }
 __device__ __forceinline__ float4 as_float4(uint4 v) {
     return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
@@ -157,6 +161,17 @@ __device__ __forceinline__ uint32_t take1(const Waiter &w, const uint32_t *p) {
         const uint32_t u = look1(p);
         if (u != EMPTY || ((++it & 255u) == 0 && w.give_up(t0))) return u;
     }
+}
+
+// One thread of the block, which the others meet at a barrier next: `fenced` has reached `target`, and what the blocks did
+// before their part of it is ordered before what this block does from that barrier on.
+__device__ __forceinline__ void settled(const Waiter &w, const uint32_t *fenced, uint32_t target) {
+    unsigned it = 0;
+    long long t0 = 0;
+#pragma unroll 1
+    while ((int)(look1(fenced) - target) < 0)
+        if ((++it & 255u) == 0 && w.give_up(t0)) break;
+    __threadfence();
 }
 
 // Barrier of the compute warps, whose lanes may have parted (they poll word by word).
@@ -336,6 +351,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_few_kernel(const __grid_con
 
     const Waiter wait{&abort_flag, P.dev_err, P.state + 2, P.wait_cycles};
     const uint32_t ring0 = P.state[0] % RING, par0 = P.state[1] & 1; // (EMPTY, the last of its kind, after a restart)
+    uint32_t all_fenced = P.state[3]; // `fenced` when every block has passed the middle of the layer before this one
     uint32_t *picks = P.words + (size_t)RING * P.slot_words;
     const int gq = lane >> 2, tq = lane & 3;
     const int c4 = tid * COLS; // this thread's places in the residual rows
@@ -394,7 +410,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_few_kernel(const __grid_con
         }
         norm_params(lp[0].ln[0], lp[0].ln[1]);
 #pragma unroll 1
-        for (int l = 0; l < P.n_layer && !gone; ++l, rp = (rp + 1) % RING) {
+        for (int l = 0; l < P.n_layer && !gone; ++l, rp = (rp + 1) % RING, all_fenced += nblk) {
             uint32_t *slot = P.words + (size_t)rp * P.slot_words, *later = P.words + (size_t)((rp + 2) % RING) * P.slot_words;
             const bool last = l + 1 == P.n_layer;
 #pragma unroll 1
@@ -404,6 +420,11 @@ __global__ void __launch_bounds__(THREADS, 1) decode_few_kernel(const __grid_con
                 const int parts = min(mt.cpi, WARPS), off = g != HEAD ? off_s[g][tid] : -1;
                 if (g != HEAD && bias_s[g][tid] >= 0 && lp[l].bias[g]) bias = __ldg(lp[l].bias[g] + bias_s[g][tid]);
                 const int items = items_s[g];
+
+                // OUT: words of the second half of this layer and of the first of the next one (under the wait for the attention,
+                // which is the longest: in the wait for the output projection's words it cost 0.3 us a layer).  HEAD: picks,
+                // the last layer's cached rows.
+                if ((g == OUT || g == HEAD) && tid == CT - 1) settled(wait, P.fenced, g == OUT ? all_fenced : all_fenced + nblk);
 
                 // ---- the product's input ----
                 if (g == OUT || g == FP) {
@@ -660,8 +681,12 @@ __global__ void __launch_bounds__(THREADS, 1) decode_few_kernel(const __grid_con
                         put(later + off, EMPTY);
                         if (g == QKV && kv_at >= 0) ((is_v ? P.vc : P.kc) + (size_t)l * P.kv_layer)[kv_at + (long long)pos * 64] = __float2half_rn(f);
                     }
-                    // what this block has returned to EMPTY (and its cache rows) before what it publishes from here on
-                    if (g == FC && tid == CT - 1) __threadfence();
+                    // behind the barrier: all that this block has read, its cache rows, and what it has returned to EMPTY but for
+                    // this product's words, which the next layer's fence covers
+                    if (g == FC && tid == CT - 1) {
+                        __threadfence();
+                        count(P.fenced);
+                    }
                 }
                 if (g == QKV) {
                     // ---- attention: a (sequence, head) pair and a part of its context per block ----
@@ -875,8 +900,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_few_kernel(const __grid_con
         csync();
         gone = ended_s != 0; // nothing of a step that was given up is stored
         if (gone) break;
-        // every block's candidates of this step are there, so those of the step before have been read; a layer's fence
-        // comes before the next ones
+        // those of the step before have been read: every block has fenced in this step's last layer
         if (tid < 2 * MT) put(picks + (size_t)((par0 + step + 1) & 1) * nblk * MT * 2 + (size_t)blk * MT * 2 + tid, EMPTY);
         if (blk == 0 && tid < M && step0 + step < P.hist_cap) P.history[(size_t)tid * P.hist_cap + step0 + step] = tok_s[tid];
     }
@@ -889,6 +913,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_few_kernel(const __grid_con
             P.counters[1] = step0 + P.n_steps;
             P.state[0] = rp;
             P.state[1] = (par0 + P.n_steps) & 1;
+            P.state[3] = all_fenced;
         }
     }
 }
@@ -924,8 +949,9 @@ static bool make_plan(const b200nn_gpt2 *m, int M, int cap, Plan *out) {
     }
     for (const BlockW &b : m->blocks)
         if (!fits(b.qkv, *lin[QKV]) || !fits(b.proj, *lin[OUT]) || !fits(b.fc, *lin[FC]) || !fits(b.fcproj, *lin[FP])) return false;
-    // every block owns a tile of the q/k/v product: no block can fall behind the reuse of the words unnoticed
+    // every block owns a tile of the q/k/v product and of the wide MLP product, in which it counts itself past the middle of a layer
     p.grid = std::min(ctx->sm_count, p.mat[QKV].tiles);
+    if (p.mat[FC].tiles < p.grid) return false;
     // the projections back to the model width have few tiles: their K is split where that gives idle blocks work
     for (int g : {OUT, FP})
         for (int s = std::min(3, p.grid / p.mat[g].tiles); s > 1; --s)
@@ -1023,7 +1049,7 @@ bool decode_few_supported(const b200nn_gpt2 *m, int rows, int cap) {
     return per_sm * ctx->sm_count >= p.grid;
 }
 
-// All words EMPTY (the ring's position and the parity too: any are as good; not BROKEN): before the first step after a
+// All words EMPTY (the ring's position, the parity and the counter too: any are as good; not BROKEN): before the first step after a
 // prompt or a rewind.
 int decode_few_restart(b200nn_session *s) {
     CK(s->m->ctx, cudaMemsetAsync(s->few_words->p, 0xff, s->few_words->bytes, s->m->ctx->stream));
@@ -1035,7 +1061,7 @@ int decode_few_prepare(b200nn_session *s) {
     b200nn_ctx *ctx = m->ctx;
     few::Plan p;
     if (!few::make_plan(m, (int)s->batch, (int)s->kv.cap, &p)) return set_error(ctx, B200NN_ERR_UNSUPPORTED, "decode_few: no plan");
-    TRY(dev_alloc(ctx, p.words * 4 + 16, &s->few_words));
+    TRY(dev_alloc(ctx, p.words * 4 + 256, &s->few_words));
     s->few_broken = (const uint32_t *)s->few_words->p + p.words + 2;
     TRY(decode_few_restart(s));
     if (m->few_maps) return B200NN_OK; // the chunks' shapes depend on the model alone
@@ -1103,6 +1129,7 @@ int launch_decode_few(b200nn_session *s, int n_steps) {
     P.o_fc = (int)p.o_fc;
     P.o_fp = (int)p.o_fp;
     P.state = P.words + p.words;
+    P.fenced = P.state + 32; // in a line of its own
     P.dev_err = ctx->dev_err;
     P.wait_cycles = ctx->persist_wait_cycles > 0 ? ctx->persist_wait_cycles : 2000000000LL;
     P.fault_layer = ctx->few_fault_layer;
