@@ -342,9 +342,15 @@ __global__ void __launch_bounds__(THREADS, 1) decode_few_kernel(const __grid_con
                         }
                     }
                 }
-            if (abort_flag) // copies still in flight land before the block's memory is released
+            // the last filling of every slot lands before the block's memory is released, also if the other warps gave up
 #pragma unroll 1
-                for (int i = 0; i < 64; ++i) __nanosleep(1000);
+            for (int i = min(n, P.slots); i > 0; --i) {
+                if (--s < 0) {
+                    s = P.slots - 1;
+                    ph ^= 1;
+                }
+                tc::mbar_drain(full + 8 * s, ph ^ 1);
+            }
         }
         return;
     }

@@ -549,8 +549,9 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_const
         }
         if (tid >= one) stages[b ^ 1].s[st_t][st_j] = next;
         __syncthreads();
-        if (*(volatile int *)&abort_flag) { // a copy did not come: reported; leave once none is under way
-            for (int i = 0; i < 2; ++i) tc::mbar_try(tc::smem_u32(&full[i]), (t0 / TOK + 1 + i) / 2 & 1);
+        if (*(volatile int *)&abort_flag) { // a copy did not come: reported; leave once this stage's and the next one's are through
+            if (tid == 0)
+                for (int i = t0 / TOK; i <= t0 / TOK + 1 && i * TOK < n; ++i) tc::mbar_drain(tc::smem_u32(&full[i & 1]), i >> 1 & 1);
             return;
         }
     }

@@ -94,6 +94,14 @@ __device__ __forceinline__ bool mbar_wait1(uint32_t bar, uint32_t parity, volati
     return true;
 }
 
+// For a thread that is to leave although nobody waits any more for copies under way: until the phase has completed, a tenth
+// of the bound of a wait at most.
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
+    const long long t0 = clock64();
+    while (!mbar_try(bar, parity) && clock64() - t0 < WAIT_CYCLES / 10) {
+    }
+}
+
 // ---- proxies / fences -------------------------------------------------------------------------
 // generic-proxy shared-memory writes -> visible to the async proxy (TMA, tcgen05.mma operand reads)
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
