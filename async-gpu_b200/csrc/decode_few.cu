@@ -1047,12 +1047,15 @@ bool decode_few_supported(const b200nn_gpt2 *m, int rows, int cap) {
     b200nn_ctx *ctx = m->ctx;
     if (!ctx->few || model_act_half(m, rows) || !few::make_plan(m, rows, cap, &p)) return false;
     int coop = 0, per_sm = 0;
-    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device) != cudaSuccess || !coop) return false;
     const few::Kernel k = few::kernel_of(m->int4, p.MT);
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, few::SMEM_MAX) != cudaSuccess) return false;
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device) != cudaSuccess ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, few::SMEM_MAX) != cudaSuccess) {
+        cudaGetLastError(); // (launches look at the last error)
+        return false;
+    }
     prefer_max_smem(k);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, few::THREADS, p.smem) != cudaSuccess) return false;
-    return per_sm * ctx->sm_count >= p.grid;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, few::THREADS, p.smem) != cudaSuccess) cudaGetLastError();
+    return coop && per_sm * ctx->sm_count >= p.grid;
 }
 
 // All words EMPTY (the ring's position, the parity and the counter too: any are as good; not BROKEN): before the first step after a

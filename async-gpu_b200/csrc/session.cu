@@ -145,8 +145,12 @@ extern "C" int32_t b200nn_lm_session_create(b200nn_lm *m, size_t batch, size_t c
         s->persist = true;
     }
     if (s->gpt2 && decode_few_supported(s->gpt2, (int)batch, (int)capacity)) {
-        TRY(decode_few_prepare(s.get()));
-        s->few = true;
+        s->few = decode_few_prepare(s.get()) == B200NN_OK; // (a tensor map refused, no room for the words: one kernel per operation)
+        if (!s->few) {
+            cudaGetLastError(); // (launches look at the last error)
+            s->few_words.reset();
+            s->few_broken = nullptr;
+        }
     }
     *out = s.release();
     return B200NN_OK;
