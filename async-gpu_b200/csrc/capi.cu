@@ -119,7 +119,7 @@ extern "C" int32_t b200nn_ctx_set_tuning(b200nn_ctx *ctx, const char *key, int32
     else if (!strcmp(key, "ln_rows_min")) ctx->ln_rows_min = value > 0 ? value : 1024;
     else if (!strcmp(key, "persist")) ctx->persist = value ? 1 : 0;
     else if (!strcmp(key, "int4_rows_max")) ctx->int4_rows_max = value < 0 ? 8 : std::min(value, 8);
-    else if (!strcmp(key, "few")) ctx->few = value ? 1 : 0;
+    else if (!strcmp(key, "few")) ctx->few = value < 0 ? 2 : std::min(value, 2);
     else if (!strcmp(key, "few_fault_layer")) ctx->few_fault_layer = value;
     else if (!strcmp(key, "persist_min_rows")) ctx->persist_min_rows = value < 1 ? 3 : value;
     else if (!strcmp(key, "persist_max_rows")) ctx->persist_max_rows = value < 1 ? 256 : value;

@@ -87,7 +87,7 @@ struct b200nn_ctx {
     int persist_prefetch_mb = 48; // KV-cache megabytes per layer it asks into L2 ahead of the attention phase
     long long persist_wait_cycles = 0; // bound of its grid-wide waits in SM clocks (0: about a second)
     void *persist_trace = nullptr; // optional stamp buffer [148][32][2] u64 (measurement aid, "persist_trace")
-    int few = 1;                  // decode steps of few rows run as one persistent kernel (decode_few.cu; 0: one kernel per operation)
+    int few = 2;                  // decode steps of few rows as one persistent kernel (decode_few.cu): 2 where it is the faster way, 1 wherever its plan fits, 0 never
     int few_fault_layer = -1;     // test hook: block 0 publishes no q/k/v word of that layer, so the bounded waits run out (-1: never)
     int persist_fault_phase = -1; // test hook: block 0 leaves out its arrival after this phase, so the bounded
                                   // waits of every other block run out (-1: never)

@@ -1058,6 +1058,18 @@ bool decode_few_supported(const b200nn_gpt2 *m, int rows, int cap) {
     return coop && per_sm * ctx->sm_count >= p.grid;
 }
 
+// Whether the steps are faster this way.  A layer gains up to 40 us here (int4 of 512 to 1600 columns: 3 to 10), a launch costs 20
+// to 25 us more than a graph's, and the output matrix has fewer blocks (those of the q/k/v product) and one read of its
+// weights for them all.  Steps taken and read one by one, us, here / one kernel per operation, 50257 tokens: width 64, 2 layers
+// int4 150 / 49, f32 116 / 50; 256, 4 layers 88 / 79, 106 / 87; 512, 8 layers 125 / 145, 163 / 188; 1024 int4, 6 layers 148 / 143; 1920 int4, 8
+// layers 286 / 275, f32 460 / 679.  In runs of 32 steps: 118 / 37, 89 / 37; 58 / 68, 84 / 76; 99 / 131, 136 / 177; 118 / 130; 255 / 264, 438 / 666.
+// Below 512 columns a layer gains little or (several sequences, long contexts) nothing.  A larger vocabulary asks for as many
+// more layers.
+bool decode_few_pays(const b200nn_gpt2 *m) {
+    const int d = m->cfg.n_embd, need = m->int4 && (d < 640 || d > 1600) ? 12 : 6;
+    return d >= 512 && (long long)m->cfg.n_layer * 65536 >= (long long)need * std::max(65536, (int)m->cfg.vocab_size);
+}
+
 // All words EMPTY (the ring's position, the parity and the counter too: any are as good; not BROKEN): before the first step after a
 // prompt or a rewind.
 int decode_few_restart(b200nn_session *s) {

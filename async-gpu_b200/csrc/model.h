@@ -242,6 +242,7 @@ struct b200nn_session {
     bool few = false;
     std::shared_ptr<DevBuf> few_words;
     const uint32_t *few_broken = nullptr; // 1: steps were given up, until a prompt or a rewind
+    bool few_pays = false;                // the faster way (decode_few_pays)
     int *pos_ptr() const { return static_cast<int *>(counters->p); }
     int *step_ptr() const { return static_cast<int *>(counters->p) + 1; }
 };
@@ -253,6 +254,7 @@ int launch_decode_layers(b200nn_session *s, bool profile);
 
 // Decode steps of few rows, layers, head and pick, as one persistent cooperative kernel; restart: after a prompt or a rewind.
 bool decode_few_supported(const b200nn_gpt2 *m, int rows, int cap);
+bool decode_few_pays(const b200nn_gpt2 *m);
 int decode_few_prepare(b200nn_session *s);
 int decode_few_restart(b200nn_session *s);
 int launch_decode_few(b200nn_session *s, int n_steps);

@@ -146,6 +146,7 @@ extern "C" int32_t b200nn_lm_session_create(b200nn_lm *m, size_t batch, size_t c
     }
     if (s->gpt2 && decode_few_supported(s->gpt2, (int)batch, (int)capacity)) {
         s->few = decode_few_prepare(s.get()) == B200NN_OK; // (a tensor map refused, no room for the words: one kernel per operation)
+        s->few_pays = s->few && decode_few_pays(s->gpt2);
         if (!s->few) {
             cudaGetLastError(); // (launches look at the last error)
             s->few_words.reset();
@@ -257,7 +258,8 @@ extern "C" int32_t b200nn_session_step(b200nn_session *s, size_t n_steps) {
     if (s->position + n_steps > s->cap) return set_error(ctx, B200NN_ERR_DIM, "session_step: capacity exceeded");
     CK(ctx, cudaSetDevice(ctx->device));
     size_t done = 0;
-    if (s->few && ctx->few && !model_act_half(s->gpt2, (int)s->batch)) {
+    const bool few = ctx->few == 1 || (ctx->few && (s->few_pays || ctx->few_fault_layer >= 0));
+    if (s->few && few && !model_act_half(s->gpt2, (int)s->batch)) {
         // whole steps in one launch, not too many of them: the kernel holds every SM until it ends
         for (; done < n_steps; done += std::min<size_t>(32, n_steps - done)) TRY(launch_decode_few(s, (int)std::min<size_t>(32, n_steps - done)));
         s->position += n_steps;

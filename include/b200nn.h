@@ -139,9 +139,10 @@ B200NN_API int32_t b200nn_ctx_set_gemv_max_rows(b200nn_ctx *ctx, int32_t rows);
  * the mLSTM (1 or 2).
  * "int4_rows_max" (default 8, at most that; negative restores it): a stand-alone int4 Linear of three f32 rows to this many runs as
  * one mma.sync kernel (no conversion launch); 0: always the conversion and the tcgen05 GEMM.
- * "few" (default 1): the steps of a GPT-2 decode session of few sequences (int4 at most 2, f32 at most 4; all Linears and
- * the output matrix of one kind) run as one persistent cooperative kernel, up to 32 steps per launch; 0: one kernel
- * per operation.  "few_fault_layer" (test aid): one block leaves out its q/k/v words of that layer, so that the bounded
+ * "few" (default 2; negative restores it): the steps of a GPT-2 decode session of few sequences (int4 at most 2, f32 at most 4;
+ * all Linears and the output matrix of one kind) run as one persistent cooperative kernel, up to 32 steps per launch, where that is
+ * the faster way (512 columns and six layers or more; int4 under 640 or over 1600 columns twelve; more with vocabularies over 65536);
+ * 1: wherever the kernel takes the shape; 0: one kernel per operation.  "few_fault_layer" (test aid): one block leaves out its q/k/v words of that layer, so that the bounded
  * waits ("persist_wait_kcycles") run out and B200NN_ERR_DEVICE is reported.
  * "persist" (default 0): decode steps of an int4 model run all transformer blocks as one cooperative
  * kernel (decode sessions whose shape it supports).  Measured slower than the per-op CUDA graph.

@@ -104,6 +104,7 @@ def test_steps_given_up_are_reported_until_the_session_starts_over(reg):
     cfg = Gpt2Config(n_layer=3, n_embd=128, n_head=2, vocab_size=257, n_positions=64)
     m = Gpt2Model(synth.gpt2_weights(cfg, base_seed=77, std=0.08, random_ln=True), cfg, reg)
     prompts = synth.token_ids(5, (2, 9), cfg.vocab_size)
+    reg.set_tuning("few", 1)
     s, other = (DecodeSession(m, batch=2, capacity=40) for _ in range(2))
 
     def read(x):
@@ -137,3 +138,18 @@ def test_steps_given_up_are_reported_until_the_session_starts_over(reg):
         s.step(6)  # the prompt's pick is still in place: what was given up has stored nothing
         assert all(np.array_equal(a, b) for a, b in zip(read(s), good)) and reg.device_error() == 0
         other.prefill(prompts)
+
+
+# one layer less than the rule asks for, and as many; narrower than any; a vocabulary that asks for twice the layers
+@pytest.mark.parametrize("family,d,layers,vocab,one", [
+    ("f32", 512, 6, 300, True), ("f32", 512, 5, 300, False), ("f32", 448, 12, 300, False), ("int4", 512, 11, 300, False), ("int4", 512, 12, 300, True),
+    ("int4", 640, 6, 300, True), ("f32", 512, 11, 131072, False), ("f32", 512, 12, 131072, True)])
+def test_steps_in_one_kernel_only_where_they_are_faster(reg, family, d, layers, vocab, one):
+    cfg = Gpt2Config(n_layer=layers, n_embd=d, n_head=d // 64, vocab_size=vocab, n_positions=64)
+    w = synth.gpt2_weights(cfg, base_seed=1, std=0.05)
+    m = Gpt2Model(w, cfg, reg) if family == "f32" else Int4Gpt2Model(w, cfg, reg, flags=b200nn.QUANT_LM_HEAD, group_size=64)
+    prompts = synth.token_ids(2, (1, 5), vocab)
+    default = _steps(reg, m, prompts, 10, -1)
+    assert (default[2] == 1) is one
+    forced = _steps(reg, m, prompts, 10, 1)
+    assert forced[2] == 1 and np.array_equal(forced[0], default[0]) and np.abs(forced[1] - default[1]).max() < 1e-3
