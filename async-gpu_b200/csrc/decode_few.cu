@@ -1070,6 +1070,13 @@ bool decode_few_pays(const b200nn_gpt2 *m) {
     return d >= 512 && (long long)m->cfg.n_layer * 65536 >= (long long)need * std::max(65536, (int)m->cfg.vocab_size);
 }
 
+// Steps of a launch.  The kernel holds every SM until it ends, and other streams wait for it: about 5 ms, by the 10 to 30 us
+// (int4, growing with the width) and 12 to 60 us (f32) that a layer was measured at.
+int decode_few_steps(const b200nn_gpt2 *m) {
+    const int layer_us = std::max(15, m->cfg.n_embd / (m->int4 ? 70 : 32));
+    return std::max(1, std::min(32, 5000 / (layer_us * m->cfg.n_layer)));
+}
+
 // All words EMPTY (the ring's position, the parity and the counter too: any are as good; not BROKEN): before the first step after a
 // prompt or a rewind.
 int decode_few_restart(b200nn_session *s) {

@@ -255,6 +255,7 @@ int launch_decode_layers(b200nn_session *s, bool profile);
 // Decode steps of few rows, layers, head and pick, as one persistent cooperative kernel; restart: after a prompt or a rewind.
 bool decode_few_supported(const b200nn_gpt2 *m, int rows, int cap);
 bool decode_few_pays(const b200nn_gpt2 *m);
+int decode_few_steps(const b200nn_gpt2 *m);
 int decode_few_prepare(b200nn_session *s);
 int decode_few_restart(b200nn_session *s);
 int launch_decode_few(b200nn_session *s, int n_steps);

@@ -260,8 +260,8 @@ extern "C" int32_t b200nn_session_step(b200nn_session *s, size_t n_steps) {
     size_t done = 0;
     const bool few = ctx->few == 1 || (ctx->few && (s->few_pays || ctx->few_fault_layer >= 0));
     if (s->few && few && !model_act_half(s->gpt2, (int)s->batch)) {
-        // whole steps in one launch, not too many of them: the kernel holds every SM until it ends
-        for (; done < n_steps; done += std::min<size_t>(32, n_steps - done)) TRY(launch_decode_few(s, (int)std::min<size_t>(32, n_steps - done)));
+        for (const size_t most = decode_few_steps(s->gpt2); done < n_steps; done += std::min(most, n_steps - done))
+            TRY(launch_decode_few(s, (int)std::min(most, n_steps - done)));
         s->position += n_steps;
         s->steps_done += n_steps;
         s->kv.len = s->position;

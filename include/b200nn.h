@@ -140,10 +140,12 @@ B200NN_API int32_t b200nn_ctx_set_gemv_max_rows(b200nn_ctx *ctx, int32_t rows);
  * "int4_rows_max" (default 8, at most that; negative restores it): a stand-alone int4 Linear of three f32 rows to this many runs as
  * one mma.sync kernel (no conversion launch); 0: always the conversion and the tcgen05 GEMM.
  * "few" (default 2; negative restores it): the steps of a GPT-2 decode session of few sequences (int4 at most 2, f32 at most 4;
- * all Linears and the output matrix of one kind) run as one persistent cooperative kernel, up to 32 steps per launch, where that is
+ * all Linears and the output matrix of one kind) run as one persistent cooperative kernel, where that is
  * the faster way (512 columns and six layers or more; int4 under 640 or over 1600 columns twelve; more with vocabularies over 65536);
- * 1: wherever the kernel takes the shape; 0: one kernel per operation.  "few_fault_layer" (test aid): one block leaves out its q/k/v words of that layer, so that the bounded
- * waits ("persist_wait_kcycles") run out and B200NN_ERR_DEVICE is reported.
+ * 1: wherever the kernel takes the shape; 0: one kernel per operation.  A launch takes up to 32 steps, but no more than about 5 ms
+ * worth: it has every SM of the GPU until it ends, and the work of other streams waits for it.  "few_fault_layer" (test aid):
+ * one block leaves out its q/k/v words of that layer, so that the bounded waits ("persist_wait_kcycles") run out and
+ * B200NN_ERR_DEVICE is reported, by this session's tokens and logits until a prompt or a rewind.
  * "persist" (default 0): decode steps of an int4 model run all transformer blocks as one cooperative
  * kernel (decode sessions whose shape it supports).  Measured slower than the per-op CUDA graph.
  * Its aids: "persist_min_rows" / "persist_max_rows" (batch range it is used for), "persist_prefetch_mb",

@@ -153,3 +153,14 @@ def test_steps_in_one_kernel_only_where_they_are_faster(reg, family, d, layers, 
     assert (default[2] == 1) is one
     forced = _steps(reg, m, prompts, 10, 1)
     assert forced[2] == 1 and np.array_equal(forced[0], default[0]) and np.abs(forced[1] - default[1]).max() < 1e-3
+
+
+@pytest.mark.parametrize("layers,steps", [(3, 32), (48, 6), (400, 1)])
+def test_a_launch_takes_no_more_steps_than_about_five_milliseconds(reg, layers, steps):
+    cfg = Gpt2Config(n_layer=layers, n_embd=64, n_head=1, vocab_size=99, n_positions=128)
+    m = Gpt2Model(synth.gpt2_weights(cfg, base_seed=1, std=0.05), cfg, reg)
+    prompts = synth.token_ids(2, (1, 5), 99)
+    tok, lg, launches = _steps(reg, m, prompts, 2 * steps + 3, 1)  # two steps are not counted
+    assert launches == 3 and reg.device_error() == 0
+    tok_o, lg_o, _ = _steps(reg, m, prompts, 2 * steps + 3, 0)
+    assert np.array_equal(tok, tok_o) and np.abs(lg - lg_o).max() < 1e-3
