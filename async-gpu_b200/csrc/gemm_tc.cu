@@ -458,8 +458,8 @@ int launch_cfg(b200nn_ctx *ctx, const Int4Weight &w, const __half *x, int M, con
     const int base_ctas = w.n_tiles * m_tiles;
     // shared memory without the scale buffer, which is sized per launch below
     constexpr size_t smem_fixed = 1024 + ring + bar_bytes;
-    // Blocks an SM holds at once: two for the variants with two dequant groups (352 threads, built
-    // for at most 93 registers) when their shared memory and TMEM columns fit twice, else one.
+    // Blocks an SM holds at once: four for the variants with one dequant group (224 threads, built for at most 73 registers, 128 TMEM
+    // columns), two for those with two (352 threads, 93 registers) when their shared memory and TMEM columns fit twice, else one.
     const int ctas_per_sm = NG == 1 ? 4 : (NG == 2 && smem_fixed + 8192 <= 113 * 1024 && 2 * TC <= 512) ? 2 : 1;
     // K split: fills the GPU when there are few (feature tile x token tile) pairs.  The count is
     // rounded down, because one block more than the SMs can hold costs a whole second wave.  The
@@ -536,13 +536,16 @@ int launch_int4_gemm_tc(b200nn_ctx *ctx, const Int4Weight &w, const __half *x, i
     switch (mb) { //            MB  NS  NP NG  TMEM columns
         case 32:
             // more tiles than two blocks per SM hold (an output matrix): four blocks with a dequant group each leave no second
-            // wave (768 x 50257, 32 rows with their conversion 14.8 -> 11.4 us); from about 20 K blocks on the one group is what
-            // a block waits for (1600 x 50257: 20.9 and 21.7 us)
+            // wave, and where they do the larger ones have a third.  32 rows with their conversion, weights beyond L2, us, larger / these:
+            // 768 x 50257 15.1 / 11.8, x 100000 24.1 / 21.3, x 200064 46.7 / 36.3; 1024 x 38001 15.2 / 15.1, x 50257 16.2 / 15.1,
+            // x 200064 48.0 / 41.8; from about 20 K blocks on the one group is what a block waits for (1600 x 50257: 20.9 / 21.7)
             if (w.n_tiles > 2 * ctx->sm_count && w.k_blocks <= 16) return launch_cfg<32, 3, 8, 1, 128>(ctx, w, x, M, epi);
             return launch_cfg<32, 7, 16, 2, 256>(ctx, w, x, M, epi);
         case 64:
-            // as for 32 rows (768 x 50257, 64 rows: 14.0 -> 12.5 us; with 1600 inputs the two larger blocks stay the better ones)
-            if (w.n_tiles > 2 * ctx->sm_count && w.k_blocks <= 16) return launch_cfg<64, 2, 8, 1, 128>(ctx, w, x, M, epi);
+            // as for 32 rows (768 x 50257, 64 rows: 16.5 / 13.8 us, x 80000 24.0 / 22.2, x 200064 52.1 / 41.4; 1024 x 50257 18.0 / 17.0,
+            // x 200064 52.2 / 46.2; 896 x 38001 16.2 / 15.5), but with 15 and 16 K blocks a wave that is hardly more than full of the
+            // larger ones stays theirs (1024 x 38001: 16.7 / 17.3)
+            if (w.n_tiles > 2 * ctx->sm_count && w.k_blocks <= (2 * w.n_tiles > 5 * ctx->sm_count ? 16 : 14)) return launch_cfg<64, 2, 8, 1, 128>(ctx, w, x, M, epi);
             // more tiles than SMs (an output matrix): two smaller blocks per SM, so that one's epilogue runs under the other's loop
             if (w.n_tiles > ctx->sm_count) return launch_cfg<64, 4, 8, 2, 256>(ctx, w, x, M, epi);
             return launch_cfg<64, 6, 12, 4, 256>(ctx, w, x, M, epi);

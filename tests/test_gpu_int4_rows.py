@@ -98,3 +98,15 @@ def test_int4_linear_of_few_rows_over_its_own_rows(reg, k, n, at):
     reg.synchronize()
     assert reg.launch_count() - launches == 2  # conversion, GEMM
     assert np.array_equal(buf[start + at:start + at + m * n].cpu().numpy().reshape(m, n), want)
+
+
+# 64 rows of sixteen K blocks: one tile fewer and one more than two and a half per SM
+@pytest.mark.parametrize("n", [370 * 128, 370 * 128 + 1])
+def test_int4_output_matrix_of_64_rows_and_16_k_blocks(reg, n):
+    packed, scales, x, _ = synth.int4_linear_case(7, 64, 1024, n, 128)
+    layer = b200nn.Int4Linear(packed, scales, None, 1024, n, 128, reg)
+    y = layer.forward(GpuTensor.from_host(x, (64, 1024), reg)).to_host()
+    ref = oracle.int4_linear(x, packed, scales, None, 64, n, 1024, 128)
+    # rows and scaled weights rounded to fp16: 2.8e-4 of a product on average each
+    assert np.sqrt(((y - ref) ** 2).mean()) / np.sqrt((ref ** 2).mean()) < 5e-4
+    assert reg.device_error() == 0
