@@ -217,11 +217,15 @@ int rows_launch(b200nn_ctx *ctx, const Int4Weight &w, const float *x, int M, con
 }  // namespace
 
 // Not for more tiles than four per block leave, nor for parts of K whose rows take longer to stage than the GEMM's start
-// (6400 x 1600, eight rows: 8.1 us conversion + GEMM, 8.5 us here; four rows 7.9 and 7.3).
+// (6400 x 1600, eight rows: 8.1 us conversion + GEMM, 8.5 us here; four rows 7.9 and 7.3).  Blocks of several tiles fill the GPU
+// without a split of K, and a warp's units then come one after another; weights beyond L2, conversion + GEMM / here, us.  Two
+// tiles: 2048 x 6400 8 rows 7.9 / 7.1, 3072 x 6400 4 rows 9.2 / 9.4, 5 rows 8.9 / 9.6, 4096 x 6400 4 rows 10.1 / 12.3.  Four: 1280 x 9500
+// 8 rows 7.5 / 7.2, 1600 x 9500 4 rows 8.4 / 8.5, 8 rows 8.3 / 9.0, 2048 x 9500 4 rows 9.2 / 10.1.
 bool int4_rows_supported(const b200nn_ctx *ctx, const Int4Weight &w, const float *x, int M) {
     if (!w.fast || w.group % 128 != 0 || M <= std::max(2, ctx->gemv_max_rows) || M > ctx->int4_rows_max || ((uintptr_t)x & 15)) return false;
     const RowsPlan p = rows_plan(ctx, w);
-    return p.tpb <= MAX_TPB && M * p.per <= 128;
+    const int most = p.tpb == 1 ? 128 : p.tpb == 2 ? (M <= 4 ? 24 : 16) : M <= 4 ? 13 : 10; // units of 128 inputs per block
+    return p.tpb <= MAX_TPB && M * p.per <= 128 && p.per <= most;
 }
 
 int launch_int4_rows(b200nn_ctx *ctx, const Int4Weight &w, const float *x, int M, const Epilogue &epi) {

@@ -110,3 +110,17 @@ def test_int4_output_matrix_of_64_rows_and_16_k_blocks(reg, n):
     # rows and scaled weights rounded to fp16: 2.8e-4 of a product on average each
     assert np.sqrt(((y - ref) ** 2).mean()) / np.sqrt((ref ** 2).mean()) < 5e-4
     assert reg.device_error() == 0
+
+
+# the longest parts of K that the kernel of few rows takes with two and four tiles a block, and one unit of 128 inputs more
+@pytest.mark.parametrize("m,k,n,launches", [(8, 2048, 4737, 1), (8, 2049 + 63, 4737, 2), (4, 3072, 4737, 1), (4, 3136, 4737, 2),
+                                            (5, 1280, 9473, 1), (5, 1344, 9473, 2), (4, 1664, 9473, 1), (4, 1728, 9473, 2)])
+def test_int4_linear_of_few_rows_stays_with_the_gemm_for_long_parts_of_k(reg, m, k, n, launches):
+    packed, scales, x, _ = synth.int4_linear_case(m + k, m, k, n, 128)
+    layer = b200nn.Int4Linear(packed, scales, None, k, n, 128, reg)
+    before = reg.launch_count()
+    y = layer.forward(GpuTensor.from_host(x, (m, k), reg)).to_host()
+    assert reg.launch_count() - before == launches
+    ref = oracle.int4_linear(x, packed, scales, None, m, n, k, 128)
+    # rows (and, by the GEMM, scaled weights) rounded to fp16: 2.8e-4 of a product on average each
+    assert np.sqrt(((y - ref) ** 2).mean()) / np.sqrt((ref ** 2).mean()) < 5e-4
