@@ -335,7 +335,9 @@ struct alignas(128) ScanStage { // the parts that tensor copies fill start on 12
 // What bounds it: the packed multiply-adds read three different operand pairs and issue every 3 to 3.5 cycles (two when operands
 // repeat): 96 of them and 60 other instructions per warp and pair; and, per stage, 600 cycles of copies announced, cross
 // products and two barriers.  One token at a time, copies by cp.async, four warps a block: 16 sequences of 1024 tokens, 8 heads of
-// 128, 591 us, now 515; one of 512 133 / 100.  Tried: four lanes for two columns (half the reductions, half the warps: 506, and
+// 128, 591 us, now 515; one of 512 133 / 100; decays per channel 2 sequences of 250 67.6 / 61.5, 8 137 / 105, but 32 287 / 293 and 64 of 50
+// 135 / 140; up to 16 tokens of few sequences cost up to a microsecond more (2 of 16: 9.0 / 9.8).  Asking for the first stage ahead of
+// the state's loads: 0.05 us less there, and 2 % more for 64 sequences of 100.  Tried: four lanes for two columns (half the reductions, half the warps: 506, and
 // 170 for one sequence), plain multiply-adds (576), a bulk copy per token and vector (920: one lane issues them), the
 // cross products with the pair (longer chains), pairs unrolled (spills).
 // Also leaves the convolution's last inputs in the cache (blocks of column group 0).
@@ -666,10 +668,13 @@ int prompt_launch(b200nn_ctx *ctx, const DeltaDims &d, bool b16, const float *pr
         launch_ordered(ctx, delta_conv_kernel<2, CH>, cgrid, dim3(256), 0, d, proj, ldp, ext, w, conv_state, rows, sm, row_seq, n_rows, conv);
     CK_LAUNCH(ctx, "delta_conv_kernel");
     // columns per lane: one (shorter chains, more instructions) while that gives an SM no more than three blocks; 512 tokens,
-    // 8 heads of 128, one / two columns, us: 2 sequences 112 / 119, 4 149 / 126, 8 213 / 168, 16 404 / 267
+    // 8 heads of 128, one / two columns, us: 2 sequences 112 / 119, 4 149 / 126, 8 213 / 168, 16 404 / 267.  Decays per channel cost a
+    // multiplication per entry and column and no reduction: three blocks up to a dim of 64, two up to 96, one above (8 heads, 250
+    // tokens: dim 128 1 sequence 55 / 61, 2 64.6 / 61.5, 3 77.8 / 67.5; dim 96 2 54 / 55, 3 63.7 / 59.7; dim 64 2 45 / 51, 4 61 / 54).
     const long long columns = (long long)d.vdim_p * d.heads * sm.n_seq;
     const int dm = (d.dim_p + 31) / 32;
-    const int nc = dm > 4 ? 1 : ctx->delta_cols ? ctx->delta_cols : columns > 8LL * 3 * ctx->sm_count ? 2 : 1;
+    const int blocks = CH ? std::min(3, std::max(1, 5 - dm)) : 3;
+    const int nc = dm > 4 ? 1 : ctx->delta_cols ? ctx->delta_cols : columns > 8LL * blocks * ctx->sm_count ? 2 : 1;
     CUtensorMap map_qk, map_v, map_g;
     const int dp = dm <= 4 ? dm * 32 : dm <= 6 ? 192 : 256;
     if (int e = map_rows(ctx, &map_qk, conv + d.q_at(), d.dim_p, d.kv_heads, 2, n_rows, d.conv_ld(), dp)) return e;
