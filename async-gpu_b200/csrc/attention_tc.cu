@@ -18,7 +18,8 @@
 // exponentials, 300 of hand-overs.  Against one block per item, two threads per row, scores read twice, O folded into
 // registers every step, 12 / 12 / 25 heads, us: 8 prompts of 1024 37.6 / 31.4 now, 32 of 512 49.7 / 37.6, 16 of 400 behind 100
 // 59.1 / 45.1.  A reference that moves only past 2^8 saves another microsecond, and loses the exactness of the
-// largest probabilities (error 2.51e-4 -> 2.55e-4): not taken.  A quarter of the exponentials as polynomials: no gain.
+// largest probabilities (error 2.51e-4 -> 2.55e-4): not taken.  A quarter of the exponentials as polynomials: 29.8 us for the 8 prompts
+// of 1024, slower at every other size.  A single step in few blocks gains nothing (8 prompts of 128, 12 heads, the kernel alone: 5.9 / 6.1).
 //
 // TMEM (256 columns per block): S at columns 0..127, P (fp16 pairs) at 128..191, O at 192..255.
 //
@@ -26,7 +27,7 @@
 // cuda/flash_attn_v3.cu:29-283) for the model path, where q and the output are fp16.
 //
 // Every mbarrier wait is bounded: on expiry the block records a code in the device error word, all
-// roles leave their loops, nothing is stored, the TMEM columns are freed and the kernel returns.
+// roles leave their loops, nothing more is stored (items it had finished are), the TMEM columns are freed and the kernel returns.
 #include <cuda.h>
 
 #include <algorithm>

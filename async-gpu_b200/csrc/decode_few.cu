@@ -22,14 +22,17 @@
 // Products: 16 output features x a run of K are a chunk (one tensor copy, one warp).  f32 weights multiply with FMAs.  int4
 // weights stay bytes: the nibbles are the unsigned bytes of mma.sync m16n8k32, the activations its signed columns, each
 // f32 value as four balanced base-256 digits of a 30-bit integer scaled by the largest of its 64 neighbours.  The integer
-// sums are exact, so a product loses less than a chain of f32 FMAs, and a weight costs three instructions per eight.
+// sums are exact, so a product usually loses less than a chain of f32 FMAs (every input is off by 2^-30 of that largest one at
+// most, which is more than an f32's own rounding for inputs below 2^-6 of it: a feature whose weights are zero where the large
+// inputs are sees that), and a weight costs three instructions per eight.  An infinity makes the products of its 64 NaN.
 // Group scales multiply the sums of 64 inputs in f32.
 //
 // What bounds a step: five hand-overs per layer of 0.9 us (a store and a load through L2 and a barrier, measured alone;
 // 1.6 us with a counter), and the chain of a block's own reductions between them: LayerNorm, products, sums over warps.
-// The weight bytes are hidden under that.  Steps after a prompt of 64, one / two / four sequences, us: GPT-2 Small f32 315 /
-// 350 / 582 launched per operation, 186 / 239 / 309 here; GPT-2 Small int4 212 / 262, here 165 / 180; GPT-2 XL int4
-// 1235 / 1579, here 1000 / 1296.  More rows: the tensor-core GEMMs take over (their activations are fp16).
+// The weight bytes are hidden under that.  Steps after a prompt of 64, one / two / four sequences, us: GPT-2 Small f32 321 /
+// 349 / 582 launched per operation, 192 / 232 / 307 here; GPT-2 Small int4 212 / 264, here 167 / 182; GPT-2 XL int4
+// 1230 / 1635, here 976 / 1322.  At contexts of 1000 (three or two splits of a head, several turns of rows a block): Small f32 332 /
+// 379 / 621, here 221 / 289 / 396.  More rows: the tensor-core GEMMs take over (their activations are fp16).
 //
 // Every wait is bounded: when one runs out the block records a code in the device error word, marks the session's exchanged
 // words as broken (what was published and not taken back would pass for later values), waits for nothing more and leaves;

@@ -480,7 +480,8 @@ B200NN_API int32_t b200nn_session_tokens(b200nn_session *s, uint32_t *out, size_
 B200NN_API int32_t b200nn_session_logits(b200nn_session *s, float *out);
 /* Per-kernel-family device time of ONE decode step at the current position, measured with CUDA
  * events around each launch (Gpt2Model::forward_profiled, gpt2.rs:529-568).  times_ms has
- * B200NN_PROF_COUNT entries.  Where a block's two LayerNorms ride along with the Linears behind them (models of up to
+ * B200NN_PROF_COUNT entries.  The step is launched as one kernel per operation, also in a session of few sequences, whose own steps
+ * run as one kernel (tuning key "few") that has no such parts; the same holds for b200nn_session_time_family.  Where a block's two LayerNorms ride along with the Linears behind them (models of up to
  * 2048 columns with one or two sequences, f32 models up to four) their work counts as B200NN_PROF_LINEAR, here and in
  * b200nn_session_time_family; B200NN_PROF_LAYERNORM is then the final norm alone. */
 enum {
@@ -593,7 +594,7 @@ B200NN_API int32_t b200nn_latent_decode_attention(b200nn_ctx *ctx, const b200nn_
  * f32 on the device: conv [taps][2 kv_heads dim + heads vdim], a_exp [heads] = exp(A_log), dt_bias [heads],
  * norm [vdim]; conv_state f32 [slots][taps][2 kv_heads dim + heads vdim], state f32 [slots][heads][dim][vdim];
  * out [n_rows][heads][vdim].  n_seq 0: one token per row.  Else prompt portions: seq [4][n_seq] (slot, first row,
- * rows, past) followed by the sequence index of every row, slot per row given, and scratch f32 of
+ * rows, which may be none, past) followed by the sequence index of every row, slot per row given, and scratch f32 of
  * n_rows * (2 kv_heads dim + 2 heads vdim + 2 heads + kv_heads + 4). */
 typedef struct {
     int32_t heads, kv_heads, dim, vdim, conv;
