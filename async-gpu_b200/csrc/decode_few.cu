@@ -1048,7 +1048,7 @@ static Kernel kernel_of(bool int4, int MT) {
 bool decode_few_supported(const b200nn_gpt2 *m, int rows, int cap) {
     few::Plan p;
     b200nn_ctx *ctx = m->ctx;
-    if (!ctx->few || model_act_half(m, rows) || !few::make_plan(m, rows, cap, &p)) return false;
+    if (model_act_half(m, rows) || !few::make_plan(m, rows, cap, &p)) return false;
     int coop = 0, per_sm = 0;
     const few::Kernel k = few::kernel_of(m->int4, p.MT);
     if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device) != cudaSuccess ||

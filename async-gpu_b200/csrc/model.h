@@ -242,7 +242,7 @@ struct b200nn_session {
     bool few = false;
     std::shared_ptr<DevBuf> few_words;
     const uint32_t *few_broken = nullptr; // 1: steps were given up, until a prompt or a rewind
-    bool few_pays = false;                // the faster way (decode_few_pays)
+    bool few_pays = false, few_asked = false; // the faster way (decode_few_pays); whether it is known if it can be taken
     int *pos_ptr() const { return static_cast<int *>(counters->p); }
     int *step_ptr() const { return static_cast<int *>(counters->p) + 1; }
 };

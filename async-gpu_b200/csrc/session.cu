@@ -117,6 +117,24 @@ extern "C" int32_t b200nn_gpt2_forward_cached(b200nn_gpt2 *m, const uint32_t *id
 // ---------------------------------------------------------------------------------------------
 static constexpr size_t PREFILL_ROWS = 16384; // rows per prefill pass (bounds the activation buffers)
 
+// Whether this session's steps are to run as one kernel (decode_few.cu), and whether they can, which is found out and prepared for once.
+static bool few_wanted(const b200nn_session *s) {
+    const b200nn_ctx *ctx = s->m->ctx;
+    return s->gpt2 && (ctx->few == 1 || (ctx->few && (s->few_pays || ctx->few_fault_layer >= 0)));
+}
+static bool few_ready(b200nn_session *s) {
+    if (s->few_asked) return s->few;
+    s->few_asked = true;
+    if (!decode_few_supported(s->gpt2, (int)s->batch, (int)s->cap)) return false;
+    s->few = decode_few_prepare(s) == B200NN_OK; // (a tensor map refused, no room for the words: one kernel per operation)
+    if (!s->few) {
+        cudaGetLastError(); // (launches look at the last error)
+        s->few_words.reset();
+        s->few_broken = nullptr;
+    }
+    return s->few;
+}
+
 extern "C" int32_t b200nn_session_create(b200nn_gpt2 *m, size_t batch, size_t capacity, uint32_t flags,
                                          b200nn_session **out) {
     return b200nn_lm_session_create(m, batch, capacity, flags, out);
@@ -144,15 +162,8 @@ extern "C" int32_t b200nn_lm_session_create(b200nn_lm *m, size_t batch, size_t c
         TRY(decode_persistent_prepare(s.get()));
         s->persist = true;
     }
-    if (s->gpt2 && decode_few_supported(s->gpt2, (int)batch, (int)capacity)) {
-        s->few = decode_few_prepare(s.get()) == B200NN_OK; // (a tensor map refused, no room for the words: one kernel per operation)
-        s->few_pays = s->few && decode_few_pays(s->gpt2);
-        if (!s->few) {
-            cudaGetLastError(); // (launches look at the last error)
-            s->few_words.reset();
-            s->few_broken = nullptr;
-        }
-    }
+    s->few_pays = s->gpt2 && decode_few_pays(s->gpt2);
+    if (few_wanted(s.get())) few_ready(s.get()); // the others' sessions do without the words and maps (10 us of a session's creation)
     *out = s.release();
     return B200NN_OK;
 }
@@ -258,8 +269,7 @@ extern "C" int32_t b200nn_session_step(b200nn_session *s, size_t n_steps) {
     if (s->position + n_steps > s->cap) return set_error(ctx, B200NN_ERR_DIM, "session_step: capacity exceeded");
     CK(ctx, cudaSetDevice(ctx->device));
     size_t done = 0;
-    const bool few = ctx->few == 1 || (ctx->few && (s->few_pays || ctx->few_fault_layer >= 0));
-    if (s->few && few && !model_act_half(s->gpt2, (int)s->batch)) {
+    if (few_wanted(s) && !model_act_half(s->gpt2, (int)s->batch) && few_ready(s)) {
         for (const size_t most = decode_few_steps(s->gpt2); done < n_steps; done += std::min(most, n_steps - done))
             TRY(launch_decode_few(s, (int)std::min(most, n_steps - done)));
         s->position += n_steps;

@@ -194,3 +194,26 @@ def test_steps_in_one_kernel_with_long_contexts(reg, family, d, layers, B, P, N,
     same = (tok == tok_o).all(axis=1)
     assert same.sum() >= B - 1  # a near-tie may turn a pick
     assert np.abs(lg - lg_o)[same].max() < 1e-3
+
+
+def test_a_session_turns_to_steps_in_one_kernel_and_back(reg):
+    """A narrow model's session prepares nothing until it is asked to; each way goes on where the other has stopped."""
+    cfg = Gpt2Config(n_layer=2, n_embd=128, n_head=2, vocab_size=257, n_positions=64)
+    m = Gpt2Model(synth.gpt2_weights(cfg, base_seed=8, std=0.08, random_ln=True), cfg, reg)
+    prompts = synth.token_ids(6, (2, 9), cfg.vocab_size)
+
+    def run(ways):
+        try:
+            reg.set_tuning("few", ways[0])
+            s = DecodeSession(m, batch=2, capacity=60)
+            s.prefill(prompts)
+            for few in ways:
+                reg.set_tuning("few", few)
+                launches = reg.launch_count()
+                s.step(3)
+                assert (reg.launch_count() - launches == 1) is (few == 1)
+            return s.tokens(), s.logits()
+        finally:
+            reg.set_tuning("few", 1)
+    a, b = run((-1, 1, 0, 1, -1, 1, 1)), run((0,) * 7)
+    assert np.array_equal(a[0], b[0]) and np.abs(a[1] - b[1]).max() < 1e-3 and reg.device_error() == 0
