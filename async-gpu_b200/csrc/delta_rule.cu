@@ -331,21 +331,23 @@ struct alignas(128) ScanStage { // the parts that tensor copies fill start on 12
 // one lane reduction for the eight values (transposing: each lane ends with one of them) and one chain for two tokens.
 // The state is held divided by the decay G accumulated since it was last rescaled (S = G s), so that a token costs three
 // multiply-adds per entry; a pair that brings G below 2^-20 applies its decays to the state instead.
-// With CH the decays differ along dim and are multiplied in directly (one multiply more per entry).
+// With CH the decays differ along dim and are multiplied in directly (one multiply more per entry); !PAIRS (CH only) takes its
+// tokens one at a time.
 // What bounds it: the packed multiply-adds read three different operand pairs and issue every 3 to 3.5 cycles (two when operands
 // repeat): 96 of them and 60 other instructions per warp and pair; and, per stage, 600 cycles of copies announced, cross
 // products and two barriers.  One token at a time, copies by cp.async, four warps a block: 16 sequences of 1024 tokens, 8 heads of
-// 128, 591 us, now 515; one of 512 133 / 100; decays per channel 2 sequences of 250 67.6 / 61.5, 8 137 / 105, but 32 287 / 293 and 64 of 50
-// 135 / 140; up to 16 tokens of few sequences cost up to a microsecond more (2 of 16: 9.0 / 9.8).  Asking for the first stage ahead of
+// 128, 591 us, now 515; one of 512 133 / 100; decays per channel 2 sequences of 250 67.6 / 61.5, 8 137 / 105, one
+// at a time 32 287 / 289; up to 16 tokens of few sequences cost up to a microsecond more (2 of 16: 9.0 / 9.8).  Asking for the first stage ahead of
 // the state's loads: 0.05 us less there, and 2 % more for 64 sequences of 100.  Tried: four lanes for two columns (half the reductions, half the warps: 506, and
 // 170 for one sequence), plain multiply-adds (576), a bulk copy per token and vector (920: one lane issues them), the
 // cross products with the pair (longer chains), pairs unrolled (spills).
 // Also leaves the convolution's last inputs in the cache (blocks of column group 0).
-template <int DM, int NC, bool CH>
+template <int DM, int NC, bool CH, bool PAIRS>
 __global__ void __launch_bounds__(SCAN_THREADS, DM > 4 ? 4 : 8)
 delta_scan_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_g,
                   DeltaDims d, const float *__restrict__ proj, int ldp, const float *__restrict__ conv, float *__restrict__ conv_state,
                   float *__restrict__ state, SeqMap sm, float *__restrict__ heads_out, uint32_t *__restrict__ dev_err) {
+    static_assert(CH || PAIRS, "one decay a head: pairs are the faster way for any number of sequences");
     constexpr int TOK = SCAN_TOKENS, T = SCAN_THREADS, DP = DM * 32, CB = T / 8 * NC;
     using Stage = ScanStage<DM, NC, CH>;
     extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -413,7 +415,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_const
         Stage &st = stages[b];
         const int nt = min(TOK, n - t0);
         tc::mbar_wait(tc::smem_u32(&full[b]), t0 / (2 * TOK) & 1, &abort_flag, dev_err, ERR_SCAN);
-        if (nt & 1) { // the last token's partner: nothing read, nothing written
+        if (PAIRS && (nt & 1)) { // the last token's partner: nothing read, nothing written
             for (int j = tid; j < DP; j += T) {
                 st.qk[nt][0][j] = st.qk[nt][1][j] = 0.0f;
                 if constexpr (CH) st.g[nt][j] = 1.0f;
@@ -422,7 +424,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_const
             if (tid < 3) st.s[nt][tid] = tid == 0 ? 1.0f : 0.0f;
             __syncthreads();
         }
-        { // k1 . k2 (even groups) and k1 . q2 (odd ones) of pair `at`, k1 under the second token's decay
+        if constexpr (PAIRS) { // k1 . k2 (even groups) and k1 . q2 (odd ones) of pair `at`, k1 under the second token's decay
             const int g = tid >> 3, at = g & ~1;
             const float *y = st.qk[at + 1][~g & 1];
             uint64_t a[2] = {};
@@ -443,8 +445,65 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap map_qk, const __grid_const
 #pragma unroll
             for (int sh = 4; sh; sh >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, sh);
             if (part == 0) st.cross[at >> 1][g & 1] = dot;
+            __syncthreads();
         }
-        __syncthreads();
+        if constexpr (!PAIRS) {
+#pragma unroll 2
+            for (int t = 0; t < nt; ++t) {
+                const float4 sc = *reinterpret_cast<const float4 *>(st.s[t]);
+                uint64_t k[DM * 2];
+                float r[2 * NC]; // s^T k of the NC columns, then s^T q
+                {
+                    uint64_t acc[2 * NC];
+#pragma unroll
+                    for (int i = 0; i < 2 * NC; ++i) acc[i] = 0ull;
+#pragma unroll
+                    for (int m = 0; m < DM; ++m) {
+                        const int at = 32 * m + 4 * part;
+                        const ulonglong2 gg = *reinterpret_cast<const ulonglong2 *>(&st.g[t][at]);
+                        const ulonglong2 kk = *reinterpret_cast<const ulonglong2 *>(&st.qk[t][1][at]), qq = *reinterpret_cast<const ulonglong2 *>(&st.qk[t][0][at]);
+                        k[2 * m] = kk.x;
+                        k[2 * m + 1] = kk.y;
+#pragma unroll
+                        for (int e = 0; e < 2; ++e)
+#pragma unroll
+                            for (int c = 0; c < NC; ++c) {
+                                s[c][2 * m + e] = mul2(e ? gg.y : gg.x, s[c][2 * m + e]);
+                                acc[c] = fma2(s[c][2 * m + e], e ? kk.y : kk.x, acc[c]);
+                                acc[NC + c] = fma2(s[c][2 * m + e], e ? qq.y : qq.x, acc[NC + c]);
+                            }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 2 * NC; ++i) {
+                        const float2 a = f32x2_parts(acc[i]);
+                        r[i] = a.x + a.y;
+                    }
+                }
+#pragma unroll
+                for (int sh = 4, w = NC; sh; sh >>= 1, w >>= 1) {
+                    const bool up = (lane & sh) != 0;
+#pragma unroll
+                    for (int i = 0; i < w; ++i) {
+                        const float send = up ? r[i] : r[i + w], keep = up ? r[i + w] : r[i];
+                        r[i] = keep + __shfl_xor_sync(0xffffffffu, send, sh);
+                    }
+                    if (w == 0) r[0] += __shfl_xor_sync(0xffffffffu, r[0], sh);
+                }
+                // lanes with bit 4 clear hold s^T k, the others s^T q, of column `at`
+                const int at = NC == 1 ? 0 : (lane >> 1) & 1;
+                const float other = __shfl_xor_sync(0xffffffffu, r[0], 4);
+                const float u = sc.y * (st.v[t][cl + at] - ((lane & 4) ? other : r[0]));
+                if ((lane & 4) && !(lane & 1) && (NC == 2 || !(lane & 2)) && col + at < d.vdim_p)
+                    heads_out[((size_t)(row0 + t0 + t) * d.heads + h) * d.vdim_p + col + at] = fmaf(sc.z, u, r[0]);
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const float uc = NC == 1 ? u : __shfl_sync(0xffffffffu, u, (lane & 24) | (c << 1));
+                    const uint64_t w2 = f32x2(uc, uc);
+#pragma unroll
+                    for (int m = 0; m < DM * 2; ++m) s[c][m] = fma2(k[m], w2, s[c][m]);
+                }
+            }
+        } else
 #pragma unroll 1
         for (int t = 0; t < nt; t += 2) {
             const float4 sc1 = *reinterpret_cast<const float4 *>(st.s[t]), sc2 = *reinterpret_cast<const float4 *>(st.s[t + 1]);
@@ -675,6 +734,11 @@ int prompt_launch(b200nn_ctx *ctx, const DeltaDims &d, bool b16, const float *pr
     const int dm = (d.dim_p + 31) / 32;
     const int blocks = CH ? std::min(3, std::max(1, 5 - dm)) : 3;
     const int nc = dm > 4 ? 1 : ctx->delta_cols ? ctx->delta_cols : columns > 8LL * blocks * ctx->sm_count ? 2 : 1;
+    // decays per channel: tokens one at a time (two columns a lane) in passes of a few tokens, where a pair's cross products are most of
+    // the work, and for heads of more than 96 in passes that fill the GPU several times over, where its longer chains hide nothing.
+    // In pairs / one at a time, us: 128 sequences of 1 40.8 / 34.7, 32 of 3 18.0 / 15.9, 4 of 3 7.3 / 7.1, of 6 8.5 / 8.6; 8 heads of 128, 8
+    // sequences of 50 27.3 / 27.7, 12 34.8 / 34.3, 16 41.6 / 40.1, 64 140 / 138; 8 heads of 64, 64 sequences of 50 86.8 / 89.6
+    const bool pairs = !CH || !(sm.max_n <= 3 || (dm == 4 && columns > 8LL * 10 * ctx->sm_count));
     CUtensorMap map_qk, map_v, map_g;
     const int dp = dm <= 4 ? dm * 32 : dm <= 6 ? 192 : 256;
     if (int e = map_rows(ctx, &map_qk, conv + d.q_at(), d.dim_p, d.kv_heads, 2, n_rows, d.conv_ld(), dp)) return e;
@@ -682,29 +746,30 @@ int prompt_launch(b200nn_ctx *ctx, const DeltaDims &d, bool b16, const float *pr
     map_g = map_v; // not read
     if (CH)
         if (int e = map_rows(ctx, &map_g, conv + d.decay_at(), d.dim_p, d.heads, 1, n_rows, d.conv_ld(), dp)) return e;
-#define DSCAN(M, C)                                                                                                           \
+#define DSCAN(M, C, P)                                                                                                        \
     do {                                                                                                                      \
         constexpr size_t smem = 2 * sizeof(ScanStage<M, C, CH>) + 128;                                                            \
         static bool done[16] = {};                                                                                            \
         if (!done[ctx->device & 15]) {                                                                                        \
-            CK(ctx, cudaFuncSetAttribute(delta_scan_kernel<M, C, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-            prefer_max_smem(delta_scan_kernel<M, C, CH>);                                                                     \
+            CK(ctx, cudaFuncSetAttribute(delta_scan_kernel<M, C, CH, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+            prefer_max_smem(delta_scan_kernel<M, C, CH, P>);                                                                     \
             done[ctx->device & 15] = true;                                                                                    \
         }                                                                                                                     \
-        CK(ctx, launch_ordered(ctx, delta_scan_kernel<M, C, CH>, dim3((d.vdim_p + 8 * C - 1) / (8 * C), d.heads, sm.n_seq), \
+        CK(ctx, launch_ordered(ctx, delta_scan_kernel<M, C, CH, P>, dim3((d.vdim_p + 8 * C - 1) / (8 * C), d.heads, sm.n_seq), \
                                dim3(SCAN_THREADS), smem, map_qk, map_v, map_g, d, proj, ldp, conv, conv_state, state, sm, heads_out, ctx->dev_err));            \
     } while (0)
 #define DSCAN_C(M)                                                                                                            \
     do {                                                                                                                      \
-        if (nc == 2) DSCAN(M, 2);                                                                                             \
-        else DSCAN(M, 1);                                                                                                     \
+        if (CH && nc == 2 && !pairs) DSCAN(M, 2, !CH);                                                                        \
+        else if (nc == 2) DSCAN(M, 2, true);                                                                                  \
+        else DSCAN(M, 1, true);                                                                                                     \
     } while (0)
     if (dm <= 1) DSCAN_C(1);
     else if (dm <= 2) DSCAN_C(2);
     else if (dm <= 3) DSCAN_C(3);
     else if (dm <= 4) DSCAN_C(4);
-    else if (dm <= 6) DSCAN(6, 1);
-    else DSCAN(8, 1);
+    else if (dm <= 6) DSCAN(6, 1, true);
+    else DSCAN(8, 1, true);
 #undef DSCAN_C
 #undef DSCAN
     CK_LAUNCH(ctx, "delta_scan_kernel");

@@ -105,3 +105,12 @@ def test_sequences_of_no_rows_change_nothing(reg, channel):
     for i in (0, 2, 3, 5):
         assert torch.equal(got[1][i], first[0][i]) and torch.equal(got[2][i], first[1][i])
     assert not torch.equal(got[2][1], first[1][1]) and reg.device_error() == 0
+
+
+# passes of at most three tokens a sequence take them one at a time where the decays are per channel (one and two columns a lane,
+# every share of dim per lane); one of four does not
+@pytest.mark.parametrize("longest", [3, 4])
+@pytest.mark.parametrize("H,KH,dim,vdim", [(8, 4, 32, 128), (16, 4, 64, 64), (8, 8, 96, 96), (6, 2, 128, 128), (2, 1, 128, 16)])
+def test_short_prompts_agree_with_single_tokens(reg, monkeypatch, H, KH, dim, vdim, longest):
+    monkeypatch.setitem(globals(), "LENGTHS", [1, 2, longest, 3, 1, 2])
+    test_prompts_agree_with_single_tokens(reg, H, KH, dim, vdim, True)
